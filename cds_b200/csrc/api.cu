@@ -449,7 +449,7 @@ cds_status cds_list_cliques(cds_ctx *c, cds_graph *g, uint32_t k, uint32_t p_siz
     dag.outdeg = DBuf<uint32_t>(c, s, 0);
     dag.off = DBuf<uint64_t>(c, s, 0);
     dag.adj = DBuf<uint32_t>(c, s, 0);
-    build_dag(c, s, g->d_off, g->d_adj, g->n, dag);
+    build_dag(c, s, g->d_off, g->d_adj, g->n, k, dag);
     Cliques cl;
     list_cliques(c, s, dag, k, false, c->tune[k < 2 ? 2 : (k > CDS_MAX_K ? CDS_MAX_K : k)], cl);
     if (count) *count = cl.count;
@@ -473,7 +473,7 @@ cds_status cds_clique_core(cds_ctx *c, cds_graph *g, uint32_t k, uint32_t gl_buf
     dag.outdeg = DBuf<uint32_t>(c, s, 0);
     dag.off = DBuf<uint64_t>(c, s, 0);
     dag.adj = DBuf<uint32_t>(c, s, 0);
-    build_dag(c, s, u.off, u.adj, u.n, dag);
+    build_dag(c, s, u.off, u.adj, u.n, k, dag);
     Cliques cl;
     list_cliques(c, s, dag, k, true, c->tune[k], cl);
     PeelOut pe;
@@ -504,7 +504,7 @@ cds_status cds_densest_core(cds_ctx *c, cds_graph *g, uint32_t k, uint64_t *thre
     dag.outdeg = DBuf<uint32_t>(c, s, 0);
     dag.off = DBuf<uint64_t>(c, s, 0);
     dag.adj = DBuf<uint32_t>(c, s, 0);
-    build_dag(c, s, u.off, u.adj, u.n, dag);
+    build_dag(c, s, u.off, u.adj, u.n, k, dag);
     Cliques cl;
     list_cliques(c, s, dag, k, true, c->tune[k], cl);
     PeelOut pe;
@@ -538,7 +538,7 @@ cds_status cds_components(cds_ctx *c, cds_graph *g, uint32_t k, uint64_t *core_c
     dag.outdeg = DBuf<uint32_t>(c, s, 0);
     dag.off = DBuf<uint64_t>(c, s, 0);
     dag.adj = DBuf<uint32_t>(c, s, 0);
-    build_dag(c, s, u.off, u.adj, u.n, dag);
+    build_dag(c, s, u.off, u.adj, u.n, k, dag);
     Cliques cl;
     list_cliques(c, s, dag, k, true, c->tune[k], cl);
     PeelOut pe;

@@ -2,6 +2,7 @@
 // for the method).  Included by every translation unit that launches it.
 #pragma once
 #include "device_util.cuh"
+#include "dag_kernels.cuh"
 #include "cds.h"
 
 namespace {
@@ -14,6 +15,7 @@ struct ListParams {
   const uint64_t *doff;
   const uint32_t *dadj;
   const uint32_t *outdeg;
+  const uint32_t *deg;             // undirected degree
   const uint32_t *roots;
   const uint32_t *nroots;          // root count, on the device
   uint32_t *work;                  // dynamic scheduling cursor
@@ -24,6 +26,7 @@ struct ListParams {
   uint32_t *out;                   // pass 2: clique records
   uint32_t dmax;                   // team capacity (entries)
   uint32_t team_words;             // shared-memory words per team
+  HeavyBits heavy;                 // adjacency among the heavy vertices
   uint32_t *rows_global;           // block teams: rows outside shared memory
   uint64_t rows_slab;              // words per block slab
   uint32_t *err;
@@ -36,6 +39,12 @@ struct Team {
   __device__ __forceinline__ static int rank() { return TB ? (int)threadIdx.x : (int)lane_id(); }
   __device__ __forceinline__ static int warps() { return TB ? (int)(blockDim.x >> 5) : 1; }
   __device__ __forceinline__ static int warp() { return TB ? (int)(threadIdx.x >> 5) : 0; }
+  __device__ __forceinline__ static bool any(bool x) {  // over the team, which it synchronises
+    if (TB) return __syncthreads_or(x) != 0;
+    const bool r = __any_sync(CDS_FULL, x);
+    __syncwarp();
+    return r;
+  }
   __device__ __forceinline__ static void sync() {
     if (TB) __syncthreads();
     else __syncwarp();
@@ -72,6 +81,369 @@ __device__ __forceinline__ uint32_t nth_in_row(const uint32_t *row, uint32_t r) 
     const uint32_t c = __popc(row[w]);
     if (r < c) return (w << 5) + (uint32_t)select_bit(row[w], (int)r);
     r -= c;
+  }
+}
+
+template <int K>
+struct CountOf {
+  using type = uint32_t;  // a local count times k-2 stays below 2^32 (at most 1,024 local vertices at k = 5)
+};
+template <>
+struct CountOf<0> {
+  using type = unsigned long long;
+};
+
+// The local graph of a sorted vertex set A[0..d): hit(i, j) for every DAG arc
+// A[i] -> A[j] whose tail is light.  (Arcs between heavy vertices are in the
+// adjacency bitmap of the heavy vertices, and every arc out of a heavy vertex
+// ends in one: arcs climb in degree.)  A warp takes a group of up to 32 rows and
+// walks their out-lists laid end to end (a prefix over their lengths in
+// registers), two steps of 32 entries in flight; light lists are short, and a
+// step per list would leave most lanes idle and wait for three dependent loads
+// (vertex, offset, entry) per row.  Team-wide; the caller synchronises after.
+constexpr uint32_t LIGHT = 0xFFFFFFFFu;  // no heavy id
+template <bool TB, class Hit>
+__device__ __forceinline__ void light_arcs(const uint32_t *A, const uint32_t *hid, uint32_t d,
+                                           const uint64_t *__restrict__ doff, const uint32_t *__restrict__ dadj,
+                                           const uint32_t *__restrict__ outdeg, Hit hit) {
+  constexpr int U = 2;
+  const uint32_t lane = lane_id(), nw = Team<TB>::warps();
+  uint32_t g = (d + nw - 1) / nw;
+  g = g > 32 ? 32 : g;
+  const uint32_t lo_id = A[0], hi_id = A[d - 1];
+  for (uint32_t r0 = Team<TB>::warp() * g; r0 < d; r0 += nw * g) {
+    const uint32_t n = min(g, d - r0);
+    uint32_t len = 0;
+    const uint32_t *list = nullptr;
+    if (lane < n && hid[r0 + lane] == LIGHT) {
+      const uint32_t a = A[r0 + lane];
+      len = outdeg[a];
+      list = dadj + doff[a];
+    }
+    const uint32_t incl = warp_inclusive_scan(len), ex = incl - len;
+    const uint32_t total = __shfl_sync(CDS_FULL, incl, 31);
+    for (uint32_t f0 = 0; f0 < total; f0 += 32 * U) {
+      uint32_t r[U], b[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const uint32_t f = f0 + 32u * u + lane;
+        r[u] = 0;
+#pragma unroll
+        for (uint32_t s = 16; s > 0; s >>= 1) {  // the last row that starts at or before f
+          const uint32_t e = __shfl_sync(CDS_FULL, ex, (r[u] + s) & 31u);
+          if (r[u] + s < n && e <= f) r[u] += s;
+        }
+        const uint32_t *p = reinterpret_cast<const uint32_t *>(
+            __shfl_sync(CDS_FULL, reinterpret_cast<unsigned long long>(list), r[u]));
+        const uint32_t at = f - __shfl_sync(CDS_FULL, ex, r[u]);
+        b[u] = f < total ? p[at] : 0xFFFFFFFFu;
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        if (b[u] < lo_id || b[u] > hi_id) continue;
+        uint32_t lo = 0, hi = d;
+        while (lo < hi) {
+          const uint32_t mid = (lo + hi) >> 1;
+          if (A[mid] < b[u]) lo = mid + 1;
+          else hi = mid;
+        }
+        if (lo < d && A[lo] == b[u]) hit(r0 + r[u], lo);
+      }
+    }
+  }
+}
+
+// Heavy part of the local graph: one word at a time of each row, word(i, w, m)
+// with bit l of m set when A[i] and A[32 w + l] are adjacent heavy vertices.  A
+// lane reads the bit of its column from row i of the heavy bitmap and a ballot
+// makes the word, so 32 pairs cost one load and no search or atomic.  Word-
+// uniform calls, every word of every row once (zero where nothing is heavy).
+// Returns whether the calling warp met a light vertex.
+template <bool TB, class Word>
+__device__ __forceinline__ bool heavy_words(const HeavyBits &hb, const uint32_t *hid, uint32_t d, Word word) {
+  const uint32_t lane = lane_id(), W = (d + 31) >> 5;
+  bool light = false;
+  for (uint32_t i = Team<TB>::warp(); i < d; i += Team<TB>::warps()) {
+    const uint32_t hi = hid[i];
+    light |= hi == LIGHT;
+    const uint32_t *row = hb.bits + (size_t)hi * hb.words;
+#pragma unroll 4
+    for (uint32_t w = 0; w < W; w++) {
+      const uint32_t j = w * 32 + lane;
+      const uint32_t hj = j < d && hi != LIGHT ? hid[j] : LIGHT;
+      const bool on = hj != LIGHT && (row[hj >> 5] >> (hj & 31)) & 1u;
+      word(i, w, __ballot_sync(CDS_FULL, on));
+    }
+  }
+  return light;
+}
+
+// Depth-first enumeration of the `depth`-cliques {l1 < l2 < ...} inside mask M
+// from position `first` on, over symmetric rows; leaf(path, s) for each, with
+// s = the vertices adjacent to all of the path inside M.  Only for k >= 6.
+template <class Leaf>
+__device__ void dfs_common(const uint32_t *rows, uint32_t rs, uint32_t W, const uint32_t *M, uint32_t first,
+                           int depth, Leaf leaf) {
+  uint32_t stack[CDS_MAX_K][DFS_WMAX];
+  uint32_t path[CDS_MAX_K];
+  uint32_t pos[CDS_MAX_K];
+  for (uint32_t w = 0; w < W; w++) stack[0][w] = M[w];
+  int lvl = 0;
+  pos[0] = first;
+  while (lvl >= 0) {
+    uint32_t b = pos[lvl];
+    uint32_t found = 0xFFFFFFFFu;
+    while ((b >> 5) < W) {
+      const uint32_t word = stack[lvl][b >> 5] & (0xFFFFFFFFu << (b & 31));
+      if (word) { found = ((b >> 5) << 5) + (uint32_t)(__ffs(word) - 1); break; }
+      b = ((b >> 5) + 1) << 5;
+    }
+    if (found == 0xFFFFFFFFu) { lvl--; continue; }
+    pos[lvl] = found + 1;
+    path[lvl] = found;
+    const uint32_t *row = rows + found * rs;
+    uint32_t c = 0;
+    if (lvl + 1 == depth) {
+      for (uint32_t w = 0; w < W; w++) c += __popc(stack[lvl][w] & row[w]);
+      if (c) leaf(path, c);
+      continue;
+    }
+    for (uint32_t w = 0; w < W; w++) {
+      stack[lvl + 1][w] = stack[lvl][w] & row[w];
+      c |= stack[lvl + 1][w];
+    }
+    if (c) {
+      lvl++;
+      pos[lvl] = found + 1;
+    }
+  }
+}
+
+// Words from one symmetric row to the next: a row of more than one word is
+// padded with zeros to whole 16-byte pieces, an odd number of them apart, so that
+// eight lanes reading a piece each of different rows meet different banks.
+__host__ __device__ constexpr uint32_t row_stride(uint32_t W) { return W <= 1 ? 1u : 4u * (((W + 3) / 4) | 1u); }
+
+// What a counting team keeps in shared memory: the local vertices, their
+// heavy ids and counts (64-bit for the generic k >= 6) and, for k >= 4, the rows
+// unless they live in global memory.
+__host__ __device__ constexpr uint32_t count_team_words(int K, uint32_t dmax, bool rows_in_smem) {
+  const uint32_t d4 = (dmax + 3) & ~3u;
+  uint32_t words = d4 * (K == 0 ? 4 : 3);
+  if (K != 3 && rows_in_smem) words += dmax * row_stride((dmax + 31) / 32);
+  return (words + 3) & ~3u;
+}
+// bits common to two (three) rows
+__device__ __forceinline__ uint32_t common(const uint32_t *a, const uint32_t *b, uint32_t W) {
+  if (W == 1) return __popc(*a & *b);
+  uint32_t s = 0;
+  for (uint32_t w = 0; w < W; w += 4) {
+    const uint4 x = *reinterpret_cast<const uint4 *>(a + w), y = *reinterpret_cast<const uint4 *>(b + w);
+    s += __popc(x.x & y.x) + __popc(x.y & y.y) + __popc(x.z & y.z) + __popc(x.w & y.w);
+  }
+  return s;
+}
+__device__ __forceinline__ uint32_t common(const uint32_t *a, const uint32_t *b, const uint32_t *c, uint32_t W) {
+  if (W == 1) return __popc(*a & *b & *c);
+  uint32_t s = 0;
+  for (uint32_t w = 0; w < W; w += 4) {
+    const uint4 x = *reinterpret_cast<const uint4 *>(a + w), y = *reinterpret_cast<const uint4 *>(b + w),
+                z = *reinterpret_cast<const uint4 *>(c + w);
+    s += __popc(x.x & y.x & z.x) + __popc(x.y & y.y & z.y) + __popc(x.z & y.z & z.z) + __popc(x.w & y.w & z.w);
+  }
+  return s;
+}
+
+// A writing team: the local vertices and heavy ids, the prefix over the rows'
+// popcounts, the rows.
+__host__ __device__ constexpr uint32_t write_team_words(uint32_t dmax, bool rows_in_smem) {
+  const uint32_t d4 = (dmax + 3) & ~3u;
+  return (3 * d4 + 4 + (rows_in_smem ? dmax * (((dmax + 31) / 32) | 1u) : 0u) + 3) & ~3u;
+}
+
+// The (k-1)-cliques of the local graph G[A]: cnt[i] = those that hold A[i],
+// times k-2 (divided out by the caller), for K = 3, 4, 5 and any k (K = 0).
+//
+// Rows are symmetric (both directions of an arc), so a pair (i, j) of adjacent
+// vertices with s = |row_i & row_j| adds s to both ends and every clique is met
+// once per edge (k = 4), with no step per clique: the oriented rows this
+// replaces found each clique once and then paid a shared-memory atomic for its
+// last member.  For k = 5 the same with triangles i < j < l, for k >= 6 with the
+// (k-2)-cliques of a depth-first search.  k = 3 counts local degrees and needs
+// no rows.  A warp takes a row and gives each word's 32 vertices to its lanes
+// (where cliques are many the rows are dense: about two in three of the pairs at
+// R-MAT scale 18, edge factor 16); neighbourhoods of at most 32 need one word a
+// row and a lane each.  Bound by instruction issue (2.9 of 4 slots with the
+// searched rows), so the step that counts is the row building: by binary
+// search of every out-list 5.9 ms for the 2.29 G 4-cliques of that graph, by
+// bitmap words and ballots 2.2 ms.
+template <int K, bool TB, class C>
+__device__ void local_count(const uint32_t *A, const uint32_t *hid, uint32_t d, const HeavyBits &hb,
+                            const uint64_t *doff, const uint32_t *dadj, const uint32_t *outdeg, uint32_t *rows,
+                            C *cnt, int kk) {
+  using T = Team<TB>;
+  const int tr = T::rank(), ts = T::size();
+  const uint32_t lane = lane_id(), W = (d + 31) >> 5, rs = row_stride(W);
+  bool light;
+  if (K == 3) {
+    uint32_t deg = 0;
+    light = heavy_words<TB>(hb, hid, d, [&](uint32_t i, uint32_t w, uint32_t m) {
+      deg = (w ? deg : 0u) + __popc(m);
+      if (w + 1 == W && lane == 0) cnt[i] = deg;
+    });
+  } else {
+    light = heavy_words<TB>(hb, hid, d, [&](uint32_t i, uint32_t w, uint32_t m) {
+      if (lane == 0) rows[i * rs + w] = m;
+    });
+    const uint32_t pad = (rs == 1 ? 1u : (W + 3) & ~3u) - W;  // words read past the row's last
+    for (uint32_t i = tr; i < d * pad; i += ts) rows[(i / pad) * rs + W + i % pad] = 0;
+    for (uint32_t i = tr; i < d; i += ts) cnt[i] = 0;
+  }
+  if (T::any(light)) {  // synchronises the team
+    light_arcs<TB>(A, hid, d, doff, dadj, outdeg, [&](uint32_t i, uint32_t j) {
+      if (K == 3) {
+        atomicAdd(&cnt[i], C(1));
+        atomicAdd(&cnt[j], C(1));
+      } else {
+        atomicOr(&rows[i * rs + (j >> 5)], 1u << (j & 31));
+        atomicOr(&rows[j * rs + (i >> 5)], 1u << (i & 31));
+      }
+    });
+    T::sync();
+  }
+  if (K == 3) return;
+  if (!TB && (K == 4 || K == 5) && W == 1) {
+    const uint32_t row = lane < d ? rows[lane * rs] : 0u;
+    uint32_t s = 0;
+    if (K == 4) {
+      for (uint32_t j = 0; j < d; j++) {
+        const uint32_t rj = __shfl_sync(CDS_FULL, row, j);
+        if ((row >> j) & 1u) s += __popc(row & rj);
+      }
+    } else {
+      for (uint32_t m = row; m; m &= m - 1) {
+        const uint32_t j = __ffs(m) - 1;
+        const uint32_t mj = row & rows[j * rs] & ~((2u << j) - 1u);
+        for (uint32_t q = mj; q; q &= q - 1) s += __popc(mj & rows[(__ffs(q) - 1) * rs]);
+      }
+      s = s / 2 * 3;  // each triangle of the row was met from two of its pairs' first ends
+    }
+    if (lane < d) cnt[lane] = s;
+    T::sync();
+    return;
+  }
+  for (uint32_t i = T::warp(); i < d; i += T::warps()) {
+    const uint32_t *ri = rows + i * rs;
+    C mine = 0;
+    for (uint32_t w0 = i >> 5; w0 < W; w0++) {
+      uint32_t m = ri[w0];
+      if (w0 == (i >> 5)) m &= ~((2u << (i & 31)) - 1u);  // neighbours after i
+      if (!((m >> lane) & 1u)) continue;
+      const uint32_t j = w0 * 32 + lane;
+      const uint32_t *rj = rows + j * rs;
+      C sum = 0;
+      if (K == 4) {
+        sum = common(ri, rj, W);
+      } else if (K == 5) {
+        uint32_t all = 0;
+        for (uint32_t w = w0; w < W; w++) {
+          uint32_t m2 = ri[w] & rj[w];
+          if (w == w0) m2 &= ~((2u << lane) - 1u);
+          for (; m2; m2 &= m2 - 1) {
+            const uint32_t l = (w << 5) + (uint32_t)(__ffs(m2) - 1);
+            const uint32_t s = common(ri, rj, rows + l * rs, W);
+            if (s) atomicAdd(&cnt[l], C(s));
+            all += s;
+          }
+        }
+        sum = all;
+      } else {
+        uint32_t M[DFS_WMAX], any = 0;
+        for (uint32_t w = 0; w < W; w++) {
+          M[w] = ri[w] & rj[w];
+          any |= M[w];
+        }
+        if (any)
+          dfs_common(rows, rs, W, M, j + 1, kk - 4, [&](const uint32_t *path, uint32_t s) {
+            for (int t = 0; t < kk - 4; t++) atomicAdd(&cnt[path[t]], C(s));
+            sum += s;
+          });
+      }
+      if (sum) atomicAdd(&cnt[j], sum);
+      mine += sum;
+    }
+    mine = warp_sum(mine);
+    if (lane == 0 && mine) atomicAdd(&cnt[i], mine);
+  }
+  T::sync();
+}
+
+// Pass 1: cliques of each root, and clique degrees.  Warp teams take roots of
+// out-degree up to p.dmax, block teams larger ones.
+template <int K, bool TB>
+__global__ void k_count(ListParams p) {
+  using T = Team<TB>;
+  using C = typename CountOf<K>::type;
+  const int KK = K ? K : (int)p.k;
+  extern __shared__ __align__(16) uint32_t sm[];
+  __shared__ uint32_t s_root;
+  uint32_t *S = sm + (TB ? 0u : (threadIdx.x >> 5) * p.team_words);
+  const uint32_t d4 = (p.dmax + 3) & ~3u;
+  C *cnt = reinterpret_cast<C *>(S);
+  uint32_t *A = S + d4 * (sizeof(C) / 4);
+  uint32_t *hid = A + d4;
+  uint32_t *rows = (TB && p.rows_global) ? p.rows_global + (uint64_t)blockIdx.x * p.rows_slab : hid + d4;
+  const int tr = T::rank(), ts = T::size();
+  const uint32_t nroots = *p.nroots;
+  for (;;) {
+    uint32_t r;
+    if (TB) {
+      if (threadIdx.x == 0) s_root = atomicAdd(p.work, 1u);
+      __syncthreads();
+      r = s_root;
+      __syncthreads();
+    } else {
+      if (lane_id() == 0) r = atomicAdd(p.work, 1u);
+      r = __shfl_sync(CDS_FULL, r, 0);
+    }
+    if (r >= nroots) break;
+    const uint32_t u = p.roots[r];
+    const uint32_t d = p.outdeg[u];
+    const uint32_t W = (d + 31) >> 5;
+    if ((K == 0 || K == 5) && W > (uint32_t)DFS_WMAX) {  // k >= 5 is limited to DFS_WMAX words
+      if (tr == 0) atomicOr(p.err, DEV_ERR_OVERFLOW);
+      continue;
+    }
+    if (d > p.dmax) {  // classification guarantees d <= dmax
+      if (tr == 0) atomicOr(p.err, DEV_ERR_INTERNAL);
+      continue;
+    }
+    const uint32_t *Au = p.dadj + p.doff[u];
+    for (uint32_t i = tr; i < d; i += ts) {
+      const uint32_t a = Au[i];
+      A[i] = a;
+      hid[i] = p.heavy.id(a);
+    }
+    T::sync();
+    local_count<K, TB, C>(A, hid, d, p.heavy, p.doff, p.dadj, p.outdeg, rows, cnt, KK);
+    unsigned long long mine = 0;
+    for (uint32_t i = tr; i < d; i += ts) {
+      const unsigned long long c = (unsigned long long)cnt[i] / (unsigned)(KK - 2);
+      mine += c;
+      if (c) {
+        if (p.cdeg64) atomicAdd(&p.cdeg64[A[i]], c);
+        else atomicAdd(&p.cdeg[A[i]], (uint32_t)c);
+      }
+    }
+    const unsigned long long total = T::template sum<unsigned long long>(mine) / (unsigned)(KK - 1);
+    if (tr == 0) {
+      p.root_cnt[u] = total;
+      if (total) {
+        if (p.cdeg64) atomicAdd(&p.cdeg64[u], total);
+        else atomicAdd(&p.cdeg[u], (uint32_t)total);
+      }
+    }
+    T::sync();
   }
 }
 
@@ -115,19 +487,20 @@ __device__ void dfs_cliques(const uint32_t *rows, uint32_t rs, uint32_t W, const
   }
 }
 
-// K = 3 and K = 4 are specialised; K = 0 is the generic path for k >= 5.
-template <int K, bool WRITE, bool TB>
-__global__ void k_list(ListParams p) {
+// Pass 2: clique records at each root's offset.  K = 3 and K = 4 are
+// specialised; K = 0 is the generic path for k >= 5.
+template <int K, bool TB>
+__global__ void k_list_write(ListParams p) {
   using T = Team<TB>;
   const int KK = K ? K : (int)p.k;
-  extern __shared__ uint32_t sm[];
+  extern __shared__ __align__(16) uint32_t sm[];
   __shared__ uint32_t s_root;
   uint32_t *S = sm + (TB ? 0u : (threadIdx.x >> 5) * p.team_words);
-  uint32_t *A = S;                  // [dmax]
-  uint32_t *P = A + p.dmax;         // [dmax+1] row-popcount prefix
-  uint32_t *cnt = P + p.dmax + 1;   // [dmax] local clique degrees
-  uint32_t *rows = (TB && p.rows_global) ? p.rows_global + (uint64_t)blockIdx.x * p.rows_slab
-                                         : cnt + p.dmax;
+  const uint32_t d4 = (p.dmax + 3) & ~3u;
+  uint32_t *A = S;               // [dmax]
+  uint32_t *P = A + d4;          // [dmax+1] row-popcount prefix
+  uint32_t *hid = P + d4 + 4;
+  uint32_t *rows = (TB && p.rows_global) ? p.rows_global + (uint64_t)blockIdx.x * p.rows_slab : hid + d4;
   const int tr = T::rank(), ts = T::size();
   const uint32_t nroots = *p.nroots;
   for (;;) {
@@ -143,48 +516,42 @@ __global__ void k_list(ListParams p) {
     }
     if (r >= nroots) break;
     const uint32_t u = p.roots[r];
+    const unsigned long long b0 = p.base[u];
+    if (p.base[u + 1] == b0) continue;  // no clique has this root
     const uint32_t d = p.outdeg[u];
-    if (d > p.dmax) {  // classification guarantees d <= dmax
-      if (tr == 0) atomicOr(p.err, DEV_ERR_INTERNAL);
-      continue;
-    }
     const uint32_t W = (d + 31) >> 5;
     if (K == 0 && W > (uint32_t)DFS_WMAX) {  // DFS masks are limited to DFS_WMAX words
       if (tr == 0) atomicOr(p.err, DEV_ERR_OVERFLOW);
       continue;
     }
+    if (d > p.dmax) {  // classification guarantees d <= dmax
+      if (tr == 0) atomicOr(p.err, DEV_ERR_INTERNAL);
+      continue;
+    }
     const uint32_t rs = W | 1u;  // odd stride: lanes reading different rows hit different banks
     const uint32_t *Au = p.dadj + p.doff[u];
-    for (uint32_t i = (uint32_t)tr * 4; i < d; i += (uint32_t)ts * 4) {
-      const uint4 q = *reinterpret_cast<const uint4 *>(Au + i);
-      A[i] = q.x;
-      if (i + 1 < d) A[i + 1] = q.y;
-      if (i + 2 < d) A[i + 2] = q.z;
-      if (i + 3 < d) A[i + 3] = q.w;
-    }
-    for (uint32_t i = tr; i < d * rs; i += ts) rows[i] = 0;
-    T::sync();
-    // local adjacency bitmap
-    for (uint32_t i = T::warp(); i < d; i += T::warps()) {
-      const uint32_t a = A[i];
-      const uint32_t da = p.outdeg[a];
-      const uint32_t *Aa = p.dadj + p.doff[a];
-      uint32_t *row = rows + i * rs;
-      const uint32_t lo_id = A[0], hi_id = A[d - 1];
-      for (uint32_t t = lane_id(); t < da; t += 32) {
-        const uint32_t b = Aa[t];
-        if (b < lo_id || b > hi_id) continue;
-        uint32_t lo = 0, hi = d;
-        while (lo < hi) {
-          const uint32_t mid = (lo + hi) >> 1;
-          if (A[mid] < b) lo = mid + 1;
-          else hi = mid;
-        }
-        if (lo < d && A[lo] == b) atomicOr(&row[lo >> 5], 1u << (lo & 31));
-      }
+    for (uint32_t i = tr; i < d; i += ts) {
+      const uint32_t a = Au[i];
+      A[i] = a;
+      hid[i] = p.heavy.id(a);
     }
     T::sync();
-    // P = exclusive prefix of row popcounts; cnt[i] = popcount (pass 1, k = 3)
+    // local adjacency bitmap, oriented (a record's members follow DAG arcs): of
+    // an adjacent heavy pair the arc is the one that climbs in (degree, id)
+    const bool light = heavy_words<TB>(p.heavy, hid, d, [&](uint32_t i, uint32_t w, uint32_t m) {
+      const uint32_t j = w * 32 + lane_id();
+      bool on = (m >> lane_id()) & 1u;
+      if (on) on = above(p.deg[A[j]], A[j], p.deg[A[i]], A[i]);
+      m = __ballot_sync(CDS_FULL, on);
+      if (lane_id() == 0) rows[i * rs + w] = m;
+    });
+    if (T::any(light)) {
+      light_arcs<TB>(A, hid, d, p.doff, p.dadj, p.outdeg, [&](uint32_t i, uint32_t j) {
+        atomicOr(&rows[i * rs + (j >> 5)], 1u << (j & 31));
+      });
+      T::sync();
+    }
+    // P = exclusive prefix of row popcounts
     uint32_t carry = 0;
     for (uint32_t i0 = 0; i0 < d; i0 += ts) {
       const uint32_t i = i0 + tr;
@@ -193,37 +560,23 @@ __global__ void k_list(ListParams p) {
         for (uint32_t w = 0; w < W; w++) v += __popc(rows[i * rs + w]);
       uint32_t tot;
       const uint32_t ex = T::template scan<uint32_t>(v, &tot);
-      if (i < d) {
-        P[i] = carry + ex;
-        if (!WRITE) cnt[i] = (K == 3) ? v : 0u;
-      }
+      if (i < d) P[i] = carry + ex;
       carry += tot;
     }
     if (tr == 0) P[d] = carry;
     T::sync();
     const uint32_t npairs = carry;
-    unsigned long long mine = 0;  // cliques counted by this thread
     if (K == 3) {
-      if (!WRITE) {
-        for (uint32_t q = tr; q < npairs; q += ts) {
-          const uint32_t i = find_row(P, d, q);
-          const uint32_t j = nth_in_row(rows + i * rs, q - P[i]);
-          atomicAdd(&cnt[j], 1u);
-        }
-        mine = (tr == 0) ? npairs : 0;
-      } else {
-        const unsigned long long b0 = p.base[u];
-        for (uint32_t q = tr; q < npairs; q += ts) {
-          const uint32_t i = find_row(P, d, q);
-          const uint32_t j = nth_in_row(rows + i * rs, q - P[i]);
-          uint32_t *o = p.out + (b0 + q) * 3;
-          o[0] = u;
-          o[1] = A[i];
-          o[2] = A[j];
-        }
+      for (uint32_t q = tr; q < npairs; q += ts) {
+        const uint32_t i = find_row(P, d, q);
+        const uint32_t j = nth_in_row(rows + i * rs, q - P[i]);
+        uint32_t *o = p.out + (b0 + q) * 3;
+        o[0] = u;
+        o[1] = A[i];
+        o[2] = A[j];
       }
     } else {
-      unsigned long long wcarry = WRITE ? p.base[u] : 0ull;
+      unsigned long long wcarry = b0;
       for (uint32_t q0 = 0; q0 < npairs; q0 += ts) {
         const uint32_t q = q0 + tr;
         uint32_t i = 0, j = 0;
@@ -254,87 +607,49 @@ __global__ void k_list(ListParams p) {
                           [&](const uint32_t *, int) { c++; });
           }
         }
-        if (!WRITE) {
-          if (c) {
-            mine += c;
-            atomicAdd(&cnt[i], (uint32_t)c);
-            atomicAdd(&cnt[j], (uint32_t)c);
+        unsigned long long tot;
+        const unsigned long long ex = T::template scan<unsigned long long>(c, &tot);
+        if (c) {
+          unsigned long long o = wcarry + ex;
+          const uint32_t ai = A[i], aj = A[j];
+          if (K == 4) {
+            // a record that starts a 32-byte sector waits for its successor,
+            // and the two go out as one 32-byte store (a whole sector)
+            // instead of two half-sector stores
             const uint32_t *ri = rows + i * rs, *rj = rows + j * rs;
-            if (K == 4) {
-              for (uint32_t w = 0; w < W; w++) {
-                uint32_t m = ri[w] & rj[w];
-                while (m) {
-                  atomicAdd(&cnt[(w << 5) + (uint32_t)(__ffs(m) - 1)], 1u);
-                  m &= m - 1;
+            uint4 pend = make_uint4(0u, 0u, 0u, 0u);
+            bool has = false;
+            for (uint32_t w = 0; w < W; w++) {
+              uint32_t m = small ? M[w] : (ri[w] & rj[w]);
+              while (m) {
+                const uint32_t l = (w << 5) + (uint32_t)(__ffs(m) - 1);
+                m &= m - 1;
+                const uint4 r = make_uint4(u, ai, aj, A[l]);
+                if (has) {
+                  store_sector(p.out + (o - 1) * 4, pend, r);
+                  has = false;
+                } else if ((reinterpret_cast<uintptr_t>(p.out + o * 4) & 31u) == 0) {
+                  pend = r;
+                  has = true;
+                } else {
+                  *reinterpret_cast<uint4 *>(p.out + o * 4) = r;
                 }
-              }
-            } else {
-              dfs_cliques(rows, rs, W, M, KK - 3, [&](const uint32_t *path, int depth) {
-                for (int t = 0; t < depth; t++) atomicAdd(&cnt[path[t]], 1u);
-              });
-            }
-          }
-        } else {
-          unsigned long long tot;
-          const unsigned long long ex = T::template scan<unsigned long long>(c, &tot);
-          if (c) {
-            unsigned long long o = wcarry + ex;
-            const uint32_t ai = A[i], aj = A[j];
-            if (K == 4) {
-              // a record that starts a 32-byte sector waits for its successor,
-              // and the two go out as one 32-byte store (a whole sector)
-              // instead of two half-sector stores
-              const uint32_t *ri = rows + i * rs, *rj = rows + j * rs;
-              uint4 pend = make_uint4(0u, 0u, 0u, 0u);
-              bool has = false;
-              for (uint32_t w = 0; w < W; w++) {
-                uint32_t m = small ? M[w] : (ri[w] & rj[w]);
-                while (m) {
-                  const uint32_t l = (w << 5) + (uint32_t)(__ffs(m) - 1);
-                  m &= m - 1;
-                  const uint4 r = make_uint4(u, ai, aj, A[l]);
-                  if (has) {
-                    store_sector(p.out + (o - 1) * 4, pend, r);
-                    has = false;
-                  } else if ((reinterpret_cast<uintptr_t>(p.out + o * 4) & 31u) == 0) {
-                    pend = r;
-                    has = true;
-                  } else {
-                    *reinterpret_cast<uint4 *>(p.out + o * 4) = r;
-                  }
-                  o++;
-                }
-              }
-              if (has) *reinterpret_cast<uint4 *>(p.out + (o - 1) * 4) = pend;
-            } else {
-              dfs_cliques(rows, rs, W, M, KK - 3, [&](const uint32_t *path, int depth) {
-                uint32_t *rec = p.out + o * (unsigned long long)KK;
-                rec[0] = u;
-                rec[1] = ai;
-                rec[2] = aj;
-                for (int t = 0; t < depth; t++) rec[3 + t] = A[path[t]];
                 o++;
-              });
+              }
             }
+            if (has) *reinterpret_cast<uint4 *>(p.out + (o - 1) * 4) = pend;
+          } else {
+            dfs_cliques(rows, rs, W, M, KK - 3, [&](const uint32_t *path, int depth) {
+              uint32_t *rec = p.out + o * (unsigned long long)KK;
+              rec[0] = u;
+              rec[1] = ai;
+              rec[2] = aj;
+              for (int t = 0; t < depth; t++) rec[3 + t] = A[path[t]];
+              o++;
+            });
           }
-          wcarry += tot;
         }
-      }
-    }
-    if (!WRITE) {
-      T::sync();
-      for (uint32_t i = tr; i < d; i += ts)
-        if (cnt[i]) {
-          if (p.cdeg64) atomicAdd(&p.cdeg64[A[i]], (unsigned long long)cnt[i]);
-          else atomicAdd(&p.cdeg[A[i]], cnt[i]);
-        }
-      const unsigned long long total = T::template sum<unsigned long long>(mine);
-      if (tr == 0) {
-        p.root_cnt[u] = total;
-        if (total) {
-          if (p.cdeg64) atomicAdd(&p.cdeg64[u], total);
-          else atomicAdd(&p.cdeg[u], (uint32_t)total);
-        }
+        wcarry += tot;
       }
     }
     T::sync();

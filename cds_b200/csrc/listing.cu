@@ -71,8 +71,9 @@ void launch_pass(cds_ctx *c, cudaStream_t s, const cds::Tuning &t, ListParams p,
     smem = (size_t)p.team_words * 4 * (threads / 32);
   }
   void (*fn)(ListParams);
-  if (block_team) fn = write ? k_list<K, true, true> : k_list<K, false, true>;
-  else fn = write ? k_list<K, true, false> : k_list<K, false, false>;
+  constexpr int KW = K == 5 ? 0 : K;  // records of k >= 5 are written by the generic kernel
+  if (block_team) fn = write ? k_list_write<KW, true> : k_count<K, true>;
+  else fn = write ? k_list_write<KW, false> : k_count<K, false>;
   // The limit is a property of the kernel shared by every thread of the
   // process: concurrent solves (server workers) launch it with different
   // sizes, so it is raised to the device's maximum rather than set to this
@@ -121,6 +122,8 @@ void run_listing(cds_ctx *c, cudaStream_t s, const cds::Dag &dag, bool materiali
   p.doff = dag.off.p;
   p.dadj = dag.adj.p;
   p.outdeg = dag.outdeg.p;
+  p.deg = dag.deg.p;
+  p.heavy = dag.heavy;
   p.cdeg = nullptr;
   p.cdeg64 = out.cdeg64.p;
   p.root_cnt = root_cnt.p;
@@ -128,11 +131,12 @@ void run_listing(cds_ctx *c, cudaStream_t s, const cds::Dag &dag, bool materiali
   p.k = k;
 
   // block-team geometry
-  const uint32_t bdmax = std::max<uint32_t>(dag.max_out, warp_dmax + 1);
+  // (k >= 5 refuses roots of out-degree above its masks' reach)
+  uint32_t bdmax = std::max<uint32_t>(dag.max_out, warp_dmax + 1);
+  if (K == 0 || K == 5) bdmax = std::min<uint32_t>(bdmax, DFS_WMAX * 32);
   const bool rows_in_smem = bdmax <= (uint32_t)BLOCK_DMAX;
-  const uint32_t bw = (bdmax + 31) / 32;
-  const uint64_t brow_words = (uint64_t)bdmax * (bw | 1u);
-  DBuf<uint32_t> rows_global;
+  const uint64_t brow_words = ((uint64_t)bdmax * row_stride((bdmax + 31) / 32) + 3) & ~3ull;  // 16-byte aligned slabs
+  DBuf<uint32_t> rows_global(c, s, 0);
   uint32_t bgrid_cap = 0;
   const bool any_block = dag.max_out > warp_dmax;
   if (any_block && !rows_in_smem) {
@@ -147,8 +151,7 @@ void run_listing(cds_ctx *c, cudaStream_t s, const cds::Dag &dag, bool materiali
       q.nroots = counters.p;
       q.work = counters.p + 2 + (write ? 1 : 0);
       q.dmax = warp_dmax;
-      q.team_words = warp_dmax + (warp_dmax + 1) + warp_dmax + warp_dmax * (((warp_dmax + 31) / 32) | 1u);
-      q.team_words = (q.team_words + 3) & ~3u;
+      q.team_words = write ? write_team_words(warp_dmax, true) : count_team_words(K, warp_dmax, true);
       launch_pass<K>(c, s, t, q, write, false, 0);
     }
     if (any_block) {
@@ -157,8 +160,8 @@ void run_listing(cds_ctx *c, cudaStream_t s, const cds::Dag &dag, bool materiali
       q.nroots = counters.p + 1;
       q.work = counters.p + 4 + (write ? 1 : 0);
       q.dmax = bdmax;
-      q.team_words = bdmax + (bdmax + 1) + bdmax + (rows_in_smem ? (uint32_t)brow_words : 0u);
-      q.team_words = (q.team_words + 3) & ~3u;
+      q.team_words = write ? write_team_words(bdmax, rows_in_smem)
+                           : count_team_words(K, bdmax, rows_in_smem);
       q.rows_global = rows_in_smem ? nullptr : rows_global.p;
       q.rows_slab = brow_words;
       launch_pass<K>(c, s, t, q, write, true, bgrid_cap);
@@ -228,6 +231,7 @@ void list_cliques(cds_ctx *c, cudaStream_t s, const Dag &dag, uint32_t k, bool m
   }
   if (k == 3) run_listing<3>(c, s, dag, materialize, t, out, err.p, k, on_count);
   else if (k == 4) run_listing<4>(c, s, dag, materialize, t, out, err.p, k, on_count);
+  else if (k == 5) run_listing<5>(c, s, dag, materialize, t, out, err.p, k, on_count);
   else run_listing<0>(c, s, dag, materialize, t, out, err.p, k, on_count);
   const uint32_t e = d2h(err.p, s);
   if (e & DEV_ERR_OVERFLOW)

@@ -143,7 +143,7 @@ template <int K>
 cds_status launch_count(ListParams p, bool block_team, int sms, cudaStream_t s) {
   const int threads = block_team ? 512 : 256;
   const size_t smem = block_team ? (size_t)p.team_words * 4 : (size_t)p.team_words * 4 * (threads / 32);
-  void (*fn)(ListParams) = block_team ? k_list<K, false, true> : k_list<K, false, false>;
+  void (*fn)(ListParams) = block_team ? k_count<K, true> : k_count<K, false>;
   // raised to the device maximum, never lowered: the listing kernels are
   // shared with the allocating entry points, which may run in other threads
   int dev = 0, optin = 0;
@@ -175,8 +175,7 @@ cds_status count_pass(ListParams p, uint32_t nw, uint32_t nb, const uint32_t *d_
     q.nroots = d_nw;
     q.work = work;
     q.dmax = NA_WARP_DMAX;
-    q.team_words = (NA_WARP_DMAX + (NA_WARP_DMAX + 1) + NA_WARP_DMAX +
-                    NA_WARP_DMAX * (((NA_WARP_DMAX + 31) / 32) | 1u) + 3) & ~3u;
+    q.team_words = count_team_words(K, NA_WARP_DMAX, true);
     st = launch_count<K>(q, false, sms, s);
     if (st != CDS_OK) return st;
   }
@@ -186,7 +185,7 @@ cds_status count_pass(ListParams p, uint32_t nw, uint32_t nb, const uint32_t *d_
     q.nroots = d_nb;
     q.work = work + 1;
     q.dmax = bdmax;
-    q.team_words = (bdmax + (bdmax + 1) + bdmax + bdmax * (((bdmax + 31) / 32) | 1u) + 3) & ~3u;
+    q.team_words = count_team_words(K, bdmax, true);
     q.rows_global = nullptr;
     st = launch_count<K>(q, true, sms, s);
   }
@@ -277,7 +276,7 @@ extern "C" cds_status cds_count_cliques_noalloc(const uint64_t *d_off, const uin
   NA_TRY(cudaStreamSynchronize(s));
   if (hctl[C_MAXOUT] > NA_MAX_OUT) return CDS_ERR_INPUT;
   if (dag_arcs > NA_MAX_ARCS / 2 + 3 * (uint64_t)NA_MAX_N + 4) return CDS_ERR_INPUT;
-  k_dag_fill<<<grid, 256, 0, s>>>(d_off, d_adj, deg, n, doff, dadj);
+  k_dag_fill<<<grid, 256, 0, s>>>(d_off, d_adj, deg, n, doff, dadj, HeavyBits{}, nullptr);  // all light: no memory for a bitmap
   cds::count_launch();
   NA_TRY(cudaGetLastError());
   if (k == 2) {  // every edge is a 2-clique
@@ -303,6 +302,7 @@ extern "C" cds_status cds_count_cliques_noalloc(const uint64_t *d_off, const uin
   cds_status st;
   if (k == 3) st = count_pass<3>(p, hn[0], hn[1], ctl + C_NW, ctl + C_NB, bdmax, wl, bl, ctl + C_WORK, sms, s);
   else if (k == 4) st = count_pass<4>(p, hn[0], hn[1], ctl + C_NW, ctl + C_NB, bdmax, wl, bl, ctl + C_WORK, sms, s);
+  else if (k == 5) st = count_pass<5>(p, hn[0], hn[1], ctl + C_NW, ctl + C_NB, bdmax, wl, bl, ctl + C_WORK, sms, s);
   else st = count_pass<0>(p, hn[0], hn[1], ctl + C_NW, ctl + C_NB, bdmax, wl, bl, ctl + C_WORK, sms, s);
   if (st != CDS_OK) return st;
   k_na_sum<<<sms, 256, 0, s>>>(rcnt, n, d_count);

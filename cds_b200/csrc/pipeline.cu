@@ -214,7 +214,7 @@ void run_problem(cds_ctx *c, cudaStream_t s, UnionGraph &u, const cds_params &pr
   dag.outdeg = DBuf<uint32_t>(c, s, 0);
   dag.off = DBuf<uint64_t>(c, s, 0);
   dag.adj = DBuf<uint32_t>(c, s, 0);
-  build_dag(c, s, u.off, u.adj, u.n, dag);
+  build_dag(c, s, u.off, u.adj, u.n, k, dag);
   const int m1 = clk.mark();
 
   Cliques cl;

@@ -9,6 +9,21 @@
 
 namespace cds {
 
+// Adjacency bitmap of a graph's heavy vertices (both directions of an arc):
+// bit hj of row hi, rows of `words` words.  hid gives a vertex its heavy id or
+// 0xFFFFFFFF; null: ids are the vertices themselves (words > 0), or there are
+// no heavy vertices (words = 0).
+struct HeavyBits {
+  const uint32_t *bits = nullptr;
+  const uint32_t *hid = nullptr;
+  uint32_t words = 0;
+#ifdef __CUDACC__
+  __device__ __forceinline__ uint32_t id(uint32_t v) const {
+    return hid ? hid[v] : words ? v : 0xFFFFFFFFu;
+  }
+#endif
+};
+
 struct Dag {
   uint32_t n = 0;
   uint32_t max_out = 0;
@@ -16,9 +31,11 @@ struct Dag {
   DBuf<uint32_t> outdeg;  // [n] out-degree
   DBuf<uint64_t> off;     // [n+1] row starts (rows padded to 4 entries)
   DBuf<uint32_t> adj;     // out-neighbours, ascending id, 0xFFFFFFFF padding
+  DBuf<uint32_t> hid, hbits;  // storage of `heavy`
+  HeavyBits heavy;        // (k >= 3)
 };
 void build_dag(cds_ctx *c, cudaStream_t s, const uint64_t *off, const uint32_t *adj,
-               uint32_t n, Dag &dag);
+               uint32_t n, uint32_t k, Dag &dag);
 
 struct Cliques {
   uint32_t k = 0;
