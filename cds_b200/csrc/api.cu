@@ -317,18 +317,10 @@ cds_status cds_create(const cds_config *cfg, cds_ctx **out) {
     // per-k launch shapes measured on R-MAT graphs (cds_autotune refines
     // them): for k >= 3 roots of out-degree above 32 go to block teams, whose
     // 512 threads share a dense neighbourhood's pairs, more push/relabel
-    // rounds pass between global relabels, and peel items hold up to 1,024
-    // incidences (fewer hub flushes; k = 2 keeps 512); for k <= 3 peel items
-    // go in ascending clique-degree order (for k >= 4 that costs sweeps)
+    // rounds pass between global relabels
     for (uint32_t k = 0; k <= CDS_MAX_K; k++) {
       if (k >= 3) c->tune[k].list_warp_dmax = 32;
       if (k >= 3) c->tune[k].flow_rounds = 32;
-      if (k >= 3) c->tune[k].peel_chunk = 1024;
-      if (k <= 3) c->tune[k].peel_order = 1;  // fewer, cheaper sweeps for k = 2, 3
-      // k >= 4: half the peel items dealt round-robin, the rest by a counter
-      // (R-MAT-18 k = 4: 736 -> 640 ms; R-MAT-14 k = 4: 2.25 -> 1.82 ms; at
-      // k = 2, 3 the counter costs more than the balance gains)
-      if (k >= 4) c->tune[k].peel_static = 50;
     }
     uint64_t keep = ~0ull;  // keep freed blocks cached in the pool
     CDS_CUDA(cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep));
@@ -451,7 +443,7 @@ cds_status cds_list_cliques(cds_ctx *c, cds_graph *g, uint32_t k, uint32_t p_siz
     dag.adj = DBuf<uint32_t>(c, s, 0);
     build_dag(c, s, g->d_off, g->d_adj, g->n, k, dag);
     Cliques cl;
-    list_cliques(c, s, dag, k, false, c->tune[k < 2 ? 2 : (k > CDS_MAX_K ? CDS_MAX_K : k)], cl);
+    list_cliques(c, s, dag, k, LIST_COUNT, c->tune[k < 2 ? 2 : (k > CDS_MAX_K ? CDS_MAX_K : k)], cl);
     if (count) *count = cl.count;
     if (clique_degree && g->n)
       CDS_CUDA(cudaMemcpyAsync(clique_degree, cl.cdeg64.p, (size_t)g->n * 8, cudaMemcpyDeviceToHost, s));
@@ -475,9 +467,9 @@ cds_status cds_clique_core(cds_ctx *c, cds_graph *g, uint32_t k, uint32_t gl_buf
     dag.adj = DBuf<uint32_t>(c, s, 0);
     build_dag(c, s, u.off, u.adj, u.n, k, dag);
     Cliques cl;
-    list_cliques(c, s, dag, k, true, c->tune[k], cl);
+    list_cliques(c, s, dag, k, LIST_NARROW, c->tune[k], cl);
     PeelOut pe;
-    peel(c, s, u.n, cl, u.inst, c->tune[k], gl_buffer_size, pe);
+    peel(c, s, u.off, u.adj, u.nnz, dag, cl, u.inst, gl_buffer_size, pe);
     if (count) *count = cl.count;
     if (max_core) *max_core = pe.max_core;
     if (core && g->n) {
@@ -506,9 +498,9 @@ cds_status cds_densest_core(cds_ctx *c, cds_graph *g, uint32_t k, uint64_t *thre
     dag.adj = DBuf<uint32_t>(c, s, 0);
     build_dag(c, s, u.off, u.adj, u.n, k, dag);
     Cliques cl;
-    list_cliques(c, s, dag, k, true, c->tune[k], cl);
+    list_cliques(c, s, dag, k, LIST_NARROW, c->tune[k], cl);
     PeelOut pe;
-    peel(c, s, u.n, cl, u.inst, c->tune[k], 0, pe);
+    peel(c, s, u.off, u.adj, u.nnz, dag, cl, u.inst, 0, pe);
     const uint64_t bn = pe.best_num[0], bd = pe.best_den[0];
     const uint64_t t = (bd && bn) ? (bn + bd - 1) / bd : 0;
     if (threshold) *threshold = t;
@@ -540,11 +532,11 @@ cds_status cds_components(cds_ctx *c, cds_graph *g, uint32_t k, uint64_t *core_c
     dag.adj = DBuf<uint32_t>(c, s, 0);
     build_dag(c, s, u.off, u.adj, u.n, k, dag);
     Cliques cl;
-    list_cliques(c, s, dag, k, true, c->tune[k], cl);
+    list_cliques(c, s, dag, k, LIST_NARROW, c->tune[k], cl);
     PeelOut pe;
-    peel(c, s, u.n, cl, u.inst, c->tune[k], 0, pe);
+    peel(c, s, u.off, u.adj, u.nnz, dag, cl, u.inst, 0, pe);
     CoreOut co;
-    densest_core_and_components(c, s, dag, cl, pe, u.inst, k, co, true, nullptr);
+    densest_core_and_components(c, s, dag, pe, u.inst, k, c->tune[k], co, true);
     CDS_CUDA(cudaStreamSynchronize(s));
     if (core_cliques) *core_cliques = co.core_cliques[0];
     if (pruned_edges) *pruned_edges = co.pruned_edges[0];

@@ -113,11 +113,8 @@ extern "C" cds_status cds_autotune(cds_ctx *c, cds_graph *const *graphs, size_t 
         {&t.list_team_block, {256, 512}},
         {&t.flow_rounds, {4, 8, 16, 32}},
         {&t.flow_block, {256, 512}},
-        {&t.peel_chunk, {256, 512, 1024}},
         {&t.flow_warm, {-1, 0, 1, 3, 6}},
         {&t.flow_inc_per_block, {0, 4096, 16384, 65536}},
-        {&t.peel_order, {0, 1}},
-        {&t.peel_static, {100, 75, 50}},
     };
     // coordinate descent: one field at a time, the others at their best
     for (auto &cd : cands) {

@@ -35,9 +35,8 @@ struct Tuning {
   int flow_inc_per_block = 0;  // push-relabel grid: a block per this many incidences
                                // (0: the whole device); small networks then
                                // meet at cheaper grid barriers
-  int peel_chunk = 512;        // incidences per peel work item
-  int peel_order = 0;          // peel items by ascending clique-degree class (1) or vertex id (0)
-  int peel_static = 100;       // percent of peel items dealt round-robin; the rest by a counter
+  // kept in tuning caches, without effect (the peel has no such work items any more)
+  int peel_chunk = 512, peel_order = 0, peel_static = 100;
 };
 
 }  // namespace cds

@@ -10,8 +10,8 @@
 // (cpuCode/c++/src/helpers.cpp:710-1116).
 //
 //  - The (k',Psi)-core is every vertex with core number >= k' where
-//    k' = ceil(best core density); its cliques are the stored cliques whose
-//    members are all in it, so nothing is listed a second time.
+//    k' = ceil(best core density); its cliques are listed from the core's part
+//    of the DAG (no other clique of the graph is ever written).
 //  - Pruning marks each DAG arc covered by a core clique (clique records are
 //    in orientation order, so member x -> member y is an arc for x < y).
 //  - Components come from a lock-free union-find over the kept arcs (which
@@ -55,28 +55,45 @@ __global__ void k_core_flags(const uint32_t *__restrict__ core, uint32_t n,
   }
 }
 
-// A clique lies in the (k',Psi)-core when its smallest member core (cmin,
-// from the peel) is at least its instance's k' > 0; the flag overwrites cmin.
-// One instance: no record is read at all.
-__global__ void k_clique_flags(const uint32_t *__restrict__ members, uint64_t m, uint32_t k,
-                               const unsigned long long *__restrict__ kp, uint32_t *__restrict__ flag,
-                               const uint32_t *__restrict__ of_vertex,
-                               unsigned long long *__restrict__ core_cliques) {
-  const unsigned long long kp0 = kp[0];
-  RunCount run;
-  for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x; b < m; b += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t c = b + threadIdx.x;
-    bool in = false;
-    uint32_t i = 0;
-    if (c < m) {
-      i = inst_of(of_vertex, of_vertex ? members[c * k] : 0u);
-      const unsigned long long t = of_vertex ? kp[i] : kp0;
-      in = t > 0 && (unsigned long long)flag[c] >= t;
-      flag[c] = in;
-    }
-    run.add(core_cliques, i, in);
+// The core's part of the DAG: out-lists of core vertices, core neighbours only
+// (ids as they are; other vertices get empty lists).  Warp per vertex, lists
+// ascending and padded as the DAG's.
+__global__ void k_core_outdeg(const uint64_t *__restrict__ doff, const uint32_t *__restrict__ dadj,
+                              const uint32_t *__restrict__ outdeg, const uint8_t *__restrict__ in_core, uint32_t n,
+                              uint32_t *__restrict__ cout) {
+  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+  for (uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < n; u += warps) {
+    uint32_t c = 0;
+    if (in_core[u])
+      for (uint32_t t = lane_id(); t < outdeg[u]; t += 32) c += in_core[dadj[doff[u] + t]];
+    c = __reduce_add_sync(CDS_FULL, c);
+    if (lane_id() == 0) cout[u] = c;
   }
-  run.flush(core_cliques);
+}
+__global__ void k_core_dag(const uint64_t *__restrict__ doff, const uint32_t *__restrict__ dadj,
+                           const uint32_t *__restrict__ outdeg, const uint8_t *__restrict__ in_core, uint32_t n,
+                           const uint64_t *__restrict__ coff, uint32_t *__restrict__ cadj) {
+  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+  for (uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < n; u += warps) {
+    if (!in_core[u]) continue;
+    uint64_t at = coff[u];
+    const uint64_t end = coff[u + 1];
+    for (uint32_t t0 = 0; t0 < outdeg[u]; t0 += 32) {
+      const uint32_t t = t0 + lane_id();
+      const uint32_t w = t < outdeg[u] ? dadj[doff[u] + t] : 0u;
+      const bool in = t < outdeg[u] && in_core[w];
+      const uint32_t m = __ballot_sync(CDS_FULL, in);
+      if (in) cadj[at + __popc(m & ((1u << lane_id()) - 1u))] = w;
+      at += __popc(m);
+    }
+    for (uint64_t i = at + lane_id(); i < end; i += 32) cadj[i] = NONE;
+  }
+}
+// cliques of each instance, from the listing's offsets
+__global__ void k_inst_cliques(const uint64_t *__restrict__ base, const uint32_t *__restrict__ vbeg, uint32_t ninst,
+                               unsigned long long *__restrict__ out) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < ninst; i += gridDim.x * blockDim.x)
+    out[i] = base[vbeg[i + 1]] - base[vbeg[i]];
 }
 
 // arc u -> w of the DAG (w in the out-list of u), or NONE
@@ -92,12 +109,11 @@ __device__ __forceinline__ uint64_t find_arc(const uint64_t *doff, const uint32_
 }
 
 __global__ void k_mark_arcs(const uint32_t *__restrict__ members, uint64_t m, uint32_t k,
-                            const uint32_t *__restrict__ flag, const uint64_t *__restrict__ doff,
-                            const uint32_t *__restrict__ dadj, const uint32_t *__restrict__ outdeg,
+                            const uint64_t *__restrict__ doff, const uint32_t *__restrict__ dadj,
+                            const uint32_t *__restrict__ outdeg,
                             uint8_t *__restrict__ arc_keep, uint32_t *__restrict__ err) {
   for (uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; c < m;
        c += (uint64_t)gridDim.x * blockDim.x) {
-    if (!flag[c]) continue;
     const uint32_t *r = members + c * k;
     for (uint32_t x = 0; x < k; x++)
       for (uint32_t y = x + 1; y < k; y++) {
@@ -185,11 +201,9 @@ __global__ void k_comp_from_roots(const uint8_t *__restrict__ in_core, const uin
 }
 
 __global__ void k_mark_pairs(const uint32_t *__restrict__ members, uint64_t m, uint32_t k,
-                             const uint32_t *__restrict__ flag, const uint64_t *__restrict__ lid,
-                             uint32_t words, uint32_t *__restrict__ bits) {
+                             const uint64_t *__restrict__ lid, uint32_t words, uint32_t *__restrict__ bits) {
   for (uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; c < m;
        c += (uint64_t)gridDim.x * blockDim.x) {
-    if (!flag[c]) continue;
     auto mark = [&](uint32_t a, uint32_t b) {
       uint32_t *w = bits + (uint64_t)a * words + (b >> 5);
       const uint32_t bit = 1u << (b & 31);
@@ -289,41 +303,19 @@ __global__ void k_roots(uint32_t *parent, const uint8_t *__restrict__ in_core, u
     comp[v] = in_core[v] ? uf_find(parent, v) : NONE;
 }
 
-// Core cliques per component: the records are stored by root vertex
-// (cliques [base[u], base[u+1]) have u first), and a core clique lies in its
-// root's component, so only the flags are read -- no record.  A warp takes
-// a chunk of clique indices (a hub root's range of tens of millions of
-// cliques is shared by many warps; `chunk` shrinks with the clique count so
-// that small problems still have a chunk per warp and few roots per chunk),
-// finds the chunk's first root by binary search, and adds the flag sum of
-// each root's part of the chunk to that root's component.
-__global__ void k_comp_cliques(const unsigned long long *__restrict__ base, uint32_t n, uint64_t m,
-                               uint32_t chunk, const uint32_t *__restrict__ flag,
-                               const uint32_t *__restrict__ comp, unsigned long long *__restrict__ ccount) {
-  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  const uint64_t nchunks = (m + chunk - 1) / chunk;
-  for (uint64_t ch = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; ch < nchunks; ch += warps) {
-    uint64_t c0 = ch * chunk;
-    const uint64_t c1 = min(m, c0 + chunk);
-    // the last root u with base[u] <= c0 (base[0] = 0, base[n] = m)
-    uint32_t lo = 0, hi = n;
-    while (hi - lo > 1) {
-      const uint32_t mid = (lo + hi) >> 1;
-      if (base[mid] <= c0) lo = mid;
-      else hi = mid;
-    }
-    uint32_t u = lo;
-    while (c0 < c1) {
-      const uint64_t e = min(c1, (uint64_t)base[u + 1]);
-      const uint32_t r = comp[u];
-      if (e > c0 && r != NONE) {  // a root outside the core has no core clique
-        unsigned long long cnt = 0;
-        for (uint64_t c = c0 + lane_id(); c < e; c += 32) cnt += flag[c];
-        cnt = warp_sum(cnt);
-        if (lane_id() == 0 && cnt) atomicAdd(&ccount[r], cnt);
-      }
-      c0 = e;
-      u++;
+// Core cliques per component: every core clique lies in its root's component.
+__global__ void k_comp_cliques(const uint64_t *__restrict__ base, uint32_t n, const uint32_t *__restrict__ comp,
+                               unsigned long long *__restrict__ ccount) {
+  for (uint32_t b = blockIdx.x * blockDim.x; b < n; b += gridDim.x * blockDim.x) {
+    const uint32_t u = b + threadIdx.x;
+    const unsigned long long c = u < n ? base[u + 1] - base[u] : 0ull;
+    const uint32_t r = c ? comp[u] : NONE;
+    const uint32_t r0 = __shfl_sync(CDS_FULL, r, __ffs(__ballot_sync(CDS_FULL, c != 0) | 0x80000000u) - 1);
+    if (__all_sync(CDS_FULL, c == 0 || r == r0)) {  // one component in the warp, mostly
+      const unsigned long long sum = warp_sum(c);
+      if (lane_id() == 0 && sum) atomicAdd(&ccount[r0], sum);
+    } else if (c) {
+      atomicAdd(&ccount[r], c);
     }
   }
 }
@@ -399,8 +391,8 @@ constexpr uint32_t SMALL_NV = 2048;
 // A block whose core cliques all lie in one component (the usual case) takes
 // its slots with one atomic; otherwise each warp takes its own.
 __global__ void k_bucket_cliques(const uint32_t *__restrict__ members, uint64_t m, uint32_t k,
-                                 const uint32_t *__restrict__ flag, const uint32_t *__restrict__ comp,
-                                 const uint64_t *__restrict__ cidx, const uint64_t *__restrict__ cbeg,
+                                 const uint32_t *__restrict__ comp, const uint64_t *__restrict__ cidx,
+                                 const uint64_t *__restrict__ cbeg,
                                  unsigned long long *__restrict__ ccur, const uint32_t *__restrict__ local,
                                  uint32_t nv, uint32_t *__restrict__ rec, uint32_t *__restrict__ ldeg) {
   __shared__ uint32_t s_lo, s_hi;
@@ -413,7 +405,7 @@ __global__ void k_bucket_cliques(const uint32_t *__restrict__ members, uint64_t 
   }
   for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x; b < m; b += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t c = b + threadIdx.x;
-    const bool in = c < m && flag[c];
+    const bool in = c < m;
     const uint32_t *r = members + (in ? c : 0) * k;
     const uint32_t ci = in ? (uint32_t)cidx[comp[r[0]]] : 0u;
     if (threadIdx.x == 0) {
@@ -549,11 +541,10 @@ __global__ void k_gather_roots(const uint32_t *__restrict__ is_root, const uint6
 
 namespace cds {
 
-void densest_core_and_components(cds_ctx *c, cudaStream_t s, const Dag &dag, const Cliques &cl,
-                                 const PeelOut &pe, const Instances &inst, uint32_t k,
-                                 CoreOut &out, bool need_networks, StageClock *clk) {
-  const uint32_t n = dag.n;
-  const uint64_t m = cl.count;
+void densest_core_and_components(cds_ctx *c, cudaStream_t s, const Dag &gdag, const PeelOut &pe,
+                                 const Instances &inst, uint32_t k, const Tuning &t, CoreOut &out,
+                                 bool need_networks, StageClock *clk, const CountHook *on_count) {
+  const uint32_t n = gdag.n;
   const uint32_t ninst = inst.count;
   const uint32_t *of_vertex = ninst > 1 ? inst.of_vertex.p : nullptr;
   const int G = c->sm_count * 8;
@@ -567,15 +558,34 @@ void densest_core_and_components(cds_ctx *c, cudaStream_t s, const Dag &dag, con
   DBuf<unsigned long long> stats(c, s, 4 * (size_t)ninst);  // core size, core cliques, arcs, comps
   stats.zero();
   DBuf<uint8_t> in_core(c, s, n + 1);
-  uint32_t *flag = pe.cmin.p;  // becomes the core-clique flags
   DBuf<uint32_t> err(c, s, 1);
   err.zero();
+  Dag dag;  // of the core
+  dag.n = n;
+  dag.max_out = gdag.max_out;
+  dag.heavy = gdag.heavy;
+  dag.degree = gdag.degree;
+  dag.outdeg = DBuf<uint32_t>(c, s, n + 1);
+  dag.off = DBuf<uint64_t>(c, s, n + 1);
+  dag.adj = DBuf<uint32_t>(c, s, gdag.adj.n);
   {
-    ProfScope ps(c, s, "core_flags");
-    if (n) k_core_flags<<<G, 256, 0, s>>>(pe.core.p, n, of_vertex, kp.p, in_core.p, stats.p);
-    if (m) k_clique_flags<<<G, 256, 0, s>>>(cl.members.p, m, k, kp.p, flag, of_vertex, stats.p + ninst);
+    ProfScope ps(c, s, "core_dag");
+    if (n) {
+      k_core_flags<<<G, 256, 0, s>>>(pe.core.p, n, of_vertex, kp.p, in_core.p, stats.p);
+      k_core_outdeg<<<G, 256, 0, s>>>(gdag.off.p, gdag.adj.p, gdag.outdeg.p, in_core.p, n, dag.outdeg.p);
+    }
+    scan_u32_pad4(dag.outdeg.p, dag.off.p, n, c, s);
+    if (n)
+      k_core_dag<<<G, 256, 0, s>>>(gdag.off.p, gdag.adj.p, gdag.outdeg.p, in_core.p, n, dag.off.p, dag.adj.p);
+    count_launch(3);
+    CDS_CUDA(cudaGetLastError());
   }
-  count_launch(2);
+  // its cliques, the only ones that are ever written
+  Cliques cl;
+  list_cliques(c, s, dag, k, LIST_WRITE, t, cl, on_count);
+  const uint64_t m = cl.count;
+  k_inst_cliques<<<std::max(1u, (ninst + 255) / 256), 256, 0, s>>>(cl.base.p, inst.vbeg.p, ninst, stats.p + ninst);
+  count_launch();
   CDS_CUDA(cudaGetLastError());
   if (clk) out.mk_core = clk->mark();
 
@@ -604,12 +614,12 @@ void densest_core_and_components(cds_ctx *c, cudaStream_t s, const Dag &dag, con
       }
       bits.zero();
       k_core_vertex<<<G, 256, 0, s>>>(in_core.p, lid.p, n, core_vertex.p);
-      k_mark_pairs<<<G, 256, 0, s>>>(cl.members.p, m, k, flag, lid.p, words, bits.p);
+      k_mark_pairs<<<G, 256, 0, s>>>(cl.members.p, m, k, lid.p, words, bits.p);
       k_pairs_to_arcs<<<G, 256, 0, s>>>(dag.off.p, dag.adj.p, dag.outdeg.p, in_core.p, lid.p, n, words, bits.p,
                                         keep.p);
       count_launch(4);
     } else if (m) {
-      k_mark_arcs<<<G, 256, 0, s>>>(cl.members.p, m, k, flag, dag.off.p, dag.adj.p, dag.outdeg.p, keep.p,
+      k_mark_arcs<<<G, 256, 0, s>>>(cl.members.p, m, k, dag.off.p, dag.adj.p, dag.outdeg.p, keep.p,
                                     err.p);
       count_launch();
     }
@@ -639,10 +649,7 @@ void densest_core_and_components(cds_ctx *c, cudaStream_t s, const Dag &dag, con
       k_union<<<G, 256, 0, s>>>(dag.off.p, dag.adj.p, dag.outdeg.p, keep.p, n, parent.p, err.p);
       k_roots<<<G, 256, 0, s>>>(parent.p, in_core.p, n, comp.p);
     }
-    if (m)
-      k_comp_cliques<<<G, 256, 0, s>>>(reinterpret_cast<const unsigned long long *>(cl.base.p), n, m,
-                                       (uint32_t)std::min<uint64_t>(8192, std::max<uint64_t>(64, m / (4ull * G * 8))),
-                                       flag, comp.p, ccount.p);
+    if (n) k_comp_cliques<<<G, 256, 0, s>>>(cl.base.p, n, comp.p, ccount.p);
     if (n) k_root_flags<<<G, 256, 0, s>>>(comp.p, ccount.p, n, of_vertex, is_root.p, stats.p + 3 * ninst);
   }
   count_launch(4);
@@ -724,7 +731,7 @@ void densest_core_and_components(cds_ctx *c, cudaStream_t s, const Dag &dag, con
     ProfScope ps_b(c, s, "components_bucket");
     k_local_ids<<<G, 256, 0, s>>>(comp.p, cidx.p, ccount.p, n, vbeg.p, vcur.p, local.p, out.vmap.p,
                                  out.vcnet.p);
-    if (m) k_bucket_cliques<<<G, 256, 0, s>>>(cl.members.p, m, k, flag, comp.p, cidx.p, cbeg.p,
+    if (m) k_bucket_cliques<<<G, 256, 0, s>>>(cl.members.p, m, k, comp.p, cidx.p, cbeg.p,
                                              ccur.p, local.p, nv, out.rec.p, ldeg.p);
   }
   count_launch(2);

@@ -62,6 +62,7 @@ void build_dag(cds_ctx *c, cudaStream_t s, const uint64_t *off, const uint32_t *
                uint32_t n, uint32_t k, Dag &dag) {
   dag.n = n;
   dag.deg.alloc(n + 1);
+  dag.degree = dag.deg.p;
   dag.outdeg.alloc(n + 1);
   dag.off.alloc(n + 1);
   DBuf<uint32_t> maxout(c, s, 1);

@@ -156,24 +156,54 @@ __device__ __forceinline__ void light_arcs(const uint32_t *A, const uint32_t *hi
 // Heavy part of the local graph: one word at a time of each row, word(i, w, m)
 // with bit l of m set when A[i] and A[32 w + l] are adjacent heavy vertices.  A
 // lane reads the bit of its column from row i of the heavy bitmap and a ballot
-// makes the word, so 32 pairs cost one load and no search or atomic.  Word-
-// uniform calls, every word of every row once (zero where nothing is heavy).
-// Returns whether the calling warp met a light vertex.
+// makes the word, so 32 pairs cost one load and no search or atomic.  Rows of
+// fewer than four words are taken as one sequence with HEAVY_U loads in flight
+// (each comes from L2); longer ones a row at a time, which saves instructions.
+// Word-uniform calls, every word of every row once, a row's words in order (zero
+// where nothing is heavy).  Returns whether the calling warp met a light vertex.
+constexpr int HEAVY_U = 8;
 template <bool TB, class Word>
 __device__ __forceinline__ bool heavy_words(const HeavyBits &hb, const uint32_t *hid, uint32_t d, Word word) {
-  const uint32_t lane = lane_id(), W = (d + 31) >> 5;
+  const uint32_t lane = lane_id(), W = (d + 31) >> 5, step = Team<TB>::warps();
   bool light = false;
-  for (uint32_t i = Team<TB>::warp(); i < d; i += Team<TB>::warps()) {
-    const uint32_t hi = hid[i];
-    light |= hi == LIGHT;
-    const uint32_t *row = hb.bits + (size_t)hi * hb.words;
+  uint32_t i = Team<TB>::warp(), w = 0;
+  if (W >= 4) {
+    for (; i < d; i += step) {
+      const uint32_t hi = hid[i];
+      light |= hi == LIGHT;
+      const uint32_t *row = hb.bits + (size_t)hi * hb.words;
 #pragma unroll 4
-    for (uint32_t w = 0; w < W; w++) {
-      const uint32_t j = w * 32 + lane;
-      const uint32_t hj = j < d && hi != LIGHT ? hid[j] : LIGHT;
-      const bool on = hj != LIGHT && (row[hj >> 5] >> (hj & 31)) & 1u;
-      word(i, w, __ballot_sync(CDS_FULL, on));
+      for (w = 0; w < W; w++) {
+        const uint32_t j = w * 32 + lane;
+        const uint32_t hj = j < d && hi != LIGHT ? hid[j] : LIGHT;
+        const bool on = hj != LIGHT && (row[hj >> 5] >> (hj & 31)) & 1u;
+        word(i, w, __ballot_sync(CDS_FULL, on));
+      }
     }
+    return light;
+  }
+  while (i < d) {
+    uint32_t x[HEAVY_U], row[HEAVY_U], at[HEAVY_U];
+    bool on[HEAVY_U];
+#pragma unroll
+    for (int u = 0; u < HEAVY_U; u++) {
+      row[u] = i;
+      at[u] = w;
+      x[u] = 0;
+      on[u] = i < d;
+      if (on[u]) {
+        const uint32_t hi = hid[i], j = w * 32 + lane, hj = j < d ? hid[j] : LIGHT;
+        light |= hi == LIGHT;
+        if (hi != LIGHT && hj != LIGHT) x[u] = hb.bits[(size_t)hi * hb.words + (hj >> 5)] >> (hj & 31);
+        if (++w == W) {
+          w = 0;
+          i += step;
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < HEAVY_U; u++)
+      if (on[u]) word(row[u], at[u], __ballot_sync(CDS_FULL, x[u] & 1u));
   }
   return light;
 }

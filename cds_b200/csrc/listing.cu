@@ -97,7 +97,7 @@ void launch_pass(cds_ctx *c, cudaStream_t s, const cds::Tuning &t, ListParams p,
 }
 
 template <int K>
-void run_listing(cds_ctx *c, cudaStream_t s, const cds::Dag &dag, bool materialize,
+void run_listing(cds_ctx *c, cudaStream_t s, const cds::Dag &dag, cds::ListMode mode,
                  const cds::Tuning &t, cds::Cliques &out, uint32_t *err, uint32_t k,
                  const cds::CountHook *on_count) {
   using namespace cds;
@@ -122,7 +122,7 @@ void run_listing(cds_ctx *c, cudaStream_t s, const cds::Dag &dag, bool materiali
   p.doff = dag.off.p;
   p.dadj = dag.adj.p;
   p.outdeg = dag.outdeg.p;
-  p.deg = dag.deg.p;
+  p.deg = dag.degree;
   p.heavy = dag.heavy;
   p.cdeg = nullptr;
   p.cdeg64 = out.cdeg64.p;
@@ -170,15 +170,25 @@ void run_listing(cds_ctx *c, cudaStream_t s, const cds::Dag &dag, bool materiali
   pass(false);
   out.base.alloc(n + 1);
   scan_u64(reinterpret_cast<const uint64_t *>(root_cnt.p), out.base.p, n, c, s);
-  out.count = d2h(out.base.p + n, s);
-  if (on_count) (*on_count)(out.count);
-  if (!materialize) return;
-  // later stages keep clique degrees (and core numbers) as u32
-  if (n) {
+  // the peel keeps clique degrees (and core numbers) as u32
+  if (mode == LIST_NARROW && n) {
     k_narrow<<<c->sm_count * 4, 256, 0, s>>>(out.cdeg64.p, out.cdeg.p, n, err);
     count_launch();
     CDS_CUDA(cudaGetLastError());
   }
+  uint32_t e = 0;
+  {
+    HostReads r(s);
+    r.add(&out.count, out.base.p + n);
+    r.add(&e, err);
+    r.wait();
+  }
+  if (e & DEV_ERR_OVERFLOW)
+    fail(CDS_ERR_OVERFLOW, "a root's out-degree exceeds the k >= 5 listing's masks, or a clique degree "
+                           "reaches 2^32 (the later stages keep clique degrees as u32)");
+  if (e) fail(CDS_ERR_CUDA, "listing kernel reported an internal error");
+  if (on_count) (*on_count)(out.count);
+  if (mode != LIST_WRITE) return;
   out.members.alloc((size_t)out.count * k + 4);
   p.base = reinterpret_cast<const unsigned long long *>(out.base.p);
   p.out = out.members.p;
@@ -189,7 +199,7 @@ void run_listing(cds_ctx *c, cudaStream_t s, const cds::Dag &dag, bool materiali
 
 namespace cds {
 
-void list_cliques(cds_ctx *c, cudaStream_t s, const Dag &dag, uint32_t k, bool materialize,
+void list_cliques(cds_ctx *c, cudaStream_t s, const Dag &dag, uint32_t k, ListMode mode,
                   const Tuning &t, Cliques &out, const CountHook *on_count) {
   if (k < 2 || k > CDS_MAX_K) fail(CDS_ERR_INPUT, "k must be in [2, 16]");
   const uint32_t n = dag.n;
@@ -203,7 +213,7 @@ void list_cliques(cds_ctx *c, cudaStream_t s, const Dag &dag, uint32_t k, bool m
   out.members.c = c;
   out.members.s = s;
   out.cdeg64.alloc(n + 1);
-  if (materialize) out.cdeg.alloc(n + 1);
+  if (mode == LIST_NARROW) out.cdeg.alloc(n + 1);
   DBuf<uint32_t> err(c, s, 1);
   err.zero();
   if (k == 2) {
@@ -213,11 +223,11 @@ void list_cliques(cds_ctx *c, cudaStream_t s, const Dag &dag, uint32_t k, bool m
     out.count = d2h(out.base.p + n, s);
     if (on_count) (*on_count)(out.count);
     if (n) {
-      k_widen<<<c->sm_count * 4, 256, 0, s>>>(dag.deg.p, out.cdeg64.p, n);
-      if (materialize) k_copy_u32<<<c->sm_count * 4, 256, 0, s>>>(dag.deg.p, out.cdeg.p, n);
-      count_launch(materialize ? 2 : 1);
+      if (mode == LIST_COUNT) k_widen<<<c->sm_count * 4, 256, 0, s>>>(dag.deg.p, out.cdeg64.p, n);
+      if (mode == LIST_NARROW) k_copy_u32<<<c->sm_count * 4, 256, 0, s>>>(dag.deg.p, out.cdeg.p, n);
+      if (mode != LIST_WRITE) count_launch();
     }
-    if (materialize) {
+    if (mode == LIST_WRITE) {
       out.members.alloc((size_t)out.count * 2 + 4);
       if (n) {
         ProfScope ps(c, s, "list_write_edges");
@@ -229,15 +239,10 @@ void list_cliques(cds_ctx *c, cudaStream_t s, const Dag &dag, uint32_t k, bool m
     CDS_CUDA(cudaGetLastError());
     return;
   }
-  if (k == 3) run_listing<3>(c, s, dag, materialize, t, out, err.p, k, on_count);
-  else if (k == 4) run_listing<4>(c, s, dag, materialize, t, out, err.p, k, on_count);
-  else if (k == 5) run_listing<5>(c, s, dag, materialize, t, out, err.p, k, on_count);
-  else run_listing<0>(c, s, dag, materialize, t, out, err.p, k, on_count);
-  const uint32_t e = d2h(err.p, s);
-  if (e & DEV_ERR_OVERFLOW)
-    fail(CDS_ERR_OVERFLOW, "a root's out-degree exceeds the k >= 5 listing's masks, or a clique degree "
-                           "reaches 2^32 (the later stages keep clique degrees as u32)");
-  if (e) fail(CDS_ERR_CUDA, "listing kernel reported an internal error");
+  if (k == 3) run_listing<3>(c, s, dag, mode, t, out, err.p, k, on_count);
+  else if (k == 4) run_listing<4>(c, s, dag, mode, t, out, err.p, k, on_count);
+  else if (k == 5) run_listing<5>(c, s, dag, mode, t, out, err.p, k, on_count);
+  else run_listing<0>(c, s, dag, mode, t, out, err.p, k, on_count);
 }
 
 }  // namespace cds

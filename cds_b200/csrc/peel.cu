@@ -16,659 +16,675 @@
 // lie in the h-core), and every iterate stays >= core (H is monotone and
 // core is its fixpoint).  This is the local characterisation of nucleus
 // decompositions (Sariyuce, Seshadhri, Pinar, VLDB 2018) for 1-vertex
-// nuclei of k-cliques.  A sweep over all incidences is bulk-parallel work:
-// the number of sweeps (about 30 on R-MAT graphs) replaces the number of
-// peel levels (hundreds to thousands), each of which needs a grid-wide
-// synchronisation.
+// nuclei of k-cliques.
 //
-// A sweep splits every vertex's incidence list into items of at most
-// `chunk` incidences, one warp per item.  A vertex with one item gets an
-// exact histogram of its x_C and its exact H, stored at once (later items of
-// the sweep read it).  The items of a larger vertex (a hub) count x_C >=
-// tau(v), the exact values tau-1 .. tau-32, and the rest in log-scale bins of
-// sixteen per octave of the distance below that window, summed in global
-// memory; the warp adding the last item computes the new value -- exact in
-// the window, else the least upper bound the bins allow (still >= core, so
-// the fixpoint is unchanged, and within about a seventeenth of the gap, which the
-// next sweep refines).  A sweep in which no value changes saw every value in
-// its final state, so it ends the loop.
+// H without the cliques.  Order the vertices by tau (ties in any order) and give
+// every clique to its first member, its root u.  Then x_C = tau(u) for every other member v of
+// it, and x_C >= tau(u) for u itself, so
+//     H(v) = the largest h <= tau(v) with R(v) + sum{ c(u,v) : tau(u) >= h } >= h
+// where R(v) counts the cliques rooted at v and c(u,v) those rooted at u that
+// hold v.  c(u,.) is what the counting pass computes from u's later neighbours
+// N+(u) by bitmaps: 32 cliques an instruction, nothing stored per clique.  It
+// depends on the set N+(u) alone, so a root is counted again only when a
+// neighbour crossed it in the order.  With weights that are older than the
+// values, tau(u) of the old root is at least the true x_C (it is one of the
+// members the minimum is over), so an update with them is still an upper bound
+// >= core: values may be lowered several times between two counts, and only a
+// pass over current weights that lowers nothing ends the loop.
+//
+// Sweep (one cooperative launch, a grid barrier after each phase):
+//   order   every vertex a change can have reached compares itself with its neighbours
+//           before and after; where its later set changed, small sets are
+//           counted at once by the warp, larger ones queued
+//   count   blocks take the queued roots
+//   lower   (twice) weighted h-index of every vertex a change can have reached
+// Ties keep the order they had: a vertex that arrives at a value goes behind those
+// that were there (its key's low half holds the sweep it arrived in and how far
+// it fell).  With ids to break ties a plateau of equal values turns around as it
+// forms: R-MAT 200k k = 3 took 56 sweeps and 15 ms with ids, 46 and
+// 10.4 ms this way.
+// A change of a value from `old` to `new` reaches only vertices with new <= tau
+// <= old: above old, both values are below tau; below new, the order around the
+// vertex and the minimum with its own value stay as they were.
+//
+// Measured against sweeps over stored cliques (8-byte member tuples of every
+// incidence, 17 to 21 passes): R-MAT scale 18, edge factor 16, k = 4 (2.29 G
+// cliques, 9.1 G incidences) 605 ms for tuples and sweeps against 11 ms; R-MAT scale
+// 16, edge factor 12, k = 4 37 against 2.1; R-MAT scale 14, edge factor 8: k = 4
+// 2.2 against 1.0, k = 2 0.54 against 0.37.  Small graphs are bound by the chains
+// of L2 reads in a phase and its barrier (about 50 us a sweep whatever the
+// grid): k = 3 at scale 14 0.80 against 1.2.
 //
 // Densities: the alive set at each level of a peel is a core {v : core(v) >=
-// L}; |V_L| and |Psi_L| (cliques whose smallest member core is >= L) come
-// from two histograms and suffix sums, and the best level keeps the first
-// (smallest) L with the largest |Psi_L| / |V_L|, as the level-by-level peel
-// records it.  Instances of a batch (disjoint vertex ranges) are
-// independent and share every sweep.
+// L}; |V_L| and |Psi_L| come from two histograms by core number, of the vertices
+// and of the cliques rooted at them (a root is a member of smallest core), and
+// suffix sums; the best level keeps the first (smallest) L with the largest
+// |Psi_L| / |V_L|, as the level-by-level peel records it.  Instances of a batch
+// (disjoint vertex ranges) are independent and share every sweep.
 #include "device_util.cuh"
 #include "stages.h"
+
+#include "list_kernels.cuh"
 
 #include <algorithm>
 #include <cstdio>
 
 namespace {
 
-constexpr uint32_t UNSET = 0xFFFFFFFFu;
-constexpr int WIN = 32;                       // exact values t-1 .. t-32 of a hub
-constexpr int SUB_BITS = 4;
-constexpr int SUB = 1 << SUB_BITS;            // bins per octave below them
-constexpr int NLOG = 32 * SUB;                // log-scale bins below the window
-constexpr int ACC_WORDS = 1 + WIN + NLOG;     // [0] count >= t, window, log bins
-constexpr int MAX_CHUNK = 1024;               // incidences per item, at most
-constexpr uint32_t MAX_READ_SWEEPS = 64;      // sweeps whose reads profiling records
-constexpr int PACK_BITS = 21;                 // member id field of the packed layout
-constexpr unsigned long long PACK_MASK = (1ull << PACK_BITS) - 1;
-constexpr uint32_t PACK_MAX_N = 1u << PACK_BITS;  // vertices the packed layout can name
+constexpr int THREADS = 512, WARPS = THREADS / 32;
+constexpr uint32_t ROW_BLOCK = 512;   // a row of more entries is a block's work, else a warp's
+constexpr uint32_t WARP_SET = 32;     // later sets up to this size are counted by a warp at once
+constexpr uint32_t BINS_WARP = 256, BINS_BLOCK = 1024;
+constexpr int LOWER = 2;              // lowering passes between two counts
+constexpr uint32_t PAIR_ITEM = 64;    // later neighbours per item of a set too large for one team
+constexpr int SLOTS = 4;              // control words of a phase, by its number modulo SLOTS
 
-struct HParams {
+// control words: per lowering pass what changed, per sweep the queues
+enum { P_CHANGED = 0, P_LOW, P_HIGH, P_WORDS = 32 };       // P_LOW holds ~(smallest new value)
+enum { Q_ROOTS = 0, Q_PAIRS, Q_NEXT_ROOT, Q_NEXT_PAIR, Q_WORDS = 32 };
+
+struct CoreParams {
   uint32_t n, k;
-  const uint32_t *members;    // [m*k]
-  const uint64_t *inc_off;    // [n+1]
-  const uint32_t *inc;        // [k*m] clique ids, by vertex (clique layout)
-  const unsigned long long *inc64;  // the same as u64 ids (2^32 or more cliques)
-  const uint32_t *tup;        // [(k-1) * k*m] the other members, slot-major (member layout)
-  const uint16_t *tup16;      // the same as 16-bit ids (graphs of at most 65,536 vertices)
-  const unsigned long long *tup64;  // [k*m] the other members packed as 21-bit fields (k = 3, 4)
-  uint64_t tup_stride;        // k*m
-  uint32_t *tau;              // [n] upper bound of the core number
-  const uint32_t *item_v;     // [nitems] vertex of each item
-  const uint32_t *item_c;     // [nitems] its index among the vertex's items
-  const uint32_t *vitems;     // [n] items of each vertex
-  const uint64_t *nitems;     // items in all: item_off[n], on the device
-  uint32_t chunk;             // a vertex with at most this many incidences is one item
-  uint32_t warp_words;        // shared words per warp: max(chunk + 1, ACC_WORDS), rounded to 4
-  uint32_t hub_chunk;         // incidences per item of a larger vertex (a hub)
-  const uint32_t *big_slot;   // [n] slot of a vertex with several items
-  const uint32_t *big_v;      // [nbig]
-  uint32_t nbig;
-  uint32_t *acc;              // [nbig * ACC_WORDS] counts of the current sweep
-  uint32_t *big_done;         // [nbig] items counted in the current sweep
-  uint32_t *ctl;              // [3 * 32] change flag, ~(smallest new value), by sweep mod 3
-  const uint32_t *of_vertex;  // [n] instance of each vertex (null: one instance)
-  uint32_t ninst;
-  uint32_t *ichg;             // [3 * ninst] per-instance change flags, by sweep mod 3
+  const uint64_t *off;      // [n+1] undirected rows
+  const uint32_t *adj;      // [nnz]
+  const uint32_t *rel;      // [nnz] position of the row's vertex in its neighbour's row
+  ListParams dag;           // the degree-ordered DAG and heavy bitmap (counting)
+  uint32_t *tau;            // [n] values now
+  unsigned long long *key;  // [n] place in the order when it was last taken: value, then tie-break
+  uint32_t *R;              // [n] cliques rooted at each vertex
+  uint32_t *cin;            // [nnz] c(u, v) at the position of u in v's row
+  uint32_t *later;          // [nnz] positions of a queued root's later neighbours, from its row start
+  uint32_t *dplus;          // [n] how many
+  const uint32_t *wide;     // [*nwide] vertices with more than ROW_BLOCK neighbours
+  const uint32_t *nwide;
+  uint32_t *queue;          // [n] roots to count
+  uint2 *pairs;             // [..] (root, first of PAIR_ITEM later neighbours) of large sets
+  uint32_t dmax;            // largest set a block counts by itself
+  uint32_t *rows_global;    // rows outside shared memory (dmax > BLOCK_DMAX)
+  uint64_t rows_slab;
+  uint32_t *pass_ctl;       // [SLOTS * P_WORDS]
+  uint32_t *sweep_ctl;      // [SLOTS * Q_WORDS]
   GridBarrier *bar;
   uint32_t *err;
   unsigned long long spin_limit;
   uint32_t max_sweeps;
   unsigned long long time_budget_ns;
-  uint32_t *sweeps;           // sweeps run
-  unsigned long long *reads;  // [MAX_READ_SWEEPS] incidences read per sweep (profiling; null: off)
-  uint32_t static_pct;        // this percent of the items goes round-robin to the
-                              // warps; the rest are taken from a per-sweep counter
+  uint32_t *sweeps;         // sweeps run
+  unsigned long long *phase_ns;  // [3] block 0's time per phase, barrier included (profiling; null: off)
 };
 
-template <bool CG>
-__device__ __forceinline__ uint32_t ld_tau(const uint32_t *a) {
-  return CG ? __ldcg(a) : *a;
+// the order: keys, then ids
+__device__ __forceinline__ bool after(unsigned long long kw, uint32_t w, unsigned long long ku, uint32_t u) {
+  return kw > ku || (kw == ku && w > u);
+}
+// The key of a vertex of value t in this sweep's order, from its last one: the
+// same while the value stands, else t, the sweep (up to 65,535) and on a log
+// scale, 2,048 steps an octave, how far the value fell.
+__device__ __forceinline__ unsigned long long key_now(unsigned long long key, uint32_t t, uint32_t sweep) {
+  const uint32_t old = (uint32_t)(key >> 32);
+  if (old == t) return key;
+  uint32_t low = 0;
+  if (sweep) {
+    const uint32_t f = old - t, e = 31 - __clz(f | 1u);
+    low = min(sweep, 65535u) << 16 | (e >= 11 ? e << 11 | ((f >> (e - 11)) & 2047u) : e << 11 | ((f << (11 - e)) & 2047u));
+  }
+  return (unsigned long long)t << 32 | low;
+}
+__device__ __forceinline__ unsigned long long key_of(const CoreParams &p, uint32_t v, uint32_t sweep) {
+  return key_now(__ldcg(p.key + v), __ldcg(p.tau + v), sweep);
 }
 
-// x_C for incidence i of vertex v: the smallest tau over the other members of
-// its clique (CG: read at L2, never from a possibly older L1 copy).  TUP 1
-// (2): the other members are stored per incidence as u32 (u16) ids, k-1
-// coalesced streams; TUP 3: the k-1 <= 3 other members packed into one u64
-// per incidence (21-bit ids); TUP 0 (4): the u32 (u64) clique id leads to
-// its member record.
-template <int K, int TUP, bool CG>
-__device__ __forceinline__ uint32_t other_min(const HParams &p, uint64_t i, uint32_t v) {
-  uint32_t x = UNSET;
-  if (TUP == 3) {
-    const unsigned long long q = __ldcs(p.tup64 + i);
-#pragma unroll
-    for (int j = 0; j < K - 1; j++) x = min(x, ld_tau<CG>(p.tau + (uint32_t)((q >> (PACK_BITS * j)) & PACK_MASK)));
-    return x;
-  }
-  if (TUP == 1 || TUP == 2) {
-#pragma unroll
-    for (int j = 0; j < K - 1; j++) {
-      const uint32_t w = TUP == 2 ? (uint32_t)__ldcs(p.tup16 + j * p.tup_stride + i)
-                                  : __ldcs(p.tup + j * p.tup_stride + i);
-      x = min(x, ld_tau<CG>(p.tau + w));
-    }
-    return x;
-  }
-  const uint64_t c = TUP == 4 ? (uint64_t)__ldg(p.inc64 + i) : (uint64_t)__ldg(p.inc + i);
-  if (K == 4) {
-    const uint4 q = __ldg(reinterpret_cast<const uint4 *>(p.members) + c);
-    const uint32_t a = q.x != v ? ld_tau<CG>(p.tau + q.x) : UNSET;
-    const uint32_t b = q.y != v ? ld_tau<CG>(p.tau + q.y) : UNSET;
-    const uint32_t d = q.z != v ? ld_tau<CG>(p.tau + q.z) : UNSET;
-    const uint32_t e = q.w != v ? ld_tau<CG>(p.tau + q.w) : UNSET;
-    x = min(min(a, b), min(d, e));
-  } else if (K == 2) {
-    const uint2 q = __ldg(reinterpret_cast<const uint2 *>(p.members) + c);
-    x = ld_tau<CG>(p.tau + (q.x != v ? q.x : q.y));
-  } else {
-    const uint32_t k = K ? K : p.k;
-    const uint32_t *mc = p.members + (uint64_t)c * k;
-#pragma unroll 4
-    for (uint32_t j = 0; j < k; j++) {
-      const uint32_t w = __ldg(mc + j);
-      if (w != v) x = min(x, ld_tau<CG>(p.tau + w));
-    }
-  }
-  return x;
+struct Range {  // of the changes since some point: [low new value, high old value]
+  uint32_t lo, hi;
+  __device__ __forceinline__ bool reaches(uint32_t t) const { return t >= lo && t <= hi; }
+};
+__device__ __forceinline__ Range pass_range(const uint32_t *pass_ctl, uint32_t pass) {
+  const uint32_t *w = pass_ctl + (pass % SLOTS) * P_WORDS;
+  return {~__ldcg(w + P_LOW), __ldcg(w + P_HIGH)};
 }
 
-// x_C of incidences i, i+32, ..., i+32(U-1) (those below e; UNSET for the
-// rest), with every load of the U incidences issued before any is used
-constexpr int UNROLL = 4;
-template <int K, int TUP, bool CG>
-__device__ __forceinline__ void other_min_x4(const HParams &p, uint64_t i, uint64_t e, uint32_t v,
-                                             uint32_t (&x)[UNROLL]) {
-  if (TUP == 3) {
-    unsigned long long q[UNROLL];
-#pragma unroll
-    for (int u = 0; u < UNROLL; u++) q[u] = i + 32u * u < e ? __ldcs(p.tup64 + i + 32u * u) : 0ull;
-#pragma unroll
-    for (int u = 0; u < UNROLL; u++) {
-      x[u] = UNSET;
-      if (i + 32u * u < e) {
-#pragma unroll
-        for (int j = 0; j < K - 1; j++)
-          x[u] = min(x[u], ld_tau<CG>(p.tau + (uint32_t)((q[u] >> (PACK_BITS * j)) & PACK_MASK)));
-      }
-    }
-  } else if (TUP == 1 || TUP == 2) {
-    constexpr int KM = K > 1 ? K - 1 : 1;
-    uint32_t w[UNROLL][KM];
-#pragma unroll
-    for (int u = 0; u < UNROLL; u++) {
-      const uint64_t iu = i + 32u * u;
-#pragma unroll
-      for (int j = 0; j < KM; j++)
-        w[u][j] = iu >= e ? 0u
-                  : TUP == 2 ? (uint32_t)__ldcs(p.tup16 + j * p.tup_stride + iu)
-                             : __ldcs(p.tup + j * p.tup_stride + iu);
-    }
-#pragma unroll
-    for (int u = 0; u < UNROLL; u++) {
-      x[u] = UNSET;
-      if (i + 32u * u < e) {
-#pragma unroll
-        for (int j = 0; j < KM; j++) x[u] = min(x[u], ld_tau<CG>(p.tau + w[u][j]));
-      }
-    }
-  } else {
-#pragma unroll
-    for (int u = 0; u < UNROLL; u++)
-      x[u] = i + 32u * u < e ? other_min<K, TUP, CG>(p, i + 32u * u, v) : UNSET;
+// Calls visit(v) warp-uniformly for every vertex with want(v), each by one warp.
+// A warp takes vertices a stride apart (ids correlate with degree in many graphs).
+// The first `busy` blocks have other work: they take none where the rest can hold
+// the vertices 32 a warp.
+template <class Want, class Visit>
+__device__ __forceinline__ void each_vertex(uint32_t n, uint32_t busy, Want want, Visit visit) {
+  uint32_t gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t skip = min(busy, gridDim.x / 2) * (blockDim.x >> 5);
+  if (n <= 32 * (nwarps - skip)) {
+    if (gwarp < skip) return;
+    gwarp -= skip;
+    nwarps -= skip;
+  }
+  const uint32_t per = min(32u, (n + nwarps - 1) / nwarps), groups = (n + per - 1) / per;
+  for (uint32_t g = gwarp; g < groups; g += nwarps) {
+    const uint64_t v64 = g + (uint64_t)lane_id() * groups;
+    const bool on = lane_id() < per && v64 < n && want((uint32_t)v64);
+    for (uint32_t m = __ballot_sync(CDS_FULL, on); m; m &= m - 1)
+      visit(__shfl_sync(CDS_FULL, (uint32_t)v64, __ffs(m) - 1));
   }
 }
 
-// An item's packed member tuples [b, e) brought from DRAM into L2 ahead of
-// its loads by one bulk prefetch (16-byte aligned: b rounded down and e up to
-// even; the array holds one spare element past its end).  The sweep's loads
-// then meet L2 latency after the first window instead of DRAM latency for
-// every window, with no register or shared memory held for it.
-__device__ __forceinline__ void prefetch_tuples(const unsigned long long *tup64, uint64_t b, uint64_t e) {
-  const uint64_t b0 = b & ~1ull, e0 = (e + 1) & ~1ull;
-  if (e0 > b0)
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(tup64 + b0), "r"((uint32_t)((e0 - b0) * 8))
-                 : "memory");
-}
-
-// Exact histogram of one single-item vertex: hist[min(x_C, t)] += 1 over
-// its incidences; returns H exactly.  hist has t+1 <= chunk+1 words.
-template <int K, int TUP, bool CG>
-__device__ __forceinline__ uint32_t h_exact(const HParams &p, uint32_t v, uint32_t t, uint64_t b,
-                                            uint64_t e, uint32_t *hist, uint64_t &read) {
-  const uint32_t lane = lane_id();
-  for (uint32_t i = lane; i <= t; i += 32) hist[i] = 0;
-  __syncwarp();
-  // x >= t (most cliques of a vertex at its fixpoint) is counted in a
-  // register: as a shared-memory atomic every lane would hit hist[t]
-  uint32_t ge = 0;
-  for (uint64_t i0 = b; i0 < e; i0 += 32 * UNROLL) {
-    const uint64_t i = i0 + lane;
-    uint32_t x[UNROLL];
-    other_min_x4<K, TUP, CG>(p, i, e, v, x);
+// Order phase for one vertex whose value or neighbours changed: has its later set
+// changed?  (Yes in the first sweep, before which there is no order.)  The counts of neighbours that left
+// the set are cleared.  tr of ts threads take part; the result is per thread.
+__device__ __forceinline__ bool set_changed(const CoreParams &p, uint32_t u, uint32_t sweep, uint32_t tr,
+                                            uint32_t ts) {
+  if (sweep == 0) return true;
+  constexpr int U = 4;
+  const uint64_t b = p.off[u];
+  const uint32_t len = (uint32_t)(p.off[u + 1] - b);
+  const unsigned long long ku = __ldcg(p.key + u), nu = key_now(ku, __ldcg(p.tau + u), sweep);
+  bool any = false;
+  for (uint32_t i0 = tr; i0 < len; i0 += ts * U) {
+    uint32_t w[U], tw[U];
+    unsigned long long kw[U];
 #pragma unroll
-    for (int u = 0; u < UNROLL; u++) {
-      if (i + 32u * u >= e) continue;
-      if (x[u] >= t) ge++;
-      else atomicAdd(&hist[x[u]], 1u);
-    }
-    // t cliques with x >= t already give H >= t, and H <= t: the value
-    // stands, and the rest of the list cannot change that
-    if (__reduce_add_sync(CDS_FULL, ge) >= t) {
-      __syncwarp();
-      read += min(e, i0 + 32 * UNROLL) - b;
-      return t;
-    }
-  }
-  read += e - b;
-  ge = __reduce_add_sync(CDS_FULL, ge);
-  __syncwarp();
-  if (lane == 0) hist[t] += ge;
-  __syncwarp();
-  // largest h with (values >= h) >= h, 32 candidates at a time from the top;
-  // h = 0 always qualifies, so the loop ends by top = 31 at the latest
-  uint32_t acc = 0;
-  for (int top = (int)t;; top -= 32) {
-    const int h = top - (int)lane;
-    const uint32_t c = h >= 0 ? hist[h] : 0u;
-    const uint32_t incl = warp_inclusive_scan(c);
-    const bool ok = h <= 0 || acc + incl >= (uint32_t)h;
-    const uint32_t m = __ballot_sync(CDS_FULL, ok);
-    if (m) {
-      __syncwarp();
-      return (uint32_t)(top - (__ffs(m) - 1));
-    }
-    acc += __shfl_sync(CDS_FULL, incl, 31);
-  }
-}
-
-// Log-scale bin of a distance e = t-WIN-x >= 1 below the window: octave j =
-// floor(log2 e) split into SUB = 16 parts by the four bits after the
-// leading one, so bin (j, s) holds e in [ceil((16+s) 2^j / 16),
-// ceil((17+s) 2^j / 16)) (empty for some s when j < 4).  Bins grow with e.
-__device__ __forceinline__ uint32_t log_bin(uint32_t e) {
-  const uint32_t j = 31 - __clz(e);
-  const uint32_t s = j >= SUB_BITS ? (e >> (j - SUB_BITS)) & (SUB - 1u) : (e << (SUB_BITS - j)) & (SUB - 1u);
-  return j * SUB + s;
-}
-__device__ __forceinline__ unsigned long long log_bin_lo(uint32_t b) {  // smallest e of bin b
-  return (((unsigned long long)(SUB + b % SUB) << (b / SUB)) + SUB - 1) >> SUB_BITS;
-}
-
-// Counts of one item of a hub (t fixed for the sweep): [0] x >= t,
-// [1 + d] x = t-1-d for d < WIN, [1 + WIN + log_bin(t-WIN-x)] x < t-WIN.
-template <int K, int TUP, bool CG>
-__device__ __forceinline__ void hub_counts(const HParams &p, uint32_t v, uint32_t t, uint64_t b,
-                                           uint64_t e, uint32_t *cnt) {
-  const uint32_t lane = lane_id();
-  for (uint32_t i = lane; i < ACC_WORDS; i += 32) cnt[i] = 0;
-  __syncwarp();
-  uint32_t ge = 0;
-  for (uint64_t i = b + lane; i < e; i += 32 * UNROLL) {
-    uint32_t x[UNROLL];
-    other_min_x4<K, TUP, CG>(p, i, e, v, x);
+    for (int x = 0; x < U; x++) w[x] = i0 + ts * x < len ? __ldg(p.adj + b + i0 + ts * x) : u;
 #pragma unroll
-    for (int u = 0; u < UNROLL; u++) {
-      if (i + 32u * u >= e) continue;
-      if (x[u] >= t) {
-        ge++;
-      } else {
-        const uint32_t d = t - 1u - x[u];
-        atomicAdd(&cnt[d < WIN ? 1 + d : 1 + WIN + log_bin(d + 1u - WIN)], 1u);
-      }
+    for (int x = 0; x < U; x++) {
+      tw[x] = __ldcg(p.tau + w[x]);
+      kw[x] = __ldcg(p.key + w[x]);
     }
-  }
-  ge = __reduce_add_sync(CDS_FULL, ge);
-  __syncwarp();
-  if (lane == 0) cnt[0] = ge;
-  __syncwarp();
-}
-
-// New value of a hub from its summed counts: H exactly when it lies in the
-// window, else the least upper bound the log bins give (H < t - WIN there):
-// the top value of the first bin, from the top, whose lowest value h has
-// at least h counts at or above it -- every h above it fails -- so that a
-// drop far below the window shrinks the gap about seventeenfold per sweep.
-__device__ __forceinline__ uint32_t hub_tau(uint32_t t, const uint32_t *acc) {
-  const uint32_t lane = lane_id();
-  const uint32_t ge = __ldcg(acc);
-  if (ge >= t) return t;
-  // window: lane d checks h = t-1-d
-  const uint32_t wi = warp_inclusive_scan(__ldcg(acc + 1 + lane));
-  const long long h = (long long)t - 1 - lane;
-  uint32_t m = __ballot_sync(CDS_FULL, h <= 0 || (long long)ge + wi >= h);
-  if (m) return (uint32_t)(t - 1 - (__ffs(m) - 1));
-  // below the window, 32 bins at a time; bin (j, s) holds x in
-  // [t-WIN-hi+1, t-WIN-lo] for its e range [lo, hi).  The last bins reach
-  // x <= 0, so some bin qualifies.
-  unsigned long long base = (unsigned long long)ge + __shfl_sync(CDS_FULL, wi, 31);
-  for (uint32_t b0 = 0; b0 < NLOG; b0 += 32) {
-    const uint32_t b = b0 + lane;
-    const uint32_t cnt = __ldcg(acc + 1 + WIN + b);
-    const unsigned long long incl = base + warp_inclusive_scan(cnt);
-    const unsigned long long lo = log_bin_lo(b), hi = log_bin_lo(b + 1);  // bin NLOG starts at 2^32
-    const long long xlo = (long long)t - WIN - (long long)hi + 1;
-    const bool ok = hi > lo && (xlo <= 0 || (long long)incl >= xlo);
-    m = __ballot_sync(CDS_FULL, ok);
-    if (m) {
-      const uint32_t bb = b0 + (__ffs(m) - 1);
-      const long long xhi = (long long)t - WIN - (long long)log_bin_lo(bb);
-      return xhi > 0 ? (uint32_t)xhi : 0u;
-    }
-    base = __shfl_sync(CDS_FULL, incl, 31);
-  }
-  return 0;  // not reached: the last bin reaches x <= 0
-}
-
-template <int K, int TUP>
-__global__ void __launch_bounds__(512, 2) k_hindex(HParams p) {
-  extern __shared__ uint32_t s_hist[];
-  __shared__ uint32_t s_any, s_low;  // per-sweep block summary of changes
-  uint32_t *hist = s_hist + (threadIdx.x >> 5) * p.warp_words;
-  if (threadIdx.x == 0) {
-    s_any = 0;
-    s_low = 0;
-  }
-  __syncthreads();
-  const uint32_t lane = lane_id();
-  const uint32_t gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  const bool leader = blockIdx.x == 0 && threadIdx.x == 0;
-  const unsigned long long t0 = globaltimer_ns();
-  const uint32_t nitems = (uint32_t)*p.nitems;
-  uint32_t it = 0;
-  // After a sweep without change, one more reads every value at L2: only a
-  // sweep that saw the current values and changed nothing ends the loop.
-  bool verify = false;
-  for (; it < p.max_sweeps; it++) {
-    uint32_t *changed = p.ctl + (it % 3) * 32;
-    uint32_t *ichg = p.ichg + (it % 3) * p.ninst;
-    // an instance none of whose values changed in the last sweep is at its
-    // fixpoint (its vertices read only its own values): skip it, except in
-    // a verifying sweep
-    const uint32_t *quiet_src = it > 0 && !verify ? p.ichg + ((it + 2) % 3) * p.ninst : nullptr;
-    if (leader) {
-      // slot (it+1)%3 was last read right after the barrier of sweep it-2,
-      // before every block passed the barrier of sweep it-1
-      p.ctl[((it + 1) % 3) * 32] = 0;
-      p.ctl[((it + 1) % 3) * 32 + 2] = 0;
-      p.ctl[((it + 1) % 3) * 32 + 3] = 0;  // the item counter of that sweep
-      if (globaltimer_ns() - t0 > p.time_budget_ns) atomicOr(p.err, DEV_ERR_TIMEOUT);
-    }
-    if (blockIdx.x == 0)  // the per-instance flags of slot (it+1)%3 likewise
-      for (uint32_t i = threadIdx.x; i < p.ninst; i += blockDim.x) p.ichg[((it + 1) % 3) * p.ninst + i] = 0;
-    bool any = false;
-    // Every value that changed in the last sweep ended at or above `low`
-    // (slot word 2 holds ~min, so zero means none).  A vertex with tau < low
-    // reads each clique through min(x_C, tau), which those changes cannot
-    // move (old and new values are both >= tau), and it did not change
-    // itself (its value would be >= low), so its value is still exact: skip
-    // it.  The verifying sweep recounts everything.
-    const uint32_t low = it > 0 && !verify ? ~*(volatile uint32_t *)(p.ctl + ((it + 2) % 3) * 32 + 2) : 0u;
-    uint32_t wmin = UNSET;  // smallest new value this warp stored
-    uint64_t wread = 0;     // incidences this warp read (profiling)
-    // items in the static part go to the warps round-robin; then each warp
-    // takes the next item of the tail from the sweep's counter (early exits
-    // make item costs uneven, and a warp left idle waits at the barrier)
-    const uint32_t stat = (uint32_t)((uint64_t)nitems * p.static_pct / 100u);
-    uint32_t *tail = p.ctl + (it % 3) * 32 + 3;
-    auto next_tail = [&]() -> uint32_t {
-      uint32_t got = 0;
-      if (lane == 0) got = atomicAdd(tail, 1u);
-      return stat + __shfl_sync(CDS_FULL, got, 0);
-    };
-    for (uint32_t r = gwarp < stat ? gwarp : next_tail(); r < nitems;
-         r = r + nwarps < stat ? r + nwarps : next_tail()) {
-      const uint32_t v = p.item_v[r];
-      // the vertex's own value at L2: every item of a hub must count against
-      // the same t, and an L1 line filled before another SM stored the
-      // hub's new value would give an older one
-      const uint32_t t = __ldcg(p.tau + v);
-      if (t < low || t == 0) continue;
-      const uint32_t inst = p.of_vertex ? p.of_vertex[v] : 0u;
-      if (quiet_src && !__ldcg(quiet_src + inst)) continue;
-      const uint32_t nit = p.vitems[v];
-      const uint64_t ib = p.inc_off[v], ie = p.inc_off[v + 1];
-      const bool hub = ie - ib > p.chunk;
-      const uint32_t len = hub ? p.hub_chunk : p.chunk;
-      const uint64_t b = ib + (uint64_t)p.item_c[r] * len;
-      const uint64_t e = min(b + len, ie);
-      uint32_t nt = t;
-      if (!hub) {
-        // the whole list (t <= clique degree <= chunk): exact, and visible
-        // to the rest of the sweep at once
-        if (TUP == 3 && lane == 0) prefetch_tuples(p.tup64, b, e);
-        nt = verify ? h_exact<K, TUP, true>(p, v, t, b, e, hist, wread)
-                    : h_exact<K, TUP, false>(p, v, t, b, e, hist, wread);
-      } else {
-        // a hub: add this item's counts; the warp adding the last item
-        // computes the new value, so it too is visible within the sweep,
-        // and no item of the hub reads its value after that
-        const uint32_t bi = p.big_slot[v];
-        uint32_t *a = p.acc + (uint64_t)bi * ACC_WORDS;
-        // items that finished earlier in this sweep may already have found
-        // t cliques with x >= t: then H = t whatever this item holds, and
-        // it only reports that it is done
-        const uint32_t have = __shfl_sync(CDS_FULL, lane == 0 ? __ldcg(a) : 0u, 0);
-        if (have < t) {
-          if (TUP == 3 && lane == 0) prefetch_tuples(p.tup64, b, e);
-          if (verify) hub_counts<K, TUP, true>(p, v, t, b, e, hist);
-          else hub_counts<K, TUP, false>(p, v, t, b, e, hist);
-          wread += e - b;
-          for (uint32_t i = lane; i < ACC_WORDS; i += 32)
-            if (hist[i]) atomicAdd(a + i, hist[i]);
-        }
-        __syncwarp();
-        uint32_t prev = 0;
-        if (lane == 0) {
-          __threadfence();  // the counts above, then the item's completion
-          prev = atomicAdd(p.big_done + bi, 1u);
-          if (prev + 1 == nit) __threadfence();  // the last item's reader sees every count
-        }
-        prev = __shfl_sync(CDS_FULL, prev, 0);
-        __syncwarp();
-        if (prev + 1 < nit) continue;
-        nt = hub_tau(t, a);
-        __syncwarp();
-        for (uint32_t i = lane; i < ACC_WORDS; i += 32) a[i] = 0;
-        if (lane == 0) p.big_done[bi] = 0;
-      }
-      if (nt < t) {
-        if (lane == 0) {
-          p.tau[v] = nt;
-          ichg[inst] = 1;
-        }
+#pragma unroll
+    for (int x = 0; x < U; x++) {  // (past the end: u against itself, which does not change)
+      const bool now = after(key_now(kw[x], tw[x], sweep), w[x], nu, u), was = after(kw[x], w[x], ku, u);
+      if (now != was) {
         any = true;
-        wmin = min(wmin, nt);
+        if (was) p.cin[p.off[w[x]] + __ldg(p.rel + b + i0 + ts * x)] = 0;
       }
     }
-    if (p.reads && lane == 0 && wread && it < MAX_READ_SWEEPS) atomicAdd(p.reads + it, (unsigned long long)wread);
-    // the block's change flag and smallest new value, then one global update
-    if (any && lane == 0) {
-      s_any = 1;
-      atomicMax(&s_low, ~wmin);
+  }
+  return any;
+}
+
+// The weights of root u over its counted later set (positions pos(r)).
+template <int K, class Pos, class C>
+__device__ __forceinline__ unsigned long long store_weights(const CoreParams &p, uint64_t b, uint32_t d, uint32_t tr,
+                                                            uint32_t ts, Pos pos, const uint32_t *A, const C *cnt) {
+  const uint32_t div = (K ? K : p.k) - 2;
+  unsigned long long mine = 0;
+  for (uint32_t r = tr; r < d; r += ts) {
+    const uint32_t c = (uint32_t)(cnt[r] / div);
+    mine += c;
+    p.cin[p.off[A[r]] + __ldg(p.rel + b + pos(r))] = c;
+  }
+  return mine;
+}
+
+// Queues root u, whose later set (dplus, later) is in global memory.
+__device__ __forceinline__ void queue_root(const CoreParams &p, uint32_t *sctl, uint32_t u, uint32_t d) {
+  if (d <= p.dmax) {
+    p.queue[atomicAdd(sctl + Q_ROOTS, 1u)] = u;
+  } else {
+    const uint32_t items = (d + PAIR_ITEM - 1) / PAIR_ITEM;
+    const uint32_t at = atomicAdd(sctl + Q_PAIRS, items);
+    for (uint32_t i = 0; i < items; i++) p.pairs[at + i] = make_uint2(u, i * PAIR_ITEM);
+  }
+}
+
+// A set too small for a clique, or one whose items will add to its weights.
+__device__ __forceinline__ void clear_weights(const CoreParams &p, uint32_t u, uint64_t b, uint32_t d, uint32_t tr,
+                                              uint32_t ts) {
+  for (uint32_t r = tr; r < d; r += ts) {
+    const uint32_t i = __ldcg(p.later + b + r);
+    p.cin[p.off[p.adj[b + i]] + p.rel[b + i]] = 0;
+  }
+  if (tr == 0) p.R[u] = 0;
+}
+
+// One item of a root whose later set is too large for a team: the cliques whose
+// first member in the degree order is one of PAIR_ITEM later neighbours a, from
+// the local graph of N+(a) inside the set (at most the DAG's largest out-degree).
+template <int K>
+__device__ void count_pairs(const CoreParams &p, uint2 item, uint32_t sweep, uint32_t *sm, uint32_t *rows) {
+  using C = typename CountOf<K>::type;
+  const uint32_t u = item.x, d = __ldcg(p.dplus + u);
+  const unsigned long long nu = key_of(p, u, sweep);
+  const uint64_t b = p.off[u];
+  const uint32_t len = (uint32_t)(p.off[u + 1] - b), d4 = (p.dmax + 3) & ~3u;
+  C *cnt = reinterpret_cast<C *>(sm);
+  uint32_t *A = sm + d4 * (sizeof(C) / 4), *hid = A + d4;
+  for (uint32_t r = item.y; r < min(d, item.y + PAIR_ITEM); r++) {
+    const uint32_t ia = __ldcg(p.later + b + r), a = p.adj[b + ia];
+    const uint32_t *list = p.dag.dadj + p.dag.doff[a];
+    const uint32_t la = p.dag.outdeg[a];
+    uint32_t m = 0;
+    for (uint32_t i0 = 0; i0 < la; i0 += blockDim.x) {
+      const uint32_t w = i0 + threadIdx.x < la ? list[i0 + threadIdx.x] : 0u;
+      bool in = false;
+      if (i0 + threadIdx.x < la && after(key_of(p, w, sweep), w, nu, u)) {
+        uint32_t lo = 0, hi = len;
+        while (lo < hi) {
+          const uint32_t mid = (lo + hi) >> 1;
+          if (p.adj[b + mid] < w) lo = mid + 1;
+          else hi = mid;
+        }
+        in = lo < len && p.adj[b + lo] == w;
+      }
+      uint32_t total;
+      const uint32_t at = m + block_exclusive_scan<uint32_t>(in ? 1u : 0u, &total);
+      if (in) {
+        A[at] = w;
+        hid[at] = p.dag.heavy.id(w);
+      }
+      m += total;
     }
     __syncthreads();
-    if (threadIdx.x == 0 && s_any) {
-      changed[0] = 1;
-      atomicMax(changed + 2, s_low);
-      s_any = 0;  // read again only after the next sweep's items
-      s_low = 0;
+    if (m == 0 || m < (K ? K : p.k) - 2) continue;
+    unsigned long long mine = 0;
+    if (K != 3) {
+      constexpr int KS = K == 4 ? 3 : K == 5 ? 4 : 0;
+      local_count<KS, true, C>(A, hid, m, p.dag.heavy, p.dag.doff, p.dag.dadj, p.dag.outdeg, rows, cnt,
+                               (int)(K ? K : p.k) - 1);
     }
-    if (!grid_sync(p.bar, p.err, p.spin_limit)) break;
-    if (*(volatile uint32_t *)changed == 0) {
-      if (verify) {
-        it++;
+    const uint32_t div = K == 3 ? 1u : (K ? K : p.k) - 3;
+    for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
+      const uint32_t c = K == 3 ? 1u : (uint32_t)(cnt[i] / div), w = A[i];
+      mine += c;
+      if (c) {
+        uint32_t lo = 0, hi = len;  // w's position in u's row
+        while (lo < hi) {
+          const uint32_t mid = (lo + hi) >> 1;
+          if (p.adj[b + mid] < w) lo = mid + 1;
+          else hi = mid;
+        }
+        atomicAdd(p.cin + p.off[w] + p.rel[b + lo], c);
+      }
+    }
+    const unsigned long long total = Team<true>::sum<unsigned long long>(mine) / ((K ? K : p.k) - 2);
+    if (threadIdx.x == 0 && total) {
+      atomicAdd(p.cin + p.off[a] + p.rel[b + ia], (uint32_t)total);
+      atomicAdd(p.R + u, (uint32_t)total);
+    }
+    __syncthreads();
+  }
+}
+
+// Sum over a row of the weights whose value passes `test`, calling use(x, c) on
+// the others; tr of ts threads take part, the sum is per thread.
+template <int K, class Use>
+__device__ __forceinline__ uint32_t row_sum(const CoreParams &p, uint64_t b, uint32_t len, uint32_t t, uint32_t tr,
+                                            uint32_t ts, Use use) {
+  constexpr int U = 4;
+  uint32_t ge = 0;
+  for (uint32_t i0 = tr; i0 < len; i0 += ts * U) {
+    uint32_t w[U], c[U], x[U];
+#pragma unroll
+    for (int j = 0; j < U; j++) {
+      const bool in = i0 + ts * j < len;
+      w[j] = in ? __ldg(p.adj + b + i0 + ts * j) : 0u;
+      c[j] = !in ? 0u : K == 2 ? 1u : __ldcg(p.cin + b + i0 + ts * j);
+    }
+#pragma unroll
+    for (int j = 0; j < U; j++) x[j] = c[j] ? __ldcg(p.tau + w[j]) : 0u;
+#pragma unroll
+    for (int j = 0; j < U; j++) {
+      if (x[j] >= t) ge += c[j];
+      else use(x[j], c[j]);
+    }
+  }
+  return ge;
+}
+
+// Weighted h-index of a vertex whose weight S at values >= t falls short of t.
+// S itself is feasible, so the answer lies in [lo, hi) = [S, t).  The weights in
+// that range go into bins of 2^s values from hi - 1 down; the first bin whose
+// lowest value has enough weight at or above it holds the answer, exactly for
+// s = 0, and is the next range otherwise.  (A bound from one pass would do for
+// the fixpoint, but many values just below t leave S far under the answer, and
+// the sweeps then creep: 2,312 of them instead of 16 on R-MAT scale 18.)
+struct BinSearch {
+  uint32_t hi, lo, S, s;  // S: weight at values >= hi
+  template <uint32_t BINS>
+  __device__ __forceinline__ void shift() {
+    s = 0;
+    while (((hi - lo - 1) >> s) >= BINS) s++;
+  }
+  __device__ __forceinline__ void add(uint32_t *bin, uint32_t x, uint32_t c) const {
+    if (x >= lo && x < hi && c) atomicAdd(&bin[(hi - 1 - x) >> s], c);
+  }
+  // weight Sb at or above bin b's lowest value is enough (or that is below lo)
+  __device__ __forceinline__ bool found(uint32_t b, uint32_t Sb) const {
+    const unsigned long long down = (unsigned long long)(b + 1) << s;
+    return down >= hi - lo || Sb >= (uint32_t)(hi - down);
+  }
+  // on to bin b, with the weight above it; true when hi - 1 is the answer
+  __device__ __forceinline__ bool narrow(uint32_t b, uint32_t above_b) {
+    const unsigned long long down = (unsigned long long)(b + 1) << s;
+    if (down < hi - lo) lo = hi - (uint32_t)down;
+    hi -= b << s;
+    S = above_b;
+    return s == 0;
+  }
+};
+
+template <int K>
+__device__ __forceinline__ uint32_t lower_warp(const CoreParams &p, uint32_t v, uint32_t t, uint32_t *bin) {
+  const uint32_t lane = lane_id();
+  const uint64_t b = p.off[v];
+  const uint32_t len = (uint32_t)(p.off[v + 1] - b);
+  uint32_t ge = row_sum<K>(p, b, len, t, lane, 32, [](uint32_t, uint32_t) {});
+  ge = __reduce_add_sync(CDS_FULL, ge) + (K == 2 ? 0u : __ldcg(p.R + v));
+  if (ge >= t) return t;
+  BinSearch bs{t, ge, ge, 0};
+  for (;;) {
+    bs.shift<BINS_WARP>();
+    for (uint32_t i = lane; i < BINS_WARP; i += 32) bin[i] = 0;
+    __syncwarp();
+    row_sum<K>(p, b, len, 0xFFFFFFFFu, lane, 32, [&](uint32_t x, uint32_t c) { bs.add(bin, x, c); });
+    __syncwarp();
+    uint32_t base = bs.S, m = 0, S = 0, x = 0, b0 = 0;
+    for (;; b0 += 32) {  // the last bin reaches lo, so some bin is found
+      x = bin[b0 + lane];
+      S = base + warp_inclusive_scan(x);
+      m = __ballot_sync(CDS_FULL, bs.found(b0 + lane, S));
+      if (m) break;
+      base = __shfl_sync(CDS_FULL, S, 31);
+    }
+    const uint32_t at = __ffs(m) - 1;
+    const bool exact = bs.narrow(b0 + at, __shfl_sync(CDS_FULL, S - x, at));
+    __syncwarp();  // the bins are reused
+    if (exact) return bs.hi - 1;
+  }
+}
+
+template <int K>
+__device__ __forceinline__ uint32_t lower_block(const CoreParams &p, uint32_t v, uint32_t t, uint32_t *bin) {
+  __shared__ uint32_t s_first, s_above;
+  const uint64_t b = p.off[v];
+  const uint32_t len = (uint32_t)(p.off[v + 1] - b);
+  const uint32_t mine = row_sum<K>(p, b, len, t, threadIdx.x, blockDim.x, [](uint32_t, uint32_t) {});
+  uint32_t ge;
+  block_exclusive_scan<uint32_t>(mine, &ge);
+  ge += K == 2 ? 0u : __ldcg(p.R + v);
+  if (ge >= t) return t;
+  BinSearch bs{t, ge, ge, 0};
+  for (;;) {
+    bs.shift<BINS_BLOCK>();
+    for (uint32_t i = threadIdx.x; i < BINS_BLOCK; i += blockDim.x) bin[i] = 0;
+    if (threadIdx.x == 0) s_first = 0xFFFFFFFFu;
+    __syncthreads();
+    row_sum<K>(p, b, len, 0xFFFFFFFFu, threadIdx.x, blockDim.x, [&](uint32_t x, uint32_t c) { bs.add(bin, x, c); });
+    __syncthreads();
+    static_assert(BINS_BLOCK == 2 * THREADS, "two bins a thread");
+    const uint32_t b0 = 2 * threadIdx.x, x0 = bin[b0], x1 = bin[b0 + 1];
+    uint32_t total;
+    const uint32_t S0 = bs.S + block_exclusive_scan<uint32_t>(x0 + x1, &total) + x0, S1 = S0 + x1;
+    const bool f0 = bs.found(b0, S0), f1 = bs.found(b0 + 1, S1);
+    if (f0 || f1) atomicMin(&s_first, f0 ? b0 : b0 + 1);
+    __syncthreads();
+    if (s_first / 2 == threadIdx.x) s_above = s_first == b0 ? S0 - x0 : S0;
+    __syncthreads();
+    const bool exact = bs.narrow(s_first, s_above);
+    __syncthreads();  // s_first, s_above and the bins are reused
+    if (exact) return bs.hi - 1;
+  }
+}
+
+template <int K>
+__global__ void __launch_bounds__(THREADS, 2) k_core(CoreParams p) {
+  using C = typename CountOf<K>::type;
+  extern __shared__ __align__(16) uint32_t sm[];
+  __shared__ uint32_t s_changed, s_low, s_high, s_item;
+  const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+  const bool leader = blockIdx.x == 0 && threadIdx.x == 0;
+  const unsigned long long t0 = globaltimer_ns();
+  const uint32_t nwide = *p.nwide, kmin = (K ? K : p.k) - 1;
+  if (threadIdx.x == 0) {
+    s_changed = 0;
+    s_low = 0;
+    s_high = 0;
+  }
+  __syncthreads();
+  uint32_t pass = 0, sweep = 0;
+  bool done = false;
+  unsigned long long tprev = t0;
+  auto phase_end = [&](int i) {
+    if (p.phase_ns && leader) {
+      const unsigned long long now = globaltimer_ns();
+      p.phase_ns[i] += now - tprev;
+      tprev = now;
+    }
+  };
+  for (; sweep < p.max_sweeps && !done; sweep++) {
+    if (leader && globaltimer_ns() - t0 > p.time_budget_ns) atomicOr(p.err, DEV_ERR_TIMEOUT);
+    const bool first = sweep == 0;
+    // what changed since the vertices were last ordered (all of it, at first)
+    Range since{0u, 0xFFFFFFFFu};
+    if (!first) {
+      since = pass_range(p.pass_ctl, pass - 1);
+      if (K != 2) {  // every sweep but the last makes LOWER = 2 passes
+        const Range r2 = pass_range(p.pass_ctl, pass - 2);
+        since.lo = min(since.lo, r2.lo);
+        since.hi = max(since.hi, r2.hi);
+      }
+    }
+    if constexpr (K != 2) {
+      uint32_t *sctl = p.sweep_ctl + (sweep % SLOTS) * Q_WORDS;
+      if (leader)  // of the next sweep: no block reads or writes them in this one
+        for (int i = 0; i < 4; i++) p.sweep_ctl[((sweep + 1) % SLOTS) * Q_WORDS + i] = 0;
+      // ---- order: long rows by blocks, then the others by warps
+      for (uint32_t x = blockIdx.x; x < nwide; x += gridDim.x) {
+        const uint32_t u = p.wide[x], t = __ldcg(p.tau + u);
+        if (t == 0 || !since.reaches(t)) continue;
+        if (!__syncthreads_or(set_changed(p, u, sweep, threadIdx.x, blockDim.x))) continue;
+        const uint64_t b = p.off[u];
+        const unsigned long long nu = key_of(p, u, sweep);
+        const uint32_t len = (uint32_t)(p.off[u + 1] - b);
+        uint32_t d = 0;
+        for (uint32_t i0 = 0; i0 < len; i0 += 4 * blockDim.x) {  // four consecutive entries a thread
+          const uint32_t i = i0 + 4 * threadIdx.x;
+          uint32_t w[4], m = 0, total;
+#pragma unroll
+          for (int x = 0; x < 4; x++) w[x] = i + x < len ? __ldg(p.adj + b + i + x) : u;
+#pragma unroll
+          for (int x = 0; x < 4; x++) m |= after(key_of(p, w[x], sweep), w[x], nu, u) ? 1u << x : 0u;
+          uint32_t at = d + block_exclusive_scan<uint32_t>(__popc(m), &total);
+          for (; m; m &= m - 1) p.later[b + at++] = i + __ffs(m) - 1;
+          d += total;
+        }
+        __syncthreads();  // the list, for the block's own reads below
+        if (threadIdx.x == 0) p.dplus[u] = d;
+        if (d < kmin || d > p.dmax) clear_weights(p, u, b, d, threadIdx.x, blockDim.x);
+        if (d >= kmin && threadIdx.x == 0) queue_root(p, sctl, u, d);
+      }
+      {
+        constexpr uint32_t CW = sizeof(C) / 4;
+        uint32_t *area = sm + warp * ((CW + 3) * WARP_SET);
+        C *cnt = reinterpret_cast<C *>(area);
+        uint32_t *A = area + CW * WARP_SET, *hid = A + WARP_SET, *rows = hid + WARP_SET;
+        each_vertex(
+            p.n, nwide,
+            [&](uint32_t v) {
+              const uint32_t t = __ldcg(p.tau + v);
+              return t && since.reaches(t) && p.off[v + 1] - p.off[v] <= ROW_BLOCK;
+            },
+            [&](uint32_t u) {
+              if (!__any_sync(CDS_FULL, set_changed(p, u, sweep, lane, 32))) return;
+              const uint64_t b = p.off[u];
+              const unsigned long long nu = key_of(p, u, sweep);
+              const uint32_t len = (uint32_t)(p.off[u + 1] - b);
+              uint32_t d = 0, pos = 0;  // pos: lane r holds the set's r-th position (sets up to 32)
+              for (uint32_t i0 = 0; i0 < len; i0 += 128) {
+                uint32_t w[4];
+                bool in[4];
+#pragma unroll
+                for (int x = 0; x < 4; x++)
+                  w[x] = i0 + 32 * x + lane < len ? __ldg(p.adj + b + i0 + 32 * x + lane) : u;
+#pragma unroll
+                for (int x = 0; x < 4; x++) in[x] = after(key_of(p, w[x], sweep), w[x], nu, u);
+#pragma unroll
+                for (int x = 0; x < 4; x++) {
+                  const uint32_t m = __ballot_sync(CDS_FULL, in[x]);
+                  if (in[x]) p.later[b + d + __popc(m & ((1u << lane) - 1u))] = i0 + 32 * x + lane;
+                  if (lane >= d && lane - d < __popc(m)) pos = i0 + 32 * x + select_bit(m, lane - d);
+                  d += __popc(m);
+                }
+              }
+              __syncwarp();
+              if (d < kmin) {
+                clear_weights(p, u, b, d, lane, 32);
+              } else if (d <= WARP_SET) {
+                if (lane < d) {
+                  const uint32_t a = p.adj[b + pos];
+                  A[lane] = a;
+                  hid[lane] = p.dag.heavy.id(a);
+                }
+                __syncwarp();
+                local_count<K, false, C>(A, hid, d, p.dag.heavy, p.dag.doff, p.dag.dadj, p.dag.outdeg,
+                                                      rows, cnt, (int)kmin + 1);
+                const unsigned long long total =
+                    warp_sum(store_weights<K>(p, b, d, lane, 32, [&](uint32_t) { return pos; }, A, cnt)) / kmin;
+                if (lane == 0) p.R[u] = (uint32_t)total;
+                __syncwarp();
+              } else if (lane == 0) {
+                p.dplus[u] = d;
+                queue_root(p, sctl, u, d);
+              }
+            });
+      }
+      if (!grid_sync(p.bar, p.err, p.spin_limit)) return;
+      phase_end(0);
+      // ---- count: the queued roots by blocks
+      {
+        const uint32_t nroots = __ldcg(sctl + Q_ROOTS), npairs = __ldcg(sctl + Q_PAIRS);
+        const uint32_t d4 = (p.dmax + 3) & ~3u;
+        C *cnt = reinterpret_cast<C *>(sm);
+        uint32_t *A = sm + d4 * (sizeof(C) / 4), *hid = A + d4;
+        uint32_t *rows = p.rows_global ? p.rows_global + (uint64_t)blockIdx.x * p.rows_slab : hid + d4;
+        for (int kind = 0; kind < 2; kind++) {
+          const uint32_t total_items = kind ? npairs : nroots;
+          for (uint32_t r = blockIdx.x; r < total_items;) {
+            if (kind) {
+              count_pairs<K>(p, __ldcg(p.pairs + r), sweep, sm, rows);
+            } else {
+              const uint32_t u = __ldcg(p.queue + r), d = __ldcg(p.dplus + u);
+              const uint64_t b = p.off[u];
+              for (uint32_t i = threadIdx.x; i < d; i += blockDim.x) {
+                const uint32_t a = p.adj[b + __ldcg(p.later + b + i)];
+                A[i] = a;
+                hid[i] = p.dag.heavy.id(a);
+              }
+              __syncthreads();
+              local_count<K, true, C>(A, hid, d, p.dag.heavy, p.dag.doff, p.dag.dadj, p.dag.outdeg,
+                                                   rows, cnt, (int)kmin + 1);
+              const unsigned long long total =
+                  Team<true>::sum<unsigned long long>(store_weights<K>(
+                      p, b, d, threadIdx.x, blockDim.x,
+                      [&](uint32_t i) { return __ldcg(p.later + b + i); }, A, cnt)) / kmin;
+              if (threadIdx.x == 0) p.R[u] = (uint32_t)total;
+            }
+            // the first items go by block number, the rest by a counter
+            if (threadIdx.x == 0) s_item = gridDim.x + atomicAdd(sctl + (kind ? Q_NEXT_PAIR : Q_NEXT_ROOT), 1u);
+            __syncthreads();
+            r = s_item;
+            __syncthreads();
+          }
+        }
+      }
+      // (every block read the same sizes; with nothing queued nothing was written)
+      if (__ldcg(sctl + Q_ROOTS) + __ldcg(sctl + Q_PAIRS) && !grid_sync(p.bar, p.err, p.spin_limit)) return;
+      phase_end(1);
+    }
+    // ---- lower
+    for (int x = 0; x < (K == 2 ? 1 : LOWER); x++, pass++) {
+      uint32_t *pctl = p.pass_ctl + (pass % SLOTS) * P_WORDS;
+      if (leader)  // of the next pass: last read two passes ago
+        for (int i = 0; i < 3; i++) p.pass_ctl[((pass + 1) % SLOTS) * P_WORDS + i] = 0;
+      const Range reach = x == 0 ? since : pass_range(p.pass_ctl, pass - 1);
+      for (uint32_t i = blockIdx.x; i < nwide; i += gridDim.x) {
+        const uint32_t v = p.wide[i], t = __ldcg(p.tau + v);
+        if (t == 0 || !reach.reaches(t)) continue;
+        const uint32_t nt = lower_block<K>(p, v, t, sm);
+        if (threadIdx.x == 0) {
+          if (x == 0 && K != 2) p.key[v] = key_now(__ldcg(p.key + v), t, sweep);
+          if (nt < t) {
+            p.tau[v] = nt;
+            s_changed = 1;
+            atomicMax(&s_low, ~nt);
+            atomicMax(&s_high, t);
+          }
+        }
+      }
+      __syncthreads();
+      each_vertex(
+          p.n, nwide,
+          [&](uint32_t v) {
+            const uint32_t t = __ldcg(p.tau + v);
+            return t && reach.reaches(t) && p.off[v + 1] - p.off[v] <= ROW_BLOCK;
+          },
+          [&](uint32_t v) {
+            const uint32_t t = __ldcg(p.tau + v);
+            const uint32_t nt = lower_warp<K>(p, v, t, sm + warp * BINS_WARP);
+            if (lane == 0) {
+              if (x == 0 && K != 2) p.key[v] = key_now(__ldcg(p.key + v), t, sweep);
+              if (nt < t) {
+                p.tau[v] = nt;
+                s_changed = 1;
+                atomicMax(&s_low, ~nt);
+                atomicMax(&s_high, t);
+              }
+            }
+          });
+      __syncthreads();
+      if (threadIdx.x == 0 && s_changed) {
+        pctl[P_CHANGED] = 1;
+        atomicMax(pctl + P_LOW, s_low);
+        atomicMax(pctl + P_HIGH, s_high);
+        s_changed = 0;
+        s_low = 0;
+        s_high = 0;
+      }
+      if (!grid_sync(p.bar, p.err, p.spin_limit)) return;
+      phase_end(2);
+      if (x == 0 && !__ldcg(pctl + P_CHANGED)) {  // current weights, and nothing to lower
+        done = true;
         break;
       }
-      verify = true;
-    } else {
-      verify = false;
     }
   }
   if (leader) {
-    *p.sweeps = it;
-    if (it >= p.max_sweeps) atomicOr(p.err, DEV_ERR_TIMEOUT);
+    *p.sweeps = sweep;
+    if (!done) atomicOr(p.err, DEV_ERR_TIMEOUT);
   }
 }
 
-// incidence lists: slot j of clique c goes to members[c*k+j]'s list (ids
-// as u32, or as u64 when there are 2^32 or more cliques)
-template <typename I>
-__global__ void k_fill_incidence(const uint32_t *__restrict__ members, uint64_t m, uint32_t k,
-                                 const uint64_t *__restrict__ inc_off, uint32_t *__restrict__ cursor,
-                                 I *__restrict__ inc) {
-  const uint64_t total = m * k;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < total; base += stride) {
-    const uint64_t t = base + threadIdx.x;
-    // slot-major order: lanes see the same slot of consecutive cliques, which
-    // share their root, so the cursor atomics aggregate
-    const bool ok = t < total;
-    uint32_t v = UNSET;
-    uint64_t c = 0;
-    if (ok) {
-      const uint64_t j = t / m;
-      c = t - j * m;
-      v = members[c * k + j];
+// rel[e], for e = the position of w in u's row: the position of u in w's row.
+// Each edge once, from its end of larger (degree, id), searching the shorter row.
+__global__ void k_rel(const uint64_t *__restrict__ off, const uint32_t *__restrict__ adj, uint32_t n, uint64_t nnz,
+                      uint32_t *__restrict__ rel) {
+  const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  for (uint64_t c = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; c * 32 < nnz; c += warps) {
+    uint32_t lo = 0, hi = n;  // the row of the first of 32 arcs
+    while (hi - lo > 1) {
+      const uint32_t mid = lo + (hi - lo) / 2;
+      if (off[mid] <= c * 32) lo = mid;
+      else hi = mid;
     }
-    const uint32_t grp = __match_any_sync(CDS_FULL, v);
-    const uint32_t leader = __ffs(grp) - 1;
-    uint32_t at = 0;
-    if (ok && leader == lane_id()) at = atomicAdd(&cursor[v], (uint32_t)__popc(grp));
-    at = __shfl_sync(grp, at, leader);
-    if (ok) inc[inc_off[v] + at + __popc(grp & ((1u << lane_id()) - 1u))] = (I)c;
+    const uint64_t e = c * 32 + lane_id();
+    if (e >= nnz) continue;
+    uint32_t u = lo;
+    while (off[u + 1] <= e) u++;
+    const uint32_t w = adj[e];
+    const uint64_t bu = off[u], bw = off[w];
+    const uint32_t du = (uint32_t)(off[u + 1] - bu), dw = (uint32_t)(off[w + 1] - bw);
+    if (!above(du, u, dw, w)) continue;
+    uint32_t a = 0, z = dw;
+    while (a < z) {
+      const uint32_t mid = (a + z) >> 1;
+      if (adj[bw + mid] < u) a = mid + 1;
+      else z = mid;
+    }
+    rel[e] = a;
+    rel[bw + a] = (uint32_t)(e - bu);
   }
 }
 
-// member layout: incidence (v, c) stores the k-1 other members of c, in
-// slot order, in k-1 arrays of k*m entries
-template <typename T>
-__global__ void k_fill_tuples(const uint32_t *__restrict__ members, uint64_t m, uint32_t k,
-                              const uint64_t *__restrict__ inc_off, uint32_t *__restrict__ cursor,
-                              T *__restrict__ tup) {
-  const uint64_t total = m * k;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < total; base += stride) {
-    const uint64_t t = base + threadIdx.x;
-    const bool ok = t < total;
-    uint32_t v = UNSET, j = 0;
-    uint64_t c = 0;
-    if (ok) {
-      j = (uint32_t)(t / m);
-      c = t - (uint64_t)j * m;
-      v = members[c * k + j];
-    }
-    const uint32_t grp = __match_any_sync(CDS_FULL, v);
-    const uint32_t leader = __ffs(grp) - 1;
-    uint32_t at = 0;
-    if (ok && leader == lane_id()) at = atomicAdd(&cursor[v], (uint32_t)__popc(grp));
-    at = __shfl_sync(grp, at, leader);
-    if (ok) {
-      const uint64_t pos = inc_off[v] + at + __popc(grp & ((1u << lane_id()) - 1u));
-      for (uint32_t s = 0; s + 1 < k; s++) tup[s * total + pos] = (T)members[c * k + (s < j ? s : s + 1)];
-    }
-  }
-}
-
-// packed member layout: incidence (v, c) stores the k-1 <= 3 other members
-// of c, in slot order, as 21-bit fields of one u64
-__global__ void k_fill_tuples64(const uint32_t *__restrict__ members, uint64_t m, uint32_t k,
-                                const uint64_t *__restrict__ inc_off, uint32_t *__restrict__ cursor,
-                                unsigned long long *__restrict__ tup) {
-  // clique-major: a thread reads its clique's record once and places the k
-  // incidences, one warp-aggregated cursor round per slot (consecutive
-  // records share their root and, in runs, their next members)
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < m; base += stride) {
-    const uint64_t c = base + threadIdx.x;
-    const bool ok = c < m;
-    uint32_t mem[4] = {UNSET, UNSET, UNSET, UNSET};
-    if (ok) {
-      if (k == 4) {
-        const uint4 r = *reinterpret_cast<const uint4 *>(members + c * 4);
-        mem[0] = r.x;
-        mem[1] = r.y;
-        mem[2] = r.z;
-        mem[3] = r.w;
-      } else {
-        for (uint32_t j = 0; j < k; j++) mem[j] = members[c * k + j];
-      }
-    }
-    // every slot's cursor atomic and list offset are issued before any is
-    // used: the k round trips to L2 overlap instead of following each other
-    uint32_t grp[4], at[4];
-    uint64_t off[4];
-#pragma unroll
-    for (uint32_t j = 0; j < 4; j++) {
-      grp[j] = 0;
-      at[j] = 0;
-      off[j] = 0;
-      if (j >= k) continue;
-      const uint32_t v = ok ? mem[j] : UNSET;
-      grp[j] = __match_any_sync(CDS_FULL, v);
-      if (ok && __ffs(grp[j]) - 1 == (int)lane_id()) at[j] = atomicAdd(&cursor[v], (uint32_t)__popc(grp[j]));
-      if (ok) off[j] = inc_off[v];
-    }
-#pragma unroll
-    for (uint32_t j = 0; j < 4; j++) {
-      if (j >= k) continue;
-      const uint32_t leader = __ffs(grp[j]) - 1;
-      const uint32_t base = __shfl_sync(grp[j], at[j], leader);
-      if (ok) {
-        const uint64_t pos = off[j] + base + __popc(grp[j] & ((1u << lane_id()) - 1u));
-        unsigned long long q = 0;
-        uint32_t f = 0;
-#pragma unroll
-        for (uint32_t s2 = 0; s2 < 4; s2++)
-          if (s2 < k && s2 != j) q |= (unsigned long long)mem[s2] << (PACK_BITS * f++);
-        tup[pos] = q;
-      }
-    }
-  }
-}
-
-// items of each vertex: one up to `chunk` incidences (an exact histogram in
-// shared memory), else ceil(clique degree / hub_chunk) hub items
-__global__ void k_item_count(const uint32_t *__restrict__ cdeg, uint32_t n, uint32_t chunk,
-                             uint32_t hub_chunk, uint32_t *__restrict__ items,
-                             uint32_t *__restrict__ multi) {
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-    const uint32_t d = cdeg[v];
-    const bool hub = d > chunk;
-    items[v] = hub ? (d + hub_chunk - 1) / hub_chunk : (d ? 1u : 0u);
-    multi[v] = hub ? 1u : 0u;
-  }
-}
-
-// Item order.  With `peel_order` set, vertices go in ascending classes of
-// clique degree (powers of two): a single-item vertex's new value is visible
-// to the rest of the sweep, so low-degree vertices settle first and the hubs,
-// counted last, read fresher values.  Otherwise items follow vertex ids.
-// bcur[32] counts, then places, the vertices of each class.
-__global__ void k_class_count(const uint32_t *__restrict__ cdeg, uint32_t n, uint32_t *__restrict__ bcur) {
-  for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
-    const uint32_t v = base + threadIdx.x;
-    const uint32_t d = v < n ? cdeg[v] : 0u;
-    agg_add_u32(bcur, d ? 31u - __clz(d) : 0u, d != 0);
-  }
-}
-__global__ void k_class_scan(uint32_t *bcur) {  // one warp: exclusive scan of the 32 counts
-  const uint32_t x = bcur[lane_id()];
-  bcur[lane_id()] = warp_inclusive_scan(x) - x;
-}
-__global__ void k_class_place(const uint32_t *__restrict__ cdeg, const uint32_t *__restrict__ items,
-                              uint32_t n, uint32_t *__restrict__ bcur, uint32_t *__restrict__ perm,
-                              uint32_t *__restrict__ pitems) {
-  for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
-    const uint32_t v = base + threadIdx.x;
-    const uint32_t d = v < n ? cdeg[v] : 0u;
-    const uint32_t at = agg_inc(bcur, d ? 31u - __clz(d) : 0u, d != 0);
-    if (d) {
-      perm[at] = v;
-      pitems[at] = items[v];
-    }
-  }
-}
-
-// item_v / item_c of the vertices in order (perm null: ids, n of them; else
-// the bcur[31] placed ones), and each hub's accumulator slot
-__global__ void k_item_fill(const uint32_t *__restrict__ perm, const uint32_t *__restrict__ nplaced,
-                            const uint64_t *__restrict__ item_off, const uint64_t *__restrict__ big_off,
-                            uint32_t n, uint32_t *__restrict__ item_v, uint32_t *__restrict__ item_c,
-                            uint32_t *__restrict__ big_slot, uint32_t *__restrict__ big_v) {
-  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t np = perm ? nplaced[31] : n;
-  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < np; i += warps) {
-    const uint32_t v = perm ? perm[i] : i;
-    const uint64_t b = item_off[i], e = item_off[i + 1];
-    for (uint64_t r = b + lane_id(); r < e; r += 32) {
-      item_v[r] = v;
-      item_c[r] = (uint32_t)(r - b);
-    }
-  }
-  for (uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < n; v += warps)
-    if (lane_id() == 0) {
-      const bool multi = big_off[v + 1] > big_off[v];
-      big_slot[v] = multi ? (uint32_t)big_off[v] : UNSET;
-      if (multi) big_v[big_off[v]] = v;
-    }
+__global__ void k_wide(const uint64_t *__restrict__ off, uint32_t n, uint32_t *__restrict__ wide,
+                       uint32_t *__restrict__ nwide) {
+  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
+    if (off[v + 1] - off[v] > ROW_BLOCK) wide[atomicAdd(nwide, 1u)] = v;
 }
 
 // largest core per instance and the vertex histogram of core numbers
@@ -678,18 +694,18 @@ __global__ void k_inst_maxcore(const uint32_t *__restrict__ core, uint32_t n,
   for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
     const uint32_t v = base + threadIdx.x;
     const bool ok = v < n;
-    const uint32_t key = ok ? (of_vertex ? of_vertex[v] : 0u) : UNSET;
+    const uint32_t key = ok ? (of_vertex ? of_vertex[v] : 0u) : 0xFFFFFFFFu;
     const uint32_t grp = __match_any_sync(CDS_FULL, key);
     const uint32_t m = __reduce_max_sync(grp, ok ? core[v] : 0u);
     if (ok && (__ffs(grp) - 1) == (int)lane_id()) atomicMax(out + key, m);
   }
 }
 
-// hv[hoff[i] + L] = vertices of instance i with core L; hc likewise for
-// cliques by their smallest member core
-__global__ void k_core_hist(const uint32_t *__restrict__ core, uint32_t n,
-                            const uint32_t *__restrict__ of_vertex,
-                            const uint64_t *__restrict__ hoff, unsigned long long *__restrict__ hv) {
+// hv[hoff[i] + L] = vertices of instance i with core L, hc likewise the cliques
+// rooted at them (k = 2: a vertex roots the edges to later neighbours)
+__global__ void k_core_hist(const uint32_t *__restrict__ core, const uint32_t *__restrict__ R, uint32_t n,
+                            const uint32_t *__restrict__ of_vertex, const uint64_t *__restrict__ hoff,
+                            unsigned long long *__restrict__ hv, unsigned long long *__restrict__ hc) {
   const uint32_t stride = gridDim.x * blockDim.x;
   for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
     const uint32_t v = base + threadIdx.x;
@@ -698,55 +714,22 @@ __global__ void k_core_hist(const uint32_t *__restrict__ core, uint32_t n,
     if (ok) key = hoff[of_vertex ? of_vertex[v] : 0u] + core[v];
     const uint32_t grp = __match_any_sync(CDS_FULL, key);
     if (ok && (__ffs(grp) - 1) == (int)lane_id()) atomicAdd(hv + key, (unsigned long long)__popc(grp));
+    if (ok && R[v]) atomicAdd(hc + key, (unsigned long long)R[v]);
   }
 }
-
-// (cmin[c] = that smallest member core: the densest-core stage derives its
-// clique flags from it without reading the records again)
-__global__ void k_clique_hist(const uint32_t *__restrict__ members, uint64_t m, uint32_t k,
-                              const uint32_t *__restrict__ core, const uint32_t *__restrict__ of_vertex,
-                              const uint64_t *__restrict__ hoff, unsigned long long *__restrict__ hc,
-                              uint32_t *__restrict__ cmin) {
-  // A warp whose 32 cliques share one level (the cliques inside a dense
-  // core) adds to a count its lane 0 keeps while the level stays the same,
-  // instead of an atomic per step on that level's word.
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  uint64_t wkey = ~0ull;
-  unsigned long long wn = 0;
-  for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < m; base += stride) {
-    const uint64_t c = base + threadIdx.x;
-    const bool ok = c < m;
-    uint64_t key = ~0ull;
-    if (ok) {
-      const uint32_t *mc = members + c * k;
-      uint32_t lo = UNSET, first;
-      if (k == 4) {  // the record in one 16-byte load
-        const uint4 q = *reinterpret_cast<const uint4 *>(mc);
-        lo = min(min(core[q.x], core[q.y]), min(core[q.z], core[q.w]));
-        first = q.x;
-      } else {
-        for (uint32_t j = 0; j < k; j++) lo = min(lo, core[mc[j]]);
-        first = mc[0];
-      }
-      cmin[c] = lo;
-      key = hoff[of_vertex ? of_vertex[first] : 0u] + lo;
+__global__ void k_edge_roots(const uint64_t *__restrict__ off, const uint32_t *__restrict__ adj,
+                             const uint32_t *__restrict__ core, uint32_t n, uint32_t *__restrict__ R) {
+  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+  for (uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < n; v += warps) {
+    const uint32_t t = core[v];
+    uint32_t c = 0;
+    for (uint64_t i = off[v] + lane_id(); i < off[v + 1]; i += 32) {
+      const uint32_t w = adj[i], tw = core[w];
+      c += tw > t || (tw == t && w > v);
     }
-    const uint64_t k0 = __shfl_sync(CDS_FULL, key, 0);
-    if (__all_sync(CDS_FULL, ok && key == k0)) {
-      if (lane_id() == 0) {
-        if (k0 != wkey) {
-          if (wn) atomicAdd(hc + wkey, wn);
-          wkey = k0;
-          wn = 0;
-        }
-        wn += 32;
-      }
-      continue;
-    }
-    const uint32_t grp = __match_any_sync(CDS_FULL, key);
-    if (ok && (__ffs(grp) - 1) == (int)lane_id()) atomicAdd(hc + key, (unsigned long long)__popc(grp));
+    c = __reduce_add_sync(CDS_FULL, c);
+    if (lane_id() == 0) R[v] = c;
   }
-  if (lane_id() == 0 && wn) atomicAdd(hc + wkey, wn);
 }
 
 // One block per instance: suffix sums over L of both histograms give the
@@ -873,12 +856,13 @@ __global__ void __launch_bounds__(512) k_best_level(const uint64_t *__restrict__
 
 namespace cds {
 
-void peel(cds_ctx *c, cudaStream_t s, uint32_t n, const Cliques &cl, const Instances &inst,
-          const Tuning &t, uint32_t gl_buffer_size, PeelOut &out) {
-  const uint32_t k = cl.k;
+void peel(cds_ctx *c, cudaStream_t s, const uint64_t *off, const uint32_t *adj, uint64_t nnz, const Dag &dag,
+          const Cliques &cl, const Instances &inst, uint32_t gl_buffer_size, PeelOut &out) {
+  const uint32_t n = dag.n, k = cl.k;
   const uint64_t m = cl.count;
   const uint32_t ninst = inst.count;
   const uint32_t *of_vertex = ninst > 1 ? inst.of_vertex.p : nullptr;
+  (void)gl_buffer_size;  // the reference's per-block removal buffer length has no counterpart
   out.core.c = c;
   out.core.s = s;
   out.core.alloc(n + 1);
@@ -890,189 +874,112 @@ void peel(cds_ctx *c, cudaStream_t s, uint32_t n, const Cliques &cl, const Insta
   out.levels = 0;
   out.max_core = 0;
   if (n == 0) return;
+  DBuf<unsigned long long> phase(c, s, c->prof ? 3 : 0);
+  phase.zero();
+  CDS_CUDA(cudaMemcpyAsync(out.core.p, cl.cdeg.p, (size_t)n * 4, cudaMemcpyDeviceToDevice, s));
 
-  // vertex -> clique incidence CSR: for k <= 4 the other members of each
-  // incidence (streamed by every sweep), falling back to clique ids (one
-  // member record gathered per incidence) when that does not fit the budget
-  DBuf<uint64_t> inc_off(c, s, n + 1);
-  scan_u32(cl.cdeg.p, inc_off.p, n, c, s);
-  DBuf<uint32_t> inc, tup;
-  DBuf<uint16_t> tup16;
-  DBuf<unsigned long long> tup64, inc64;
-  inc.c = tup.c = tup16.c = tup64.c = inc64.c = c;
-  inc.s = tup.s = tup16.s = tup64.s = inc64.s = s;
-  // clique ids past 32 bits: 2^32 or more cliques (or the flag that forces
-  // that layout); the member layouts below need no clique ids at all
-  const bool wide_ids = m >= 0xFFFFFFFFull || (c->flags & CDS_CONFIG_WIDE_CLIQUE_IDS);
-  bool tuple = false;
-  const bool narrow = n <= 65536;  // member ids fit 16 bits
-  // k = 3, 4 above that: the other members packed into one u64 (8 bytes an
-  // incidence instead of 4(k-1)), while ids fit 21 bits
-  const bool packed = !narrow && (k == 3 || k == 4) && n <= PACK_MAX_N;
-  if (k <= 4 && m && !(c->flags & (CDS_CONFIG_COMPACT_PEEL | CDS_CONFIG_WIDE_CLIQUE_IDS))) {
-    try {
-      if (narrow) tup16.alloc(m * k * (k - 1) + 1);
-      else if (packed) tup64.alloc(m * k + 1);
-      else tup.alloc(m * k * (k - 1) + 1);
-      tuple = true;
-    } catch (const Error &e) {
-      if (e.status != CDS_ERR_OOM) throw;
-    }
-  }
-  if (!tuple && wide_ids) inc64.alloc(m * k + 1);
-  else if (!tuple) inc.alloc(m * k + 1);
+  // work words in one zeroed block: barrier, status, control slots, queue sizes
+  constexpr size_t CTL = 32 + SLOTS * (P_WORDS + Q_WORDS) + 4;
+  DBuf<uint32_t> ctl(c, s, CTL), R(c, s, n), wide(c, s, n);
+  ctl.zero();
+  R.zero();
+  uint32_t *const ctl_err = ctl.p + CTL - 1, *const ctl_sweeps = ctl.p + CTL - 2, *const ctl_nwide = ctl.p + CTL - 3;
+  k_wide<<<c->sm_count * 2, 256, 0, s>>>(off, n, wide.p, ctl_nwide);
+  count_launch();
   {
-    DBuf<uint32_t> cursor(c, s, n);
-    cursor.zero();
+    CoreParams p{};
+    p.n = n;
+    p.k = k;
+    p.off = off;
+    p.adj = adj;
+    p.tau = out.core.p;
+    p.R = R.p;
+    p.wide = wide.p;
+    p.nwide = ctl_nwide;
+    static_assert(sizeof(GridBarrier) == 32 * sizeof(uint32_t), "the barrier takes the first line");
+    p.bar = reinterpret_cast<GridBarrier *>(ctl.p);
+    p.pass_ctl = ctl.p + 32;
+    p.sweep_ctl = p.pass_ctl + SLOTS * P_WORDS;
+    p.err = ctl_err;
+    p.sweeps = ctl_sweeps;
+    p.phase_ns = phase.p;
+    p.spin_limit = 1ull << 26;
+    p.max_sweeps = 1u << 20;
+    p.time_budget_ns = 120ull * 1000000000ull;
+    DBuf<unsigned long long> key(c, s, 0);
+    DBuf<uint32_t> rel(c, s, 0), cin(c, s, 0), later(c, s, 0), dplus(c, s, 0), queue(c, s, 0),
+        rows(c, s, 0);
+    DBuf<uint2> pairs(c, s, 0);
+    size_t smem = (size_t)std::max<uint32_t>(WARPS * BINS_WARP, BINS_BLOCK) * 4;
+    unsigned blocks = coop_grid(c, 2);
+    if (k >= 3 && m) {
+      rel.alloc(nnz + 1);
+      key.alloc(n);
+      cin.alloc(nnz + 1);
+      later.alloc(nnz + 1);
+      dplus.alloc(n);
+      queue.alloc(n);
+      cin.zero();
+      key.zero();  // (read for vertices in no clique, which are never ordered)
+      {
+        ProfScope ps(c, s, "peel_arcs");
+        k_rel<<<c->sm_count * 8, 256, 0, s>>>(off, adj, n, nnz, rel.p);
+        count_launch();
+        CDS_CUDA(cudaGetLastError());
+      }
+      // the largest later set one block counts: as far as two blocks' rows fit
+      // an SM (768: 95 KB), or the DAG's largest out-degree where that is more
+      // (count_pairs needs it); past BLOCK_DMAX the rows go to global memory
+      const int K = k <= 5 ? (int)k : 0;
+      p.dmax = std::max<uint32_t>(k == 3 ? 4096 : 768, dag.max_out);
+      const bool rows_in_smem = k == 3 || p.dmax <= (uint32_t)BLOCK_DMAX;
+      if (!rows_in_smem) {
+        p.rows_slab = ((uint64_t)p.dmax * row_stride((p.dmax + 31) / 32) + 3) & ~3ull;
+        blocks = std::min<unsigned>(blocks, coop_grid(c, 1));
+        rows.alloc((size_t)blocks * p.rows_slab);
+        p.rows_global = rows.p;
+      }
+      pairs.alloc(nnz / PAIR_ITEM + nnz / p.dmax + 1);
+      smem = std::max(smem, (size_t)count_team_words(K, p.dmax, rows_in_smem) * 4);
+      smem = std::max(smem, (size_t)WARPS * WARP_SET * 5 * 4);
+      p.rel = rel.p;
+      p.key = key.p;
+      p.cin = cin.p;
+      p.later = later.p;
+      p.dplus = dplus.p;
+      p.queue = queue.p;
+      p.pairs = pairs.p;
+      p.dag.doff = dag.off.p;
+      p.dag.dadj = dag.adj.p;
+      p.dag.outdeg = dag.outdeg.p;
+      p.dag.heavy = dag.heavy;
+    }
     if (m) {
-      ProfScope ps(c, s, "peel_incidence");
-      if (tuple && narrow)
-        k_fill_tuples<uint16_t><<<c->sm_count * 8, 256, 0, s>>>(cl.members.p, m, k, inc_off.p, cursor.p,
-                                                                tup16.p);
-      else if (tuple && packed)
-        k_fill_tuples64<<<c->sm_count * 8, 256, 0, s>>>(cl.members.p, m, k, inc_off.p, cursor.p, tup64.p);
-      else if (tuple)
-        k_fill_tuples<uint32_t><<<c->sm_count * 8, 256, 0, s>>>(cl.members.p, m, k, inc_off.p, cursor.p,
-                                                                tup.p);
-      else if (wide_ids)
-        k_fill_incidence<unsigned long long><<<c->sm_count * 8, 256, 0, s>>>(cl.members.p, m, k, inc_off.p,
-                                                                            cursor.p, inc64.p);
-      else
-        k_fill_incidence<uint32_t><<<c->sm_count * 8, 256, 0, s>>>(cl.members.p, m, k, inc_off.p, cursor.p,
-                                                                  inc.p);
+      void *kern = k == 2 ? (void *)k_core<2> : k == 3 ? (void *)k_core<3> : k == 4 ? (void *)k_core<4>
+                 : k == 5 ? (void *)k_core<5> : (void *)k_core<0>;
+      // (raised to the most any launch uses, never lowered under another thread's launch)
+      cudaFuncAttributes fa;
+      CDS_CUDA(cudaFuncGetAttributes(&fa, kern));
+      const size_t dyn_max = c->smem_optin - fa.sharedSizeBytes;
+      if (smem > dyn_max) fail(CDS_ERR_CUDA, "peel team does not fit in shared memory");
+      CDS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn_max));
+      int per_sm = 0;
+      CDS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, THREADS, smem));
+      if (per_sm < 1) fail(CDS_ERR_CUDA, "peel kernel does not fit on an SM");
+      blocks = std::min<unsigned>(blocks, coop_grid(c, std::min(per_sm, 2)));
+      void *args[] = {&p};
+      {
+        ProfScope ps(c, s, "peel");
+        CDS_CUDA(cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(THREADS), args, smem, s));
+      }
       count_launch();
       CDS_CUDA(cudaGetLastError());
     }
   }
-
-  // Work items of at most `chunk` incidences; the reference's glBufferSize
-  // (a per-block removal buffer length) has no counterpart here.
-  (void)gl_buffer_size;
-  const uint32_t chunk = (uint32_t)std::max(64, std::min(t.peel_chunk, MAX_CHUNK));
-  DBuf<uint32_t> items(c, s, n), multi(c, s, n);
-  const uint32_t hub_chunk = chunk;  // larger hub items save flushes but cost sweeps
-  k_item_count<<<c->sm_count * 4, 256, 0, s>>>(cl.cdeg.p, n, chunk, hub_chunk, items.p, multi.p);
-  count_launch();
-  // item order: by ascending degree class (t.peel_order) or by vertex id
-  DBuf<uint32_t> bcur(c, s, 32), perm, pitems;
-  perm.c = pitems.c = c;
-  perm.s = pitems.s = s;
-  if (t.peel_order) {
-    perm.alloc(n + 1);
-    pitems.alloc(n + 1);
-    bcur.zero();
-    pitems.zero();
-    k_class_count<<<c->sm_count * 4, 256, 0, s>>>(cl.cdeg.p, n, bcur.p);
-    k_class_scan<<<1, 32, 0, s>>>(bcur.p);
-    k_class_place<<<c->sm_count * 4, 256, 0, s>>>(cl.cdeg.p, items.p, n, bcur.p, perm.p, pitems.p);
-    count_launch(3);
-  }
-  DBuf<uint64_t> item_off(c, s, n + 1), big_off(c, s, n + 1);
-  scan_u32(t.peel_order ? pitems.p : items.p, item_off.p, n, c, s);
-  scan_u32(multi.p, big_off.p, n, c, s);
-  // sized by bounds known on the host, so nothing waits for the scans: a
-  // vertex has at most clique degree / item size + 1 items, and a hub more
-  // than `chunk` incidences
-  const uint64_t nitems = (uint64_t)n + (m * k) / std::min(chunk, hub_chunk) + 1;
-  const uint64_t nbig = std::min<uint64_t>(n, (m * k) / chunk + 1);
-  if (nitems >= 0xFFFFFFFFull) fail(CDS_ERR_OVERFLOW, "peel: more than 2^32-1 work items");
-  DBuf<uint32_t> item_v(c, s, nitems + 1), item_c(c, s, nitems + 1), big_slot(c, s, n),
-      big_v(c, s, nbig + 1);
-  k_item_fill<<<c->sm_count * 8, 256, 0, s>>>(t.peel_order ? perm.p : nullptr, bcur.p, item_off.p,
-                                              big_off.p, n, item_v.p, item_c.p, big_slot.p, big_v.p);
-  count_launch();
-  CDS_CUDA(cudaGetLastError());
-  DBuf<uint32_t> acc(c, s, nbig * ACC_WORDS + 1), big_done(c, s, nbig + 1);
-  acc.zero();
-  big_done.zero();
-  CDS_CUDA(cudaMemcpyAsync(out.core.p, cl.cdeg.p, (size_t)n * 4, cudaMemcpyDeviceToDevice, s));
-  DBuf<uint32_t> ctl(c, s, 3 * 32 + 1), ichg(c, s, 3 * (size_t)ninst);
-  ichg.zero();
-  DBuf<GridBarrier> bar(c, s, 1);
-  DBuf<uint32_t> err(c, s, 1);
-  ctl.zero();
-  bar.zero();
-  err.zero();
-
-  HParams p{};
-  p.n = n;
-  p.k = k;
-  p.members = cl.members.p;
-  p.inc_off = inc_off.p;
-  p.inc = inc.p;
-  p.inc64 = inc64.p;
-  p.tup = tup.p;
-  p.tup16 = tup16.p;
-  p.tup64 = tup64.p;
-  p.tup_stride = m * k;
-  p.tau = out.core.p;
-  p.item_v = item_v.p;
-  p.item_c = item_c.p;
-  p.vitems = items.p;
-  p.nitems = item_off.p + n;
-  p.chunk = chunk;
-  p.hub_chunk = hub_chunk;
-  p.big_slot = big_slot.p;
-  p.big_v = big_v.p;
-  p.nbig = (uint32_t)nbig;
-  p.acc = acc.p;
-  p.big_done = big_done.p;
-  p.ctl = ctl.p;
-  p.of_vertex = of_vertex;
-  p.ninst = ninst;
-  p.ichg = ichg.p;
-  p.bar = bar.p;
-  p.err = err.p;
-  p.spin_limit = 1ull << 26;
-  p.max_sweeps = 1u << 20;
-  p.time_budget_ns = 120ull * 1000000000ull;
-  p.sweeps = ctl.p + 3 * 32;
-  DBuf<unsigned long long> reads(c, s, c->prof ? MAX_READ_SWEEPS : 0);
-  if (c->prof) reads.zero();
-  p.reads = c->prof ? reads.p : nullptr;
-  // the static share of the items (peel_static percent, 100: all static)
-  p.static_pct = (uint32_t)std::min(100, std::max(0, t.peel_static));
-  if (m) {
-    void *kern = tuple && narrow ? (k == 2 ? (void *)k_hindex<2, 2>
-                                  : k == 3 ? (void *)k_hindex<3, 2> : (void *)k_hindex<4, 2>)
-               : tuple && packed ? (k == 3 ? (void *)k_hindex<3, 3> : (void *)k_hindex<4, 3>)
-               : tuple ? (k == 2 ? (void *)k_hindex<2, 1>
-                        : k == 3 ? (void *)k_hindex<3, 1> : (void *)k_hindex<4, 1>)
-               : wide_ids ? (k == 2 ? (void *)k_hindex<2, 4>
-                           : k == 3 ? (void *)k_hindex<3, 4>
-                           : k == 4 ? (void *)k_hindex<4, 4> : (void *)k_hindex<0, 4>)
-                       : (k == 2 ? (void *)k_hindex<2, 0>
-                        : k == 3 ? (void *)k_hindex<3, 0>
-                        : k == 4 ? (void *)k_hindex<4, 0> : (void *)k_hindex<0, 0>);
-    const int threads = 512;
-    // each warp's histogram as large as its items need (the rest of the
-    // SM's shared memory stays L1, which holds the gathered core values)
-    p.warp_words = (std::max<uint32_t>(chunk + 1, ACC_WORDS) + 3u) & ~3u;
-    const size_t smem = (size_t)(threads / 32) * p.warp_words * 4;
-    CDS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int per_sm = 0;
-    CDS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
-    if (per_sm < 1) fail(CDS_ERR_CUDA, "peel kernel does not fit on an SM");
-    per_sm = std::min(per_sm, 2);
-    dim3 grid(coop_grid(c, per_sm)), block(threads);
-    void *args[] = {&p};
-    {
-      ProfScope ps(c, s, "peel");
-      CDS_CUDA(cudaLaunchCooperativeKernel(kern, grid, block, args, smem, s));
-    }
+  if (k == 2) {
+    k_edge_roots<<<c->sm_count * 8, 256, 0, s>>>(off, adj, out.core.p, n, R.p);
     count_launch();
-    CDS_CUDA(cudaGetLastError());
   }
-  // the incidence streams are done with (stream-ordered frees), which makes
-  // room for the per-clique smallest member core
-  tup.release();
-  tup16.release();
-  tup64.release();
-  inc.release();
-  inc64.release();
-  out.cmin.c = c;
-  out.cmin.s = s;
-  out.cmin.alloc(m + 1);
   // per-instance largest core (sizes the histograms), read with the status
   DBuf<uint32_t> imax(c, s, ninst);
   imax.zero();
@@ -1082,7 +989,7 @@ void peel(cds_ctx *c, cudaStream_t s, uint32_t n, const Cliques &cl, const Insta
   {
     HostReads r(s);
     r.add(out.inst_max_core.data(), imax.p, ninst);
-    r.add(&e, err.p);
+    r.add(&e, ctl_err);
     r.wait();
   }
   if (e & DEV_ERR_TIMEOUT) fail(CDS_ERR_TIMEOUT, "peel: device iteration budget exhausted");
@@ -1101,13 +1008,10 @@ void peel(cds_ctx *c, cudaStream_t s, uint32_t n, const Cliques &cl, const Insta
   hc.zero();
   {
     ProfScope ps(c, s, "peel_levels");
-    k_core_hist<<<c->sm_count * 4, 256, 0, s>>>(out.core.p, n, of_vertex, d_hoff.p, hv.p);
-    if (m)
-      k_clique_hist<<<c->sm_count * 8, 256, 0, s>>>(cl.members.p, m, k, out.core.p, of_vertex,
-                                                    d_hoff.p, hc.p, out.cmin.p);
+    k_core_hist<<<c->sm_count * 4, 256, 0, s>>>(out.core.p, R.p, n, of_vertex, d_hoff.p, hv.p, hc.p);
     k_best_level<<<std::min<uint32_t>(ninst, c->sm_count * 4), 512, 0, s>>>(
         d_hoff.p, hv.p, hc.p, ninst, bnum.p, bden.p, ilev.p, blev.p);
-    count_launch(m ? 3 : 2);
+    count_launch(2);
   }
   CDS_CUDA(cudaGetLastError());
   std::vector<unsigned long long> hn(ninst), hd(ninst);
@@ -1118,27 +1022,25 @@ void peel(cds_ctx *c, cudaStream_t s, uint32_t n, const Cliques &cl, const Insta
     r.add(hd.data(), bden.p, ninst);
     r.add(out.inst_levels.data(), ilev.p, ninst);
     r.add(out.best_level.data(), blev.p, ninst);
-    r.add(&sweeps, p.sweeps);
+    r.add(&sweeps, ctl_sweeps);
     r.wait();
   }
   if (c->prof) {
-    std::vector<unsigned long long> hr(MAX_READ_SWEEPS);
+    unsigned long long hph[3];
     {
       HostReads r(s);
-      r.add(hr.data(), reads.p, MAX_READ_SWEEPS);
+      r.add(hph, phase.p, 3);
       r.wait();
     }
     std::lock_guard<std::mutex> g(c->mu);
     auto &slot = c->prof_done["peel_sweeps"];
     slot.first += 1;
     slot.second += sweeps;
-    // incidences each sweep read, in millions (the early exits skip the rest)
-    for (uint32_t i = 0; i < std::min(sweeps, MAX_READ_SWEEPS); i++) {
-      char name[32];
-      std::snprintf(name, sizeof(name), "peel_reads_sweep%02u", i);
-      auto &r2 = c->prof_done[name];
-      r2.first += 1;
-      r2.second += hr[i] / 1e6;
+    static const char *pn[3] = {"peel_phase_order", "peel_phase_count", "peel_phase_lower"};
+    for (int i = 0; i < 3; i++) {
+      auto &a = c->prof_done[pn[i]];
+      a.first += 1;
+      a.second += hph[i] / 1e6;
     }
   }
   for (uint32_t i = 0; i < ninst; i++) {

@@ -218,15 +218,15 @@ void run_problem(cds_ctx *c, cudaStream_t s, UnionGraph &u, const cds_params &pr
   const int m1 = clk.mark();
 
   Cliques cl;
-  list_cliques(c, s, dag, k, true, t, cl, on_count);
+  list_cliques(c, s, dag, k, LIST_NARROW, t, cl);
   const int m2 = clk.mark();
 
   PeelOut pe;
-  peel(c, s, u.n, cl, u.inst, t, prm.gl_buffer_size, pe);
+  peel(c, s, u.off, u.adj, u.nnz, dag, cl, u.inst, prm.gl_buffer_size, pe);
   const int m3 = clk.mark();
 
   CoreOut co;
-  densest_core_and_components(c, s, dag, cl, pe, u.inst, k, co, !core_only, &clk);
+  densest_core_and_components(c, s, dag, pe, u.inst, k, t, co, !core_only, &clk, on_count);
   const int m4 = clk.mark();
 
   // per-instance clique totals
@@ -240,8 +240,6 @@ void run_problem(cds_ctx *c, cudaStream_t s, UnionGraph &u, const cds_params &pr
     r.add(tot.data(), d.p, ninst);
     r.wait();
   }
-  // the clique store and incidence lists are no longer needed
-  cl.members.release();
 
   FlowAnswer fa;
   if (core_only) core_answer(s, pe, u, fa);

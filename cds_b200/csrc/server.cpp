@@ -86,26 +86,22 @@ namespace {
 
 bool is_large(const cds_server::Req &r) { return r.nnz >= LARGE_ARCS; }
 
-// Device bytes a request takes before its clique count is known: its graph
-// (when uploaded), DAG, listing work arrays and per-vertex state.
+// Device bytes a request takes before the cliques of its densest core are
+// counted: its graph (when uploaded), DAG and heavy bitmap, the peel's per-arc
+// arrays and per-vertex state.
 uint64_t pre_count_bytes(uint64_t n, uint64_t nnz, bool upload) {
-  uint64_t b = 96 * (n + 1) + 8 * nnz;
+  const uint64_t heavy = n < 16384 ? n : 16384;
+  uint64_t b = 160 * (n + 1) + 20 * nnz + heavy * heavy / 8;
   if (upload) b += 8 * (n + 1) + 4 * nnz;
   return b + (1u << 20);
 }
 
-// Device bytes sized by |Psi|: the clique store (4k per clique), and the
-// larger of the peel's incidence streams (the layout peel.cu picks) and the
-// flow networks' members, incidences and flow state (at most 12k + 4 per
-// clique); the estimate used for admission once the count is known.
-uint64_t post_count_bytes(uint64_t cliques, uint32_t k, uint64_t n) {
-  uint64_t peel;
-  if (k <= 4 && n <= 65536) peel = 2ull * k * (k - 1);
-  else if ((k == 3 || k == 4) && n <= (1u << 21)) peel = 8ull * k;
-  else if (k <= 4) peel = 4ull * k * (k - 1);
-  else peel = 4ull * k;
-  const uint64_t flow = 12ull * k + 4;
-  return cliques * (4ull * k + (peel > flow ? peel : flow)) + (16u << 20);
+// Device bytes sized by the densest cores' cliques: their store (4k per clique),
+// the networks' records (member and flow slots) and incidence lists (4k); the
+// estimate used for admission once that count is known.
+uint64_t post_count_bytes(uint64_t cliques, uint32_t k) {
+  const uint64_t slots = k <= 2 ? 2 : k <= 4 ? 4 : k <= 8 ? 8 : 16;
+  return cliques * (8ull * k + 8ull * slots) + (16u << 20);
 }
 
 void publish(cds_server *s, const std::vector<cds_server::Req> &batch, cds_status st,
@@ -211,14 +207,10 @@ void worker_main(cds_server *s, size_t wi) {
     }
     if (!batch.empty()) try {
       std::vector<const cds_graph *> gs;
-      uint64_t n_all = 0;
-      for (size_t i = 0; i < batch.size(); i++) {
-        gs.push_back(batch[i].g ? batch[i].g : uploaded[i]);
-        n_all += batch[i].n;
-      }
+      for (size_t i = 0; i < batch.size(); i++) gs.push_back(batch[i].g ? batch[i].g : uploaded[i]);
       const uint32_t k = batch[0].p.k;
       const cds::CountHook admit = [&](uint64_t cliques) {
-        const uint64_t need = post_count_bytes(cliques, k, n_all);
+        const uint64_t need = post_count_bytes(cliques, k);
         std::unique_lock<std::mutex> lk(s->mu);
         s->waiting_mem++;
         // wait while it does not fit and some other batch is still working

@@ -28,6 +28,7 @@ struct Dag {
   uint32_t n = 0;
   uint32_t max_out = 0;
   DBuf<uint32_t> deg;     // [n] undirected degree
+  const uint32_t *degree = nullptr;  // [n] the degrees the arcs climb in (a part of a DAG: the whole one's)
   DBuf<uint32_t> outdeg;  // [n] out-degree
   DBuf<uint64_t> off;     // [n+1] row starts (rows padded to 4 entries)
   DBuf<uint32_t> adj;     // out-neighbours, ascending id, 0xFFFFFFFF padding
@@ -41,8 +42,8 @@ struct Cliques {
   uint32_t k = 0;
   uint64_t count = 0;
   DBuf<unsigned long long> cdeg64;  // [n] clique degree of every vertex, exact
-  DBuf<uint32_t> cdeg;     // [n] the same as u32 (materialised listings only; every
-                           // clique degree below 2^32, else CDS_ERR_OVERFLOW)
+  DBuf<uint32_t> cdeg;     // [n] the same as u32 (LIST_NARROW only; every clique
+                           // degree below 2^32, else CDS_ERR_OVERFLOW)
   DBuf<uint64_t> base;     // [n+1] first clique rooted at each vertex
   DBuf<uint32_t> members;  // [count*k] clique records (k ids each)
 };
@@ -50,11 +51,11 @@ struct Cliques {
 // is allocated (the server reserves device memory there; it may block).
 using CountHook = std::function<void(uint64_t cliques)>;
 
-// Counts (and, if materialize, writes) every k-clique.  The count and the
-// u64 clique degrees have no 2^32 cap; a materialised listing also narrows
-// the clique degrees to u32 for the later stages (CDS_ERR_OVERFLOW when one
-// reaches 2^32).
-void list_cliques(cds_ctx *c, cudaStream_t s, const Dag &dag, uint32_t k, bool materialize,
+// Counts every k-clique; LIST_NARROW also narrows the clique degrees to u32 for
+// the peel (CDS_ERR_OVERFLOW when one reaches 2^32), LIST_WRITE writes the
+// records.  The count and the u64 clique degrees have no 2^32 cap.
+enum ListMode { LIST_COUNT, LIST_NARROW, LIST_WRITE };
+void list_cliques(cds_ctx *c, cudaStream_t s, const Dag &dag, uint32_t k, ListMode mode,
                   const Tuning &t, Cliques &out, const CountHook *on_count = nullptr);
 
 // Instance table of a problem: instance i owns vertices [vbeg[i], vbeg[i+1]).
@@ -67,7 +68,6 @@ struct Instances {
 
 struct PeelOut {
   DBuf<uint32_t> core;              // [n] clique-core number
-  DBuf<uint32_t> cmin;              // [m] smallest core number among each clique's members
   uint32_t max_core = 0;
   std::vector<uint64_t> best_num;   // per instance: best core density
   std::vector<uint64_t> best_den;
@@ -76,8 +76,9 @@ struct PeelOut {
   std::vector<uint32_t> best_level;   // per instance: L of the densest core {core >= L}
   uint32_t levels = 0;                // the largest of inst_levels
 };
-void peel(cds_ctx *c, cudaStream_t s, uint32_t n, const Cliques &cl, const Instances &inst,
-          const Tuning &t, uint32_t gl_buffer_size, PeelOut &out);
+// cl: a LIST_NARROW listing of the graph (off, adj with nnz arcs) and its DAG
+void peel(cds_ctx *c, cudaStream_t s, const uint64_t *off, const uint32_t *adj, uint64_t nnz, const Dag &dag,
+          const Cliques &cl, const Instances &inst, uint32_t gl_buffer_size, PeelOut &out);
 
 // Densest core, pruning and components; everything the flow stage needs.
 struct CoreOut {
@@ -106,9 +107,10 @@ struct CoreOut {
   int mk_core = 0, mk_prune = 0;  // StageClock marks after the core and the pruning
 };
 struct StageClock;
-void densest_core_and_components(cds_ctx *c, cudaStream_t s, const Dag &dag, const Cliques &cl,
-                                 const PeelOut &pe, const Instances &inst, uint32_t k,
-                                 CoreOut &out, bool need_networks, StageClock *clk = nullptr);
+void densest_core_and_components(cds_ctx *c, cudaStream_t s, const Dag &dag, const PeelOut &pe,
+                                 const Instances &inst, uint32_t k, const Tuning &t, CoreOut &out,
+                                 bool need_networks, StageClock *clk = nullptr,
+                                 const CountHook *on_count = nullptr);
 
 // Exact search over all component networks; per instance the answer set.
 struct FlowAnswer {

@@ -55,18 +55,14 @@ typedef struct cds_config {
 } cds_config;
 
 /* cds_config.flags.  No counterpart in the reference (its layouts are fixed). */
-/* The peel reads clique ids and gathers member records instead of streaming
- * per-incidence copies of the other members: (k-1)x less peel memory for
- * k <= 4 (the default falls back to it only when the copies do not fit),
- * slower sweeps. */
+/* Accepted, without effect: the peel stores nothing per clique, so there is no
+ * larger layout to avoid. */
 #define CDS_CONFIG_COMPACT_PEEL 1u
 /* 64-bit clique indices in the incidence lists and 64-bit flow state in
  * every flow network, whatever its size (the default narrows them to 32
  * bits when they fit). */
 #define CDS_CONFIG_WIDE_FLOW 2u
-/* 64-bit clique ids in the peel's clique-id layout, whatever the count (a
- * listing of 2^32 or more cliques always uses them; member layouts need no
- * clique ids).  Implies the clique-id layout. */
+/* Accepted, without effect: the peel uses no clique ids. */
 #define CDS_CONFIG_WIDE_CLIQUE_IDS 4u
 
 /* Solve parameters: the reference CLI's positional arguments

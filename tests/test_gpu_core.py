@@ -1,0 +1,78 @@
+"""Clique-core numbers by weighted arcs: exact against the oracle's peel where rows
+are handled by warps and by blocks, and against known values where a vertex has
+more later neighbours than one team counts (a hub of low core number among
+vertices of higher ones)."""
+from math import comb
+
+import numpy as np
+import pytest
+
+import cds_b200 as cds
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    with cds.Context(0) as c:
+        yield c
+
+
+@pytest.mark.parametrize("k", [2, 3, 4, 5, 6])
+@pytest.mark.parametrize("n,degree,plant", [(33, 6.0, 20), (600, 10.0, 33), (3001, 12.0, 0), (5000, 14.0, 70)])
+def test_against_the_oracle(ctx, n, degree, plant, k):
+    if k >= 5:
+        degree, plant = degree / 2, min(plant, 34)
+    scale = (n - 1).bit_length()
+    off, adj = cds.gen_rmat(scale, degree / 2 * n / (1 << scale), n + k, n=n)
+    if plant:
+        off, adj, _ = cds.gen_plant(off, adj, plant, 0.6, n)
+    # a hub whose row is a block's work, joined to every third vertex
+    src = np.repeat(np.arange(n), np.diff(off.astype(np.int64)))
+    hub = np.arange(1, n, 3)
+    off, adj = cds.csr_from_edges(n, np.r_[src, np.zeros_like(hub)], np.r_[adj.astype(np.int64), hub])
+    want = oracle.peel(off, adj, k)
+    g = ctx.graph(off, adj)
+    core, largest, total = ctx.clique_core(g, k)
+    g.free()
+    assert total == want["total"]
+    assert np.array_equal(core.astype(np.int64), want["core"])
+    assert largest == want["core"].max()
+
+
+@pytest.mark.parametrize("k,groups,m", [(3, 2100, 70), (4, 1000, 20), (5, 300, 12), (6, 200, 10)])
+def test_later_sets_past_one_team(ctx, k, groups, m):
+    # `groups` complete graphs of k-1 vertices, all joined to a complete graph D of
+    # m; a hub joined to every group but not to D lies in one k-clique a group
+    r = k - 1
+    u, v = [], []
+
+    def edge(a, b):
+        u.append(a)
+        v.append(b)
+
+    first = 1 + m
+    for a in range(m):
+        for b in range(a):
+            edge(1 + a, 1 + b)
+    for gi in range(groups):
+        base = first + gi * r
+        for x in range(r):
+            edge(0, base + x)
+            for y in range(x):
+                edge(base + x, base + y)
+            for d in range(m):
+                edge(base + x, 1 + d)
+    n = first + groups * r
+    off, adj = cds.csr_from_edges(n, u, v)
+    # k-cliques of a group's vertex with the rest of its group and D, without the hub
+    deg = sum(comb(r - 1, i) * comb(m, k - 1 - i) for i in range(r))
+    assert deg > groups and comb(m - 1, k - 1) < deg
+    g = ctx.graph(off, adj)
+    core, largest, _ = ctx.clique_core(g, k)
+    sol = ctx.solve(g, k, search="core")
+    g.free()
+    assert core[0] == groups
+    assert (core[1:] == deg).all() and largest == deg
+    assert sol.max_core == deg and sol.peel_levels == 2
