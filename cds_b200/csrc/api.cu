@@ -536,7 +536,7 @@ cds_status cds_components(cds_ctx *c, cds_graph *g, uint32_t k, uint64_t *core_c
     PeelOut pe;
     peel(c, s, u.off, u.adj, u.nnz, dag, cl, u.inst, 0, pe);
     CoreOut co;
-    densest_core_and_components(c, s, dag, pe, u.inst, k, c->tune[k], co, true);
+    densest_core_and_components(c, s, dag, pe, u.inst, k, c->tune[k], co);
     CDS_CUDA(cudaStreamSynchronize(s));
     if (core_cliques) *core_cliques = co.core_cliques[0];
     if (pruned_edges) *pruned_edges = co.pruned_edges[0];

@@ -37,21 +37,32 @@ __device__ __forceinline__ uint32_t inst_of(const uint32_t *of_vertex, uint32_t 
 
 // Grid-stride loops below step whole warps (base is warp-uniform), because
 // the warp-aggregated atomics need all 32 lanes.
-__global__ void k_core_flags(const uint32_t *__restrict__ core, uint32_t n,
+__global__ void k_core_flags(const uint32_t *__restrict__ core, const uint32_t *__restrict__ roots, uint32_t n,
                              const uint32_t *__restrict__ of_vertex,
-                             const unsigned long long *__restrict__ kp, uint8_t *__restrict__ in_core,
-                             unsigned long long *__restrict__ core_size) {
+                             const unsigned long long *__restrict__ kp, uint32_t *__restrict__ in_core,
+                             unsigned long long *__restrict__ core_size,
+                             unsigned long long *__restrict__ core_cliques) {
   for (uint32_t b = blockIdx.x * blockDim.x; b < n; b += gridDim.x * blockDim.x) {
     const uint32_t v = b + threadIdx.x;
-    uint32_t i = 0;
+    uint32_t i = 0, r = 0;
     bool in = false;
     if (v < n) {
       i = inst_of(of_vertex, v);
       const unsigned long long t = kp[i];
       in = t > 0 && (unsigned long long)core[v] >= t;
       in_core[v] = in;
+      r = in ? roots[v] : 0u;  // a clique is in the core when its first member is
     }
     agg_add_u64(core_size, i, in);
+    const uint32_t on = __ballot_sync(CDS_FULL, r != 0);
+    if (!on) continue;
+    const uint32_t i0 = __shfl_sync(CDS_FULL, i, __ffs(on) - 1);
+    if (__all_sync(CDS_FULL, r == 0 || i == i0)) {
+      const unsigned long long sum = warp_sum((unsigned long long)r);
+      if (lane_id() == 0) atomicAdd(&core_cliques[i0], sum);
+    } else if (r) {
+      atomicAdd(&core_cliques[i], (unsigned long long)r);
+    }
   }
 }
 
@@ -59,7 +70,7 @@ __global__ void k_core_flags(const uint32_t *__restrict__ core, uint32_t n,
 // (ids as they are; other vertices get empty lists).  Warp per vertex, lists
 // ascending and padded as the DAG's.
 __global__ void k_core_outdeg(const uint64_t *__restrict__ doff, const uint32_t *__restrict__ dadj,
-                              const uint32_t *__restrict__ outdeg, const uint8_t *__restrict__ in_core, uint32_t n,
+                              const uint32_t *__restrict__ outdeg, const uint32_t *__restrict__ in_core, uint32_t n,
                               uint32_t *__restrict__ cout) {
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
   for (uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < n; u += warps) {
@@ -71,7 +82,7 @@ __global__ void k_core_outdeg(const uint64_t *__restrict__ doff, const uint32_t 
   }
 }
 __global__ void k_core_dag(const uint64_t *__restrict__ doff, const uint32_t *__restrict__ dadj,
-                           const uint32_t *__restrict__ outdeg, const uint8_t *__restrict__ in_core, uint32_t n,
+                           const uint32_t *__restrict__ outdeg, const uint32_t *__restrict__ in_core, uint32_t n,
                            const uint64_t *__restrict__ coff, uint32_t *__restrict__ cadj) {
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
   for (uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < n; u += warps) {
@@ -89,13 +100,6 @@ __global__ void k_core_dag(const uint64_t *__restrict__ doff, const uint32_t *__
     for (uint64_t i = at + lane_id(); i < end; i += 32) cadj[i] = NONE;
   }
 }
-// cliques of each instance, from the listing's offsets
-__global__ void k_inst_cliques(const uint64_t *__restrict__ base, const uint32_t *__restrict__ vbeg, uint32_t ninst,
-                               unsigned long long *__restrict__ out) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < ninst; i += gridDim.x * blockDim.x)
-    out[i] = base[vbeg[i + 1]] - base[vbeg[i]];
-}
-
 // arc u -> w of the DAG (w in the out-list of u), or NONE
 __device__ __forceinline__ uint64_t find_arc(const uint64_t *doff, const uint32_t *dadj,
                                              const uint32_t *outdeg, uint32_t u, uint32_t w) {
@@ -124,21 +128,94 @@ __global__ void k_mark_arcs(const uint32_t *__restrict__ members, uint64_t m, ui
   }
 }
 
-// Small cores (at most PAIR_CORE_MAX vertices in all): the pairs that core
-// cliques cover are marked in a bitmap over core-local ids -- a read, and an
-// atomic only for a bit not yet set -- instead of a binary search for each
-// of a clique's k(k-1)/2 arcs; a dense core's cliques share their pairs
-// thousands of times over.  Then every DAG arc between core vertices looks
-// its pair up.
+// Small cores (at most PAIR_CORE_MAX vertices in all): adjacency and the pairs
+// that core cliques cover are bitmaps over core-local ids.  For k <= 5 a pair is
+// tested on the adjacency rows alone (does a clique of the k-2 other members fit
+// into the common neighbours?), which in a dense core the first candidate answers;
+// for larger k the listed cliques mark their pairs.
 constexpr uint32_t PAIR_CORE_MAX = 4096;
 
-// core-local ids in vertex order: f[v] = in_core[v], scanned into lid, and
-// the inverse core_vertex[lid] = v (so the smallest id of a set of core
-// vertices is its smallest vertex)
-__global__ void k_core_u32(const uint8_t *__restrict__ in_core, uint32_t n, uint32_t *__restrict__ f) {
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) f[v] = in_core[v];
+__global__ void k_core_bits(const uint64_t *__restrict__ doff, const uint32_t *__restrict__ dadj,
+                            const uint32_t *__restrict__ outdeg, const uint32_t *__restrict__ in_core,
+                            const uint64_t *__restrict__ lid, const uint32_t *__restrict__ core_vertex,
+                            uint32_t ncore, uint32_t words, uint32_t *__restrict__ adj) {
+  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+  for (uint32_t a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; a < ncore; a += warps) {
+    const uint32_t u = core_vertex[a], d = outdeg[u];
+    for (uint32_t t = lane_id(); t < d; t += 32) {
+      const uint32_t w = dadj[doff[u] + t];
+      if (!in_core[w]) continue;
+      const uint32_t b = (uint32_t)lid[w];
+      atomicOr(adj + (size_t)a * words + (b >> 5), 1u << (b & 31));
+      atomicOr(adj + (size_t)b * words + (a >> 5), 1u << (a & 31));
+    }
+  }
 }
-__global__ void k_core_vertex(const uint8_t *__restrict__ in_core, const uint64_t *__restrict__ lid, uint32_t n,
+
+// is there a D-clique among the vertices of mask M (words lane, lane + 32, ...)?
+template <int D>
+__device__ bool clique_in(const uint32_t (&M)[PAIR_CORE_MAX / 1024], const uint32_t *adj, uint32_t words) {
+  constexpr uint32_t Q = PAIR_CORE_MAX / 1024;
+  if constexpr (D == 0) {
+    return true;
+  } else if constexpr (D == 1) {
+    uint32_t any = 0;
+#pragma unroll
+    for (uint32_t q = 0; q < Q; q++) any |= M[q];
+    return __any_sync(CDS_FULL, any != 0);
+  } else {
+#pragma unroll
+    for (uint32_t q = 0; q < Q; q++)
+      for (uint32_t on = __ballot_sync(CDS_FULL, M[q] != 0); on; on &= on - 1) {
+        const uint32_t l = __ffs(on) - 1;
+        for (uint32_t m = __shfl_sync(CDS_FULL, M[q], l); m; m &= m - 1) {
+          const uint32_t j = (q * 32 + l) * 32 + __ffs(m) - 1;
+          uint32_t N[Q];
+#pragma unroll
+          for (uint32_t x = 0; x < Q; x++) {
+            const uint32_t w = x * 32 + lane_id();
+            N[x] = w < words ? M[x] & adj[(size_t)j * words + w] : 0u;
+          }
+          if (clique_in<D - 1>(N, adj, words)) return true;
+        }
+      }
+    return false;
+  }
+}
+
+// bits: the covered pairs a < b; pairs counted per instance.  Warp per row word.
+template <int K>
+__global__ void k_cover(const uint32_t *__restrict__ adj, uint32_t words, uint32_t ncore,
+                        const uint32_t *__restrict__ core_vertex, const uint32_t *__restrict__ of_vertex,
+                        uint32_t *__restrict__ bits, unsigned long long *__restrict__ pairs) {
+  constexpr uint32_t Q = PAIR_CORE_MAX / 1024;
+  const uint32_t warps = (gridDim.x * blockDim.x) >> 5, total = ncore * words;
+  for (uint32_t x = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; x < total; x += warps) {
+    const uint32_t a = x / words, w0 = x % words;
+    uint32_t m = adj[x], out = 0;
+    if (w0 < (a >> 5)) m = 0;
+    else if (w0 == (a >> 5)) m &= ~((2u << (a & 31)) - 1u);
+    for (uint32_t r = m; r; r &= r - 1) {
+      const uint32_t b = w0 * 32 + __ffs(r) - 1;
+      uint32_t M[Q];
+#pragma unroll
+      for (uint32_t q = 0; q < Q; q++) {
+        const uint32_t w = q * 32 + lane_id();
+        M[q] = w < words ? adj[(size_t)a * words + w] & adj[(size_t)b * words + w] : 0u;
+      }
+      if (clique_in<K - 2>(M, adj, words)) out |= r & (0u - r);
+    }
+    if (lane_id() == 0) {
+      bits[x] = out;
+      if (out) atomicAdd(&pairs[inst_of(of_vertex, core_vertex[a])], (unsigned long long)__popc(out));
+    }
+  }
+}
+
+// core-local ids in vertex order: in_core scanned into lid, and the inverse
+// core_vertex[lid] = v (so the smallest id of a set of core vertices is its
+// smallest vertex)
+__global__ void k_core_vertex(const uint32_t *__restrict__ in_core, const uint64_t *__restrict__ lid, uint32_t n,
                               uint32_t *__restrict__ core_vertex) {
   for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
     if (in_core[v]) core_vertex[lid[v]] = v;
@@ -193,7 +270,7 @@ __global__ void __launch_bounds__(1024) k_small_components(const uint32_t *__res
   }
 }
 
-__global__ void k_comp_from_roots(const uint8_t *__restrict__ in_core, const uint64_t *__restrict__ lid,
+__global__ void k_comp_from_roots(const uint32_t *__restrict__ in_core, const uint64_t *__restrict__ lid,
                                   const uint32_t *__restrict__ root, const uint32_t *__restrict__ core_vertex,
                                   uint32_t n, uint32_t *__restrict__ comp) {
   for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
@@ -230,7 +307,7 @@ __global__ void k_mark_pairs(const uint32_t *__restrict__ members, uint64_t m, u
 }
 
 __global__ void k_pairs_to_arcs(const uint64_t *__restrict__ doff, const uint32_t *__restrict__ dadj,
-                                const uint32_t *__restrict__ outdeg, const uint8_t *__restrict__ in_core,
+                                const uint32_t *__restrict__ outdeg, const uint32_t *__restrict__ in_core,
                                 const uint64_t *__restrict__ lid, uint32_t n, uint32_t words,
                                 const uint32_t *__restrict__ bits, uint8_t *__restrict__ arc_keep) {
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
@@ -297,23 +374,25 @@ __global__ void k_union(const uint64_t *__restrict__ doff, const uint32_t *__res
   }
 }
 
-__global__ void k_roots(uint32_t *parent, const uint8_t *__restrict__ in_core, uint32_t n,
+__global__ void k_roots(uint32_t *parent, const uint32_t *__restrict__ in_core, uint32_t n,
                         uint32_t *__restrict__ comp) {
   for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
     comp[v] = in_core[v] ? uf_find(parent, v) : NONE;
 }
 
-// Core cliques per component: every core clique lies in its root's component.
-__global__ void k_comp_cliques(const uint64_t *__restrict__ base, uint32_t n, const uint32_t *__restrict__ comp,
+// Core cliques per component: every core clique lies in its first member's.
+__global__ void k_comp_cliques(const uint32_t *__restrict__ roots, uint32_t n, const uint32_t *__restrict__ comp,
                                unsigned long long *__restrict__ ccount) {
   for (uint32_t b = blockIdx.x * blockDim.x; b < n; b += gridDim.x * blockDim.x) {
     const uint32_t u = b + threadIdx.x;
-    const unsigned long long c = u < n ? base[u + 1] - base[u] : 0ull;
-    const uint32_t r = c ? comp[u] : NONE;
-    const uint32_t r0 = __shfl_sync(CDS_FULL, r, __ffs(__ballot_sync(CDS_FULL, c != 0) | 0x80000000u) - 1);
+    const uint32_t r = u < n ? comp[u] : NONE;
+    const unsigned long long c = r != NONE ? roots[u] : 0ull;
+    const uint32_t on = __ballot_sync(CDS_FULL, c != 0);
+    if (!on) continue;
+    const uint32_t r0 = __shfl_sync(CDS_FULL, r, __ffs(on) - 1);
     if (__all_sync(CDS_FULL, c == 0 || r == r0)) {  // one component in the warp, mostly
       const unsigned long long sum = warp_sum(c);
-      if (lane_id() == 0 && sum) atomicAdd(&ccount[r0], sum);
+      if (lane_id() == 0) atomicAdd(&ccount[r0], sum);
     } else if (c) {
       atomicAdd(&ccount[r], c);
     }
@@ -392,7 +471,7 @@ constexpr uint32_t SMALL_NV = 2048;
 // its slots with one atomic; otherwise each warp takes its own.
 __global__ void k_bucket_cliques(const uint32_t *__restrict__ members, uint64_t m, uint32_t k,
                                  const uint32_t *__restrict__ comp, const uint64_t *__restrict__ cidx,
-                                 const uint64_t *__restrict__ cbeg,
+                                 const uint8_t *__restrict__ open, const uint64_t *__restrict__ cbeg,
                                  unsigned long long *__restrict__ ccur, const uint32_t *__restrict__ local,
                                  uint32_t nv, uint32_t *__restrict__ rec, uint32_t *__restrict__ ldeg) {
   __shared__ uint32_t s_lo, s_hi;
@@ -405,9 +484,10 @@ __global__ void k_bucket_cliques(const uint32_t *__restrict__ members, uint64_t 
   }
   for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x; b < m; b += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t c = b + threadIdx.x;
-    const bool in = c < m;
+    bool in = c < m;
     const uint32_t *r = members + (in ? c : 0) * k;
     const uint32_t ci = in ? (uint32_t)cidx[comp[r[0]]] : 0u;
+    in = in && open[ci];
     if (threadIdx.x == 0) {
       s_lo = 0xFFFFFFFFu;
       s_hi = 0;
@@ -541,9 +621,39 @@ __global__ void k_gather_roots(const uint32_t *__restrict__ is_root, const uint6
 
 namespace cds {
 
+namespace {
+
+// Every clique of the densest core, from the core's part of the DAG.
+void list_core_cliques(cds_ctx *c, cudaStream_t s, const Dag &gdag, uint32_t k, const Tuning &t, CoreOut &out,
+                       Dag &dag, const CountHook *on_count) {
+  const uint32_t n = gdag.n;
+  const int G = c->sm_count * 8;
+  dag.n = n;
+  dag.max_out = gdag.max_out;
+  dag.heavy = gdag.heavy;
+  dag.degree = gdag.degree;
+  dag.outdeg = DBuf<uint32_t>(c, s, n + 1);
+  dag.off = DBuf<uint64_t>(c, s, n + 1);
+  dag.adj = DBuf<uint32_t>(c, s, gdag.adj.n);
+  {
+    ProfScope ps(c, s, "core_dag");
+    if (n)
+      k_core_outdeg<<<G, 256, 0, s>>>(gdag.off.p, gdag.adj.p, gdag.outdeg.p, out.in_core.p, n, dag.outdeg.p);
+    scan_u32_pad4(dag.outdeg.p, dag.off.p, n, c, s);
+    if (n)
+      k_core_dag<<<G, 256, 0, s>>>(gdag.off.p, gdag.adj.p, gdag.outdeg.p, out.in_core.p, n, dag.off.p, dag.adj.p);
+    count_launch(2);
+    CDS_CUDA(cudaGetLastError());
+  }
+  list_cliques(c, s, dag, k, LIST_WRITE, t, out.cliques, on_count);
+  out.listed = true;
+}
+
+}  // namespace
+
 void densest_core_and_components(cds_ctx *c, cudaStream_t s, const Dag &gdag, const PeelOut &pe,
                                  const Instances &inst, uint32_t k, const Tuning &t, CoreOut &out,
-                                 bool need_networks, StageClock *clk, const CountHook *on_count) {
+                                 StageClock *clk, const CountHook *on_count) {
   const uint32_t n = gdag.n;
   const uint32_t ninst = inst.count;
   const uint32_t *of_vertex = ninst > 1 ? inst.of_vertex.p : nullptr;
@@ -555,104 +665,107 @@ void densest_core_and_components(cds_ctx *c, cudaStream_t s, const Dag &gdag, co
       out.threshold[i] = (pe.best_num[i] + pe.best_den[i] - 1) / pe.best_den[i];
   DBuf<unsigned long long> kp(c, s, ninst);
   CDS_CUDA(cudaMemcpyAsync(kp.p, out.threshold.data(), ninst * 8, cudaMemcpyHostToDevice, s));
-  DBuf<unsigned long long> stats(c, s, 4 * (size_t)ninst);  // core size, core cliques, arcs, comps
+  DBuf<unsigned long long> stats(c, s, 4 * (size_t)ninst);  // core size, core cliques, pairs, comps
   stats.zero();
-  DBuf<uint8_t> in_core(c, s, n + 1);
   DBuf<uint32_t> err(c, s, 1);
   err.zero();
-  Dag dag;  // of the core
-  dag.n = n;
-  dag.max_out = gdag.max_out;
-  dag.heavy = gdag.heavy;
-  dag.degree = gdag.degree;
-  dag.outdeg = DBuf<uint32_t>(c, s, n + 1);
-  dag.off = DBuf<uint64_t>(c, s, n + 1);
-  dag.adj = DBuf<uint32_t>(c, s, gdag.adj.n);
-  {
-    ProfScope ps(c, s, "core_dag");
-    if (n) {
-      k_core_flags<<<G, 256, 0, s>>>(pe.core.p, n, of_vertex, kp.p, in_core.p, stats.p);
-      k_core_outdeg<<<G, 256, 0, s>>>(gdag.off.p, gdag.adj.p, gdag.outdeg.p, in_core.p, n, dag.outdeg.p);
-    }
-    scan_u32_pad4(dag.outdeg.p, dag.off.p, n, c, s);
-    if (n)
-      k_core_dag<<<G, 256, 0, s>>>(gdag.off.p, gdag.adj.p, gdag.outdeg.p, in_core.p, n, dag.off.p, dag.adj.p);
-    count_launch(3);
+  out.in_core = DBuf<uint32_t>(c, s, n + 1);
+  const DBuf<uint32_t> &in_core = out.in_core;
+  if (n) {
+    ProfScope ps(c, s, "core_flags");
+    k_core_flags<<<G, 256, 0, s>>>(pe.core.p, pe.roots.p, n, of_vertex, kp.p, in_core.p, stats.p, stats.p + ninst);
+    count_launch();
     CDS_CUDA(cudaGetLastError());
   }
-  // its cliques, the only ones that are ever written
-  Cliques cl;
-  list_cliques(c, s, dag, k, LIST_WRITE, t, cl, on_count);
-  const uint64_t m = cl.count;
-  k_inst_cliques<<<std::max(1u, (ninst + 255) / 256), 256, 0, s>>>(cl.base.p, inst.vbeg.p, ninst, stats.p + ninst);
-  count_launch();
-  CDS_CUDA(cudaGetLastError());
   if (clk) out.mk_core = clk->mark();
 
-  // prune: arcs inside >= 1 core clique
-  uint64_t ncore = 0;
+  // prune: pairs inside >= 1 core clique
+  uint64_t ncore = 0, m = 0;
   {
-    std::vector<unsigned long long> h(ninst);
+    std::vector<unsigned long long> h(2 * (size_t)ninst);
     HostReads r(s);
-    r.add(h.data(), stats.p, ninst);
+    r.add(h.data(), stats.p, h.size());
     r.wait();
-    for (auto x : h) ncore += x;
+    for (uint32_t i = 0; i < ninst; i++) {
+      ncore += h[i];
+      m += h[ninst + i];
+    }
   }
-  DBuf<uint8_t> keep(c, s, dag.adj.n + 1);
-  const bool small_core = m && n && ncore <= PAIR_CORE_MAX;
-  const uint32_t words = (uint32_t)((ncore + 31) / 32);
-  DBuf<uint64_t> lid(c, s, small_core ? n + 1 : 0);
-  DBuf<uint32_t> core_vertex(c, s, small_core ? ncore + 1 : 0), bits(c, s, small_core ? ncore * words + 1 : 0);
+  const bool bitmap = m && n && ncore <= PAIR_CORE_MAX;  // marks over core-local ids
+  out.small = bitmap && k <= 5;                          // ... found on the adjacency alone
+  out.ncore = (uint32_t)ncore;
+  out.words = (uint32_t)((ncore + 31) / 32);
+  const uint32_t words = out.words;
+  DBuf<uint64_t> lid(c, s, bitmap ? n + 1 : 0);
+  DBuf<uint8_t> keep(c, s, 0);
+  Dag dag;  // of the core, when its cliques are listed
+  if (m && !out.small) list_core_cliques(c, s, gdag, k, t, out, dag, on_count);
   {
-    keep.zero();
     ProfScope ps(c, s, "prune_arcs");
-    if (small_core) {
-      {
-        DBuf<uint32_t> f(c, s, n + 1);
-        k_core_u32<<<G, 256, 0, s>>>(in_core.p, n, f.p);
-        scan_u32(f.p, lid.p, n, c, s);
-      }
-      bits.zero();
-      k_core_vertex<<<G, 256, 0, s>>>(in_core.p, lid.p, n, core_vertex.p);
-      k_mark_pairs<<<G, 256, 0, s>>>(cl.members.p, m, k, lid.p, words, bits.p);
-      k_pairs_to_arcs<<<G, 256, 0, s>>>(dag.off.p, dag.adj.p, dag.outdeg.p, in_core.p, lid.p, n, words, bits.p,
-                                        keep.p);
-      count_launch(4);
-    } else if (m) {
-      k_mark_arcs<<<G, 256, 0, s>>>(cl.members.p, m, k, dag.off.p, dag.adj.p, dag.outdeg.p, keep.p,
-                                    err.p);
+    if (bitmap) {
+      out.core_vertex = DBuf<uint32_t>(c, s, ncore + 1);
+      out.bits = DBuf<uint32_t>(c, s, ncore * words + 1);
+      scan_u32(in_core.p, lid.p, n, c, s);
+      k_core_vertex<<<G, 256, 0, s>>>(in_core.p, lid.p, n, out.core_vertex.p);
       count_launch();
     }
-    if (n) k_count_arcs<<<G, 256, 0, s>>>(dag.off.p, dag.outdeg.p, keep.p, n, of_vertex, stats.p + 2 * ninst);
-    count_launch();
+    if (out.small) {
+      DBuf<uint32_t> adj(c, s, ncore * words + 1);
+      adj.zero();
+      k_core_bits<<<G, 256, 0, s>>>(gdag.off.p, gdag.adj.p, gdag.outdeg.p, in_core.p, lid.p, out.core_vertex.p,
+                                    (uint32_t)ncore, words, adj.p);
+      void (*cover)(const uint32_t *, uint32_t, uint32_t, const uint32_t *, const uint32_t *, uint32_t *,
+                    unsigned long long *) = k == 2 ? k_cover<2> : k == 3 ? k_cover<3> : k == 4 ? k_cover<4> : k_cover<5>;
+      cover<<<G, 256, 0, s>>>(adj.p, words, (uint32_t)ncore, out.core_vertex.p, of_vertex, out.bits.p,
+                              stats.p + 2 * ninst);
+      count_launch(2);
+    } else if (m) {
+      keep.alloc(dag.adj.n + 1);
+      keep.zero();
+      const Cliques &cl = out.cliques;
+      if (bitmap) {
+        out.bits.zero();
+        k_mark_pairs<<<G, 256, 0, s>>>(cl.members.p, m, k, lid.p, words, out.bits.p);
+        k_pairs_to_arcs<<<G, 256, 0, s>>>(dag.off.p, dag.adj.p, dag.outdeg.p, in_core.p, lid.p, n, words, out.bits.p,
+                                          keep.p);
+        count_launch();
+      } else {
+        k_mark_arcs<<<G, 256, 0, s>>>(cl.members.p, m, k, dag.off.p, dag.adj.p, dag.outdeg.p, keep.p, err.p);
+      }
+      k_count_arcs<<<G, 256, 0, s>>>(dag.off.p, dag.outdeg.p, keep.p, n, of_vertex, stats.p + 2 * ninst);
+      count_launch(2);
+    }
     CDS_CUDA(cudaGetLastError());
   }
   if (clk) out.mk_prune = clk->mark();
 
   // components
-  DBuf<uint32_t> parent(c, s, n + 1), comp(c, s, n + 1);
+  out.comp = DBuf<uint32_t>(c, s, n + 1);
+  out.cidx = DBuf<uint64_t>(c, s, n + 1);
+  const DBuf<uint32_t> &comp = out.comp;
+  const DBuf<uint64_t> &cidx = out.cidx;
+  DBuf<uint32_t> parent(c, s, bitmap ? 0 : n + 1), is_root(c, s, n + 1);
   DBuf<unsigned long long> ccount(c, s, n + 1);  // core cliques per component root (may pass 2^32)
-  if (n) {
-    k_iota<<<G, 256, 0, s>>>(parent.p, n);
-    count_launch();
-  }
   ccount.zero();
-  DBuf<uint32_t> is_root(c, s, n + 1);
-  DBuf<uint64_t> cidx(c, s, n + 1);
   {
     ProfScope ps_cc(c, s, "components_unionfind");
-    if (small_core) {
+    if (bitmap) {
       DBuf<uint32_t> root(c, s, ncore + 1);
-      k_small_components<<<1, 1024, 0, s>>>(bits.p, words, (uint32_t)ncore, root.p, err.p);
-      k_comp_from_roots<<<G, 256, 0, s>>>(in_core.p, lid.p, root.p, core_vertex.p, n, comp.p);
+      k_small_components<<<1, 1024, 0, s>>>(out.bits.p, words, (uint32_t)ncore, root.p, err.p);
+      k_comp_from_roots<<<G, 256, 0, s>>>(in_core.p, lid.p, root.p, out.core_vertex.p, n, comp.p);
+      count_launch(2);
     } else if (n) {
-      k_union<<<G, 256, 0, s>>>(dag.off.p, dag.adj.p, dag.outdeg.p, keep.p, n, parent.p, err.p);
+      k_iota<<<G, 256, 0, s>>>(parent.p, n);
+      if (m) k_union<<<G, 256, 0, s>>>(dag.off.p, dag.adj.p, dag.outdeg.p, keep.p, n, parent.p, err.p);
       k_roots<<<G, 256, 0, s>>>(parent.p, in_core.p, n, comp.p);
+      count_launch(3);
     }
-    if (n) k_comp_cliques<<<G, 256, 0, s>>>(cl.base.p, n, comp.p, ccount.p);
-    if (n) k_root_flags<<<G, 256, 0, s>>>(comp.p, ccount.p, n, of_vertex, is_root.p, stats.p + 3 * ninst);
+    if (n) {
+      k_comp_cliques<<<G, 256, 0, s>>>(pe.roots.p, n, comp.p, ccount.p);
+      k_root_flags<<<G, 256, 0, s>>>(comp.p, ccount.p, n, of_vertex, is_root.p, stats.p + 3 * ninst);
+      count_launch(2);
+    }
   }
-  count_launch(4);
   CDS_CUDA(cudaGetLastError());
   scan_u32(is_root.p, cidx.p, n, c, s);
   // one wait for the component count, the per-instance statistics and the status
@@ -681,7 +794,7 @@ void densest_core_and_components(cds_ctx *c, cudaStream_t s, const Dag &gdag, co
   out.comp_cbeg.assign(ncomp + 1, 0);
   out.comp_maxcore.assign(ncomp, 0);
   out.comp_root.assign(ncomp, 0);
-  if (!need_networks || ncomp == 0) return;
+  if (ncomp == 0) return;
   DBuf<uint32_t> csize(c, s, ncomp), cmax(c, s, ncomp), roots(c, s, ncomp);
   DBuf<unsigned long long> cclq(c, s, ncomp);
   csize.zero();
@@ -689,60 +802,75 @@ void densest_core_and_components(cds_ctx *c, cudaStream_t s, const Dag &gdag, co
   cmax.zero();
   k_comp_sizes<<<G, 256, 0, s>>>(comp.p, cidx.p, ccount.p, n, csize.p, cclq.p, pe.core.p, cmax.p);
   k_gather_roots<<<G, 256, 0, s>>>(is_root.p, cidx.p, n, roots.p);
-  count_launch(2);
-  CDS_CUDA(cudaGetLastError());
-  DBuf<uint64_t> vbeg(c, s, ncomp + 1), cbeg(c, s, ncomp + 1);
+  DBuf<uint64_t> vbeg(c, s, ncomp + 1);
   scan_u32(csize.p, vbeg.p, ncomp, c, s);
-  scan_u64(reinterpret_cast<const uint64_t *>(cclq.p), cbeg.p, ncomp, c, s);
-  std::vector<uint64_t> hv(ncomp + 1), hc(ncomp + 1);
-  std::vector<uint32_t> hroots(ncomp);
+  // local ids: component by component (at most ncore of them)
+  out.vmap = DBuf<uint32_t>(c, s, ncore + 1);
+  out.vcnet = DBuf<uint32_t>(c, s, ncore + 1);
+  out.local = DBuf<uint32_t>(c, s, n + 1);
+  DBuf<uint32_t> vcur(c, s, ncomp);
+  vcur.zero();
+  k_local_ids<<<G, 256, 0, s>>>(comp.p, cidx.p, ccount.p, n, vbeg.p, vcur.p, out.local.p, out.vmap.p, out.vcnet.p);
+  count_launch(3);
+  CDS_CUDA(cudaGetLastError());
+  std::vector<uint64_t> hv(ncomp + 1);
+  std::vector<unsigned long long> hc(ncomp);
   {
     HostReads r(s);
     r.add(hv.data(), vbeg.p, ncomp + 1);
-    r.add(hc.data(), cbeg.p, ncomp + 1);
+    r.add(hc.data(), cclq.p, ncomp);
     r.add(out.comp_maxcore.data(), cmax.p, ncomp);
-    r.add(hroots.data(), roots.p, ncomp);
+    r.add(out.comp_root.data(), roots.p, ncomp);
     r.wait();
   }
-  for (uint32_t i = 0; i <= ncomp; i++) {
-    out.comp_vbeg[i] = (uint32_t)hv[i];
-    out.comp_cbeg[i] = hc[i];
-  }
-  out.comp_root = hroots;
   for (uint32_t i = 0; i < ncomp; i++) {
-    uint32_t r = hroots[i], ii = 0;
+    out.comp_vbeg[i + 1] = (uint32_t)hv[i + 1];
+    out.comp_cbeg[i + 1] = out.comp_cbeg[i] + hc[i];
     // instance of the root: binary search in the instance table
-    ii = (uint32_t)(std::upper_bound(inst.h_vbeg.begin(), inst.h_vbeg.end(), r) - inst.h_vbeg.begin()) - 1;
-    out.comp_inst[i] = ii;
+    out.comp_inst[i] = (uint32_t)(std::upper_bound(inst.h_vbeg.begin(), inst.h_vbeg.end(), out.comp_root[i]) -
+                                  inst.h_vbeg.begin()) - 1;
   }
-  const uint32_t nv = (uint32_t)hv[ncomp];
-  const uint64_t nc = hc[ncomp];
-  out.vmap.c = out.rec.c = out.vcnet.c = out.vinc_off.c = out.vinc.c = c;
-  out.vmap.s = out.rec.s = out.vcnet.s = out.vinc_off.s = out.vinc.s = s;
-  out.vmap.alloc(nv + 1);
-  out.vcnet.alloc(nv + 1);
-  out.rec.alloc((nc << rec_shift(k)) + 1);
-  DBuf<uint32_t> local(c, s, n + 1), vcur(c, s, ncomp), ldeg(c, s, nv + 1);
+}
+
+void build_networks(cds_ctx *c, cudaStream_t s, const Dag &gdag, const Instances &inst, uint32_t k,
+                    const Tuning &t, CoreOut &out, const std::vector<uint8_t> &open, const CountHook *on_count) {
+  (void)inst;
+  const uint32_t ncomp = out.ncomp, nv = out.comp_vbeg[ncomp];
+  const int G = c->sm_count * 8;
+  if (!out.listed) {
+    Dag dag;
+    list_core_cliques(c, s, gdag, k, t, out, dag, on_count);
+  }
+  const uint64_t m = out.cliques.count;
+  std::vector<uint64_t> hc(ncomp + 1, 0);  // first clique of each component's network
+  for (uint32_t i = 0; i < ncomp; i++)
+    hc[i + 1] = hc[i] + (open[i] ? out.comp_cbeg[i + 1] - out.comp_cbeg[i] : 0);
+  const uint64_t nc = out.nc = hc[ncomp];
+  DBuf<uint64_t> cbeg(c, s, ncomp + 1);
+  DBuf<uint8_t> d_open(c, s, ncomp);
+  CDS_CUDA(cudaMemcpyAsync(cbeg.p, hc.data(), (ncomp + 1) * 8, cudaMemcpyHostToDevice, s));
+  CDS_CUDA(cudaMemcpyAsync(d_open.p, open.data(), ncomp, cudaMemcpyHostToDevice, s));
+  out.rec = DBuf<uint32_t>(c, s, (nc << rec_shift(k)) + 1);
+  DBuf<uint32_t> ldeg(c, s, nv + 1);
   DBuf<unsigned long long> ccur(c, s, ncomp);
-  vcur.zero();
   ccur.zero();
   ldeg.zero();
-  {
+  if (m) {
     ProfScope ps_b(c, s, "components_bucket");
-    k_local_ids<<<G, 256, 0, s>>>(comp.p, cidx.p, ccount.p, n, vbeg.p, vcur.p, local.p, out.vmap.p,
-                                 out.vcnet.p);
-    if (m) k_bucket_cliques<<<G, 256, 0, s>>>(cl.members.p, m, k, comp.p, cidx.p, cbeg.p,
-                                             ccur.p, local.p, nv, out.rec.p, ldeg.p);
+    k_bucket_cliques<<<G, 256, 0, s>>>(out.cliques.members.p, m, k, out.comp.p, out.cidx.p, d_open.p, cbeg.p,
+                                       ccur.p, out.local.p, nv, out.rec.p, ldeg.p);
+    count_launch();
+    CDS_CUDA(cudaGetLastError());
   }
-  count_launch(2);
-  CDS_CUDA(cudaGetLastError());
-  out.vinc_off.alloc(nv + 1);
+  out.cliques.members.release();
+  out.listed = false;
+  out.vinc_off = DBuf<uint64_t>(c, s, nv + 1);
   scan_u32(ldeg.p, out.vinc_off.p, nv, c, s);
   out.flows_zero = true;
   // each vertex's cliques as u32 record indices while they fit, else u64
   // (two words each); the vertex's slot in a record is found by matching
   out.vinc_wide = nc >= 0xFFFFFFFFull || (c->flags & CDS_CONFIG_WIDE_FLOW);
-  out.vinc.alloc(nc * k * (out.vinc_wide ? 2 : 1) + 2);
+  out.vinc = DBuf<uint32_t>(c, s, nc * k * (out.vinc_wide ? 2 : 1) + 2);
   {
     ProfScope ps_v(c, s, "components_vinc");
     DBuf<uint32_t> cur(c, s, nv + 1);

@@ -48,8 +48,9 @@ __global__ void k_outdeg(const uint64_t *__restrict__ off, const uint32_t *__res
 // Heavy vertices: all of the graph, or the ones of largest degree.  Degrees are
 // binned on a log scale, sixteen bins an octave, and the heavy ones are those
 // from the lowest bin on at and above which at most `cap` vertices lie: a degree
-// threshold, so that no DAG arc leaves the set.  bins[512] is left holding the
-// threshold bin, bins[513] counts the ids given out.
+// threshold, so that no DAG arc leaves the set.  Ids go by descending bin, so that the
+// columns that the densest neighbourhoods touch lie together in every row.  bins[i] is
+// left holding the next id of bin i, bins[512] the threshold bin.
 constexpr uint32_t DEG_BINS = 512;
 __device__ __forceinline__ uint32_t deg_bin(uint32_t d) {
   if (d < 16) return d;
@@ -71,16 +72,16 @@ __global__ void __launch_bounds__(DEG_BINS) k_heavy_bin(uint32_t *__restrict__ b
   uint32_t total;
   const uint32_t x = bins[b], above_b = block_exclusive_scan<uint32_t>(x, &total);
   const int ok = __syncthreads_count(above_b + x <= cap);  // a prefix of the threads
-  if (threadIdx.x == 0) {
-    bins[DEG_BINS] = DEG_BINS - (uint32_t)ok;
-    bins[DEG_BINS + 1] = 0;
-  }
+  bins[b] = above_b;
+  if (threadIdx.x == 0) bins[DEG_BINS] = DEG_BINS - (uint32_t)ok;
 }
 __global__ void k_heavy_ids(const uint32_t *__restrict__ deg, uint32_t n, uint32_t *__restrict__ bins,
                             uint32_t *__restrict__ hid) {
   const uint32_t lo = bins[DEG_BINS];
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
-    hid[v] = deg_bin(deg[v]) >= lo ? atomicAdd(&bins[DEG_BINS + 1], 1u) : 0xFFFFFFFFu;
+  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+    const uint32_t b = deg_bin(deg[v]);
+    hid[v] = b >= lo ? atomicAdd(&bins[b], 1u) : 0xFFFFFFFFu;
+  }
 }
 
 // warp per vertex; writes the out-list in ascending id order plus padding, and

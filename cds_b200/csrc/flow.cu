@@ -533,10 +533,12 @@ __global__ void __launch_bounds__(512, 2) k_flow(FlowParams p) {
 // model tests gives these figures).
 constexpr uint32_t SPLIT_SMEM_NV = 4096;  // per-block load sums in shared memory up to here
 
-__global__ void k_split_init(FlowParams p, float *__restrict__ w) {
+// (known: weights that the balancing of certify.cu reached, 0 where it has none)
+__global__ void k_split_init(FlowParams p, const double *__restrict__ known, float *__restrict__ w) {
   for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < p.nv; v += gridDim.x * blockDim.x) {
     const uint64_t d = p.vinc_off[v + 1] - p.vinc_off[v];
-    w[v] = d ? 1.0f / (float)d : 1.0f;
+    const float x = known ? (float)known[v] : 0.0f;
+    w[v] = x > 0.0f ? x : d ? 1.0f / (float)d : 1.0f;
   }
 }
 
@@ -779,7 +781,8 @@ struct CompState {
 namespace cds {
 
 void exact_search(cds_ctx *c, cudaStream_t s, const CoreOut &co, const Instances &inst,
-                  uint32_t k, const cds_params &prm, const Tuning &t, FlowAnswer &ans) {
+                  uint32_t k, const cds_params &prm, const Tuning &t,
+                  const std::function<void(const std::vector<uint8_t> &)> &networks, FlowAnswer &ans) {
   const uint32_t ninst = inst.count;
   const uint32_t nnet = co.ncomp;
   ans.num.assign(ninst, 0);
@@ -794,7 +797,6 @@ void exact_search(cds_ctx *c, cudaStream_t s, const CoreOut &co, const Instances
   ans.comp_ub.assign(nnet, 0.0);
   if (nnet == 0) return;
   const uint32_t nv = co.comp_vbeg[nnet];
-  const uint64_t nc = co.comp_cbeg[nnet];
 
   // starting answer of every instance: its densest whole component (first on ties)
   std::vector<int64_t> best_n(ninst, 0), best_d(ninst, 0);
@@ -833,323 +835,352 @@ void exact_search(cds_ctx *c, cudaStream_t s, const CoreOut &co, const Instances
     ncand++;
   }
 
-  // flow state width: 32-bit when every probe's q keeps 2 q k^2 < 2^31 (q is
-  // a set size with Dinkelbach probes, at most n_c (n_c - 1) with bisection)
-  __int128 qbound = 1;
-  for (uint32_t i = 0; i < nnet; i++) {
-    const __int128 nci = (__int128)(co.comp_vbeg[i + 1] - co.comp_vbeg[i]);
-    qbound = std::max<__int128>(qbound, prm.search == 1 ? nci * std::max<__int128>(nci - 1, 1) : nci);
-  }
-  const bool x32_fits =
-      !(c->flags & CDS_CONFIG_WIDE_FLOW) && (__int128)2 * qbound * k * k < ((__int128)1 << 31);
-  FlowParams p{};
-  // 32-bit flow words live in the clique records; 64-bit ones in their own array
-  DBuf<long long> x(c, s, x32_fits ? 0 : nc * k + 1), ev(c, s, nv + 1), rt(c, s, nv + 1),
-      budget(c, s, nv + 1);
-  DBuf<int> d(c, s, nv + 1), dnew(c, s, nv + 1);
-  DBuf<uint8_t> sel(c, s, nv + 1), mark(c, s, nv + 1);
-  DBuf<long long> sink(c, s, nnet), P(c, s, nnet), Q(c, s, nnet);
-  DBuf<uint8_t> active(c, s, nnet), fin(c, s, nnet);
-  DBuf<uint32_t> ctl(c, s, F_WORDS + 1);
-  DBuf<GridBarrier> bar(c, s, 1);
-  DBuf<uint32_t> err(c, s, 1);
-  DBuf<unsigned long long> cut(c, s, 2 * (size_t)nnet);
-  DBuf<unsigned long long> bfsw(c, s, 4);
-  // warm start: T - 1 weight updates, then the split (t.flow_warm; < 0: by
-  // size, three for networks of a million cliques or more; 0: none)
-  const uint32_t T = (uint32_t)std::min(255, t.flow_warm < 0 ? (nc >= (1ull << 20) ? 3 : 0) : t.flow_warm);
-  DBuf<float> wgt(c, s, T ? nv + 1 : 0), wl(c, s, T ? nv + 1 : 0);
-  DBuf<unsigned long long> wload(c, s, T ? nv + 1 : 0);
-  bool wgt_init = false;
-  sel.zero();
-  mark.zero();
-  budget.zero();
-  const int threads = std::min(512, std::max(128, t.flow_block)) & ~31;  // whole warps
-  const uint64_t max_blocks = (uint64_t)c->sm_count * 2;
-  const size_t ev_bytes =
-      nv <= EV_SMEM_MAX && (uint64_t)nv * max_blocks * 8 <= nc * k ? (size_t)nv * 8 : 0;
-  int per_sm = 0;
-  {
-    int a = 0, b = 0;
-    CDS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_flow<int, uint64_t>, threads, ev_bytes));
-    CDS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_flow<long long, uint64_t>, threads, ev_bytes));
-    per_sm = std::min(a, b);
-  }
-  if (per_sm < 1) fail(CDS_ERR_CUDA, "flow kernel does not fit on an SM");
-  per_sm = std::min(per_sm, 2);
   const int G = c->sm_count * 4;
-  // the grid: the whole device, or (flow_inc_per_block) one block per that
-  // many incidences, at least 8 -- a barrier among fewer blocks is cheaper,
-  // which is what the many short phases of a small network wait on
-  unsigned blocks = coop_grid(c, per_sm);
-  if (t.flow_inc_per_block > 0) {
-    const uint64_t want = (nc * k + (uint64_t)t.flow_inc_per_block - 1) / (uint64_t)t.flow_inc_per_block;
-    blocks = (unsigned)std::max<uint64_t>(std::min<uint64_t>(8, blocks), std::min<uint64_t>(blocks, want));
-  }
-  // incidence lists cut into chunks, about four per warp of the grid
-  const uint64_t warps = (uint64_t)blocks * threads / 32;
-  uint32_t chunk = (uint32_t)std::min<uint64_t>(4096, std::max<uint64_t>(32, (nc * k) / (4 * warps + 1)));
-  chunk = (chunk + 31) & ~31u;
-  DBuf<uint32_t> nch(c, s, nv + 1);
-  DBuf<uint64_t> first(c, s, nv + 1);
-  k_chunk_count<<<G, 256, 0, s>>>(co.vinc_off.p, nv, chunk, nch.p);
-  count_launch();
-  scan_u32(nch.p, first.p, nv, c, s);
-  // sized by a bound (ceil(deg / chunk) <= deg / chunk + 1 per vertex), so
-  // nothing waits for the scan; the kernels read the count on the device
-  const uint64_t nchunks = (nc * k) / chunk + nv + 1;
-  if (nchunks >= 0xFFFFFFFFull) fail(CDS_ERR_OVERFLOW, "too many incidence chunks");
-  DBuf<uint32_t> chunk_v(c, s, nchunks + 1);
-  DBuf<uint64_t> chunk_beg(c, s, nchunks + 1);
-  k_chunk_fill<<<G, 256, 0, s>>>(co.vinc_off.p, nv, chunk, first.p, chunk_v.p, chunk_beg.p);
-  count_launch();
-  CDS_CUDA(cudaGetLastError());
-  p.nv = nv;
-  p.nc = nc;
-  p.k = k;
-  p.rec = co.rec.p;
-  p.S = rec_slots(k);
-  p.rs = rec_shift(k);
-  p.vinc_off = co.vinc_off.p;
-  p.vinc = co.vinc.p;
-  p.vcnet = co.vcnet.p;
-  p.chunk_v = chunk_v.p;
-  p.chunk_beg = chunk_beg.p;
-  p.nchunks = first.p + nv;
-  p.chunk = chunk;
-  p.x64 = x.p;
-  p.ev = ev.p;
-  p.rt = rt.p;
-  p.budget = budget.p;
-  p.d = d.p;
-  p.dnew = dnew.p;
-  p.sel = sel.p;
-  p.sink = sink.p;
-  p.P = P.p;
-  p.Q = Q.p;
-  p.active = active.p;
-  p.ctl = ctl.p;
-  p.bar = bar.p;
-  p.err = err.p;
-  p.spin_limit = 1ull << 24;
-  p.max_cycles = 1u << 20;
-  p.time_budget_ns = 120ull * 1000000000ull;
-  DBuf<unsigned long long> phase(c, s, 5);
-  phase.zero();
-  p.phase_ns = c->prof ? phase.p : nullptr;
-  p.rounds = (uint32_t)std::max(1, t.flow_rounds);
-  p.early_stop = prm.early_stop;
-  p.INF = (int)std::min<uint64_t>((uint64_t)nv + 2, 1u << 30);
-  p.ev_smem = ev_bytes ? 1u : 0u;
-  p.bfs = bfsw.p;
-
-  std::vector<long long> hP(nnet), hQ(nnet);
-  std::vector<uint8_t> hact(nnet), hfin(nnet);
-
-  bool fresh = co.flows_zero;  // record flow words untouched since they were built
-  co.flows_zero = false;
-  while (ncand) {
-    // choose the probe of every open network
+  DBuf<double> known;  // weights of components the proof gave up
+  DBuf<uint8_t> mark(c, s, nv + 1), fin(c, s, nnet);
+  mark.zero();
+  // Most components are their own densest set: where that can be proved without a
+  // network, the answer stands and no network is built.  (Flow options that were
+  // asked for are answered by the flows.)
+  if (ncand && prm.early_stop < 0 && t.flow_warm < 0 && !(c->flags & CDS_CONFIG_WIDE_FLOW)) {
+    std::vector<CertAsk> ask(nnet);
     for (uint32_t i = 0; i < nnet; i++) {
-      CompState &cs = st[i];
-      hact[i] = 0;
-      if (!cs.candidate || cs.done) continue;
-      const int64_t nci = (int64_t)(co.comp_vbeg[i + 1] - co.comp_vbeg[i]);
-      const int64_t mci = (int64_t)(co.comp_cbeg[i + 1] - co.comp_cbeg[i]);
-      cs.an = cs.lb_n;
-      cs.ad = cs.lb_d;
-      cs.certify = true;
-      if (prm.search == 1) {
-        // bisection on the grid j / D, D = n_c (n_c - 1), while a grid point
-        // lies strictly between the bounds and the scaled capacities fit
-        const int64_t D = nci * (nci - 1);
-        const bool fits = D > 0 && (__int128)D * k * mci < ((__int128)1 << 62);
-        if (fits && frac_lt(cs.lb_n, cs.lb_d, cs.ub_n, cs.ub_d)) {
-          // gap >= 1/D ?
-          const __int128 gap_num = (__int128)cs.ub_n * cs.lb_d - (__int128)cs.lb_n * cs.ub_d;
-          const __int128 gap_den = (__int128)cs.ub_d * cs.lb_d;
-          if (gap_num * D >= gap_den) {
-            const __int128 mid = ((__int128)cs.lb_n * cs.ub_d + (__int128)cs.ub_n * cs.lb_d) * D /
-                                 (2 * (__int128)cs.lb_d * cs.ub_d);
-            const int64_t j = (int64_t)mid;
-            if (frac_lt(cs.lb_n, cs.lb_d, j, D) && frac_lt(j, D, cs.ub_n, cs.ub_d)) {
-              cs.an = j;
-              cs.ad = D;
-              cs.certify = false;
+      if (!st[i].candidate) continue;
+      const int64_t g = gcd64(st[i].lb_n, st[i].lb_d);
+      ask[i] = {st[i].lb_n / g, st[i].lb_d / g};
+    }
+    std::vector<uint8_t> proven;
+    certify(c, s, co, k, ask, proven, known);
+    for (uint32_t i = 0; i < nnet; i++)
+      if (proven[i]) {
+        st[i].done = st[i].certify = true;
+        ncand--;
+        ans.flows = 1;  // an assignment that saturates the network, as one max-flow finds
+      }
+  }
+  if (ncand) {
+    std::vector<uint8_t> open(nnet);
+    for (uint32_t i = 0; i < nnet; i++) open[i] = st[i].candidate && !st[i].done;
+    networks(open);
+    ans.flows = 0;
+    const uint64_t nc = co.nc;
+    // flow state width: 32-bit when every probe's q keeps 2 q k^2 < 2^31 (q is
+    // a set size with Dinkelbach probes, at most n_c (n_c - 1) with bisection)
+    __int128 qbound = 1;
+    for (uint32_t i = 0; i < nnet; i++) {
+      const __int128 nci = (__int128)(co.comp_vbeg[i + 1] - co.comp_vbeg[i]);
+      qbound = std::max<__int128>(qbound, prm.search == 1 ? nci * std::max<__int128>(nci - 1, 1) : nci);
+    }
+    const bool x32_fits =
+        !(c->flags & CDS_CONFIG_WIDE_FLOW) && (__int128)2 * qbound * k * k < ((__int128)1 << 31);
+    FlowParams p{};
+    // 32-bit flow words live in the clique records; 64-bit ones in their own array
+    DBuf<long long> x(c, s, x32_fits ? 0 : nc * k + 1), ev(c, s, nv + 1), rt(c, s, nv + 1),
+        budget(c, s, nv + 1);
+    DBuf<int> d(c, s, nv + 1), dnew(c, s, nv + 1);
+    DBuf<uint8_t> sel(c, s, nv + 1);
+    DBuf<long long> sink(c, s, nnet), P(c, s, nnet), Q(c, s, nnet);
+    DBuf<uint8_t> active(c, s, nnet);
+    DBuf<uint32_t> ctl(c, s, F_WORDS + 1);
+    DBuf<GridBarrier> bar(c, s, 1);
+    DBuf<uint32_t> err(c, s, 1);
+    DBuf<unsigned long long> cut(c, s, 2 * (size_t)nnet);
+    DBuf<unsigned long long> bfsw(c, s, 4);
+    // warm start: T - 1 weight updates, then the split (t.flow_warm; < 0: the split
+    // alone from weights that are known, else by size, three for networks of a
+    // million cliques or more; 0: none)
+    const uint32_t T = (uint32_t)std::min(255, t.flow_warm >= 0 ? t.flow_warm : known.p ? 1 : nc >= (1ull << 20) ? 3 : 0);
+    DBuf<float> wgt(c, s, T ? nv + 1 : 0), wl(c, s, T ? nv + 1 : 0);
+    DBuf<unsigned long long> wload(c, s, T ? nv + 1 : 0);
+    bool wgt_init = false;
+    sel.zero();
+    budget.zero();
+    const int threads = std::min(512, std::max(128, t.flow_block)) & ~31;  // whole warps
+    const uint64_t max_blocks = (uint64_t)c->sm_count * 2;
+    const size_t ev_bytes =
+        nv <= EV_SMEM_MAX && (uint64_t)nv * max_blocks * 8 <= nc * k ? (size_t)nv * 8 : 0;
+    int per_sm = 0;
+    {
+      int a = 0, b = 0;
+      CDS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_flow<int, uint64_t>, threads, ev_bytes));
+      CDS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_flow<long long, uint64_t>, threads, ev_bytes));
+      per_sm = std::min(a, b);
+    }
+    if (per_sm < 1) fail(CDS_ERR_CUDA, "flow kernel does not fit on an SM");
+    per_sm = std::min(per_sm, 2);
+    // the grid: the whole device, or (flow_inc_per_block) one block per that
+    // many incidences, at least 8 -- a barrier among fewer blocks is cheaper,
+    // which is what the many short phases of a small network wait on
+    unsigned blocks = coop_grid(c, per_sm);
+    if (t.flow_inc_per_block > 0) {
+      const uint64_t want = (nc * k + (uint64_t)t.flow_inc_per_block - 1) / (uint64_t)t.flow_inc_per_block;
+      blocks = (unsigned)std::max<uint64_t>(std::min<uint64_t>(8, blocks), std::min<uint64_t>(blocks, want));
+    }
+    // incidence lists cut into chunks, about four per warp of the grid
+    const uint64_t warps = (uint64_t)blocks * threads / 32;
+    uint32_t chunk = (uint32_t)std::min<uint64_t>(4096, std::max<uint64_t>(32, (nc * k) / (4 * warps + 1)));
+    chunk = (chunk + 31) & ~31u;
+    DBuf<uint32_t> nch(c, s, nv + 1);
+    DBuf<uint64_t> first(c, s, nv + 1);
+    k_chunk_count<<<G, 256, 0, s>>>(co.vinc_off.p, nv, chunk, nch.p);
+    count_launch();
+    scan_u32(nch.p, first.p, nv, c, s);
+    // sized by a bound (ceil(deg / chunk) <= deg / chunk + 1 per vertex), so
+    // nothing waits for the scan; the kernels read the count on the device
+    const uint64_t nchunks = (nc * k) / chunk + nv + 1;
+    if (nchunks >= 0xFFFFFFFFull) fail(CDS_ERR_OVERFLOW, "too many incidence chunks");
+    DBuf<uint32_t> chunk_v(c, s, nchunks + 1);
+    DBuf<uint64_t> chunk_beg(c, s, nchunks + 1);
+    k_chunk_fill<<<G, 256, 0, s>>>(co.vinc_off.p, nv, chunk, first.p, chunk_v.p, chunk_beg.p);
+    count_launch();
+    CDS_CUDA(cudaGetLastError());
+    p.nv = nv;
+    p.nc = nc;
+    p.k = k;
+    p.rec = co.rec.p;
+    p.S = rec_slots(k);
+    p.rs = rec_shift(k);
+    p.vinc_off = co.vinc_off.p;
+    p.vinc = co.vinc.p;
+    p.vcnet = co.vcnet.p;
+    p.chunk_v = chunk_v.p;
+    p.chunk_beg = chunk_beg.p;
+    p.nchunks = first.p + nv;
+    p.chunk = chunk;
+    p.x64 = x.p;
+    p.ev = ev.p;
+    p.rt = rt.p;
+    p.budget = budget.p;
+    p.d = d.p;
+    p.dnew = dnew.p;
+    p.sel = sel.p;
+    p.sink = sink.p;
+    p.P = P.p;
+    p.Q = Q.p;
+    p.active = active.p;
+    p.ctl = ctl.p;
+    p.bar = bar.p;
+    p.err = err.p;
+    p.spin_limit = 1ull << 24;
+    p.max_cycles = 1u << 20;
+    p.time_budget_ns = 120ull * 1000000000ull;
+    DBuf<unsigned long long> phase(c, s, 5);
+    phase.zero();
+    p.phase_ns = c->prof ? phase.p : nullptr;
+    p.rounds = (uint32_t)std::max(1, t.flow_rounds);
+    p.early_stop = prm.early_stop;
+    p.INF = (int)std::min<uint64_t>((uint64_t)nv + 2, 1u << 30);
+    p.ev_smem = ev_bytes ? 1u : 0u;
+    p.bfs = bfsw.p;
+
+    std::vector<long long> hP(nnet), hQ(nnet);
+    std::vector<uint8_t> hact(nnet), hfin(nnet);
+
+    bool fresh = co.flows_zero;  // record flow words untouched since they were built
+    co.flows_zero = false;
+    while (ncand) {
+      // choose the probe of every open network
+      for (uint32_t i = 0; i < nnet; i++) {
+        CompState &cs = st[i];
+        hact[i] = 0;
+        if (!cs.candidate || cs.done) continue;
+        const int64_t nci = (int64_t)(co.comp_vbeg[i + 1] - co.comp_vbeg[i]);
+        const int64_t mci = (int64_t)(co.comp_cbeg[i + 1] - co.comp_cbeg[i]);
+        cs.an = cs.lb_n;
+        cs.ad = cs.lb_d;
+        cs.certify = true;
+        if (prm.search == 1) {
+          // bisection on the grid j / D, D = n_c (n_c - 1), while a grid point
+          // lies strictly between the bounds and the scaled capacities fit
+          const int64_t D = nci * (nci - 1);
+          const bool fits = D > 0 && (__int128)D * k * mci < ((__int128)1 << 62);
+          if (fits && frac_lt(cs.lb_n, cs.lb_d, cs.ub_n, cs.ub_d)) {
+            // gap >= 1/D ?
+            const __int128 gap_num = (__int128)cs.ub_n * cs.lb_d - (__int128)cs.lb_n * cs.ub_d;
+            const __int128 gap_den = (__int128)cs.ub_d * cs.lb_d;
+            if (gap_num * D >= gap_den) {
+              const __int128 mid = ((__int128)cs.lb_n * cs.ub_d + (__int128)cs.ub_n * cs.lb_d) * D /
+                                   (2 * (__int128)cs.lb_d * cs.ub_d);
+              const int64_t j = (int64_t)mid;
+              if (frac_lt(cs.lb_n, cs.lb_d, j, D) && frac_lt(j, D, cs.ub_n, cs.ub_d)) {
+                cs.an = j;
+                cs.ad = D;
+                cs.certify = false;
+              }
             }
           }
         }
+        const int64_t g = gcd64(cs.an, cs.ad);
+        hP[i] = cs.an / g;
+        hQ[i] = cs.ad / g;
+        if ((__int128)hQ[i] * k * mci >= ((__int128)1 << 62) || (__int128)hP[i] * k >= ((__int128)1 << 62))
+          fail(CDS_ERR_OVERFLOW, "flow capacities exceed 62 bits");
+        hact[i] = 1;
       }
-      const int64_t g = gcd64(cs.an, cs.ad);
-      hP[i] = cs.an / g;
-      hQ[i] = cs.ad / g;
-      if ((__int128)hQ[i] * k * mci >= ((__int128)1 << 62) || (__int128)hP[i] * k >= ((__int128)1 << 62))
-        fail(CDS_ERR_OVERFLOW, "flow capacities exceed 62 bits");
-      hact[i] = 1;
-    }
-    CDS_CUDA(cudaMemcpyAsync(P.p, hP.data(), nnet * 8, cudaMemcpyHostToDevice, s));
-    CDS_CUDA(cudaMemcpyAsync(Q.p, hQ.data(), nnet * 8, cudaMemcpyHostToDevice, s));
-    CDS_CUDA(cudaMemcpyAsync(active.p, hact.data(), nnet, cudaMemcpyHostToDevice, s));
-    sink.zero();
-    ctl.zero();
-    bar.zero();
-    err.zero();
-    bfsw.zero();
-    {
-      uint32_t nn = nnet;
-      CDS_CUDA(cudaMemcpyAsync(ctl.p + F_WORDS, &nn, 4, cudaMemcpyHostToDevice, s));
-    }
-    // 32-bit flow state when every excursion of x fits: |x| <= q(k-1) plus
-    // at most k-1 concurrent reservations of up to qk each
-    long long qmax = 1;
-    for (uint32_t i = 0; i < nnet; i++)
-      if (hact[i]) qmax = std::max<long long>(qmax, hQ[i]);
-    const bool x32 = x32_fits && (__int128)2 * qmax * k * k < ((__int128)1 << 31);
-    if (x32_fits && !x32) fail(CDS_ERR_OVERFLOW, "flow probe outside the bound its state was sized for");
-    if (!T && !(x32 && fresh)) {  // the split writes every active clique's flows
-      if (x32) k_reset_flow<int><<<G, 256, 0, s>>>(p);
-      else k_reset_flow<long long><<<G, 256, 0, s>>>(p);
-      count_launch();
-    }
-    fresh = false;
-    if (T) {
-      ProfScope ps(c, s, "flow_warm");
-      if (!wgt_init) {  // the weights carry over between the probes
-        wl.zero();
-        k_split_init<<<G, 256, 0, s>>>(p, wgt.p);
+      CDS_CUDA(cudaMemcpyAsync(P.p, hP.data(), nnet * 8, cudaMemcpyHostToDevice, s));
+      CDS_CUDA(cudaMemcpyAsync(Q.p, hQ.data(), nnet * 8, cudaMemcpyHostToDevice, s));
+      CDS_CUDA(cudaMemcpyAsync(active.p, hact.data(), nnet, cudaMemcpyHostToDevice, s));
+      sink.zero();
+      ctl.zero();
+      bar.zero();
+      err.zero();
+      bfsw.zero();
+      {
+        uint32_t nn = nnet;
+        CDS_CUDA(cudaMemcpyAsync(ctl.p + F_WORDS, &nn, 4, cudaMemcpyHostToDevice, s));
+      }
+      // 32-bit flow state when every excursion of x fits: |x| <= q(k-1) plus
+      // at most k-1 concurrent reservations of up to qk each
+      long long qmax = 1;
+      for (uint32_t i = 0; i < nnet; i++)
+        if (hact[i]) qmax = std::max<long long>(qmax, hQ[i]);
+      const bool x32 = x32_fits && (__int128)2 * qmax * k * k < ((__int128)1 << 31);
+      if (x32_fits && !x32) fail(CDS_ERR_OVERFLOW, "flow probe outside the bound its state was sized for");
+      if (!T && !(x32 && fresh)) {  // the split writes every active clique's flows
+        if (x32) k_reset_flow<int><<<G, 256, 0, s>>>(p);
+        else k_reset_flow<long long><<<G, 256, 0, s>>>(p);
         count_launch();
-        wgt_init = true;
       }
-      for (uint32_t r = 1; r < T; r++) {
-        if (k == 3) k_split_loads<3><<<G, 256, 0, s>>>(p, wgt.p, wl.p);
-        else if (k == 4) k_split_loads<4><<<G, 256, 0, s>>>(p, wgt.p, wl.p);
-        else k_split_loads<0><<<G, 256, 0, s>>>(p, wgt.p, wl.p);
-        k_split_update<<<G, 256, 0, s>>>(p, wgt.p, wl.p);
-        count_launch(2);
+      fresh = false;
+      if (T) {
+        ProfScope ps(c, s, "flow_warm");
+        if (!wgt_init) {  // the weights carry over between the probes
+          wl.zero();
+          k_split_init<<<G, 256, 0, s>>>(p, known.p, wgt.p);
+          count_launch();
+          wgt_init = true;
+        }
+        for (uint32_t r = 1; r < T; r++) {
+          if (k == 3) k_split_loads<3><<<G, 256, 0, s>>>(p, wgt.p, wl.p);
+          else if (k == 4) k_split_loads<4><<<G, 256, 0, s>>>(p, wgt.p, wl.p);
+          else k_split_loads<0><<<G, 256, 0, s>>>(p, wgt.p, wl.p);
+          k_split_update<<<G, 256, 0, s>>>(p, wgt.p, wl.p);
+          count_launch(2);
+        }
+        wload.zero();
+        if (x32 && k == 3) k_split_apply<int, 3><<<G, 256, 0, s>>>(p, wgt.p, wload.p);
+        else if (x32 && k == 4) k_split_apply<int, 4><<<G, 256, 0, s>>>(p, wgt.p, wload.p);
+        else if (x32) k_split_apply<int, 0><<<G, 256, 0, s>>>(p, wgt.p, wload.p);
+        else k_split_apply<long long, 0><<<G, 256, 0, s>>>(p, wgt.p, wload.p);
+        count_launch();
       }
-      wload.zero();
-      if (x32 && k == 3) k_split_apply<int, 3><<<G, 256, 0, s>>>(p, wgt.p, wload.p);
-      else if (x32 && k == 4) k_split_apply<int, 4><<<G, 256, 0, s>>>(p, wgt.p, wload.p);
-      else if (x32) k_split_apply<int, 0><<<G, 256, 0, s>>>(p, wgt.p, wload.p);
-      else k_split_apply<long long, 0><<<G, 256, 0, s>>>(p, wgt.p, wload.p);
+      k_preflow<<<G, 256, 0, s>>>(p, T ? wload.p : nullptr);
       count_launch();
-    }
-    k_preflow<<<G, 256, 0, s>>>(p, T ? wload.p : nullptr);
-    count_launch();
-    CDS_CUDA(cudaGetLastError());
-    dim3 grid(blocks), block((unsigned)threads);
-    void *args[] = {&p};
-    {
-      ProfScope ps(c, s, "push_relabel");
-      void *kern = co.vinc_wide ? (x32 ? (void *)k_flow<int, uint64_t> : (void *)k_flow<long long, uint64_t>)
-                                : (x32 ? (void *)k_flow<int, uint32_t> : (void *)k_flow<long long, uint32_t>);
-      CDS_CUDA(cudaLaunchCooperativeKernel(kern, grid, block, args, ev_bytes, s));
-    }
-    count_launch();
-    CDS_CUDA(cudaGetLastError());
-    cut.zero();
-    k_cut_stats<<<G, 256, 0, s>>>(p, cut.p, cut.p + nnet);
-    count_launch();
-    CDS_CUDA(cudaGetLastError());
-    std::vector<long long> hsink(nnet);
-    std::vector<unsigned long long> hcut(2 * (size_t)nnet);
-    uint32_t hctl[F_WORDS];
-    uint32_t herr = 0;
-    {
-      HostReads r(s);
-      r.add(hsink.data(), sink.p, nnet);
-      r.add(hcut.data(), cut.p, 2 * (size_t)nnet);
-      r.add(hctl, ctl.p, F_WORDS);
-      r.add(&herr, err.p);
-      r.wait();
-    }
-    if (herr & DEV_ERR_TIMEOUT) fail(CDS_ERR_TIMEOUT, "push-relabel: device iteration budget exhausted");
-    if (herr) fail(CDS_ERR_CUDA, "push-relabel: device error");
-    const bool stopped = hctl[F_STOPPED] != 0;
-    if (stopped) ans.early_stopped = 1;
-    if (c->prof) {
-      // cycles (global relabel + rounds) and BFS levels of this max-flow
-      std::lock_guard<std::mutex> g(c->mu);
-      auto &a = c->prof_done["flow_cycles"];
-      a.first += 1;
-      a.second += hctl[F_CYCLES];
-      auto &b = c->prof_done["flow_bfs_levels"];
-      b.first += 1;
-      b.second += hctl[F_BFS];
-      auto &r = c->prof_done["flow_rounds"];
-      r.first += 1;
-      r.second += hctl[F_ROUNDS];
-      unsigned long long hph[5];
+      CDS_CUDA(cudaGetLastError());
+      dim3 grid(blocks), block((unsigned)threads);
+      void *args[] = {&p};
+      {
+        ProfScope ps(c, s, "push_relabel");
+        void *kern = co.vinc_wide ? (x32 ? (void *)k_flow<int, uint64_t> : (void *)k_flow<long long, uint64_t>)
+                                  : (x32 ? (void *)k_flow<int, uint32_t> : (void *)k_flow<long long, uint32_t>);
+        CDS_CUDA(cudaLaunchCooperativeKernel(kern, grid, block, args, ev_bytes, s));
+      }
+      count_launch();
+      CDS_CUDA(cudaGetLastError());
+      cut.zero();
+      k_cut_stats<<<G, 256, 0, s>>>(p, cut.p, cut.p + nnet);
+      count_launch();
+      CDS_CUDA(cudaGetLastError());
+      std::vector<long long> hsink(nnet);
+      std::vector<unsigned long long> hcut(2 * (size_t)nnet);
+      uint32_t hctl[F_WORDS];
+      uint32_t herr = 0;
       {
         HostReads r(s);
-        r.add(hph, phase.p, 5);
+        r.add(hsink.data(), sink.p, nnet);
+        r.add(hcut.data(), cut.p, 2 * (size_t)nnet);
+        r.add(hctl, ctl.p, F_WORDS);
+        r.add(&herr, err.p);
         r.wait();
       }
-      CDS_CUDA(cudaMemsetAsync(phase.p, 0, sizeof(hph), s));
-      static const char *pn[5] = {"flow_phase_bfs", "flow_phase_check", "flow_phase_prepare",
-                                  "flow_phase_push", "flow_phase_relabel"};
-      for (int i = 0; i < 5; i++) {
-        auto &a2 = c->prof_done[pn[i]];
-        a2.first += 1;
-        a2.second += hph[i] / 1e6;
+      if (herr & DEV_ERR_TIMEOUT) fail(CDS_ERR_TIMEOUT, "push-relabel: device iteration budget exhausted");
+      if (herr) fail(CDS_ERR_CUDA, "push-relabel: device error");
+      const bool stopped = hctl[F_STOPPED] != 0;
+      if (stopped) ans.early_stopped = 1;
+      if (c->prof) {
+        // cycles (global relabel + rounds) and BFS levels of this max-flow
+        std::lock_guard<std::mutex> g(c->mu);
+        auto &a = c->prof_done["flow_cycles"];
+        a.first += 1;
+        a.second += hctl[F_CYCLES];
+        auto &b = c->prof_done["flow_bfs_levels"];
+        b.first += 1;
+        b.second += hctl[F_BFS];
+        auto &r = c->prof_done["flow_rounds"];
+        r.first += 1;
+        r.second += hctl[F_ROUNDS];
+        unsigned long long hph[5];
+        {
+          HostReads r(s);
+          r.add(hph, phase.p, 5);
+          r.wait();
+        }
+        CDS_CUDA(cudaMemsetAsync(phase.p, 0, sizeof(hph), s));
+        static const char *pn[5] = {"flow_phase_bfs", "flow_phase_check", "flow_phase_prepare",
+                                    "flow_phase_push", "flow_phase_relabel"};
+        for (int i = 0; i < 5; i++) {
+          auto &a2 = c->prof_done[pn[i]];
+          a2.first += 1;
+          a2.second += hph[i] / 1e6;
+        }
       }
-    }
-    ans.flows++;
-    // decide every open network
-    bool any_fin = false;
-    for (uint32_t i = 0; i < nnet; i++) {
-      hfin[i] = 0;
-      if (!hact[i]) continue;
-      CompState &cs = st[i];
-      const int64_t mci = (int64_t)(co.comp_cbeg[i + 1] - co.comp_cbeg[i]);
-      const bool saturated = hsink[i] == (long long)hQ[i] * (long long)k * mci;
-      const int64_t sz = (int64_t)hcut[i], cnt = (int64_t)hcut[nnet + i];
-      if (saturated) {
-        if (cs.certify) {
+      ans.flows++;
+      // decide every open network
+      bool any_fin = false;
+      for (uint32_t i = 0; i < nnet; i++) {
+        hfin[i] = 0;
+        if (!hact[i]) continue;
+        CompState &cs = st[i];
+        const int64_t mci = (int64_t)(co.comp_cbeg[i + 1] - co.comp_cbeg[i]);
+        const bool saturated = hsink[i] == (long long)hQ[i] * (long long)k * mci;
+        const int64_t sz = (int64_t)hcut[i], cnt = (int64_t)hcut[nnet + i];
+        if (saturated) {
+          if (cs.certify) {
+            cs.done = true;
+            ncand--;
+            if (cs.improved) {
+              // the unreachable side at alpha = rho* is the maximal densest set
+              if (sz == 0 || (__int128)cnt * cs.lb_d != (__int128)cs.lb_n * sz)
+                fail(CDS_ERR_CUDA, "flow certificate does not match the found density");
+              cs.lb_n = cnt;
+              cs.lb_d = sz;
+              hfin[i] = 1;
+              any_fin = true;
+            }
+          } else {
+            cs.ub_n = cs.an;
+            cs.ub_d = cs.ad;
+          }
+        } else if (sz > 0 && frac_lt(cs.an, cs.ad, cnt, sz)) {
+          cs.lb_n = cnt;
+          cs.lb_d = sz;
+          cs.improved = true;
+        } else if (stopped) {
+          // the flow was cut short and found nothing denser: keep what we have
           cs.done = true;
+          cs.cut_short = true;
           ncand--;
           if (cs.improved) {
-            // the unreachable side at alpha = rho* is the maximal densest set
-            if (sz == 0 || (__int128)cnt * cs.lb_d != (__int128)cs.lb_n * sz)
-              fail(CDS_ERR_CUDA, "flow certificate does not match the found density");
-            cs.lb_n = cnt;
-            cs.lb_d = sz;
             hfin[i] = 1;
             any_fin = true;
           }
         } else {
-          cs.ub_n = cs.an;
-          cs.ub_d = cs.ad;
+          fail(CDS_ERR_CUDA, "flow cut is not denser than alpha");
         }
-      } else if (sz > 0 && frac_lt(cs.an, cs.ad, cnt, sz)) {
-        cs.lb_n = cnt;
-        cs.lb_d = sz;
-        cs.improved = true;
-      } else if (stopped) {
-        // the flow was cut short and found nothing denser: keep what we have
-        cs.done = true;
-        cs.cut_short = true;
-        ncand--;
-        if (cs.improved) {
-          hfin[i] = 1;
-          any_fin = true;
-        }
-      } else {
-        fail(CDS_ERR_CUDA, "flow cut is not denser than alpha");
       }
-    }
-    if (any_fin) {
-      CDS_CUDA(cudaMemcpyAsync(fin.p, hfin.data(), nnet, cudaMemcpyHostToDevice, s));
-      k_mark_answer<<<G, 256, 0, s>>>(p, fin.p, mark.p);
-      count_launch();
-      CDS_CUDA(cudaGetLastError());
-    }
-    if (stopped) {
-      // sets from an early-stopped flow are only as good as that flow
-      for (uint32_t i = 0; i < nnet; i++)
-        if (hact[i] && !st[i].done && st[i].improved && !hfin[i]) {
-          // keep iterating: the next flow starts from the improved bound
-        }
+      if (any_fin) {
+        CDS_CUDA(cudaMemcpyAsync(fin.p, hfin.data(), nnet, cudaMemcpyHostToDevice, s));
+        k_mark_answer<<<G, 256, 0, s>>>(p, fin.p, mark.p);
+        count_launch();
+        CDS_CUDA(cudaGetLastError());
+      }
+      if (stopped) {
+        // sets from an early-stopped flow are only as good as that flow
+        for (uint32_t i = 0; i < nnet; i++)
+          if (hact[i] && !st[i].done && st[i].improved && !hfin[i]) {
+            // keep iterating: the next flow starts from the improved bound
+          }
+      }
     }
   }
 

@@ -72,7 +72,13 @@
 namespace {
 
 constexpr int THREADS = 512, WARPS = THREADS / 32;
-constexpr uint32_t ROW_BLOCK = 512;   // a row of more entries is a block's work, else a warp's
+// A row of more entries than this is a block's work, else a warp's.  Lowering takes
+// the first (its searches walk a row several times); ordering the first where such
+// rows are few (a block each, or two), else the second: a block's time on a row is a
+// chain of L2 reads and synchronisations, and 16 warps take 16 rows meanwhile (R-MAT
+// 200k k = 3: 2.9 -> 2.0 ms ordering, but 2.8 -> 3.2 ms lowering).
+constexpr uint32_t ROW_FEW = 512, ROW_MANY = 2048;
+constexpr uint32_t SEGMENT = 16384;   // row entries a block looks at before it writes positions
 constexpr uint32_t WARP_SET = 32;     // later sets up to this size are counted by a warp at once
 constexpr uint32_t BINS_WARP = 256, BINS_BLOCK = 1024;
 constexpr int LOWER = 2;              // lowering passes between two counts
@@ -95,8 +101,8 @@ struct CoreParams {
   uint32_t *cin;            // [nnz] c(u, v) at the position of u in v's row
   uint32_t *later;          // [nnz] positions of a queued root's later neighbours, from its row start
   uint32_t *dplus;          // [n] how many
-  const uint32_t *wide;     // [*nwide] vertices with more than ROW_BLOCK neighbours
-  const uint32_t *nwide;
+  const uint32_t *wide;     // [2 n] vertices with more than ROW_FEW (from n: ROW_MANY) neighbours
+  const uint32_t *nwide;    // [2] how many
   uint32_t *queue;          // [n] roots to count
   uint2 *pairs;             // [..] (root, first of PAIR_ITEM later neighbours) of large sets
   uint32_t dmax;            // largest set a block counts by itself
@@ -165,37 +171,34 @@ __device__ __forceinline__ void each_vertex(uint32_t n, uint32_t busy, Want want
   }
 }
 
-// Order phase for one vertex whose value or neighbours changed: has its later set
-// changed?  (Yes in the first sweep, before which there is no order.)  The counts of neighbours that left
-// the set are cleared.  tr of ts threads take part; the result is per thread.
-__device__ __forceinline__ bool set_changed(const CoreParams &p, uint32_t u, uint32_t sweep, uint32_t tr,
-                                            uint32_t ts) {
-  if (sweep == 0) return true;
-  constexpr int U = 4;
-  const uint64_t b = p.off[u];
-  const uint32_t len = (uint32_t)(p.off[u + 1] - b);
-  const unsigned long long ku = __ldcg(p.key + u), nu = key_now(ku, __ldcg(p.tau + u), sweep);
-  bool any = false;
-  for (uint32_t i0 = tr; i0 < len; i0 += ts * U) {
-    uint32_t w[U], tw[U];
-    unsigned long long kw[U];
+// Order phase for entries i0 + lane, i0 + 32 + lane, ... (U of them) of u's row: which
+// neighbours come after u now (bit x: the x-th), and whether any changed sides (in
+// the first sweep, before which there is no order, all count as changed).  The
+// counts of neighbours that went before u are cleared.
+constexpr int ORDER_U = 8;
+__device__ __forceinline__ uint32_t row_after(const CoreParams &p, uint32_t u, uint64_t b, uint32_t len,
+                                              unsigned long long ku, unsigned long long nu, uint32_t sweep,
+                                              uint32_t i0, bool &changed) {
+  uint32_t w[ORDER_U], tw[ORDER_U], now = 0;
+  unsigned long long kw[ORDER_U];
 #pragma unroll
-    for (int x = 0; x < U; x++) w[x] = i0 + ts * x < len ? __ldg(p.adj + b + i0 + ts * x) : u;
+  for (int x = 0; x < ORDER_U; x++) w[x] = i0 + 32 * x < len ? __ldg(p.adj + b + i0 + 32 * x) : u;
 #pragma unroll
-    for (int x = 0; x < U; x++) {
-      tw[x] = __ldcg(p.tau + w[x]);
-      kw[x] = __ldcg(p.key + w[x]);
-    }
+  for (int x = 0; x < ORDER_U; x++) {
+    tw[x] = __ldcg(p.tau + w[x]);
+    kw[x] = __ldcg(p.key + w[x]);
+  }
 #pragma unroll
-    for (int x = 0; x < U; x++) {  // (past the end: u against itself, which does not change)
-      const bool now = after(key_now(kw[x], tw[x], sweep), w[x], nu, u), was = after(kw[x], w[x], ku, u);
-      if (now != was) {
-        any = true;
-        if (was) p.cin[p.off[w[x]] + __ldg(p.rel + b + i0 + ts * x)] = 0;
-      }
+  for (int x = 0; x < ORDER_U; x++) {  // (past the end: u against itself, on neither side)
+    const bool is = after(key_now(kw[x], tw[x], sweep), w[x], nu, u);
+    const bool was = sweep ? after(kw[x], w[x], ku, u) : false;
+    now |= is ? 1u << x : 0u;
+    if (is != was) {
+      changed = true;
+      if (was) p.cin[p.off[w[x]] + __ldg(p.rel + b + i0 + 32 * x)] = 0;
     }
   }
-  return any;
+  return now;
 }
 
 // The weights of root u over its counted later set (positions pos(r)).
@@ -422,6 +425,11 @@ __device__ __forceinline__ uint32_t lower_block(const CoreParams &p, uint32_t v,
   }
 }
 
+// shared words a warp uses in the order phase: counts, set, heavy ids, rows of up to
+// WARP_SET vertices, and the sides of a row
+template <class C>
+constexpr uint32_t ORDER_WORDS = (sizeof(C) / 4 + 3) * WARP_SET + ROW_MANY / 32;
+
 template <int K>
 __global__ void __launch_bounds__(THREADS, 2) k_core(CoreParams p) {
   using C = typename CountOf<K>::type;
@@ -430,7 +438,10 @@ __global__ void __launch_bounds__(THREADS, 2) k_core(CoreParams p) {
   const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
   const bool leader = blockIdx.x == 0 && threadIdx.x == 0;
   const unsigned long long t0 = globaltimer_ns();
-  const uint32_t nwide = *p.nwide, kmin = (K ? K : p.k) - 1;
+  const uint32_t nlong = p.nwide[0];
+  const bool many = nlong > 2 * gridDim.x;
+  const uint32_t nwide = p.nwide[many ? 1 : 0], row_max = many ? ROW_MANY : ROW_FEW;
+  const uint32_t *wide = p.wide + (many ? p.n : 0), kmin = (K ? K : p.k) - 1;
   if (threadIdx.x == 0) {
     s_changed = 0;
     s_low = 0;
@@ -464,68 +475,81 @@ __global__ void __launch_bounds__(THREADS, 2) k_core(CoreParams p) {
       uint32_t *sctl = p.sweep_ctl + (sweep % SLOTS) * Q_WORDS;
       if (leader)  // of the next sweep: no block reads or writes them in this one
         for (int i = 0; i < 4; i++) p.sweep_ctl[((sweep + 1) % SLOTS) * Q_WORDS + i] = 0;
-      // ---- order: long rows by blocks, then the others by warps
+      // ---- order: long rows by blocks, then the others by warps.  One look at a
+      // row gives the side of every entry, as words in shared memory; positions
+      // are written from them.
       for (uint32_t x = blockIdx.x; x < nwide; x += gridDim.x) {
-        const uint32_t u = p.wide[x], t = __ldcg(p.tau + u);
+        const uint32_t u = wide[x], t = __ldcg(p.tau + u);
         if (t == 0 || !since.reaches(t)) continue;
-        if (!__syncthreads_or(set_changed(p, u, sweep, threadIdx.x, blockDim.x))) continue;
         const uint64_t b = p.off[u];
-        const unsigned long long nu = key_of(p, u, sweep);
         const uint32_t len = (uint32_t)(p.off[u + 1] - b);
+        const unsigned long long ku = __ldcg(p.key + u), nu = key_now(ku, t, sweep);
         uint32_t d = 0;
-        for (uint32_t i0 = 0; i0 < len; i0 += 4 * blockDim.x) {  // four consecutive entries a thread
-          const uint32_t i = i0 + 4 * threadIdx.x;
-          uint32_t w[4], m = 0, total;
+        bool changed = false;
+        for (uint32_t s0 = 0; s0 < len; s0 += SEGMENT) {
+          const uint32_t n = min(SEGMENT, len - s0);
+          for (uint32_t i0 = warp * 32 * ORDER_U; i0 < n; i0 += THREADS * ORDER_U) {
+            const uint32_t now = row_after(p, u, b, s0 + n, ku, nu, sweep, s0 + i0 + lane, changed);
 #pragma unroll
-          for (int x = 0; x < 4; x++) w[x] = i + x < len ? __ldg(p.adj + b + i + x) : u;
-#pragma unroll
-          for (int x = 0; x < 4; x++) m |= after(key_of(p, w[x], sweep), w[x], nu, u) ? 1u << x : 0u;
+            for (int y = 0; y < ORDER_U; y++) {
+              const uint32_t m = __ballot_sync(CDS_FULL, (now >> y) & 1u);
+              if (lane == y) sm[(i0 >> 5) + y] = m;  // (SEGMENT is a multiple of the step)
+            }
+          }
+          __syncthreads();
+          uint32_t m = threadIdx.x < (n + 31) / 32 ? sm[threadIdx.x] : 0u, total;
+          static_assert(SEGMENT / 32 == THREADS, "a word a thread");
           uint32_t at = d + block_exclusive_scan<uint32_t>(__popc(m), &total);
-          for (; m; m &= m - 1) p.later[b + at++] = i + __ffs(m) - 1;
+          for (; m; m &= m - 1) p.later[b + at++] = s0 + threadIdx.x * 32 + __ffs(m) - 1;
           d += total;
         }
-        __syncthreads();  // the list, for the block's own reads below
+        if (!__syncthreads_or(changed)) continue;  // (and the list, for the block's own reads below)
         if (threadIdx.x == 0) p.dplus[u] = d;
         if (d < kmin || d > p.dmax) clear_weights(p, u, b, d, threadIdx.x, blockDim.x);
         if (d >= kmin && threadIdx.x == 0) queue_root(p, sctl, u, d);
       }
+      __syncthreads();
       {
-        constexpr uint32_t CW = sizeof(C) / 4;
-        uint32_t *area = sm + warp * ((CW + 3) * WARP_SET);
+        constexpr uint32_t CW = sizeof(C) / 4, MW = ROW_MANY / 32;
+        uint32_t *area = sm + warp * ORDER_WORDS<C>;
         C *cnt = reinterpret_cast<C *>(area);
-        uint32_t *A = area + CW * WARP_SET, *hid = A + WARP_SET, *rows = hid + WARP_SET;
+        uint32_t *A = area + CW * WARP_SET, *hid = A + WARP_SET, *rows = hid + WARP_SET, *side = rows + WARP_SET;
         each_vertex(
             p.n, nwide,
             [&](uint32_t v) {
               const uint32_t t = __ldcg(p.tau + v);
-              return t && since.reaches(t) && p.off[v + 1] - p.off[v] <= ROW_BLOCK;
+              return t && since.reaches(t) && p.off[v + 1] - p.off[v] <= row_max;
             },
             [&](uint32_t u) {
-              if (!__any_sync(CDS_FULL, set_changed(p, u, sweep, lane, 32))) return;
               const uint64_t b = p.off[u];
-              const unsigned long long nu = key_of(p, u, sweep);
               const uint32_t len = (uint32_t)(p.off[u + 1] - b);
-              uint32_t d = 0, pos = 0;  // pos: lane r holds the set's r-th position (sets up to 32)
-              for (uint32_t i0 = 0; i0 < len; i0 += 128) {
-                uint32_t w[4];
-                bool in[4];
+              const unsigned long long ku = __ldcg(p.key + u), nu = key_now(ku, __ldcg(p.tau + u), sweep);
+              bool changed = false;
+              for (uint32_t i0 = 0; i0 < len; i0 += 32 * ORDER_U) {
+                const uint32_t now = row_after(p, u, b, len, ku, nu, sweep, i0 + lane, changed);
 #pragma unroll
-                for (int x = 0; x < 4; x++)
-                  w[x] = i0 + 32 * x + lane < len ? __ldg(p.adj + b + i0 + 32 * x + lane) : u;
-#pragma unroll
-                for (int x = 0; x < 4; x++) in[x] = after(key_of(p, w[x], sweep), w[x], nu, u);
-#pragma unroll
-                for (int x = 0; x < 4; x++) {
-                  const uint32_t m = __ballot_sync(CDS_FULL, in[x]);
-                  if (in[x]) p.later[b + d + __popc(m & ((1u << lane) - 1u))] = i0 + 32 * x + lane;
-                  if (lane >= d && lane - d < __popc(m)) pos = i0 + 32 * x + select_bit(m, lane - d);
-                  d += __popc(m);
+                for (int y = 0; y < ORDER_U; y++) {
+                  const uint32_t m = __ballot_sync(CDS_FULL, (now >> y) & 1u);
+                  if (lane == y) side[(i0 >> 5) + y] = m;
                 }
               }
+              if (!__any_sync(CDS_FULL, changed)) return;
+              __syncwarp();
+              // lane l holds words l and l + 32 of the row's sides
+              static_assert(MW == 64, "two words a lane");
+              const uint32_t nw = (len + 31) / 32;
+              const uint32_t m0 = lane < nw ? side[lane] : 0u, m1 = lane + 32 < nw ? side[lane + 32] : 0u;
+              const uint32_t i0 = warp_inclusive_scan((uint32_t)__popc(m0)), n0 = __shfl_sync(CDS_FULL, i0, 31);
+              const uint32_t i1 = n0 + warp_inclusive_scan((uint32_t)__popc(m1)), d = __shfl_sync(CDS_FULL, i1, 31);
+              uint32_t at = i0 - __popc(m0);
+              for (uint32_t m = m0; m; m &= m - 1) p.later[b + at++] = lane * 32 + __ffs(m) - 1;
+              at = i1 - __popc(m1);
+              for (uint32_t m = m1; m; m &= m - 1) p.later[b + at++] = (lane + 32) * 32 + __ffs(m) - 1;
               __syncwarp();
               if (d < kmin) {
                 clear_weights(p, u, b, d, lane, 32);
               } else if (d <= WARP_SET) {
+                const uint32_t pos = lane < d ? __ldcg(p.later + b + lane) : 0u;
                 if (lane < d) {
                   const uint32_t a = p.adj[b + pos];
                   A[lane] = a;
@@ -533,7 +557,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_core(CoreParams p) {
                 }
                 __syncwarp();
                 local_count<K, false, C>(A, hid, d, p.dag.heavy, p.dag.doff, p.dag.dadj, p.dag.outdeg,
-                                                      rows, cnt, (int)kmin + 1);
+                                         rows, cnt, (int)kmin + 1);
                 const unsigned long long total =
                     warp_sum(store_weights<K>(p, b, d, lane, 32, [&](uint32_t) { return pos; }, A, cnt)) / kmin;
                 if (lane == 0) p.R[u] = (uint32_t)total;
@@ -593,7 +617,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_core(CoreParams p) {
       if (leader)  // of the next pass: last read two passes ago
         for (int i = 0; i < 3; i++) p.pass_ctl[((pass + 1) % SLOTS) * P_WORDS + i] = 0;
       const Range reach = x == 0 ? since : pass_range(p.pass_ctl, pass - 1);
-      for (uint32_t i = blockIdx.x; i < nwide; i += gridDim.x) {
+      for (uint32_t i = blockIdx.x; i < nlong; i += gridDim.x) {
         const uint32_t v = p.wide[i], t = __ldcg(p.tau + v);
         if (t == 0 || !reach.reaches(t)) continue;
         const uint32_t nt = lower_block<K>(p, v, t, sm);
@@ -609,10 +633,10 @@ __global__ void __launch_bounds__(THREADS, 2) k_core(CoreParams p) {
       }
       __syncthreads();
       each_vertex(
-          p.n, nwide,
+          p.n, nlong,
           [&](uint32_t v) {
             const uint32_t t = __ldcg(p.tau + v);
-            return t && reach.reaches(t) && p.off[v + 1] - p.off[v] <= ROW_BLOCK;
+            return t && reach.reaches(t) && p.off[v + 1] - p.off[v] <= ROW_FEW;
           },
           [&](uint32_t v) {
             const uint32_t t = __ldcg(p.tau + v);
@@ -683,8 +707,11 @@ __global__ void k_rel(const uint64_t *__restrict__ off, const uint32_t *__restri
 
 __global__ void k_wide(const uint64_t *__restrict__ off, uint32_t n, uint32_t *__restrict__ wide,
                        uint32_t *__restrict__ nwide) {
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
-    if (off[v + 1] - off[v] > ROW_BLOCK) wide[atomicAdd(nwide, 1u)] = v;
+  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+    const uint64_t d = off[v + 1] - off[v];
+    if (d > ROW_FEW) wide[atomicAdd(nwide, 1u)] = v;
+    if (d > ROW_MANY) wide[n + atomicAdd(nwide + 1, 1u)] = v;
+  }
 }
 
 // largest core per instance and the vertex histogram of core numbers
@@ -879,11 +906,15 @@ void peel(cds_ctx *c, cudaStream_t s, const uint64_t *off, const uint32_t *adj, 
   CDS_CUDA(cudaMemcpyAsync(out.core.p, cl.cdeg.p, (size_t)n * 4, cudaMemcpyDeviceToDevice, s));
 
   // work words in one zeroed block: barrier, status, control slots, queue sizes
-  constexpr size_t CTL = 32 + SLOTS * (P_WORDS + Q_WORDS) + 4;
-  DBuf<uint32_t> ctl(c, s, CTL), R(c, s, n), wide(c, s, n);
+  constexpr size_t CTL = 32 + SLOTS * (P_WORDS + Q_WORDS) + 4;  // nwide[2], sweeps, err
+  DBuf<uint32_t> ctl(c, s, CTL), wide(c, s, 2 * (size_t)n);
+  out.roots.c = c;
+  out.roots.s = s;
+  out.roots.alloc(n + 1);
+  DBuf<uint32_t> &R = out.roots;
   ctl.zero();
   R.zero();
-  uint32_t *const ctl_err = ctl.p + CTL - 1, *const ctl_sweeps = ctl.p + CTL - 2, *const ctl_nwide = ctl.p + CTL - 3;
+  uint32_t *const ctl_err = ctl.p + CTL - 1, *const ctl_sweeps = ctl.p + CTL - 2, *const ctl_nwide = ctl.p + CTL - 4;
   k_wide<<<c->sm_count * 2, 256, 0, s>>>(off, n, wide.p, ctl_nwide);
   count_launch();
   {
@@ -941,7 +972,7 @@ void peel(cds_ctx *c, cudaStream_t s, const uint64_t *off, const uint32_t *adj, 
       }
       pairs.alloc(nnz / PAIR_ITEM + nnz / p.dmax + 1);
       smem = std::max(smem, (size_t)count_team_words(K, p.dmax, rows_in_smem) * 4);
-      smem = std::max(smem, (size_t)WARPS * WARP_SET * 5 * 4);
+      smem = std::max({smem, (size_t)WARPS * ORDER_WORDS<unsigned long long> * 4, (size_t)SEGMENT / 8});
       p.rel = rel.p;
       p.key = key.p;
       p.cin = cin.p;

@@ -226,7 +226,7 @@ void run_problem(cds_ctx *c, cudaStream_t s, UnionGraph &u, const cds_params &pr
   const int m3 = clk.mark();
 
   CoreOut co;
-  densest_core_and_components(c, s, dag, pe, u.inst, k, t, co, !core_only, &clk, on_count);
+  densest_core_and_components(c, s, dag, pe, u.inst, k, t, co, &clk, on_count);
   const int m4 = clk.mark();
 
   // per-instance clique totals
@@ -243,7 +243,9 @@ void run_problem(cds_ctx *c, cudaStream_t s, UnionGraph &u, const cds_params &pr
 
   FlowAnswer fa;
   if (core_only) core_answer(s, pe, u, fa);
-  else exact_search(c, s, co, u.inst, k, prm, t, fa);
+  else
+    exact_search(c, s, co, u.inst, k, prm, t,
+                 [&](const std::vector<uint8_t> &open) { build_networks(c, s, dag, u.inst, k, t, co, open, on_count); }, fa);
   const int m5 = clk.mark();
   clk.wait();
   tms[CDS_T_DAG] = clk.ms(m0, m1);

@@ -68,6 +68,7 @@ struct Instances {
 
 struct PeelOut {
   DBuf<uint32_t> core;              // [n] clique-core number
+  DBuf<uint32_t> roots;             // [n] cliques whose first member by core number each vertex is
   uint32_t max_core = 0;
   std::vector<uint64_t> best_num;   // per instance: best core density
   std::vector<uint64_t> best_den;
@@ -94,7 +95,20 @@ struct CoreOut {
   std::vector<uint64_t> comp_cbeg;    // [ncomp+1] clique ranges
   std::vector<uint32_t> comp_maxcore; // largest core number inside
   std::vector<uint32_t> comp_root;    // smallest vertex (problem id) of each component
+  DBuf<uint32_t> in_core;   // [n] membership of the (k',Psi)-core
+  DBuf<uint32_t> comp;      // [n] smallest vertex of each core vertex's component
+  DBuf<uint64_t> cidx;      // [n+1] component index of a smallest vertex
+  DBuf<uint32_t> local;     // [n] local vertex of each component vertex
+  // small cores (at most 4,096 vertices, k <= 5): the pairs that core cliques
+  // cover, over core-local ids (row a, column b > a)
+  bool small = false;
+  uint32_t ncore = 0, words = 0;
+  DBuf<uint32_t> core_vertex;  // [ncore]
+  DBuf<uint32_t> bits;         // [ncore * words]
+  bool listed = false;
+  Cliques cliques;          // every core clique, once a stage needed them
   DBuf<uint32_t> vmap;      // [nv] original vertex of each local vertex
+  uint64_t nc = 0;          // cliques of the networks (build_networks)
   DBuf<uint32_t> rec;       // [nc << rec_shift(k)] clique records: rec_slots(k)
                             // member slots (local vertex ids), then as many
                             // 32-bit flow words (written by the flow stage)
@@ -109,8 +123,21 @@ struct CoreOut {
 struct StageClock;
 void densest_core_and_components(cds_ctx *c, cudaStream_t s, const Dag &dag, const PeelOut &pe,
                                  const Instances &inst, uint32_t k, const Tuning &t, CoreOut &out,
-                                 bool need_networks, StageClock *clk = nullptr,
-                                 const CountHook *on_count = nullptr);
+                                 StageClock *clk = nullptr, const CountHook *on_count = nullptr);
+// The flow networks of the components with open[i] != 0: records, incidence lists.
+void build_networks(cds_ctx *c, cudaStream_t s, const Dag &dag, const Instances &inst, uint32_t k,
+                    const Tuning &t, CoreOut &out, const std::vector<uint8_t> &open,
+                    const CountHook *on_count = nullptr);
+
+// For each component (q = 0: not asked): is no subset of it denser than p/q?
+// proven[i] = 1 only when that is proved; 0 says nothing.  weights: per local vertex,
+// how the balancing left the components it gave up (0 for others; empty when no
+// component was tried): their flows start from that split.
+struct CertAsk {
+  int64_t p = 0, q = 0;
+};
+void certify(cds_ctx *c, cudaStream_t s, const CoreOut &co, uint32_t k, const std::vector<CertAsk> &ask,
+             std::vector<uint8_t> &proven, DBuf<double> &weights);
 
 // Exact search over all component networks; per instance the answer set.
 struct FlowAnswer {
@@ -124,7 +151,9 @@ struct FlowAnswer {
   uint32_t flows = 0;
   uint32_t early_stopped = 0;
 };
+// networks(open) builds the flow networks of the components a proof is missing for
 void exact_search(cds_ctx *c, cudaStream_t s, const CoreOut &co, const Instances &inst,
-                  uint32_t k, const cds_params &prm, const Tuning &t, FlowAnswer &ans);
+                  uint32_t k, const cds_params &prm, const Tuning &t,
+                  const std::function<void(const std::vector<uint8_t> &)> &networks, FlowAnswer &ans);
 
 }  // namespace cds

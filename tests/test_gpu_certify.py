@@ -1,0 +1,114 @@
+"""Proof that a component is its own densest set, against the flow search: the
+same answers whether a context may use the proof (the default) or has to run its
+flows (64-bit flow state asked for), on components around one word of vertices,
+many words, the largest the proof takes and past it, on several components of one
+graph, on batches, and where a subset is denser than the whole by little."""
+import numpy as np
+import pytest
+
+import cds_b200 as cds
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def both():
+    with cds.Context(0) as a, cds.Context(0, flags=cds.CONFIG_WIDE_FLOW) as b:
+        yield a, b
+
+
+def answer(c, off, adj, k, **kw):
+    g = c.graph(off, adj)
+    s = c.solve(g, k, **kw)
+    g.free()
+    return (s.num, s.den, s.vertices.tolist(), s.upper_bound, s.n_components, s.pruned_edges, s.core_cliques,
+            s.early_stopped)
+
+
+def dense(n, p, seed):
+    off, adj = cds.gen_er(n, 0.0, 1)
+    off, adj, _ = cds.gen_plant(off, adj, n, p, seed)
+    return off, adj
+
+
+@pytest.mark.parametrize("k", [2, 3, 4, 5])
+@pytest.mark.parametrize("n,p", [(6, 1.0), (31, 0.6), (32, 0.6), (33, 0.6), (65, 0.5), (127, 0.4), (129, 0.35)])
+def test_one_dense_component(both, n, p, k):
+    off, adj = dense(n, p, n + k)
+    a, b = (answer(c, off, adj, k) for c in both)
+    assert a == b
+    o = oracle.solve(off, adj, k)
+    assert a[0] * o["den"] == o["num"] * a[1]
+
+
+@pytest.mark.parametrize("k,n,p", [(2, 1023, 0.05), (2, 1024, 0.05), (2, 1025, 0.05), (3, 1024, 0.06), (3, 1025, 0.06),
+                                   (4, 700, 0.12)])
+def test_large_components(both, k, n, p):
+    off, adj = dense(n, p, 5)
+    a, b = (answer(c, off, adj, k) for c in both)
+    assert a == b
+
+
+@pytest.mark.parametrize("k", [2, 3, 4, 5])
+@pytest.mark.parametrize("seed", range(4))
+def test_sparse_and_skewed(both, seed, k):
+    off, adj = cds.gen_rmat(10, 6.0, seed)
+    if seed % 2:
+        off, adj, _ = cds.gen_plant(off, adj, 30, 0.5, seed)
+    for search in ("dinkelbach", "bisect"):
+        a, b = (answer(c, off, adj, k, search=search) for c in both)
+        assert a == b
+
+
+@pytest.mark.parametrize("k", [2, 3, 4])
+def test_several_components_and_ties(both, k):
+    # copies of one dense block beside denser and sparser ones
+    parts = [dense(40, 0.5, 1), dense(40, 0.5, 1), dense(40, 0.5, 2), dense(24, 0.8, 3), dense(24, 0.8, 3)]
+    u, v, base = [], [], 0
+    for off, adj in parts:
+        n = len(off) - 1
+        u.append(np.repeat(np.arange(n), np.diff(off.astype(np.int64))) + base)
+        v.append(adj.astype(np.int64) + base)
+        base += n
+    off, adj = cds.csr_from_edges(base, np.concatenate(u), np.concatenate(v))
+    a, b = (answer(c, off, adj, k) for c in both)
+    assert a == b
+
+
+@pytest.mark.parametrize("k", [2, 3])
+def test_a_subset_barely_denser(both, k):
+    # a circulant graph is its own densest set; one chord more makes a proper
+    # subset of nothing, one vertex less attached makes a subset denser
+    n = 60
+    ring = np.arange(n)
+    for drop in (0, 1, 2):
+        u, v = [], []
+        for d in range(1, 5):
+            u.append(ring)
+            v.append((ring + d) % n)
+        u, v = np.concatenate(u), np.concatenate(v)
+        keep = ~((u == 0) & (v <= drop))
+        off, adj = cds.csr_from_edges(n, u[keep], v[keep])
+        a, b = (answer(c, off, adj, k) for c in both)
+        assert a == b
+        o = oracle.solve(off, adj, k)
+        assert (a[0], a[1]) == (o["num"], o["den"]) and a[2] == o["vertices"].tolist()
+
+
+def test_batches(both):
+    rng = np.random.default_rng(3)
+    graphs = []
+    for i in range(40):
+        n = int(rng.integers(30, 900))
+        off, adj = cds.gen_er(n, float(rng.uniform(4, 12)) / n, i)
+        off, adj, _ = cds.gen_plant(off, adj, int(rng.integers(10, 30)), 0.6, i)
+        graphs.append((off, adj, int(rng.integers(2, 6))))
+    got = []
+    for c in both:
+        gs = [(c.graph(off, adj), k) for off, adj, k in graphs]
+        got.append([(s.num, s.den, s.vertices.tolist(), s.upper_bound)
+                    for s in c.solve_batch([(g, cds.make_params(k)) for g, k in gs])])
+        for g, _ in gs:
+            g.free()
+    assert got[0] == got[1]
