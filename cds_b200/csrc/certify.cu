@@ -131,8 +131,7 @@ __device__ __forceinline__ uint32_t deal(uint32_t jmask, uint32_t incl, uint32_t
 // accumulators (the sum, and in single precision the sum of the squares) and
 // returns this lane's sums over its j (every clique twice over the
 // calls that cover all j), over words [y0, y1) of mask; of the steps of 32 j every
-// split-th from g on.  Two words at a time, two
-// visits in flight.  WIDE:
+// split-th from g on.  Two words at a time, a visit from each in flight.  WIDE:
 // double precision; else single-precision terms, summed in double per j.
 template <bool WIDE>
 __device__ __forceinline__ double pair_sums(const Shared &sh, uint32_t y0, uint32_t y1, uint32_t W, uint32_t jmask,
@@ -151,31 +150,23 @@ __device__ __forceinline__ double pair_sums(const Shared &sh, uint32_t y0, uint3
     for (uint32_t y = y0; y < y1; y += 2) {
       const uint32_t m0 = __shfl_sync(CDS_FULL, mask, y), m1 = y + 1 < y1 ? __shfl_sync(CDS_FULL, mask, y + 1) : 0u;
       if (!(m0 | m1)) continue;
-      uint64_t m = on ? (uint64_t)(m1 ? m1 & row[y + 1] : 0u) << 32 | (m0 & row[y]) : 0ull;
-      while (m) {
-        const uint32_t l = y * 32 + __ffsll((long long)m) - 1;
-        m &= m - 1;
-        const bool two = m != 0;
-        const uint32_t l2 = two ? y * 32 + __ffsll((long long)m) - 1 : l;
-        m &= m - 1;
+      // a visit from each word a step (absent ones take slot 0's weights, masked out)
+      uint32_t a0 = on ? m0 & row[y] : 0u, a1 = on && m1 ? m1 & row[y + 1] : 0u;
+      while (a0 | a1) {
+        const bool v0 = a0 != 0, v1 = a1 != 0;
+        const uint32_t l0 = v0 ? y * 32 + __ffs(a0) - 1 : 0u, l1 = v1 ? y * 32 + 31 + __ffs(a1) : 0u;
+        a0 &= a0 - 1;
+        a1 &= a1 - 1;
+        const float r0 = v0 ? rcp(bf + sh.wf[l0]) : 0.0f, r1 = v1 ? rcp(bf + sh.wf[l1]) : 0.0f;
         if (WIDE) {
-          const float a = rcp(bf + sh.wf[l]), a2 = rcp(bf + sh.wf[l2]);
-          s += newton(bj + sh.w[l], a);
-          const double z = newton(bj + sh.w[l2], a2);
-          sq = fmaf(a, a, sq);
-          if (two) {
-            s2 += z;
-            sq = fmaf(a2, a2, sq);
-          }
+          s += newton(bj + sh.w[l0], r0);  // (0 for an absent one)
+          s2 += newton(bj + sh.w[l1], r1);
         } else {
-          const float a = rcp(bf + sh.wf[l]), a2 = rcp(bf + sh.wf[l2]);
-          f += a;
-          sq = fmaf(a, a, sq);
-          if (two) {
-            f2 += a2;
-            sq = fmaf(a2, a2, sq);
-          }
+          f += r0;
+          f2 += r1;
         }
+        sq = fmaf(r0, r0, sq);
+        sq = fmaf(r1, r1, sq);
       }
     }
     if (WIDE) s += s2;
