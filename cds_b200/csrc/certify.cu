@@ -17,9 +17,18 @@
 // approach that like 1/t), accelerated by Anderson's method over the last HIST
 // differences (D. G. Anderson, "Iterative procedures for nonlinear integral
 // equations", J. ACM 12, 1965).  5 to 16 passes over the cliques reach the bound on
-// the R-MAT and planted graphs tried (7 to 36 without the derivative); components
-// whose densest set is smaller do not converge, which shows after eight passes, and
-// go to the flows.
+// the R-MAT and planted graphs tried (7 to 36 without the derivative).
+//
+// A component that some subset S of it is denser than does not balance, and shows it
+// by the eighth pass.  Its vertices by falling weight are then an order to take them
+// away in (those that want more than their cliques hold go first): a pass counts
+// every clique at its first vertex of that order, which gives the density of every
+// remainder, and the densest one is S.  From there on S and the rest balance as two
+// levels: the rest's weights are scaled up until cliques that cross give S nothing
+// that counts, S aims at its own density and the rest at what is left.  E against
+// the density of S proves it the densest, and when every other vertex stays below
+// k alpha by more than E, no densest set holds one: S is the maximal one.  What
+// does not balance after that goes to the flows, with S to start from.
 //
 // A pass never stores a clique.  The component's covered pairs are a symmetric
 // bitmap of its vertices in shared memory; a warp takes a clique of k-2 vertices
@@ -48,8 +57,9 @@ namespace {
 
 constexpr uint32_t MAX_N = 1024;   // vertices of a component: a word of a row per lane
 constexpr int THREADS = 1024, WARPS = THREADS / 32;
+constexpr uint32_t PARTS = 4;      // of the work, a block, with several components
 constexpr int HIST = 8;            // differences Anderson's method combines
-constexpr uint32_t MAX_PASSES = 32;
+constexpr uint32_t MAX_PASSES = 48, MAX_ORDERS = 5;
 constexpr uint32_t ITEM_WORDS = 2; // k <= 3: words of l an item walks
 
 struct Comp {
@@ -57,11 +67,19 @@ struct Comp {
   uint32_t W, row;        // words a row (odd: lanes on different rows meet different banks), first word
   uint32_t item, nitems;  // its items (k = 4, 5: edges, from `item` on, ...
   uint32_t split;         // ... each split this many ways)
-  double target;          // load every vertex would have at the component's own density
+};
+// The search's state of a component.
+struct Level {
+  double target[2];       // load to balance to: at the level of S (all, at first), of the rest
   double cap;             // k alpha
   double stop;            // E below this counts as reached
+  unsigned long long psi; // cliques of S ...
+  uint32_t size;          // ... and its vertices (0: none denser than asked was found)
+  uint32_t since;         // pass the present levels began at
+  uint32_t orders, split; // orders counted so far; whether one gave two levels
+  unsigned long long p, q;  // alpha
 };
-struct Part {             // a block's share of a component's prefixes
+struct Part {             // a piece of a component's items
   uint32_t comp, part, parts;
 };
 
@@ -71,23 +89,29 @@ struct CertParams {
   const uint32_t *rows;       // symmetric bitmap rows
   const uint32_t *item_u;     // k = 4, 5: the edges u < i by component (indexes in it)
   const uint32_t *item_i;
-  const uint32_t *part_off;   // [blocks+1] each block's parts
-  const Part *part;
+  const Part *part;           // [nparts] by component
+  uint32_t nparts;
+  Level *level;               // [ncomp]
+  uint32_t *rest;             // [nv] 1: not in S
+  uint32_t *rank;             // [nv] place in the order of falling weight
+  uint32_t *first;            // [nv] cliques counted at each vertex
   uint32_t *wide;             // [ncomp] sums in double precision from now on
-  uint32_t *state;            // [ncomp] 0 balancing, 1 reached, 2 given up or not asked
+  uint32_t *state;            // [ncomp] BALANCE ... NOT_ASKED
   double *w;                  // [nv]
   double *T;                  // [nv] sum of 1 / (clique's weights) over the vertex's cliques
   float *T2;                  // [nv] the same of the squares
   unsigned long long *load;   // [2 nv] integer loads: low 32-bit halves, high halves summed
   double *X, *F;              // [(HIST+1) * nv] log-weights and residuals of the last passes
   double *G;                  // [ncomp * HIST * HIST] products of residual differences
-  uint32_t *ctl;              // active components, by pass mod 3
+  uint32_t *ctl;              // by pass mod 3: active components, parts taken (sums, firsts); [9]: shares
   GridBarrier *bar;
   uint32_t *err;
   unsigned long long spin_limit;
   uint32_t *passes;
   unsigned long long *phase_ns;  // [3] block 0's time in passes, updates, the integer pass (profiling; null: off)
 };
+enum : uint32_t { BALANCE = 0, REACHED = 1, GIVEN_UP = 2, COUNT = 3, NOT_ASKED = 4 };
+constexpr double LEVEL_GAP = 28.0;  // log of the weights' ratio between the levels, at least
 constexpr int UNIT_BITS = 46;  // a clique has k 2^46 units
 
 // Shared memory of a block: the component it works on.
@@ -128,14 +152,15 @@ __device__ __forceinline__ uint32_t deal(uint32_t jmask, uint32_t incl, uint32_t
 
 // The pairs of adjacent vertices j in jmask and l in mask (lane x holds word x),
 // each with the prefix one clique.  base: the prefix's weights.  Adds to every j's
-// accumulators (the sum, and in single precision the sum of the squares) and
-// returns this lane's sums over its j (every clique twice over the
-// calls that cover all j), over words [y0, y1) of mask; of the steps of 32 j every
+// accumulators (the sum, and in single precision the sum of its squared shares) and
+// returns this lane's sums over its j (every clique twice over the calls that cover
+// all j; squares: relative to j's weight), over words [y0, y1) of mask; of the steps of 32 j every
 // split-th from g on.  Two words at a time, a visit from each in flight.  WIDE:
 // double precision; else single-precision terms, summed in double per j.
-template <bool WIDE>
+template <bool WIDE, int NP>
 __device__ __forceinline__ double pair_sums(const Shared &sh, uint32_t y0, uint32_t y1, uint32_t W, uint32_t jmask,
-                                            uint32_t mask, uint32_t g, uint32_t split, double base, float &squares) {
+                                            uint32_t mask, uint32_t g, uint32_t split, double base, const float *wp,
+                                            float *squares) {
   const uint32_t lane = lane_id(), incl = warp_inclusive_scan((uint32_t)__popc(jmask));
   const uint32_t total = __shfl_sync(CDS_FULL, incl, 31);
   double tot = 0.0;
@@ -144,7 +169,7 @@ __device__ __forceinline__ double pair_sums(const Shared &sh, uint32_t y0, uint3
     const bool on = q0 + lane < total;
     const uint32_t *row = sh.rows + jq * W;
     const double bj = base + sh.w[jq];
-    const float bf = (float)bj;
+    const float bf = (float)bj, wj = sh.wf[jq];
     double s = 0.0, s2 = 0.0;
     float f = 0.0f, f2 = 0.0f, sq = 0.0f;
     for (uint32_t y = y0; y < y1; y += 2) {
@@ -165,8 +190,9 @@ __device__ __forceinline__ double pair_sums(const Shared &sh, uint32_t y0, uint3
           f += r0;
           f2 += r1;
         }
-        sq = fmaf(r0, r0, sq);
-        sq = fmaf(r1, r1, sq);
+        const float z0 = r0 * wj, z1 = r1 * wj;  // shares: their squares stay in range
+        sq = fmaf(z0, z0, sq);
+        sq = fmaf(z1, z1, sq);
       }
     }
     if (WIDE) s += s2;
@@ -176,7 +202,11 @@ __device__ __forceinline__ double pair_sums(const Shared &sh, uint32_t y0, uint3
       atomicAdd(sh.acc2 + jq, sq);
     }
     tot += s;
-    squares += sq;
+#pragma unroll
+    for (int x = 0; x < NP; x++) {
+      const float r = wp[x] / wj;
+      squares[x] += sq * r * r;
+    }
   }
   return tot;
 }
@@ -239,35 +269,108 @@ __device__ __forceinline__ void pair_shares(const Shared &sh, uint32_t y0, uint3
   }
 }
 
-// One pass of this block over its parts of the components in state `want`.
-template <int K, bool INT>
-__device__ __noinline__ void pass_over(const CertParams &p, uint32_t want, bool reload) {
+// Every clique (once: l after j) counted at its member of smallest rank.
+template <int NP>
+__device__ __forceinline__ void pair_firsts(const Shared &sh, uint32_t y0, uint32_t y1, uint32_t W, uint32_t jmask,
+                                            uint32_t mask, uint32_t g, uint32_t split, const uint32_t *pre) {
+  const uint32_t lane = lane_id(), incl = warp_inclusive_scan((uint32_t)__popc(jmask));
+  const uint32_t total = __shfl_sync(CDS_FULL, incl, 31);
+  const uint32_t *rank = reinterpret_cast<const uint32_t *>(sh.wf);
+  uint32_t *first = reinterpret_cast<uint32_t *>(sh.acc2);
+  for (uint32_t q0 = 32 * g; q0 < total; q0 += 32 * split) {
+    const bool on = q0 + lane < total;
+    const uint32_t j = deal(jmask, incl, min(q0 + lane, total - 1));
+    const uint32_t *row = sh.rows + j * W;
+    uint32_t r0 = rank[j], v0 = j, n = 0;
+#pragma unroll
+    for (int x = 0; x < NP; x++)
+      if (rank[pre[x]] < r0) {
+        r0 = rank[pre[x]];
+        v0 = pre[x];
+      }
+    for (uint32_t y = y0; y < y1; y++) {
+      const uint32_t my = __shfl_sync(CDS_FULL, mask, y);
+      if (!my) continue;
+      uint32_t m = on && y >= (j >> 5) ? my & row[y] : 0u;
+      if (y == (j >> 5)) m &= ~((2u << (j & 31)) - 1u);
+      for (; m; m &= m - 1) {
+        const uint32_t l = y * 32 + __ffs(m) - 1;
+        if (rank[l] < r0) atomicAdd(first + l, 1u);
+        else n++;
+      }
+    }
+    if (n) atomicAdd(first + v0, n);
+  }
+}
+
+// One pass over the components in the states of `want` (a bit each).  Blocks take
+// parts from a counter (their list goes by component, so a block mostly stays with the
+// one whose rows it has) and add their sums to the component's when they leave it.
+enum Mode { SUMS, SHARES, FIRSTS };
+template <int K, Mode MODE>
+__device__ __noinline__ void pass_over(const CertParams &p, uint32_t want, uint32_t *take, uint32_t *loaded) {
+  constexpr bool INT = MODE == SHARES;
   extern __shared__ __align__(16) char smem[];
-  __shared__ uint32_t s_next;  // the next item
+  __shared__ uint32_t s_part, s_next;  // the block's next part, its warps' next item
   const uint32_t lane = lane_id();
-  for (uint32_t x = p.part_off[blockIdx.x]; x < p.part_off[blockIdx.x + 1]; x++) {
-    const Part pt = p.part[x];
-    if (__ldcg(p.state + pt.comp) != want) continue;
-    const Comp c = p.comp[pt.comp];
-    __syncthreads();
+  uint32_t cur = 0xFFFFFFFFu;
+  Comp c{};
+  // (derived from the array at each use: pointers that live across the loop lose
+  // their address space, and every access then costs a generic one)
+  auto areas = [&] {
     Shared sh;
     sh.w = reinterpret_cast<double *>(smem);
     sh.acc = sh.w + c.n;
     sh.wf = reinterpret_cast<float *>(sh.acc + c.n);
     sh.acc2 = sh.wf + c.n;
     sh.rows = reinterpret_cast<uint32_t *>(sh.acc2 + c.n);
-    if (reload || p.part_off[blockIdx.x + 1] - p.part_off[blockIdx.x] > 1) {  // else in place from the first pass
-      for (uint32_t i = threadIdx.x; i < c.n * c.W; i += blockDim.x) sh.rows[i] = p.rows[c.row + i];
-    }
-    for (uint32_t v = threadIdx.x; v < c.n; v += blockDim.x) {
-      const double w = __ldcg(p.w + c.vbeg + v);
-      sh.w[v] = w;
-      sh.wf[v] = (float)w;
-      sh.acc[v] = 0.0;
-      sh.acc2[v] = 0.0f;
-    }
-    if (threadIdx.x == 0) s_next = 0;
+    return sh;
+  };
+  auto leave = [&] {  // (every thread is past its items)
+    if (cur == 0xFFFFFFFFu) return;
+    const Shared sh = areas();
+    if (MODE == FIRSTS)
+      for (uint32_t v = threadIdx.x; v < c.n; v += blockDim.x) {
+        const uint32_t n = reinterpret_cast<uint32_t *>(sh.acc2)[v];
+        if (n) atomicAdd(p.first + c.vbeg + v, n);
+      }
+    if (MODE == SUMS)
+      for (uint32_t v = threadIdx.x; v < c.n; v += blockDim.x)
+        if (sh.acc[v] != 0.0) {
+          atomicAdd(p.T + c.vbeg + v, sh.acc[v]);
+          atomicAdd(p.T2 + c.vbeg + v, sh.acc2[v]);
+        }
     __syncthreads();
+  };
+  for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      uint32_t x = atomicAdd(take, 1u);
+      while (x < p.nparts && !((want >> __ldcg(p.state + p.part[x].comp)) & 1u)) x = atomicAdd(take, 1u);
+      s_part = x;
+      s_next = 0;
+    }
+    __syncthreads();
+    if (s_part >= p.nparts) break;
+    const Part pt = p.part[s_part];
+    if (pt.comp != cur) {
+      leave();
+      cur = pt.comp;
+      c = p.comp[cur];
+      const Shared sh = areas();
+      if (*loaded != cur)
+        for (uint32_t i = threadIdx.x; i < c.n * c.W; i += blockDim.x) sh.rows[i] = p.rows[c.row + i];
+      for (uint32_t v = threadIdx.x; v < c.n; v += blockDim.x) {
+        const double w = __ldcg(p.w + c.vbeg + v);
+        sh.w[v] = w;
+        sh.wf[v] = MODE == FIRSTS ? __uint_as_float(__ldcg(p.rank + c.vbeg + v)) : (float)w;
+        sh.acc[v] = 0.0;
+        sh.acc2[v] = 0.0f;  // (FIRSTS: a count of zero)
+      }
+      __syncthreads();
+      if (threadIdx.x == 0) *loaded = cur;
+    }
+    const Shared sh = areas();
     auto row = [&](uint32_t v) { return lane < c.W ? sh.rows[v * c.W + lane] : 0u; };
     auto later = [&](uint32_t m, uint32_t v) {  // the bits of m past v
       const uint32_t w = v >> 5;
@@ -279,18 +382,27 @@ __device__ __noinline__ void pass_over(const CertParams &p, uint32_t want, bool 
     auto leaf = [&](uint32_t jmask, uint32_t mask, uint32_t y0, uint32_t y1, uint32_t g, uint32_t split, double base,
                     const uint32_t *pre) {
       if (!__any_sync(CDS_FULL, jmask)) return;
-      if constexpr (INT) {
+      if constexpr (MODE == FIRSTS) {
+        pair_firsts<K - 2>(sh, y0, y1, c.W, jmask, mask, g, split, pre);
+      } else if constexpr (INT) {
         pair_shares<K - 2>(sh, y0, y1, c.W, jmask, mask, g, split, base, p.k, pre, lo, hi);
       } else {
-        float sq = 0.0f;
-        const double t = wide ? pair_sums<true>(sh, y0, y1, c.W, jmask, mask, g, split, base, sq)
-                              : pair_sums<false>(sh, y0, y1, c.W, jmask, mask, g, split, base, sq);
-        if constexpr (K > 2) {
-          const double h = 0.5 * warp_sum(t);
-          sq = 0.5f * warp_sum(sq);
-          if (lane < K - 2) {
-            atomicAdd(sh.acc + pre[lane < K - 2 ? lane : 0], h);
-            atomicAdd(sh.acc2 + pre[lane < K - 2 ? lane : 0], sq);
+        constexpr int NP = K - 2;
+        float wp[NP ? NP : 1], sq[NP ? NP : 1];
+#pragma unroll
+        for (int y = 0; y < NP; y++) {
+          wp[y] = sh.wf[pre[y]];
+          sq[y] = 0.0f;
+        }
+        const double t = wide ? pair_sums<true, NP>(sh, y0, y1, c.W, jmask, mask, g, split, base, wp, sq)
+                              : pair_sums<false, NP>(sh, y0, y1, c.W, jmask, mask, g, split, base, wp, sq);
+        const double h = 0.5 * warp_sum(t);
+#pragma unroll
+        for (int y = 0; y < NP; y++) {
+          const float z = 0.5f * warp_sum(sq[y]);
+          if (lane == 0) {
+            atomicAdd(sh.acc + pre[y], h);
+            atomicAdd(sh.acc2 + pre[y], z);
           }
         }
       }
@@ -328,14 +440,8 @@ __device__ __noinline__ void pass_over(const CertParams &p, uint32_t want, bool 
         }
       }
     }
-    __syncthreads();
-    if (!INT)
-      for (uint32_t v = threadIdx.x; v < c.n; v += blockDim.x)
-        if (sh.acc[v] != 0.0) {
-          atomicAdd(p.T + c.vbeg + v, sh.acc[v]);
-          atomicAdd(p.T2 + c.vbeg + v, sh.acc2[v]);
-        }
   }
+  leave();
 }
 
 __device__ __forceinline__ double block_sum(double v, double *s) {
@@ -357,43 +463,173 @@ __device__ __forceinline__ double block_max(double v, double *s) {
   return t;
 }
 
+// The order of falling weight, for a count at each clique's first vertex.
+__device__ __noinline__ void ask_order(const CertParams &p, uint32_t ci) {
+  __shared__ double s_w[MAX_N];
+  const Comp c = p.comp[ci];
+  for (uint32_t v = threadIdx.x; v < c.n; v += blockDim.x) s_w[v] = p.w[c.vbeg + v];
+  __syncthreads();
+  for (uint32_t v = threadIdx.x; v < c.n; v += blockDim.x) {
+    uint32_t r = 0;
+    for (uint32_t u = 0; u < c.n; u++) r += s_w[u] > s_w[v] || (s_w[u] == s_w[v] && u < v);
+    p.rank[c.vbeg + v] = r;
+    p.first[c.vbeg + v] = 0;
+  }
+  __syncthreads();
+}
+
+// After the count: the densest remainder of the order becomes S where it is denser
+// than the present S (the component, at first).  Returns whether it is.
+__device__ __noinline__ bool split_levels(const CertParams &p, uint32_t ci, uint32_t t, double *s) {
+  __shared__ unsigned long long s_left[MAX_N];
+  __shared__ uint32_t s_best;
+  __shared__ uint32_t s_rank[MAX_N];
+  const Comp c = p.comp[ci];
+  Level &lv = p.level[ci];
+  for (uint32_t v = threadIdx.x; v < c.n; v += blockDim.x) {
+    s_rank[v] = p.rank[c.vbeg + v];
+    s_left[s_rank[v]] = __ldcg(p.first + c.vbeg + v);
+  }
+  if (threadIdx.x == 0) s_best = 0xFFFFFFFFu;
+  __syncthreads();
+  // cliques left once the vertices of smaller rank are gone (a thread a rank)
+  static_assert(MAX_N == THREADS, "a rank a thread");
+  const uint32_t i = threadIdx.x;
+  unsigned long long total;
+  const unsigned long long gone =
+      block_exclusive_scan<unsigned long long>(i < c.n ? s_left[i] : 0ull, &total);
+  const unsigned long long left = total - gone;
+  const double density = i < c.n ? (double)left / (double)(c.n - i) : -1.0;
+  const double top = block_max(density, s);
+  if (density == top) atomicMin(&s_best, i);
+  __syncthreads();
+  const uint32_t best = s_best;
+  if (i == best) s_left[0] = left;
+  __syncthreads();
+  const unsigned long long psi = s_left[0];
+  const uint32_t size = c.n - best;
+  const double now = lv.target[0] / (double)p.k;  // density the top level aims at
+  __syncthreads();
+  if (best == 0 || !(top > now * (1.0 + 1e-12))) return false;
+  if (threadIdx.x == 0) {
+    // denser than alpha: the new alpha (in integers)
+    const unsigned long long lh = __umul64hi(psi, lv.q), ll = psi * lv.q, rh = __umul64hi(lv.p, size), rl = lv.p * size;
+    if (lh > rh || (lh == rh && ll > rl)) {
+      unsigned long long a = psi, b = size;
+      while (b) {
+        const unsigned long long r = a % b;
+        a = b;
+        b = r;
+      }
+      lv.p = psi / a;
+      lv.q = size / a;
+      lv.psi = psi;
+      lv.size = size;
+      lv.cap = (double)p.k * (double)lv.p / (double)lv.q;
+      lv.stop = 0.3 * (double)p.k / (double)lv.q;
+    }
+    lv.target[0] = (double)p.k * (double)psi / (double)size;
+    lv.target[1] = (double)p.k * (double)(total - psi) / (double)best;
+  }
+  // the rest's weights above those of S by the gap
+  double hi = -1e300, lo = 1e300;
+  for (uint32_t v = threadIdx.x; v < c.n; v += blockDim.x) {
+    const double x = log(p.w[c.vbeg + v]);
+    if (s_rank[v] < best) lo = x < lo ? x : lo;
+    else hi = x > hi ? x : hi;
+  }
+  hi = block_max(hi, s);
+  lo = -block_max(-lo, s);
+  const double down = hi - lo + LEVEL_GAP;
+  double mx = -1e300;
+  for (uint32_t v = threadIdx.x; v < c.n; v += blockDim.x) {
+    const bool out = s_rank[v] < best;
+    const double x = log(p.w[c.vbeg + v]) - (out || down < 0.0 ? 0.0 : down);
+    p.X[(size_t)((t + 1) % (HIST + 1)) * p.nv + c.vbeg + v] = x;
+    p.rest[c.vbeg + v] = out;
+    mx = x > mx ? x : mx;
+  }
+  mx = block_max(mx, s);
+  for (uint32_t v = threadIdx.x; v < c.n; v += blockDim.x) {
+    const double d = p.X[(size_t)((t + 1) % (HIST + 1)) * p.nv + c.vbeg + v] - mx;
+    p.w[c.vbeg + v] = exp(d < -60.0 ? -60.0 : d);
+  }
+  __syncthreads();
+  return true;
+}
+
 // After pass t: the loads of component ci, and its next weights.  One block; the
 // same block takes the component every time, so its history is its own.
 __device__ __noinline__ void update(const CertParams &p, uint32_t ci, uint32_t t, uint32_t *active, double *s) {
   const Comp c = p.comp[ci];
+  Level &lv = p.level[ci];
+  if (__ldcg(p.state + ci) == COUNT) {
+    const bool better = split_levels(p, ci, t, s);
+    if (threadIdx.x == 0) p.state[ci] = BALANCE;
+    if (better) {  // on from there; this pass's sums belong to the old levels
+      for (uint32_t v = threadIdx.x; v < c.n; v += blockDim.x) {
+        p.T[c.vbeg + v] = 0.0;
+        p.T2[c.vbeg + v] = 0.0f;
+      }
+      if (threadIdx.x == 0) {
+        lv.since = t + 1;
+        lv.split = 1;
+        atomicAdd(active, 1u);
+      }
+      return;
+    }
+  }
   double *sum = s, *G = s + 32;                     // G: [HIST][HIST + 1]
   double *gamma = G + HIST * (HIST + 1);
-  const uint32_t cur = t % (HIST + 1), m = min(t, (uint32_t)HIST);
+  const uint32_t cur = t % (HIST + 1), age = t - lv.since;
+  // differences to combine: none once what does not balance has given no order, as the
+  // combined steps scatter its weights (463 vertices, all but two of them S: proven in 16
+  // of 16 runs, in 5 of 12 with the differences kept)
+  const uint32_t m = age > 18 && !lv.split ? 0 : min(age, (uint32_t)HIST);
+  const double total = lv.target[0] * c.n;  // (about the units in all, for relative sizes)
   double over = 0.0;
   for (uint32_t v = threadIdx.x; v < c.n; v += blockDim.x) {
     const uint32_t g = c.vbeg + v;
     const double wv = __ldcg(p.w + g), T = __ldcg(p.T + g), l = (double)p.k * wv * T;
-    over += l > c.cap ? l - c.cap : 0.0;
-    double slope = 1.0 - wv * (double)__ldcg(p.T2 + g) / T;  // d log l / d log w
+    over += l > lv.cap ? l - lv.cap : 0.0;
+    double slope = 1.0 - (double)__ldcg(p.T2 + g) / (wv * T);  // d log l / d log w
     slope = slope > 1e-3 ? slope : 1e-3;
-    p.F[(size_t)cur * p.nv + g] = log(c.target / l) / slope;
+    p.F[(size_t)cur * p.nv + g] = log(lv.target[p.rest[g]] / l) / slope;
     p.T[g] = 0.0;
     p.T2[g] = 0.0f;
   }
   over = block_sum(over, sum);
-  const double rel = over / (c.target * c.n);
+  const double rel = over / total;
   // single-precision sums are within about 1e-7: enough while the loads are further
   // apart than that, and for bounds that are far above it
   const bool wide = __ldcg(p.wide + ci) != 0;
-  if (over + (wide ? 0.0 : 2e-7 * c.target * c.n) <= c.stop) {
-    if (threadIdx.x == 0) p.state[ci] = 1;
+  if (over + (wide ? 0.0 : 2e-7 * total) <= lv.stop) {
+    if (threadIdx.x == 0) p.state[ci] = REACHED;
     return;
   }
   if (!wide && rel < 1e-6 && threadIdx.x == 0) p.wide[ci] = 1;
-  // not on its way: a component that some subset of it is denser than
-  if (!(rel < 1e30) || (t >= 8 && rel > 1e-3) || (t >= 12 && rel > 1e-4) || (t >= 16 && rel > 1e-5) ||
-      (t >= 20 && rel > 1e-6) || t + 1 >= MAX_PASSES) {
-    if (threadIdx.x == 0) p.state[ci] = 2;
+  // not on its way: look for a denser subset, a few times
+  if (!(rel < 1e30) || t + 2 >= MAX_PASSES) {
+    if (threadIdx.x == 0) p.state[ci] = GIVEN_UP;
     return;
+  }
+  const bool slow = (age == 8 && rel > 1e-3) || (age == 13 && rel > 1e-4) || (age == 18 && rel > 1e-5) ||
+                    age == 23 || age >= 28;
+  if (slow && !(lv.split && age == 8)) {
+    if (lv.split || lv.orders >= MAX_ORDERS) {  // (S is not the densest, or the rest has levels of its own)
+      if (threadIdx.x == 0) p.state[ci] = GIVEN_UP;
+      return;
+    }
+    ask_order(p, ci);
+    if (threadIdx.x == 0) {
+      lv.orders++;
+      p.state[ci] = COUNT;
+    }
   }
   if (threadIdx.x == 0) atomicAdd(active, 1u);
   auto F = [&](uint32_t h, uint32_t v) -> double { return p.F[(size_t)(h % (HIST + 1)) * p.nv + c.vbeg + v]; };
   auto X = [&](uint32_t h, uint32_t v) -> double { return p.X[(size_t)(h % (HIST + 1)) * p.nv + c.vbeg + v]; };
+  // (over S alone once there is one: the rest, with its own plain steps, need not balance)
   // Gram matrix of the residual differences dF(h) = F(h) - F(h-1) of the last m
   // passes, by slot h mod HIST and kept from one pass to the next, and their products
   // with F(t): of the newest with every other, and of each with F(t), a warp per entry
@@ -402,6 +638,7 @@ __device__ __noinline__ void update(const CertParams &p, uint32_t ci, uint32_t t
     const uint32_t r = e >> 1, h = t - r;
     double d = 0.0;
     for (uint32_t v = lane_id(); v < c.n; v += 32) {
+      if (p.rest[c.vbeg + v]) continue;
       const double f = F(t, v);
       d += (F(h, v) - F(h - 1, v)) * ((e & 1) ? f : f - F(t - 1, v));
     }
@@ -449,7 +686,7 @@ __device__ __noinline__ void update(const CertParams &p, uint32_t ci, uint32_t t
   for (uint32_t v = threadIdx.x; v < c.n; v += blockDim.x, i++) {
     const double x = X(t, v);
     double step = F(t, v);
-    for (uint32_t r = 0; r < m; r++)
+    for (uint32_t r = 0; r < (p.rest[c.vbeg + v] ? 0 : m); r++)
       step -= gamma[r] * (X(t - r, v) - X(t - r - 1, v) + F(t - r, v) - F(t - r - 1, v));
     step = step > 1.5 ? 1.5 : step < -1.5 ? -1.5 : step == step ? step : 0.0;
     nx[i] = x + step;
@@ -476,20 +713,26 @@ __global__ void __launch_bounds__(THREADS, 1) k_certify(CertParams p) {
       tprev = now;
     }
   };
+  __shared__ uint32_t s_loaded;  // the component whose rows are in place
+  if (threadIdx.x == 0) s_loaded = 0xFFFFFFFFu;
   uint32_t t = 0;
   for (; t < MAX_PASSES; t++) {
-    if (leader) p.ctl[(t + 1) % 3] = 0;  // of the next pass
-    pass_over<K, false>(p, 0, t == 0);
+    if (leader)  // of the next pass
+      for (int i = 0; i < 3; i++) p.ctl[3 * i + (t + 1) % 3] = 0;
+    pass_over<K, SUMS>(p, 1u << BALANCE | 1u << COUNT, p.ctl + 3 + t % 3, &s_loaded);
+    pass_over<K, FIRSTS>(p, 1u << COUNT, p.ctl + 6 + t % 3, &s_loaded);
     if (!grid_sync(p.bar, p.err, p.spin_limit)) return;
     phase_end(0);
-    for (uint32_t ci = blockIdx.x; ci < p.ncomp; ci += gridDim.x)
-      if (__ldcg(p.state + ci) == 0) update(p, ci, t, p.ctl + t % 3, s_up);
+    for (uint32_t ci = blockIdx.x; ci < p.ncomp; ci += gridDim.x) {
+      const uint32_t st = __ldcg(p.state + ci);
+      if (st == BALANCE || st == COUNT) update(p, ci, t, p.ctl + t % 3, s_up);
+    }
     if (!grid_sync(p.bar, p.err, p.spin_limit)) return;
     phase_end(1);
     if (!__ldcg(p.ctl + t % 3)) break;
   }
   if (leader) *p.passes = t + 1;
-  pass_over<K, true>(p, 1, false);
+  pass_over<K, SHARES>(p, 1u << REACHED, p.ctl + 9, &s_loaded);
   phase_end(2);
 }
 
@@ -554,12 +797,14 @@ __global__ void k_cert_items(const uint32_t *__restrict__ rows, const uint32_t *
 namespace cds {
 
 void certify(cds_ctx *c, cudaStream_t s, const CoreOut &co, uint32_t k, const std::vector<CertAsk> &ask,
-             std::vector<uint8_t> &proven, DBuf<double> &weights) {
+             std::vector<CertAnswer> &out, std::vector<uint8_t> &in_set, DBuf<double> &weights) {
   const uint32_t nnet = co.ncomp, nv = nnet ? co.comp_vbeg[nnet] : 0;
-  proven.assign(nnet, 0);
+  out.assign(nnet, CertAnswer{});
+  in_set.clear();
   if (!co.small || k > 5) return;
   std::vector<Comp> hc(nnet);
-  std::vector<uint32_t> hstate(nnet, 2), asked;
+  std::vector<uint32_t> hstate(nnet, NOT_ASKED), asked;
+  std::vector<Level> hl(nnet);
   uint32_t words = 0;
   uint64_t pairs = 0, work = 0;
   size_t smem = 0;
@@ -578,65 +823,53 @@ void certify(cds_ctx *c, cudaStream_t s, const CoreOut &co, uint32_t k, const st
     h.nitems = k == 2 ? per : k == 3 ? h.n * per : 0;
     // small components have few edges: their work is dealt in finer pieces
     h.split = k == 4 && h.n <= 128 ? (h.n + 31) / 32 : k == 5 && h.n <= 256 ? 8 : 1;
-    h.target = (double)k * (double)psi / (double)h.n;
-    h.cap = (double)k * (double)ask[i].p / (double)ask[i].q;
-    h.stop = 0.3 * (double)k / (double)ask[i].q;
-    hstate[i] = 0;
+    Level &l = hl[i];
+    l = Level{};
+    l.target[0] = (double)k * (double)psi / (double)h.n;
+    l.cap = (double)k * (double)ask[i].p / (double)ask[i].q;
+    l.stop = 0.3 * (double)k / (double)ask[i].q;
+    l.p = (unsigned long long)ask[i].p;
+    l.q = (unsigned long long)ask[i].q;
+    hstate[i] = BALANCE;
     asked.push_back(i);
     work += psi;
     smem = std::max(smem, shared_bytes(h.n, h.W));
   }
   if (asked.empty()) return;
-  // Blocks: one an SM at most.  Every component gets its share of them by cliques
-  // (at least one, at most a warp per prefix); with more components than blocks,
-  // the largest go first to the block with the least work.
-  const uint32_t avail = coop_grid(c, 1);
-  std::vector<std::vector<Part>> plan;
-  if (asked.size() <= avail) {
-    for (uint32_t i : asked) {
-      const uint64_t psi = co.comp_cbeg[i + 1] - co.comp_cbeg[i];
-      const uint64_t prefixes = k <= 3 ? hc[i].nitems : std::max<uint64_t>(hc[i].n, psi / 64);
-      uint64_t parts = (avail - asked.size()) * psi / work + 1;
-      parts = std::max<uint64_t>(1, std::min(parts, (prefixes + WARPS - 1) / WARPS));
-      for (uint32_t x = 0; x < parts; x++) plan.push_back({Part{i, x, (uint32_t)parts}});
-    }
-  } else {
-    std::vector<uint32_t> order = asked;
-    std::sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) {
-      const uint64_t x = co.comp_cbeg[a + 1] - co.comp_cbeg[a], y = co.comp_cbeg[b + 1] - co.comp_cbeg[b];
-      return x != y ? x > y : a < b;
-    });
-    plan.resize(avail);
-    std::vector<uint64_t> sum(avail, 0);
-    for (uint32_t i : order) {
-      const size_t b = (size_t)(std::min_element(sum.begin(), sum.end()) - sum.begin());
-      plan[b].push_back(Part{i, 0, 1});
-      sum[b] += co.comp_cbeg[i + 1] - co.comp_cbeg[i];
-    }
-  }
-  std::vector<uint32_t> off(plan.size() + 1, 0);
+  // Parts, shared among the components by their cliques (at most a warp per prefix
+  // each): with several, some a block, so that the blocks of a finished component work
+  // for the others (19 components of 25 M 4-cliques, two of which never balance:
+  // 19.4 -> 6.2 ms).  One component is dealt to the blocks evenly in any case, and a
+  // part each spares them the ends of more (988 vertices: 55 -> 42 ms).
+  const uint32_t avail = coop_grid(c, 1), per_block = asked.size() > 1 ? PARTS : 1;
   std::vector<Part> parts;
-  for (size_t b = 0; b < plan.size(); b++) {
-    parts.insert(parts.end(), plan[b].begin(), plan[b].end());
-    off[b + 1] = (uint32_t)parts.size();
+  for (uint32_t i : asked) {
+    const uint64_t psi = co.comp_cbeg[i + 1] - co.comp_cbeg[i];
+    const uint64_t items = k <= 3 ? hc[i].nitems : std::max<uint64_t>(hc[i].n, psi / 64) * hc[i].split;
+    const uint64_t want = (uint64_t)((double)avail * per_block * (double)psi / (double)work) + (asked.size() > 1);
+    const uint32_t n = (uint32_t)std::max<uint64_t>(1, std::min(want, (items + WARPS - 1) / WARPS));
+    for (uint32_t x = 0; x < n; x++) parts.push_back(Part{i, x, n});
   }
+  const unsigned blocks = (unsigned)std::min<size_t>(avail, parts.size());
   DBuf<Comp> comp(c, s, nnet);
   DBuf<Part> d_part(c, s, parts.size());
-  DBuf<uint32_t> state(c, s, nnet), wide(c, s, nnet), rows(c, s, words), cnt(c, s, nv), item_u(c, s, k < 4 ? 0 : pairs + 1),
-      item_i(c, s, k < 4 ? 0 : pairs + 1), ctl(c, s, 32 + 3 + 2), d_off(c, s, off.size());
+  DBuf<Level> level(c, s, nnet);
+  DBuf<uint32_t> state(c, s, nnet), wide(c, s, nnet), rest(c, s, nv), rank(c, s, nv), firsts(c, s, nv), rows(c, s, words), cnt(c, s, nv), item_u(c, s, k < 4 ? 0 : pairs + 1),
+      item_i(c, s, k < 4 ? 0 : pairs + 1), ctl(c, s, 32 + 10 + 2);
   DBuf<uint64_t> first(c, s, nv + 1);
   DBuf<double> w(c, s, nv), T(c, s, nv), X(c, s, (size_t)(HIST + 1) * nv), F(c, s, (size_t)(HIST + 1) * nv),
       G(c, s, (size_t)nnet * HIST * HIST);
   DBuf<float> T2(c, s, nv);
   DBuf<unsigned long long> load(c, s, 2 * (size_t)nv);
   CDS_CUDA(cudaMemcpyAsync(comp.p, hc.data(), nnet * sizeof(Comp), cudaMemcpyHostToDevice, s));
+  CDS_CUDA(cudaMemcpyAsync(level.p, hl.data(), nnet * sizeof(Level), cudaMemcpyHostToDevice, s));
   CDS_CUDA(cudaMemcpyAsync(state.p, hstate.data(), nnet * 4, cudaMemcpyHostToDevice, s));
-  CDS_CUDA(cudaMemcpyAsync(d_off.p, off.data(), off.size() * 4, cudaMemcpyHostToDevice, s));
   CDS_CUDA(cudaMemcpyAsync(d_part.p, parts.data(), parts.size() * sizeof(Part), cudaMemcpyHostToDevice, s));
   rows.zero();
   T.zero();
   T2.zero();
   wide.zero();
+  rest.zero();
   load.zero();
   ctl.zero();
   const int grid = c->sm_count * 4;
@@ -658,10 +891,14 @@ void certify(cds_ctx *c, cudaStream_t s, const CoreOut &co, uint32_t k, const st
   p.rows = rows.p;
   p.item_u = item_u.p;
   p.item_i = item_i.p;
-  p.part_off = d_off.p;
   p.part = d_part.p;
+  p.nparts = (uint32_t)parts.size();
   p.state = state.p;
   p.wide = wide.p;
+  p.level = level.p;
+  p.rest = rest.p;
+  p.rank = rank.p;
+  p.first = firsts.p;
   p.w = w.p;
   p.T = T.p;
   p.T2 = T2.p;
@@ -672,7 +909,7 @@ void certify(cds_ctx *c, cudaStream_t s, const CoreOut &co, uint32_t k, const st
   static_assert(sizeof(GridBarrier) == 32 * sizeof(uint32_t), "the barrier takes the first line");
   p.bar = reinterpret_cast<GridBarrier *>(ctl.p);
   p.ctl = ctl.p + 32;
-  p.err = ctl.p + 35;
+  p.err = ctl.p + 42;
   p.passes = p.err + 1;
   p.spin_limit = 1ull << 26;
   DBuf<unsigned long long> phase(c, s, c->prof ? 3 : 0);
@@ -687,15 +924,18 @@ void certify(cds_ctx *c, cudaStream_t s, const CoreOut &co, uint32_t k, const st
   void *args[] = {&p};
   {
     ProfScope ps(c, s, "certify");
-    CDS_CUDA(cudaLaunchCooperativeKernel(kern, dim3((unsigned)plan.size()), dim3(THREADS), args, smem, s));
+    CDS_CUDA(cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(THREADS), args, smem, s));
   }
   count_launch();
   CDS_CUDA(cudaGetLastError());
   std::vector<unsigned long long> hload(2 * (size_t)nv);
+  std::vector<uint32_t> hrest(nv);
   uint32_t status[2] = {0, 0};
   {
     HostReads r(s);
     r.add(hstate.data(), state.p, nnet);
+    r.add(hl.data(), level.p, nnet);
+    r.add(hrest.data(), rest.p, nv);
     r.add(hload.data(), load.p, hload.size());
     r.add(status, p.err, 2);
     r.wait();
@@ -720,19 +960,38 @@ void certify(cds_ctx *c, cudaStream_t s, const CoreOut &co, uint32_t k, const st
   }
   if (status[0]) fail(CDS_ERR_TIMEOUT, "certify: device iteration budget exhausted");
   const __int128 one = (__int128)1 << UNIT_BITS;
+  in_set.assign(nv, 0);
   for (uint32_t i : asked) {
-    if (hstate[i] != 1) continue;
     const Comp &h = hc[i];
+    const Level &l = hl[i];
+    CertAnswer &o = out[i];
+    o.num = l.size ? (int64_t)l.psi : 0;
+    o.den = l.size;
+    if (hstate[i] != REACHED) continue;
     const __int128 psi = (__int128)(co.comp_cbeg[i + 1] - co.comp_cbeg[i]);
-    const __int128 cap = (__int128)k * ask[i].p * one;  // times q
-    __int128 sum = 0, over = 0;
+    const __int128 cap = (__int128)k * l.p * one;  // times q, as all below
+    __int128 sum = 0, over = 0, top = 0, room = (__int128)1 << 120;
+    uint32_t size = 0;
     for (uint32_t v = 0; v < h.n; v++) {
-      const __int128 l = (__int128)hload[h.vbeg + v] + ((__int128)hload[(size_t)nv + h.vbeg + v] << 32);
-      sum += l;
-      if (l * ask[i].q > cap) over += l * ask[i].q - cap;
+      const __int128 x = (__int128)hload[h.vbeg + v] + ((__int128)hload[(size_t)nv + h.vbeg + v] << 32);
+      sum += x;
+      if (x * l.q > cap) over += x * l.q - cap;
+      if (!hrest[h.vbeg + v]) {
+        top += x;
+        size++;
+      } else if (cap - x * l.q < room) {
+        room = cap - x * l.q;
+      }
     }
     if (sum != psi * k * one) fail(CDS_ERR_CUDA, "certify: loads do not add up to the cliques' units");
-    proven[i] = over < (__int128)k * one;
+    bool good = over < (__int128)k * one;
+    // a proper subset: it holds the cliques it was said to, and no other vertex can
+    // be in a densest set
+    if (l.size) good = good && size == l.size && top >= (__int128)k * one * l.psi && room > over;
+    if (!good) continue;
+    o.proven = true;
+    if (l.size)
+      for (uint32_t v = 0; v < h.n; v++) in_set[h.vbeg + v] = !hrest[h.vbeg + v];
   }
   weights = std::move(w);
 }

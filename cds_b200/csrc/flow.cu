@@ -849,14 +849,24 @@ void exact_search(cds_ctx *c, cudaStream_t s, const CoreOut &co, const Instances
       const int64_t g = gcd64(st[i].lb_n, st[i].lb_d);
       ask[i] = {st[i].lb_n / g, st[i].lb_d / g};
     }
-    std::vector<uint8_t> proven;
-    certify(c, s, co, k, ask, proven, known);
-    for (uint32_t i = 0; i < nnet; i++)
-      if (proven[i]) {
-        st[i].done = st[i].certify = true;
-        ncand--;
-        ans.flows = 1;  // an assignment that saturates the network, as one max-flow finds
+    std::vector<CertAnswer> found;
+    std::vector<uint8_t> in_set;
+    certify(c, s, co, k, ask, found, in_set, known);
+    bool marked = false;
+    for (uint32_t i = 0; i < nnet; i++) {
+      CompState &cs = st[i];
+      if (found[i].den) {
+        cs.lb_n = found[i].num;
+        cs.lb_d = found[i].den;
+        cs.improved = true;
       }
+      if (!found[i].proven) continue;
+      cs.done = cs.certify = true;
+      ncand--;
+      ans.flows = 1;  // an assignment that saturates the network, as one max-flow finds
+      marked |= cs.improved;
+    }
+    if (marked) CDS_CUDA(cudaMemcpyAsync(mark.p, in_set.data(), nv, cudaMemcpyHostToDevice, s));
   }
   if (ncand) {
     std::vector<uint8_t> open(nnet);

@@ -129,15 +129,21 @@ void build_networks(cds_ctx *c, cudaStream_t s, const Dag &dag, const Instances 
                     const Tuning &t, CoreOut &out, const std::vector<uint8_t> &open,
                     const CountHook *on_count = nullptr);
 
-// For each component (q = 0: not asked): is no subset of it denser than p/q?
-// proven[i] = 1 only when that is proved; 0 says nothing.  weights: per local vertex,
-// how the balancing left the components it gave up (0 for others; empty when no
-// component was tried): their flows start from that split.
+// For each component (q = 0: not asked): is no subset of it denser than p/q, or
+// which one is?  den = 0: none was found.  proven: no subset is denser than the
+// found one (or than p/q), and the found one, marked in in_set (over local vertices),
+// is the maximal such set; else nothing is known but that it exists.  weights: per
+// local vertex, how the balancing left the components (0 where it did not run;
+// empty when it ran for none): their flows start from that split.
 struct CertAsk {
   int64_t p = 0, q = 0;
 };
+struct CertAnswer {
+  bool proven = false;
+  int64_t num = 0, den = 0;
+};
 void certify(cds_ctx *c, cudaStream_t s, const CoreOut &co, uint32_t k, const std::vector<CertAsk> &ask,
-             std::vector<uint8_t> &proven, DBuf<double> &weights);
+             std::vector<CertAnswer> &out, std::vector<uint8_t> &in_set, DBuf<double> &weights);
 
 // Exact search over all component networks; per instance the answer set.
 struct FlowAnswer {
