@@ -587,6 +587,9 @@ __device__ __noinline__ void update(const CertParams &p, uint32_t ci, uint32_t t
   // of 16 runs, in 5 of 12 with the differences kept)
   const uint32_t m = age > 18 && !lv.split ? 0 : min(age, (uint32_t)HIST);
   const double total = lv.target[0] * c.n;  // (about the units in all, for relative sizes)
+  // (read before block_sum's barriers: thread 0 sets it below, and all threads have to
+  // take the same way there)
+  const bool wide = __ldcg(p.wide + ci) != 0;
   double over = 0.0;
   for (uint32_t v = threadIdx.x; v < c.n; v += blockDim.x) {
     const uint32_t g = c.vbeg + v;
@@ -602,7 +605,6 @@ __device__ __noinline__ void update(const CertParams &p, uint32_t ci, uint32_t t
   const double rel = over / total;
   // single-precision sums are within about 1e-7: enough while the loads are further
   // apart than that, and for bounds that are far above it
-  const bool wide = __ldcg(p.wide + ci) != 0;
   if (over + (wide ? 0.0 : 2e-7 * total) <= lv.stop) {
     if (threadIdx.x == 0) p.state[ci] = REACHED;
     return;
