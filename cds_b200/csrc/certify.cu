@@ -60,6 +60,7 @@ constexpr int THREADS = 1024, WARPS = THREADS / 32;
 constexpr uint32_t PARTS = 4;      // of the work, a block, with several components
 constexpr int HIST = 8;            // differences Anderson's method combines
 constexpr uint32_t MAX_PASSES = 48, MAX_ORDERS = 5;
+constexpr uint64_t MAX_CLIQUES = 0xFFFFFFFFull;  // (counts at first vertices are 32-bit)
 constexpr uint32_t ITEM_WORDS = 2; // k <= 3: words of l an item walks
 
 struct Comp {
@@ -253,19 +254,23 @@ __device__ __forceinline__ void pair_shares(const Shared &sh, uint32_t y0, uint3
       }
     }
     if (sum) give(j, sum);
-  }
-  if (NP == 0) return;
-  rem = warp_sum(rem);
-  if (lane == 0 && rem) {
-    unsigned long long left = rem;
+    // a step adds at most 1,024 cliques of k 2^46 units to a lane: given before 32
+    // lanes' sums could pass 64 bits
+    if (NP > 0 && (q0 + 32 * split >= total || __any_sync(CDS_FULL, rem >> 56))) {
+      const unsigned long long sum_rem = warp_sum(rem);
+      rem = 0;
+      if (lane == 0 && sum_rem) {
+        unsigned long long left = sum_rem;
 #pragma unroll
-    for (int x = 1; x < NP; x++) {
-      unsigned long long a = (unsigned long long)((double)rem * (sh.w[pre[x]] / base));
-      a = a < left ? a : left;
-      left -= a;
-      give(pre[x], a);
+        for (int x = 1; x < NP; x++) {
+          unsigned long long a = (unsigned long long)((double)sum_rem * (sh.w[pre[x]] / base));
+          a = a < left ? a : left;
+          left -= a;
+          give(pre[x], a);
+        }
+        if (left) give(pre[0], left);
+      }
     }
-    if (left) give(pre[0], left);
   }
 }
 
@@ -816,7 +821,7 @@ void certify(cds_ctx *c, cudaStream_t s, const CoreOut &co, uint32_t k, const st
     h.vbeg = co.comp_vbeg[i];
     h.n = co.comp_vbeg[i + 1] - h.vbeg;
     const uint64_t psi = co.comp_cbeg[i + 1] - co.comp_cbeg[i];
-    if (!ask[i].q || h.n > MAX_N || !psi) continue;
+    if (!ask[i].q || h.n > MAX_N || !psi || psi > MAX_CLIQUES) continue;
     h.W = ((h.n + 31) / 32) | 1u;
     if (h.W > 32) h.W = 32;  // a lane a word (1,024 vertices: rows share banks)
     h.row = words;

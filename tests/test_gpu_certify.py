@@ -3,6 +3,8 @@ same answers whether a context may use the proof (the default) or has to run its
 flows (64-bit flow state asked for), on components around one word of vertices,
 many words, the largest the proof takes and past it, on several components of one
 graph, on batches, and where a subset is denser than the whole by little."""
+import math
+
 import numpy as np
 import pytest
 
@@ -112,3 +114,15 @@ def test_batches(both):
         for g, _ in gs:
             g.free()
     assert got[0] == got[1]
+
+
+def test_units_of_many_cliques(both):
+    # an edge of the complete graph on 560 vertices has 155,403 4-cliques before its
+    # later neighbours': k 2^46 units of each pass 64 bits
+    n, k = 560, 4
+    off, adj = dense(n, 1.0, 1)
+    g = both[0].graph(off, adj)
+    s = both[0].solve(g, k)
+    g.free()
+    assert s.num * n == math.comb(n, k) * s.den
+    assert s.vertices.tolist() == list(range(n))
