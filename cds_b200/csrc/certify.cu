@@ -45,6 +45,7 @@
 // triangles 0.39 -> 0.14 ms, 470 vertices and 25,761 edges 0.69 -> 0.25, 112 and
 // 1.18 M 4-cliques 1.5 -> 0.38, 746 and 9.3 M triangles 4.4 -> 1.3, 988 and 1.14 G
 // 4-cliques 295 -> 47 (and 62 GB of records and lists that are not built).
+#include "core_rows.cuh"
 #include "device_util.cuh"
 #include "stages.h"
 
@@ -745,21 +746,19 @@ __global__ void __launch_bounds__(THREADS, 1) k_certify(CertParams p) {
 
 // symmetric rows of every component from the covered pairs of core-local ids
 // (bits: row a, column b > a); warp per row and word
-__global__ void k_cert_rows(const uint32_t *__restrict__ bits, uint32_t words, uint32_t ncore,
+__global__ void k_cert_rows(const uint32_t *__restrict__ bits, CoreRows r, uint32_t ncore,
                             const uint32_t *__restrict__ core_vertex, const uint32_t *__restrict__ local,
                             const uint32_t *__restrict__ vcnet, const Comp *__restrict__ comp,
                             uint32_t *__restrict__ rows) {
-  const uint32_t warps = (gridDim.x * blockDim.x) >> 5, total = ncore * words;
-  for (uint32_t x = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; x < total; x += warps) {
-    const uint32_t m = bits[x];
-    if (!((m >> lane_id()) & 1u)) continue;
-    const uint32_t la = local[core_vertex[x / words]], lb = local[core_vertex[x % words * 32 + lane_id()]];
+  each_word(r, ncore, core_vertex, bits, [&](uint32_t i, const CoreBand &bd, uint32_t w, uint32_t m) {
+    if (!((m >> lane_id()) & 1u)) return;
+    const uint32_t la = local[core_vertex[i]], lb = local[core_vertex[bd.lid + w * 32 + lane_id()]];
     const Comp c = comp[vcnet[la]];
-    if (!c.W) continue;  // not asked
+    if (!c.W) return;  // not asked
     const uint32_t a = la - c.vbeg, b = lb - c.vbeg;
     atomicOr(rows + c.row + a * c.W + (b >> 5), 1u << (b & 31));
     atomicOr(rows + c.row + b * c.W + (a >> 5), 1u << (a & 31));
-  }
+  });
 }
 // per local vertex: its later neighbours, and the start of the balancing
 __device__ __forceinline__ uint32_t later_word(const uint32_t *rows, const Comp &c, uint32_t v, uint32_t x) {
@@ -880,7 +879,7 @@ void certify(cds_ctx *c, cudaStream_t s, const CoreOut &co, uint32_t k, const st
   load.zero();
   ctl.zero();
   const int grid = c->sm_count * 4;
-  k_cert_rows<<<grid, 256, 0, s>>>(co.bits.p, co.words, co.ncore, co.core_vertex.p, co.local.p, co.vcnet.p, comp.p,
+  k_cert_rows<<<grid, 256, 0, s>>>(co.bits.p, co.rows, co.ncore, co.core_vertex.p, co.local.p, co.vcnet.p, comp.p,
                                 rows.p);
   k_cert_start<<<(nv + 255) / 256, 256, 0, s>>>(rows.p, co.vcnet.p, comp.p, nv, cnt.p, w.p, X.p);
   count_launch(2);

@@ -21,6 +21,7 @@
 //    ascending-start BFS orders them.
 //  - Counters that many threads bump at once (per component, per instance)
 //    are warp-aggregated: one atomic per distinct key in a warp.
+#include "core_rows.cuh"
 #include "device_util.cuh"
 #include "stages.h"
 #include "pipeline.h"
@@ -128,26 +129,34 @@ __global__ void k_mark_arcs(const uint32_t *__restrict__ members, uint64_t m, ui
   }
 }
 
-// Small cores (at most PAIR_CORE_MAX vertices in all): adjacency and the pairs
-// that core cliques cover are bitmaps over core-local ids.  For k <= 5 a pair is
+// Small cores (every instance's at most PAIR_CORE_MAX vertices, its bitmaps together
+// within the budget's share): adjacency and the pairs that core cliques cover are
+// bitmaps over core-local ids, an instance's rows as wide as its own core (24 graphs
+// in four batches, cores of 5,786 vertices in the largest: 66 -> 34 ms, where
+// rows over all ids left that batch to listing and flows).  For k <= 5 a pair is
 // tested on the adjacency rows alone (does a clique of the k-2 other members fit
 // into the common neighbours?), which in a dense core the first candidate answers;
-// for larger k the listed cliques mark their pairs.
-constexpr uint32_t PAIR_CORE_MAX = 4096;
+// for larger k the listed cliques mark their pairs.  An edge covers itself, so k = 2
+// needs no such test and takes larger cores.
+constexpr uint32_t PAIR_CORE_MAX = 4096, EDGE_CORE_MAX = 16384;
+constexpr uint64_t BAND_BYTES = 4ull << 20;  // of both bitmaps, whatever the budget
 
 __global__ void k_core_bits(const uint64_t *__restrict__ doff, const uint32_t *__restrict__ dadj,
                             const uint32_t *__restrict__ outdeg, const uint32_t *__restrict__ in_core,
                             const uint64_t *__restrict__ lid, const uint32_t *__restrict__ core_vertex,
-                            uint32_t ncore, uint32_t words, uint32_t *__restrict__ adj) {
+                            uint32_t ncore, CoreRows r, uint32_t *__restrict__ adj) {
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-  for (uint32_t a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; a < ncore; a += warps) {
-    const uint32_t u = core_vertex[a], d = outdeg[u];
+  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < ncore; i += warps) {
+    const uint32_t u = core_vertex[i], d = outdeg[u];
+    const CoreBand bd = band_of(r, u);
+    uint32_t *rows = adj + bd.word;
+    const uint32_t a = i - bd.lid;
     for (uint32_t t = lane_id(); t < d; t += 32) {
       const uint32_t w = dadj[doff[u] + t];
       if (!in_core[w]) continue;
-      const uint32_t b = (uint32_t)lid[w];
-      atomicOr(adj + (size_t)a * words + (b >> 5), 1u << (b & 31));
-      atomicOr(adj + (size_t)b * words + (a >> 5), 1u << (a & 31));
+      const uint32_t b = (uint32_t)lid[w] - bd.lid;
+      atomicOr(rows + a * bd.width + (b >> 5), 1u << (b & 31));
+      atomicOr(rows + b * bd.width + (a >> 5), 1u << (a & 31));
     }
   }
 }
@@ -184,106 +193,60 @@ __device__ bool clique_in(const uint32_t (&M)[PAIR_CORE_MAX / 1024], const uint3
 }
 
 // bits: the covered pairs a < b; pairs counted per instance.  Warp per row word.
+// (bits comes in zeroed.)  parent: each id's smallest partner below it, which leaves
+// the union-find over the pairs little to join.
 template <int K>
-__global__ void k_cover(const uint32_t *__restrict__ adj, uint32_t words, uint32_t ncore,
-                        const uint32_t *__restrict__ core_vertex, const uint32_t *__restrict__ of_vertex,
-                        uint32_t *__restrict__ bits, unsigned long long *__restrict__ pairs) {
+__global__ void k_cover(const uint32_t *__restrict__ all, CoreRows r, uint32_t ncore,
+                        const uint32_t *__restrict__ core_vertex, uint32_t *__restrict__ bits,
+                        uint32_t *parent, unsigned long long *__restrict__ pairs) {
   constexpr uint32_t Q = PAIR_CORE_MAX / 1024;
-  const uint32_t warps = (gridDim.x * blockDim.x) >> 5, total = ncore * words;
-  for (uint32_t x = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; x < total; x += warps) {
-    const uint32_t a = x / words, w0 = x % words;
-    uint32_t m = adj[x], out = 0;
-    if (w0 < (a >> 5)) m = 0;
-    else if (w0 == (a >> 5)) m &= ~((2u << (a & 31)) - 1u);
-    for (uint32_t r = m; r; r &= r - 1) {
-      const uint32_t b = w0 * 32 + __ffs(r) - 1;
+  each_word(r, ncore, core_vertex, all, [&](uint32_t i, const CoreBand &bd, uint32_t w0, uint32_t m) {
+    const uint32_t *adj = all + bd.word;
+    const uint32_t a = i - bd.lid, words = bd.width;
+    uint32_t out = 0;
+    if (w0 == (a >> 5)) m &= ~((2u << (a & 31)) - 1u);
+    if (K == 2) out = m;
+    for (uint32_t rest = K == 2 ? 0u : m; rest; rest &= rest - 1) {
+      const uint32_t b = w0 * 32 + __ffs(rest) - 1;
       uint32_t M[Q];
 #pragma unroll
       for (uint32_t q = 0; q < Q; q++) {
         const uint32_t w = q * 32 + lane_id();
         M[q] = w < words ? adj[(size_t)a * words + w] & adj[(size_t)b * words + w] : 0u;
       }
-      if (clique_in<K - 2>(M, adj, words)) out |= r & (0u - r);
+      if (clique_in<K - 2>(M, adj, words)) out |= rest & (0u - rest);
     }
-    if (lane_id() == 0) {
-      bits[x] = out;
-      if (out) atomicAdd(&pairs[inst_of(of_vertex, core_vertex[a])], (unsigned long long)__popc(out));
+    const uint32_t b = bd.lid + w0 * 32 + lane_id();
+    if (((out >> lane_id()) & 1u) && __ldcg(parent + b) > i) atomicMin(parent + b, i);
+    if (lane_id() == 0 && out) {
+      bits[bd.word + a * words + w0] = out;
+      atomicAdd(&pairs[inst_of(r.of_vertex, core_vertex[i])], (unsigned long long)__popc(out));
     }
-  }
+  });
 }
 
 // core-local ids in vertex order: in_core scanned into lid, and the inverse
 // core_vertex[lid] = v (so the smallest id of a set of core vertices is its
 // smallest vertex)
 __global__ void k_core_vertex(const uint32_t *__restrict__ in_core, const uint64_t *__restrict__ lid, uint32_t n,
-                              uint32_t *__restrict__ core_vertex) {
+                              uint32_t *__restrict__ core_vertex, uint32_t *__restrict__ parent) {
   for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
-    if (in_core[v]) core_vertex[lid[v]] = v;
-}
-
-// Components of a small core in one block: union-find over the covered
-// pairs of the bitmap with the parents in shared memory (smaller id wins, so
-// a root is its component's smallest vertex); root[i] = the root of core id i.
-__device__ __forceinline__ uint32_t s_find(uint32_t *par, uint32_t x) {
-  uint32_t p = par[x];
-  while (p != x) {
-    const uint32_t gp = par[p];
-    if (gp != p) par[x] = gp;
-    x = p;
-    p = gp;
-  }
-  return x;
-}
-__global__ void __launch_bounds__(1024) k_small_components(const uint32_t *__restrict__ bits, uint32_t words,
-                                                           uint32_t ncore, uint32_t *__restrict__ root,
-                                                           uint32_t *__restrict__ err) {
-  __shared__ uint32_t par[PAIR_CORE_MAX];
-  for (uint32_t i = threadIdx.x; i < ncore; i += blockDim.x) par[i] = i;
-  __syncthreads();
-  const uint64_t total = (uint64_t)ncore * words;
-  for (uint64_t w = threadIdx.x; w < total; w += blockDim.x) {
-    uint32_t word = bits[w];
-    const uint32_t a0 = (uint32_t)(w / words), b0 = (uint32_t)(w % words) * 32;
-    while (word) {
-      const uint32_t b = b0 + (uint32_t)(__ffs(word) - 1);
-      word &= word - 1;
-      uint32_t a = a0, bb = b;
-      for (int tries = 0;; tries++) {
-        if (tries > (1 << 20)) {
-          atomicOr(err, DEV_ERR_TIMEOUT);
-          break;
-        }
-        const uint32_t ra = s_find(par, a), rb = s_find(par, bb);
-        if (ra == rb) break;
-        const uint32_t lo = ra < rb ? ra : rb, hi = ra < rb ? rb : ra;
-        if (atomicCAS(&par[hi], hi, lo) == hi) break;
-        a = lo;
-        bb = hi;
-      }
+    if (in_core[v]) {
+      const uint32_t a = (uint32_t)lid[v];
+      core_vertex[a] = v;
+      parent[a] = a;
     }
-  }
-  __syncthreads();
-  for (uint32_t i = threadIdx.x; i < ncore; i += blockDim.x) {
-    uint32_t r = i;
-    while (par[r] != r) r = par[r];
-    root[i] = r;
-  }
-}
-
-__global__ void k_comp_from_roots(const uint32_t *__restrict__ in_core, const uint64_t *__restrict__ lid,
-                                  const uint32_t *__restrict__ root, const uint32_t *__restrict__ core_vertex,
-                                  uint32_t n, uint32_t *__restrict__ comp) {
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
-    comp[v] = in_core[v] ? core_vertex[root[lid[v]]] : NONE;
 }
 
 __global__ void k_mark_pairs(const uint32_t *__restrict__ members, uint64_t m, uint32_t k,
-                             const uint64_t *__restrict__ lid, uint32_t words, uint32_t *__restrict__ bits) {
+                             const uint64_t *__restrict__ lid, CoreRows rows, uint32_t *__restrict__ all) {
   for (uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; c < m;
        c += (uint64_t)gridDim.x * blockDim.x) {
+    const CoreBand bd = band_of(rows, members[c * k]);
+    uint32_t *bits = all + bd.word;
     auto mark = [&](uint32_t a, uint32_t b) {
-      uint32_t *w = bits + (uint64_t)a * words + (b >> 5);
-      const uint32_t bit = 1u << (b & 31);
+      uint32_t *w = bits + (a - bd.lid) * bd.width + ((b - bd.lid) >> 5);
+      const uint32_t bit = 1u << ((b - bd.lid) & 31);
       if (!(*(volatile uint32_t *)w & bit)) atomicOr(w, bit);
     };
     if (k == 4) {  // the record in one 16-byte load, its local ids gathered together
@@ -308,17 +271,18 @@ __global__ void k_mark_pairs(const uint32_t *__restrict__ members, uint64_t m, u
 
 __global__ void k_pairs_to_arcs(const uint64_t *__restrict__ doff, const uint32_t *__restrict__ dadj,
                                 const uint32_t *__restrict__ outdeg, const uint32_t *__restrict__ in_core,
-                                const uint64_t *__restrict__ lid, uint32_t n, uint32_t words,
+                                const uint64_t *__restrict__ lid, uint32_t n, CoreRows rows,
                                 const uint32_t *__restrict__ bits, uint8_t *__restrict__ arc_keep) {
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
   for (uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < n; u += warps) {
     if (!in_core[u]) continue;
-    const uint32_t a = (uint32_t)lid[u];
+    const CoreBand bd = band_of(rows, u);
+    const uint32_t a = (uint32_t)lid[u] - bd.lid;
     for (uint32_t t = lane_id(); t < outdeg[u]; t += 32) {
       const uint32_t w = dadj[doff[u] + t];
       if (!in_core[w]) continue;
-      const uint32_t b = (uint32_t)lid[w];
-      if (bits[(uint64_t)a * words + (b >> 5)] & (1u << (b & 31))) arc_keep[doff[u] + t] = 1;
+      const uint32_t b = (uint32_t)lid[w] - bd.lid;
+      if (bits[bd.word + a * bd.width + (b >> 5)] & (1u << (b & 31))) arc_keep[doff[u] + t] = 1;
     }
   }
 }
@@ -348,6 +312,37 @@ __device__ __forceinline__ uint32_t uf_find(uint32_t *parent, uint32_t x) {
   return x;
 }
 
+__device__ __forceinline__ void unite(uint32_t *parent, uint32_t a, uint32_t b, uint32_t *err) {
+  for (int tries = 0;; tries++) {
+    if (tries > (1 << 20)) {
+      atomicOr(err, DEV_ERR_TIMEOUT);
+      return;
+    }
+    const uint32_t ra = uf_find(parent, a), rb = uf_find(parent, b);
+    if (ra == rb) return;
+    const uint32_t lo = ra < rb ? ra : rb, hi = ra < rb ? rb : ra;
+    if (atomicCAS(&parent[hi], hi, lo) == hi) return;
+    a = lo;
+    b = hi;
+  }
+}
+
+// of a small core: union-find over the covered pairs of the bitmap, by core-local id
+// (a warp a word: one block over all of them took 62 us at 463 vertices, with its two launches; this 50)
+__global__ void k_union_bits(const uint32_t *__restrict__ bits, CoreRows r, uint32_t ncore,
+                             const uint32_t *__restrict__ core_vertex, uint32_t *parent, uint32_t *err) {
+  each_word(r, ncore, core_vertex, bits, [&](uint32_t a, const CoreBand &bd, uint32_t w, uint32_t m) {
+    if (!((m >> lane_id()) & 1u)) return;
+    const uint32_t b = bd.lid + w * 32 + lane_id();
+    if (__ldcg(parent + a) != __ldcg(parent + b)) unite(parent, a, b, err);
+  });
+}
+__global__ void k_roots_bits(uint32_t *parent, const uint32_t *__restrict__ in_core, const uint64_t *__restrict__ lid,
+                             const uint32_t *__restrict__ core_vertex, uint32_t n, uint32_t *__restrict__ comp) {
+  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
+    comp[v] = in_core[v] ? core_vertex[uf_find(parent, (uint32_t)lid[v])] : NONE;
+}
+
 // union-find over the kept arcs: they connect exactly what the core cliques
 // connect, with at most m unions instead of (k-1)|Psi|
 __global__ void k_union(const uint64_t *__restrict__ doff, const uint32_t *__restrict__ dadj,
@@ -357,19 +352,7 @@ __global__ void k_union(const uint64_t *__restrict__ doff, const uint32_t *__res
   for (uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < n; u += warps) {
     for (uint32_t t = lane_id(); t < outdeg[u]; t += 32) {
       if (!keep[doff[u] + t]) continue;
-      uint32_t a = u, b = dadj[doff[u] + t];
-      for (int tries = 0;; tries++) {
-        if (tries > (1 << 20)) {
-          atomicOr(err, DEV_ERR_TIMEOUT);
-          break;
-        }
-        const uint32_t ra = uf_find(parent, a), rb = uf_find(parent, b);
-        if (ra == rb) break;
-        const uint32_t lo = ra < rb ? ra : rb, hi = ra < rb ? rb : ra;
-        if (atomicCAS(&parent[hi], hi, lo) == hi) break;
-        a = lo;
-        b = hi;
-      }
+      unite(parent, u, dadj[doff[u] + t], err);
     }
   }
 }
@@ -681,42 +664,64 @@ void densest_core_and_components(cds_ctx *c, cudaStream_t s, const Dag &gdag, co
 
   // prune: pairs inside >= 1 core clique
   uint64_t ncore = 0, m = 0;
+  std::vector<unsigned long long> hstats(2 * (size_t)ninst);
   {
-    std::vector<unsigned long long> h(2 * (size_t)ninst);
     HostReads r(s);
-    r.add(h.data(), stats.p, h.size());
+    r.add(hstats.data(), stats.p, hstats.size());
     r.wait();
     for (uint32_t i = 0; i < ninst; i++) {
-      ncore += h[i];
-      m += h[ninst + i];
+      ncore += hstats[i];
+      m += hstats[ninst + i];
     }
   }
-  const bool bitmap = m && n && ncore <= PAIR_CORE_MAX;  // marks over core-local ids
-  out.small = bitmap && k <= 5;                          // ... found on the adjacency alone
+  // marks over core-local ids; k <= 5: ... found on the adjacency alone
+  bool bitmap = m && n;
+  uint64_t words = 0;  // of a bitmap
+  {
+    std::vector<CoreBand> band(ninst);
+    uint64_t at = 0;
+    for (uint32_t i = 0; i < ninst; i++) {
+      const uint64_t size = hstats[i], width = (size + 31) / 32;
+      if (size > (k == 2 ? EDGE_CORE_MAX : PAIR_CORE_MAX)) bitmap = false;
+      band[i] = CoreBand{(uint32_t)at, (uint32_t)width, (uint32_t)words};
+      at += size;
+      words += size * width;
+      out.rows.words = std::max(out.rows.words, (uint32_t)width);
+      if (8 * words > std::max<uint64_t>(BAND_BYTES, c->budget / 64)) bitmap = false;
+    }
+    if (bitmap) {
+      out.band = DBuf<CoreBand>(c, s, ninst);
+      CDS_CUDA(cudaMemcpyAsync(out.band.p, band.data(), ninst * sizeof(CoreBand), cudaMemcpyHostToDevice, s));
+      out.rows.of_vertex = of_vertex;
+      out.rows.band = out.band.p;
+    }
+  }
+  out.small = bitmap && k <= 5;
   out.ncore = (uint32_t)ncore;
-  out.words = (uint32_t)((ncore + 31) / 32);
-  const uint32_t words = out.words;
   DBuf<uint64_t> lid(c, s, bitmap ? n + 1 : 0);
   DBuf<uint8_t> keep(c, s, 0);
+  DBuf<uint32_t> parent(c, s, bitmap ? ncore + 1 : n + 1);  // union-find, of core-local ids or vertices
   Dag dag;  // of the core, when its cliques are listed
   if (m && !out.small) list_core_cliques(c, s, gdag, k, t, out, dag, on_count);
   {
     ProfScope ps(c, s, "prune_arcs");
     if (bitmap) {
       out.core_vertex = DBuf<uint32_t>(c, s, ncore + 1);
-      out.bits = DBuf<uint32_t>(c, s, ncore * words + 1);
+      out.bits = DBuf<uint32_t>(c, s, words + 1);
+      out.bits.zero();
       scan_u32(in_core.p, lid.p, n, c, s);
-      k_core_vertex<<<G, 256, 0, s>>>(in_core.p, lid.p, n, out.core_vertex.p);
+      k_core_vertex<<<G, 256, 0, s>>>(in_core.p, lid.p, n, out.core_vertex.p, parent.p);
       count_launch();
     }
     if (out.small) {
-      DBuf<uint32_t> adj(c, s, ncore * words + 1);
+      DBuf<uint32_t> adj(c, s, words + 1);
       adj.zero();
       k_core_bits<<<G, 256, 0, s>>>(gdag.off.p, gdag.adj.p, gdag.outdeg.p, in_core.p, lid.p, out.core_vertex.p,
-                                    (uint32_t)ncore, words, adj.p);
-      void (*cover)(const uint32_t *, uint32_t, uint32_t, const uint32_t *, const uint32_t *, uint32_t *,
-                    unsigned long long *) = k == 2 ? k_cover<2> : k == 3 ? k_cover<3> : k == 4 ? k_cover<4> : k_cover<5>;
-      cover<<<G, 256, 0, s>>>(adj.p, words, (uint32_t)ncore, out.core_vertex.p, of_vertex, out.bits.p,
+                                    (uint32_t)ncore, out.rows, adj.p);
+      void (*cover)(const uint32_t *, CoreRows, uint32_t, const uint32_t *, uint32_t *, uint32_t *,
+                    unsigned long long *) =
+           k == 2 ? k_cover<2> : k == 3 ? k_cover<3> : k == 4 ? k_cover<4> : k_cover<5>;
+      cover<<<G, 256, 0, s>>>(adj.p, out.rows, (uint32_t)ncore, out.core_vertex.p, out.bits.p, parent.p,
                               stats.p + 2 * ninst);
       count_launch(2);
     } else if (m) {
@@ -724,9 +729,8 @@ void densest_core_and_components(cds_ctx *c, cudaStream_t s, const Dag &gdag, co
       keep.zero();
       const Cliques &cl = out.cliques;
       if (bitmap) {
-        out.bits.zero();
-        k_mark_pairs<<<G, 256, 0, s>>>(cl.members.p, m, k, lid.p, words, out.bits.p);
-        k_pairs_to_arcs<<<G, 256, 0, s>>>(dag.off.p, dag.adj.p, dag.outdeg.p, in_core.p, lid.p, n, words, out.bits.p,
+        k_mark_pairs<<<G, 256, 0, s>>>(cl.members.p, m, k, lid.p, out.rows, out.bits.p);
+        k_pairs_to_arcs<<<G, 256, 0, s>>>(dag.off.p, dag.adj.p, dag.outdeg.p, in_core.p, lid.p, n, out.rows, out.bits.p,
                                           keep.p);
         count_launch();
       } else {
@@ -744,15 +748,14 @@ void densest_core_and_components(cds_ctx *c, cudaStream_t s, const Dag &gdag, co
   out.cidx = DBuf<uint64_t>(c, s, n + 1);
   const DBuf<uint32_t> &comp = out.comp;
   const DBuf<uint64_t> &cidx = out.cidx;
-  DBuf<uint32_t> parent(c, s, bitmap ? 0 : n + 1), is_root(c, s, n + 1);
+  DBuf<uint32_t> is_root(c, s, n + 1);
   DBuf<unsigned long long> ccount(c, s, n + 1);  // core cliques per component root (may pass 2^32)
   ccount.zero();
   {
     ProfScope ps_cc(c, s, "components_unionfind");
     if (bitmap) {
-      DBuf<uint32_t> root(c, s, ncore + 1);
-      k_small_components<<<1, 1024, 0, s>>>(out.bits.p, words, (uint32_t)ncore, root.p, err.p);
-      k_comp_from_roots<<<G, 256, 0, s>>>(in_core.p, lid.p, root.p, out.core_vertex.p, n, comp.p);
+      k_union_bits<<<G, 256, 0, s>>>(out.bits.p, out.rows, (uint32_t)ncore, out.core_vertex.p, parent.p, err.p);
+      k_roots_bits<<<G, 256, 0, s>>>(parent.p, in_core.p, lid.p, out.core_vertex.p, n, comp.p);
       count_launch(2);
     } else if (n) {
       k_iota<<<G, 256, 0, s>>>(parent.p, n);

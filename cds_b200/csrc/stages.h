@@ -81,6 +81,16 @@ struct PeelOut {
 void peel(cds_ctx *c, cudaStream_t s, const uint64_t *off, const uint32_t *adj, uint64_t nnz, const Dag &dag,
           const Cliques &cl, const Instances &inst, uint32_t gl_buffer_size, PeelOut &out);
 
+// Rows of core-local ids over the ids of their own instance.
+struct CoreBand {
+  uint32_t lid, width, word;  // an instance's first id, words a row, first word
+};
+struct CoreRows {
+  const uint32_t *of_vertex = nullptr;  // instance of a vertex (null: one instance)
+  const CoreBand *band = nullptr;       // [instances]
+  uint32_t words = 0;                   // of the widest row
+};
+
 // Densest core, pruning and components; everything the flow stage needs.
 struct CoreOut {
   std::vector<uint64_t> threshold;  // per instance k'
@@ -99,12 +109,14 @@ struct CoreOut {
   DBuf<uint32_t> comp;      // [n] smallest vertex of each core vertex's component
   DBuf<uint64_t> cidx;      // [n+1] component index of a smallest vertex
   DBuf<uint32_t> local;     // [n] local vertex of each component vertex
-  // small cores (at most 4,096 vertices, k <= 5): the pairs that core cliques
-  // cover, over core-local ids (row a, column b > a)
+  // small cores (k <= 5): the pairs that core cliques cover, over core-local ids
+  // (row a, column b > a)
   bool small = false;
-  uint32_t ncore = 0, words = 0;
+  uint32_t ncore = 0;
+  CoreRows rows;
+  DBuf<CoreBand> band;
   DBuf<uint32_t> core_vertex;  // [ncore]
-  DBuf<uint32_t> bits;         // [ncore * words]
+  DBuf<uint32_t> bits;
   bool listed = false;
   Cliques cliques;          // every core clique, once a stage needed them
   DBuf<uint32_t> vmap;      // [nv] original vertex of each local vertex

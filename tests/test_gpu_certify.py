@@ -126,3 +126,22 @@ def test_units_of_many_cliques(both):
     g.free()
     assert s.num * n == math.comb(n, k) * s.den
     assert s.vertices.tolist() == list(range(n))
+
+
+@pytest.mark.parametrize("k", [2, 3, 4])
+def test_cores_of_a_batch_side_by_side(both, k):
+    # every core within its own rows, however many vertices they have together (with
+    # k = 2 one core is wider than any other and past the proof's size)
+    rng = np.random.default_rng(7)
+    graphs = [cds.gen_rmat(12, float(rng.uniform(6, 12)), i) for i in range(24)]
+    graphs.insert(5, cds.gen_er(5000, 12.0 / 5000, 3))
+    graphs.insert(0, cds.gen_er(40, 0.0, 4))  # no clique at all
+    gs = [both[0].graph(*g) for g in graphs]
+    params = cds.make_params(k)
+    got = both[0].solve_batch([(g, params) for g in gs])
+    for g, b in zip(gs, got):
+        s = both[0].solve(g, k)
+        assert (s.num, s.den, s.vertices.tolist(), s.pruned_edges, s.n_components, s.core_size) == (
+            b.num, b.den, b.vertices.tolist(), b.pruned_edges, b.n_components, b.core_size)
+        g.free()
+    assert k == 4 or sum(b.core_size for b in got) > 4096
