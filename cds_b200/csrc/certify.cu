@@ -33,18 +33,22 @@
 // A pass never stores a clique.  The component's covered pairs are a symmetric
 // bitmap of its vertices in shared memory; a warp takes a clique of k-2 vertices
 // (none for k = 2, a vertex for k = 3, an edge for k = 4), deals the later common
-// neighbours j to its lanes, and lane j walks the bits l of its row inside that
-// mask, adding 1 / (sum of weights).  Every clique is so met twice, from j and from
-// l, and each lane's sum belongs to its own j: met once, the sums of the last
+// neighbours j to its lanes, and goes through that mask's members l together: lane j
+// adds 1 / (sum of weights) where its row has l.  Every clique is so met twice, from j
+// and from l, and each lane's sum belongs to its own j: met once, the sums of the last
 // members need an atomic or a reduction per prefix, which cost five times the
-// arithmetic saved.  Bound by instruction issue, about 20 a visit.  The proof itself
+// arithmetic saved.  Bound by instruction issue, about 10 a member in single and 15 in
+// double precision.  (Each lane walking the bits of its own row wastes no step, but
+// finding a bit takes two operations of the unit that has the reciprocals, at a
+// quarter of the rate: 33.6 ms for the nine passes of 1.14 G 4-cliques, 29.3 with one
+// such operation, 23.8 this way.)  The proof itself
 // is in integers: a last pass splits k 2^s units of every clique exactly, and the
 // host checks E (and that the loads add up to every clique's units) in 128 bits.
 //
 // Measured against network build, warm split and push-relabel: 40 vertices and 1,499
 // triangles 0.39 -> 0.14 ms, 470 vertices and 25,761 edges 0.69 -> 0.25, 112 and
 // 1.18 M 4-cliques 1.5 -> 0.38, 746 and 9.3 M triangles 4.4 -> 1.3, 988 and 1.14 G
-// 4-cliques 295 -> 47 (and 62 GB of records and lists that are not built).
+// 4-cliques 295 -> 31 (and 62 GB of records and lists that are not built).
 #include "core_rows.cuh"
 #include "device_util.cuh"
 #include "stages.h"
@@ -174,27 +178,20 @@ __device__ __forceinline__ double pair_sums(const Shared &sh, uint32_t y0, uint3
     const float bf = (float)bj, wj = sh.wf[jq];
     double s = 0.0, s2 = 0.0;
     float f = 0.0f, f2 = 0.0f, sq = 0.0f;
-    for (uint32_t y = y0; y < y1; y += 2) {
-      const uint32_t m0 = __shfl_sync(CDS_FULL, mask, y), m1 = y + 1 < y1 ? __shfl_sync(CDS_FULL, mask, y + 1) : 0u;
-      if (!(m0 | m1)) continue;
-      // a visit from each word a step (absent ones take slot 0's weights, masked out)
-      uint32_t a0 = on ? m0 & row[y] : 0u, a1 = on && m1 ? m1 & row[y + 1] : 0u;
-      while (a0 | a1) {
-        const bool v0 = a0 != 0, v1 = a1 != 0;
-        const uint32_t l0 = v0 ? y * 32 + __ffs(a0) - 1 : 0u, l1 = v1 ? y * 32 + 31 + __ffs(a1) : 0u;
-        a0 &= a0 - 1;
-        a1 &= a1 - 1;
-        const float r0 = v0 ? rcp(bf + sh.wf[l0]) : 0.0f, r1 = v1 ? rcp(bf + sh.wf[l1]) : 0.0f;
-        if (WIDE) {
-          s += newton(bj + sh.w[l0], r0);  // (0 for an absent one)
-          s2 += newton(bj + sh.w[l1], r1);
-        } else {
-          f += r0;
-          f2 += r1;
-        }
-        const float z0 = r0 * wj, z1 = r1 * wj;  // shares: their squares stay in range
-        sq = fmaf(z0, z0, sq);
-        sq = fmaf(z1, z1, sq);
+    for (uint32_t y = y0; y < y1; y++) {
+      uint32_t m = __reduce_or_sync(CDS_FULL, lane == y ? mask : 0u);
+      if (!m) continue;
+      const uint32_t r = on ? row[y] : 0u;
+      const float *wf = sh.wf + y * 32;
+      const double *w = sh.w + y * 32;
+#pragma unroll
+      for (uint32_t b = 0; b < 32; b++) {
+        if (!((m >> b) & 1u)) continue;  // (the whole warp)
+        const float x = (r >> b) & 1u ? rcp(bf + wf[b]) : 0.0f;  // (0 for an absent one)
+        if (WIDE) (b & 1 ? s2 : s) += newton(bj + w[b], x);
+        else (b & 1 ? f2 : f) += x;
+        const float z = x * wj;  // shares: their squares stay in range
+        sq = fmaf(z, z, sq);
       }
     }
     if (WIDE) s += s2;
@@ -240,18 +237,19 @@ __device__ __forceinline__ void pair_shares(const Shared &sh, uint32_t y0, uint3
     for (uint32_t y = y0; y < y1; y++) {
       const uint32_t my = __shfl_sync(CDS_FULL, mask, y);
       if (!my) continue;
-      for (uint32_t m = on ? my & row[y] : 0u; m; m &= m - 1) {
-        const uint32_t l = y * 32 + __ffs(m) - 1;
+      for (uint32_t m = on ? my & row[y] : 0u; m;) {
+        const uint32_t b = 31 - __clz(m), l = y * 32 + b;
+        m ^= 1u << b;
         const double wl = sh.w[l], d = base + (wj + wl), inv = newton(d, rcp((float)d));
         unsigned long long a = (unsigned long long)(units * ((j < l ? wj : wl) * inv));  // the smaller one's
         a = a < all ? a : all;
-        unsigned long long b = all - a;  // and the larger one's
+        unsigned long long c = all - a;  // and the larger one's
         if (NP > 0) {
           const unsigned long long z = (unsigned long long)(units * ((j < l ? wl : wj) * inv));
-          b = z < b ? z : b;
+          c = z < c ? z : c;
         }
-        sum += j < l ? a : b;
-        if (j < l) rem += all - a - b;
+        sum += j < l ? a : c;
+        if (j < l) rem += all - a - c;
       }
     }
     if (sum) give(j, sum);
