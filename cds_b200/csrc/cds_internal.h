@@ -46,6 +46,13 @@ struct ProfEvent {
   const char *name;
   cudaEvent_t a, b;
 };
+// Small blocks freed on a stream, kept for the next allocation on it (see dalloc_bytes).
+struct SpareBlocks {
+  static constexpr size_t MAX_BLOCK = 4ull << 20, MAX_BYTES = 64ull << 20;
+  static constexpr int SIZES = 52;  // 256, 512, 768 bytes, then four sizes an octave
+  std::vector<void *> blocks[SIZES];
+  size_t bytes = 0;
+};
 }  // namespace cds
 
 struct cds_ctx {
@@ -59,8 +66,9 @@ struct cds_ctx {
   uint64_t budget = 0;
   std::atomic<uint64_t> in_use{0};
   std::atomic<uint64_t> peak{0};
-  std::mutex mu;  // guards sizes and err
+  std::mutex mu;  // guards sizes, spare and err
   std::unordered_map<void *, size_t> sizes;
+  std::unordered_map<cudaStream_t, cds::SpareBlocks> spare;
   std::string err;
   cds::Tuning tune[CDS_MAX_K + 1];
   // Cooperative (grid-barrier) kernels use 1/coop_div of the device, so that

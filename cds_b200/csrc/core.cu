@@ -771,61 +771,81 @@ void densest_core_and_components(cds_ctx *c, cudaStream_t s, const Dag &gdag, co
   }
   CDS_CUDA(cudaGetLastError());
   scan_u32(is_root.p, cidx.p, n, c, s);
-  // one wait for the component count, the per-instance statistics and the status
-  uint64_t ncomp64 = 0;
-  uint32_t e0 = 0;
+  // The components' sizes, clique counts, largest core numbers and smallest vertices,
+  // and local ids component by component (at most ncore of them).
+  std::vector<uint64_t> hv;
+  std::vector<unsigned long long> hc;
+  uint32_t ncomp = 0;
+  DBuf<uint32_t> csize(c, s, 0), cmax(c, s, 0), roots(c, s, 0), vcur(c, s, 0);
+  DBuf<unsigned long long> cclq(c, s, 0);
+  DBuf<uint64_t> vbeg(c, s, 0);
+  auto tables = [&](uint32_t slots) {  // for up to that many components
+    csize.alloc(slots);
+    cmax.alloc(slots);
+    roots.alloc(slots);
+    vcur.alloc(slots);
+    cclq.alloc(slots);
+    vbeg.alloc(slots + 1);
+    csize.zero();
+    cclq.zero();
+    cmax.zero();
+    vcur.zero();
+    k_comp_sizes<<<G, 256, 0, s>>>(comp.p, cidx.p, ccount.p, n, csize.p, cclq.p, pe.core.p, cmax.p);
+    k_gather_roots<<<G, 256, 0, s>>>(is_root.p, cidx.p, n, roots.p);
+    scan_u32(csize.p, vbeg.p, slots, c, s);
+    out.vmap = DBuf<uint32_t>(c, s, ncore + 1);
+    out.vcnet = DBuf<uint32_t>(c, s, ncore + 1);
+    out.local = DBuf<uint32_t>(c, s, n + 1);
+    k_local_ids<<<G, 256, 0, s>>>(comp.p, cidx.p, ccount.p, n, vbeg.p, vcur.p, out.local.p, out.vmap.p, out.vcnet.p);
+    count_launch(3);
+    CDS_CUDA(cudaGetLastError());
+    hv.resize(slots + 1);
+    hc.resize(slots);
+    out.comp_maxcore.resize(slots);
+    out.comp_root.resize(slots);
+  };
+  auto read_tables = [&](HostReads &r) {
+    r.add(hv.data(), vbeg.p, hv.size());
+    r.add(hc.data(), cclq.p, hc.size());
+    r.add(out.comp_maxcore.data(), cmax.p, hc.size());
+    r.add(out.comp_root.data(), roots.p, hc.size());
+  };
+  // One wait for the component count, the per-instance statistics and the status: of
+  // a core of few vertices, which bound its components, also for the tables (24 bytes
+  // a slot; a wait and the launches behind it cost about 15 us).
+  const uint32_t early = ncore && ncore <= 1024 ? (uint32_t)ncore : 0u;
+  if (early) tables(early);
   {
+    uint64_t ncomp64 = 0;
+    uint32_t e0 = 0;
     std::vector<unsigned long long> h(4 * (size_t)ninst);
     HostReads r(s);
     r.add(&ncomp64, cidx.p + n);
     r.add(&e0, err.p);
     r.add(h.data(), stats.p, h.size());
+    if (early) read_tables(r);
     r.wait();
     out.core_size.assign(h.begin(), h.begin() + ninst);
     out.core_cliques.assign(h.begin() + ninst, h.begin() + 2 * ninst);
     out.pruned_edges.assign(h.begin() + 2 * ninst, h.begin() + 3 * ninst);
     out.n_components.resize(ninst);
     for (uint32_t i = 0; i < ninst; i++) out.n_components[i] = (uint32_t)h[3 * ninst + i];
+    ncomp = (uint32_t)ncomp64;
+    if (e0 & DEV_ERR_TIMEOUT) fail(CDS_ERR_TIMEOUT, "components: union-find retry budget exhausted");
+    if (e0) fail(CDS_ERR_CUDA, "densest core: clique record is not a DAG path");
   }
-  const uint32_t ncomp = (uint32_t)ncomp64;
   out.ncomp = ncomp;
-  if (e0 & DEV_ERR_TIMEOUT) fail(CDS_ERR_TIMEOUT, "components: union-find retry budget exhausted");
-  if (e0) fail(CDS_ERR_CUDA, "densest core: clique record is not a DAG path");
-
+  if (ncomp && !early) {
+    tables(ncomp);
+    HostReads r(s);
+    read_tables(r);
+    r.wait();
+  }
   out.comp_inst.assign(ncomp, 0);
   out.comp_vbeg.assign(ncomp + 1, 0);
   out.comp_cbeg.assign(ncomp + 1, 0);
-  out.comp_maxcore.assign(ncomp, 0);
-  out.comp_root.assign(ncomp, 0);
-  if (ncomp == 0) return;
-  DBuf<uint32_t> csize(c, s, ncomp), cmax(c, s, ncomp), roots(c, s, ncomp);
-  DBuf<unsigned long long> cclq(c, s, ncomp);
-  csize.zero();
-  cclq.zero();
-  cmax.zero();
-  k_comp_sizes<<<G, 256, 0, s>>>(comp.p, cidx.p, ccount.p, n, csize.p, cclq.p, pe.core.p, cmax.p);
-  k_gather_roots<<<G, 256, 0, s>>>(is_root.p, cidx.p, n, roots.p);
-  DBuf<uint64_t> vbeg(c, s, ncomp + 1);
-  scan_u32(csize.p, vbeg.p, ncomp, c, s);
-  // local ids: component by component (at most ncore of them)
-  out.vmap = DBuf<uint32_t>(c, s, ncore + 1);
-  out.vcnet = DBuf<uint32_t>(c, s, ncore + 1);
-  out.local = DBuf<uint32_t>(c, s, n + 1);
-  DBuf<uint32_t> vcur(c, s, ncomp);
-  vcur.zero();
-  k_local_ids<<<G, 256, 0, s>>>(comp.p, cidx.p, ccount.p, n, vbeg.p, vcur.p, out.local.p, out.vmap.p, out.vcnet.p);
-  count_launch(3);
-  CDS_CUDA(cudaGetLastError());
-  std::vector<uint64_t> hv(ncomp + 1);
-  std::vector<unsigned long long> hc(ncomp);
-  {
-    HostReads r(s);
-    r.add(hv.data(), vbeg.p, ncomp + 1);
-    r.add(hc.data(), cclq.p, ncomp);
-    r.add(out.comp_maxcore.data(), cmax.p, ncomp);
-    r.add(out.comp_root.data(), roots.p, ncomp);
-    r.wait();
-  }
+  out.comp_maxcore.resize(ncomp);
+  out.comp_root.resize(ncomp);
   for (uint32_t i = 0; i < ncomp; i++) {
     out.comp_vbeg[i + 1] = (uint32_t)hv[i + 1];
     out.comp_cbeg[i + 1] = out.comp_cbeg[i] + hc[i];

@@ -1258,13 +1258,18 @@ void exact_search(cds_ctx *c, cudaStream_t s, const CoreOut &co, const Instances
   k_collect<<<G, 256, 0, s>>>(mark.p, co.vcnet.p, co.vmap.p, nv, dwant.p, outv.p, cnt.p);
   count_launch();
   CDS_CUDA(cudaGetLastError());
-  const uint32_t total = d2h(cnt.p, s);
-  std::vector<uint32_t> hv_out(total);
-  if (total) {
+  uint64_t expected = 0;  // every answer set has its density's denominator of vertices
+  for (uint32_t in = 0; in < ninst; in++) expected += ans.den[in];
+  if (expected > nv) fail(CDS_ERR_CUDA, "answer set size does not match its density denominator");
+  uint32_t total = 0;
+  std::vector<uint32_t> hv_out(expected);
+  {
     HostReads r(s);
-    r.add(hv_out.data(), outv.p, total);
+    r.add(&total, cnt.p);
+    if (expected) r.add(hv_out.data(), outv.p, expected);
     r.wait();
   }
+  if (total != expected) fail(CDS_ERR_CUDA, "answer set size does not match its density denominator");
   // split per instance (vertex ids are union ids; instances own id ranges)
   std::sort(hv_out.begin(), hv_out.end());
   for (uint32_t v : hv_out) {

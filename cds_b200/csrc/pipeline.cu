@@ -229,23 +229,21 @@ void run_problem(cds_ctx *c, cudaStream_t s, UnionGraph &u, const cds_params &pr
   densest_core_and_components(c, s, dag, pe, u.inst, k, t, co, &clk, on_count);
   const int m4 = clk.mark();
 
-  // per-instance clique totals
+  // per-instance clique totals (the copy is queued here and waited for with the answer)
   std::vector<unsigned long long> tot(ninst);
-  {
-    DBuf<unsigned long long> d(c, s, ninst);
-    k_inst_totals<<<std::max(1u, (ninst + 255) / 256), 256, 0, s>>>(cl.base.p, u.inst.vbeg.p, ninst, d.p);
-    count_launch();
-    CDS_CUDA(cudaGetLastError());
-    HostReads r(s);
-    r.add(tot.data(), d.p, ninst);
-    r.wait();
-  }
+  DBuf<unsigned long long> d_tot(c, s, ninst);
+  k_inst_totals<<<std::max(1u, (ninst + 255) / 256), 256, 0, s>>>(cl.base.p, u.inst.vbeg.p, ninst, d_tot.p);
+  count_launch();
+  CDS_CUDA(cudaGetLastError());
+  HostReads totals(s);
+  totals.add(tot.data(), d_tot.p, ninst);
 
   FlowAnswer fa;
   if (core_only) core_answer(s, pe, u, fa);
   else
     exact_search(c, s, co, u.inst, k, prm, t,
                  [&](const std::vector<uint8_t> &open) { build_networks(c, s, dag, u.inst, k, t, co, open, on_count); }, fa);
+  totals.wait();
   const int m5 = clk.mark();
   clk.wait();
   tms[CDS_T_DAG] = clk.ms(m0, m1);
