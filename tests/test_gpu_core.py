@@ -76,3 +76,34 @@ def test_later_sets_past_one_team(ctx, k, groups, m):
     assert core[0] == groups
     assert (core[1:] == deg).all() and largest == deg
     assert sol.max_core == deg and sol.peel_levels == 2
+
+
+@pytest.mark.parametrize("k", [3, 4])
+def test_levels_of_long_histograms(ctx, k):
+    # clique-core numbers on both sides of the 32,768 values from which the levels in
+    # use are gathered first, alone and as one batch (whose values add up)
+    graphs = []
+    for m in (60, 61) if k == 4 else (256, 259):  # largest values 32,509 / 34,220; 32,385 / 33,153
+        off, adj = cds.gen_er(m, 0.0, 1)
+        graphs.append(cds.gen_plant(off, adj, m, 1.0, 1)[:2])
+    off, adj = cds.gen_er(900, 14.0 / 900, 2)
+    graphs.append(cds.gen_plant(off, adj, 90, 0.8, 3)[:2])
+    graphs.append(cds.gen_er(20, 0.0, 1))  # no clique
+    gs = [ctx.graph(off, adj) for off, adj in graphs]
+    params = cds.make_params(k)
+    batch = ctx.solve_batch([(g, params) for g in gs])
+    for (off, adj), g, b in zip(graphs, gs, batch):
+        s = ctx.solve(g, k)
+        for r in (s, b):
+            assert (r.num, r.den, r.vertices.tolist(), r.max_core, r.core_threshold) == (
+                s.num, s.den, s.vertices.tolist(), s.max_core, s.core_threshold)
+        g.free()
+        if s.num == 0:
+            continue
+        if len(off) <= 260:  # a complete graph
+            m = len(off) - 1
+            want = np.full(m, comb(m - 1, k - 1))
+        else:
+            want = oracle.peel(off, adj, k)["core"]
+        assert s.max_core == int(want.max())
+        assert s.peel_levels == len(np.unique(want))
