@@ -8,8 +8,7 @@ b=c=0.19), with a planted 300-vertex community (p = 0.5), seed 4 -- about
 Synthetic data from the library's seeded generators (cds_b200.workloads).
 
   value  solves/s with the graph resident in HBM (device time, CUDA events
-         around each solve, L2 flushed between steps; the clique store is far
-         larger than L2 anyway), max over ranks
+         around each solve, L2 flushed between steps), max over ranks
   e2e    solves/s through cds_graph_from_csr + cds_solve from pinned host
          buffers, the upload and the answer copy-back inside the timed region
   kcliques_per_s   4-cliques listed per second of the listing stage
@@ -49,23 +48,23 @@ WORKLOAD = {"workload": "rmat18-ef16-plant300-k4-seed4",
             "graph": "R-MAT scale 18, edge factor 16, a=0.57 b=c=0.19, planted 300-vertex community p=0.5, seed 4",
             "n": 262144, "k": HEADLINE_K,
             "args": "pSize=8000 cpSize=16000 glBufferSize=0 partitionSize=30000 earlyStop=-1",
-            "l2": "inputs larger than L2 (the 4-clique store is ~37 GB); L2 also flushed (256 MiB write) between steps"}
+            "l2": "L2 flushed (256 MiB write) between steps"}
 SOLVE_ARGS = dict(p_size=8000, cp_size=16000, gl_buffer_size=0, partition_size=30000, early_stop=-1)
 RMAT14_KS = (2, 3, 4)
 # DRAM bytes (read + write) per launch of a kernel on a workload, from one ncu
 # capture each (profiles/ holds the summaries and the commands that made them)
-TRAFFIC = {("rmat18", "peel", 4): 1440400000000,  # 1.44 TB read + 371.2 MB written (ncu, 3 digits)
-           ("rmat18", "push_relabel", 4): 511000000000,  # 509.5 GB read + 1.49 GB written
-           ("rmat14", "peel", 4): 2181099520, ("rmat14", "push_relabel", 4): 59505920}
-TRAFFIC_SOURCE = {("rmat18", "peel", 4): "profiles/k_hindex_rmat18_k4.md",
-                  ("rmat18", "push_relabel", 4): "profiles/k_flow_rmat18_k4.md",
-                  ("rmat14", "peel", 4): "profiles/k_hindex_rmat14_k4.md",
+TRAFFIC = {("rmat18", "push_relabel", 4): 511000000000,  # 509.5 GB read + 1.49 GB written
+           ("rmat14", "push_relabel", 4): 59505920}
+TRAFFIC_SOURCE = {("rmat18", "push_relabel", 4): "profiles/k_flow_rmat18_k4.md",
                   ("rmat14", "push_relabel", 4): "profiles/k_flow_rmat14_k4.md"}
+# Reciprocals a second of one B200: 16 a clock on each of 148 SMs at 1,965 MHz
+RECIPROCALS = 148 * 16 * 1.965e9
 REASONS = {  # nvidia-smi clocks_event_reasons bits
     0x1: "gpu_idle", 0x2: "applications_clocks_setting", 0x4: "sw_power_cap", 0x8: "hw_slowdown",
     0x10: "sync_boost", 0x20: "sw_thermal_slowdown", 0x40: "hw_thermal_slowdown",
     0x80: "hw_power_brake_slowdown", 0x100: "display_clock_setting"}
-PSEUDO = ("peel_sweeps", "peel_reads", "flow_cycles", "flow_bfs", "flow_rounds", "flow_phase")
+PSEUDO = ("peel_sweeps", "peel_phase", "certify_pass", "certify_phase", "flow_cycles", "flow_bfs", "flow_rounds",
+          "flow_phase")
 
 
 def dist_env():
@@ -138,10 +137,10 @@ def listing_bytes(off, adj, k, cliques):
     return {"count": read, "write": read + 4 * k * cliques}
 
 
-def peel_bytes(n, k, cliques):
-    """Incidence reads, clique records and status once, the atomic
-    decrements, and the per-vertex arrays."""
-    return 4 * k * cliques + (4 * k + 4) * cliques + 8 * (k - 1) * cliques + 16 * (n + 1)
+def peel_bytes(n, arcs, k):
+    """Every row's neighbours, positions and weights once, and the per-vertex
+    arrays (a sweep's least; k = 2 has no weights)."""
+    return (12 if k > 2 else 4) * arcs + 16 * (n + 1)
 
 
 def max_over_ranks(values, device=None):
@@ -215,7 +214,7 @@ def dominant_roofline(prof, off, adj, k, sol, peaks, traffic_key):
     elif name.startswith("list_write"):
         alg = listing_bytes(off, adj, k, sol.total_cliques)["write"]
     elif name == "peel":
-        alg = peel_bytes(n, k, sol.total_cliques)
+        alg = peel_bytes(n, len(adj), k)
     elif name == "push_relabel":
         # one pass over the solved network: incidence id, member and 32-bit
         # flow state of every incidence, and the per-vertex state
@@ -224,17 +223,28 @@ def dominant_roofline(prof, off, adj, k, sol, peaks, traffic_key):
         alg = 0
     peak = float(peaks.get("hbm_gbs", 6650.0))
     avg_ms = ms / max(nl, 1)
-    achieved = alg / (avg_ms / 1e3) / 1e9 if avg_ms > 0 else 0.0
     tot = sum(v[1] for v in kern.values())
+    split = {"kernel_ms": {a: round(v[1], 3) for a, v in kern.items()},
+             "share": {a: round(v[1] / tot, 4) for a, v in kern.items()},
+             "peel_sweeps": int(prof.get("peel_sweeps", (0, 0))[1])}
+    if name == "certify":
+        # no bytes to speak of (the component sits in shared memory): a reciprocal for
+        # each of two visits to every core clique in every pass and the integer one
+        passes = int(prof.get("certify_passes", (0, 0))[1])
+        ops = 2 * sol.core_cliques * (passes + 1)
+        rate = ops / (avg_ms / 1e3) if avg_ms > 0 else 0.0
+        return {"bound": "sfu", "kernel": f"{name} (k={k})", "launches": nl, "avg_launch_ms": round(avg_ms, 4),
+                "algorithmic_ops": ops, "achieved": round(rate / 1e9, 2), "peak": round(RECIPROCALS / 1e9, 2),
+                "unit": "Greciprocals/s", "frac": round(rate / RECIPROCALS, 5),
+                "peak_source": "16 a clock and SM, 148 SMs, 1,965 MHz (nominal)", "passes": passes,
+                "traffic": None, "traffic_source": "profiles/k_certify_rmat18_k3.md", **split}
+    achieved = alg / (avg_ms / 1e3) / 1e9 if avg_ms > 0 else 0.0
     key = (traffic_key, name, k)
     return {"bound": "hbm", "kernel": f"{name} (k={k})", "launches": nl, "avg_launch_ms": round(avg_ms, 4),
             "algorithmic_bytes": alg, "achieved": round(achieved, 2), "peak": peak, "unit": "GB/s",
             "frac": round(achieved / peak, 5),
             "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)" if peaks else "fallback 6.65 TB/s",
-            "traffic": TRAFFIC.get(key), "traffic_source": TRAFFIC_SOURCE.get(key),
-            "kernel_ms": {a: round(v[1], 3) for a, v in kern.items()},
-            "share": {a: round(v[1] / tot, 4) for a, v in kern.items()},
-            "peel_sweeps": int(prof.get("peel_sweeps", (0, 0))[1])}
+            "traffic": TRAFFIC.get(key), "traffic_source": TRAFFIC_SOURCE.get(key), **split}
 
 
 def load_peaks():

@@ -483,9 +483,10 @@ class Context:
         keep the fastest in this context (cds_autotune); with cache_path the
         result is written as "k key value" lines, and when the file already
         holds lines for k they are loaded and nothing is timed.  Keys: list_warp_block,
-        list_warp_dmax, list_team_block, flow_rounds, flow_block, peel_chunk,
-        flow_warm (balancing passes before each max-flow; -1: by network
-        size), peel_order, flow_inc_per_block, peel_static."""
+        list_warp_dmax, list_team_block, flow_rounds, flow_block, flow_warm
+        (balancing passes before each max-flow; -1: a proof without a flow
+        first), flow_inc_per_block; peel_chunk, peel_order and peel_static are
+        kept without effect."""
         arr = (ctypes.c_void_p * len(graphs))(*[g.handle.value for g in graphs])
         self._check(lib().cds_autotune(self.handle, arr, len(graphs), k,
                                        cache_path.encode() if cache_path else None),

@@ -14,11 +14,11 @@
 // two or more workers at least one of them never takes a large request.
 //
 // Admission by memory, in two steps.  Before a batch starts it reserves a
-// bound on what its graphs, DAGs and listing work arrays take.  After the
-// listing's count pass, when |Psi| is known and before anything sized by it
-// is allocated, the worker reserves what the clique store, the peel's
-// incidence streams and the flow networks can take, waiting while that does
-// not fit what the budget has left and another batch is running.  A batch
+// bound on what its graphs, DAGs and per-arc arrays take.  Where the densest
+// cores' cliques have to be listed for max-flows, their number is known before
+// anything sized by it is allocated, and the worker reserves what their store
+// and the networks can take, waiting while that does not fit what the budget
+// has left and another batch is running.  A batch
 // that still runs out of device memory is split: each of its requests is
 // queued again to run alone, and only a request that fails alone reports
 // its error (CDS_ERR_OOM or another).  A request whose host CSR is malformed

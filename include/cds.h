@@ -216,10 +216,10 @@ cds_status cds_solve_batch(cds_ctx *ctx, const cds_job *jobs, size_t n,
  * into batches of the same k and size class and run them on their streams;
  * graphs of at least 2^20 arcs run alone, and with two or more workers one
  * always stays free for smaller requests.  Admission is by device memory:
- * a bound on the graph and listing state before a batch starts, then, once
- * the listing has counted |Psi|, what the clique store, peel and flow
- * networks can take (the worker waits while that does not fit and another
- * batch runs).  A batch that runs out of memory is split and its requests
+ * a bound on the graph and per-arc state before a batch starts, then, where
+ * max-flows are needed, what the store and networks of the densest cores'
+ * counted cliques can take (the worker waits while that does not fit and
+ * another batch runs).  A batch that runs out of memory is split and its requests
  * run again alone. */
 typedef struct cds_server_config {
   uint32_t max_batch;       /* instances per batch (0 = 64)                   */
@@ -248,17 +248,19 @@ cds_status cds_wait(cds_server *s, uint64_t ticket, cds_result *result);
 /* Finishes every admitted request, then stops the scheduler. */
 cds_status cds_server_stop(cds_server *s);
 
-/* Autotune: times the listing, peel and max-flow launch shapes on sample
+/* Autotune: times the listing and max-flow launch shapes on sample
  * graphs and keeps the fastest per clique size; results are cached in
  * cache_path (may be NULL) as "k key value" lines and used by later solves
  * on this context.  When the file already holds lines for k they are loaded
  * and nothing is timed (so n = 0 only loads).  Keys: list_warp_block,
- * list_warp_dmax, list_team_block, flow_rounds, flow_block, peel_chunk,
- * flow_warm, peel_order, flow_inc_per_block, peel_static; unknown keys and
+ * list_warp_dmax, list_team_block, flow_rounds, flow_block, flow_warm,
+ * flow_inc_per_block, and peel_chunk, peel_order, peel_static (accepted and
+ * kept, without effect: the peel has no work items); unknown keys and
  * out-of-range values are ignored.  flow_warm is the number of balancing
  * passes before each max-flow (weight updates, then the split of every
- * clique's units it starts from): 0 none, -1 (the default) three for
- * networks of 2^20 cliques or more and none below. */
+ * clique's units it starts from): 0 none, -1 (the default) tries to prove
+ * the answer by balanced shares without a flow first, and then takes the
+ * split from the weights that reached, or by size. */
 cds_status cds_autotune(cds_ctx *ctx, cds_graph *const *graphs, size_t n, uint32_t k,
                         const char *cache_path);
 
