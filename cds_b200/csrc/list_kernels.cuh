@@ -286,10 +286,32 @@ __device__ __forceinline__ uint32_t common(const uint32_t *a, const uint32_t *b,
 
 // A writing team: the local vertices and heavy ids, the prefix over the rows'
 // popcounts, the rows.
+// Its rows are an odd number of words apart: lanes reading different rows hit
+// different banks.
+__host__ __device__ constexpr uint32_t write_stride(uint32_t W) { return W | 1u; }
 __host__ __device__ constexpr uint32_t write_team_words(uint32_t dmax, bool rows_in_smem) {
   const uint32_t d4 = (dmax + 3) & ~3u;
-  return (3 * d4 + 4 + (rows_in_smem ? dmax * (((dmax + 31) / 32) | 1u) : 0u) + 3) & ~3u;
+  return (3 * d4 + 4 + (rows_in_smem ? dmax * write_stride((dmax + 31) / 32) : 0u) + 3) & ~3u;
 }
+
+// Words of a block's rows in global memory (out-degrees past BLOCK_DMAX), a multiple
+// of 16 bytes.  Both passes use the same slabs, each with its own stride, and neither
+// stride is the larger one everywhere (36 words: 36 counting, 37 writing).
+__host__ __device__ constexpr uint64_t rows_slab_words(uint32_t dmax) {
+  const uint32_t W = (dmax + 31) / 32, a = row_stride(W), b = write_stride(W);
+  return ((uint64_t)dmax * (a > b ? a : b) + 3) & ~(uint64_t)3;
+}
+// every root up to dmax fits: d rows, as far apart as for d vertices
+constexpr bool slabs_hold_their_rows() {
+  for (uint32_t dmax = 1025; dmax <= 8192; dmax++) {
+    const uint32_t W = (dmax + 31) / 32;
+    if (dmax * (uint64_t)row_stride(W) > rows_slab_words(dmax)) return false;
+    if (dmax * (uint64_t)write_stride(W) > rows_slab_words(dmax)) return false;
+    if (row_stride(W) < row_stride(W - 1) || write_stride(W) < write_stride(W - 1)) return false;  // (smaller d)
+  }
+  return true;
+}
+static_assert(slabs_hold_their_rows(), "rows in global memory leave their block's slab");
 
 // The (k-1)-cliques of the local graph G[A]: cnt[i] = those that hold A[i],
 // times k-2 (divided out by the caller), for K = 3, 4, 5 and any k (K = 0).
@@ -558,7 +580,7 @@ __global__ void k_list_write(ListParams p) {
       if (tr == 0) atomicOr(p.err, DEV_ERR_INTERNAL);
       continue;
     }
-    const uint32_t rs = W | 1u;  // odd stride: lanes reading different rows hit different banks
+    const uint32_t rs = write_stride(W);
     const uint32_t *Au = p.dadj + p.doff[u];
     for (uint32_t i = tr; i < d; i += ts) {
       const uint32_t a = Au[i];

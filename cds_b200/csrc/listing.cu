@@ -135,7 +135,7 @@ void run_listing(cds_ctx *c, cudaStream_t s, const cds::Dag &dag, cds::ListMode 
   uint32_t bdmax = std::max<uint32_t>(dag.max_out, warp_dmax + 1);
   if (K == 0 || K == 5) bdmax = std::min<uint32_t>(bdmax, DFS_WMAX * 32);
   const bool rows_in_smem = bdmax <= (uint32_t)BLOCK_DMAX;
-  const uint64_t brow_words = ((uint64_t)bdmax * row_stride((bdmax + 31) / 32) + 3) & ~3ull;  // 16-byte aligned slabs
+  const uint64_t brow_words = rows_slab_words(bdmax);
   DBuf<uint32_t> rows_global(c, s, 0);
   uint32_t bgrid_cap = 0;
   const bool any_block = dag.max_out > warp_dmax;

@@ -996,7 +996,7 @@ void peel(cds_ctx *c, cudaStream_t s, const uint64_t *off, const uint32_t *adj, 
       p.dmax = std::max<uint32_t>(k == 3 ? 4096 : 768, dag.max_out);
       const bool rows_in_smem = k == 3 || p.dmax <= (uint32_t)BLOCK_DMAX;
       if (!rows_in_smem) {
-        p.rows_slab = ((uint64_t)p.dmax * row_stride((p.dmax + 31) / 32) + 3) & ~3ull;
+        p.rows_slab = rows_slab_words(p.dmax);
         blocks = std::min<unsigned>(blocks, coop_grid(c, 1));
         rows.alloc((size_t)blocks * p.rows_slab);
         p.rows_global = rows.p;

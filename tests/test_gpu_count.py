@@ -76,3 +76,35 @@ def test_rows_past_shared_memory(ctx, s, k):
     g.free()
     assert got == comb(s, k) + comb(40, k)
     assert deg.tolist() == [comb(s - 1, k - 1)] * s + [comb(39, k - 1)] * 40
+
+
+# Cliques are also written where the rows are in global memory: sizes on both sides of
+# a multiple of 32 and where either pass has the wider rows.  All are past the proof's
+# component size, so the core's cliques are listed for the flows.
+@pytest.mark.parametrize("k", [3, 4])
+@pytest.mark.parametrize("s", [1026, 1122, 1140, 1152, 1398])
+def test_rows_past_shared_memory_are_written(ctx, s, k):
+    # s vertices joined to s others, which form s / (k-1) cliques among themselves
+    r = k - 1
+    low, high = np.meshgrid(np.arange(s), np.arange(s, 2 * s))
+    group = np.arange(s, 2 * s).reshape(-1, r)
+    x, y = np.triu_indices(r, 1)
+    off, adj = cds.csr_from_edges(2 * s, np.r_[low.ravel(), group[:, x].ravel()],
+                                  np.r_[high.ravel(), group[:, y].ravel()])
+    g = ctx.graph(off, adj)
+    sol = ctx.solve(g, k)
+    g.free()
+    # x low vertices and y groups hold x y cliques: most of them a vertex for all
+    assert sol.total_cliques == s * (s // r) == sol.num
+    assert sol.den == 2 * s and sol.vertices.tolist() == list(range(2 * s))
+
+
+@pytest.mark.parametrize("s", [1122, 1140, 1153, 1400])
+def test_complete_graphs_past_the_proof(ctx, s):
+    off = np.arange(s + 1, dtype=np.uint64) * (s - 1)
+    adj = np.broadcast_to(np.arange(s, dtype=np.uint32), (s, s))[~np.eye(s, dtype=bool)]
+    g = ctx.graph(off, adj)
+    sol = ctx.solve(g, 3)
+    g.free()
+    assert (sol.total_cliques, sol.num, sol.den) == (comb(s, 3), comb(s, 3), s)
+    assert sol.vertices.tolist() == list(range(s))
