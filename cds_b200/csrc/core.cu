@@ -238,33 +238,22 @@ __global__ void k_core_vertex(const uint32_t *__restrict__ in_core, const uint64
     }
 }
 
+// k >= 6.  Bits are of pairs a < b, as k_cover's: a record's members are in the order
+// of the DAG, which climbs in degree and not in id.
 __global__ void k_mark_pairs(const uint32_t *__restrict__ members, uint64_t m, uint32_t k,
                              const uint64_t *__restrict__ lid, CoreRows rows, uint32_t *__restrict__ all) {
   for (uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; c < m;
        c += (uint64_t)gridDim.x * blockDim.x) {
-    const CoreBand bd = band_of(rows, members[c * k]);
-    uint32_t *bits = all + bd.word;
-    auto mark = [&](uint32_t a, uint32_t b) {
-      uint32_t *w = bits + (a - bd.lid) * bd.width + ((b - bd.lid) >> 5);
-      const uint32_t bit = 1u << ((b - bd.lid) & 31);
-      if (!(*(volatile uint32_t *)w & bit)) atomicOr(w, bit);
-    };
-    if (k == 4) {  // the record in one 16-byte load, its local ids gathered together
-      const uint4 q = *reinterpret_cast<const uint4 *>(members + c * 4);
-      const uint32_t a0 = (uint32_t)lid[q.x], a1 = (uint32_t)lid[q.y], a2 = (uint32_t)lid[q.z],
-                     a3 = (uint32_t)lid[q.w];
-      mark(a0, a1);
-      mark(a0, a2);
-      mark(a0, a3);
-      mark(a1, a2);
-      mark(a1, a3);
-      mark(a2, a3);
-      continue;
-    }
     const uint32_t *r = members + c * k;
+    const CoreBand bd = band_of(rows, r[0]);
     for (uint32_t x = 0; x < k; x++) {
-      const uint32_t a = (uint32_t)lid[r[x]];
-      for (uint32_t y = x + 1; y < k; y++) mark(a, (uint32_t)lid[r[y]]);
+      const uint32_t u = (uint32_t)lid[r[x]] - bd.lid;
+      for (uint32_t y = x + 1; y < k; y++) {
+        const uint32_t v = (uint32_t)lid[r[y]] - bd.lid, a = min(u, v), b = max(u, v);
+        uint32_t *w = all + bd.word + a * bd.width + (b >> 5);
+        const uint32_t bit = 1u << (b & 31);
+        if (!(*(volatile uint32_t *)w & bit)) atomicOr(w, bit);
+      }
     }
   }
 }
@@ -281,8 +270,8 @@ __global__ void k_pairs_to_arcs(const uint64_t *__restrict__ doff, const uint32_
     for (uint32_t t = lane_id(); t < outdeg[u]; t += 32) {
       const uint32_t w = dadj[doff[u] + t];
       if (!in_core[w]) continue;
-      const uint32_t b = (uint32_t)lid[w] - bd.lid;
-      if (bits[bd.word + a * bd.width + (b >> 5)] & (1u << (b & 31))) arc_keep[doff[u] + t] = 1;
+      const uint32_t b = (uint32_t)lid[w] - bd.lid, lo = min(a, b), hi = max(a, b);
+      if (bits[bd.word + lo * bd.width + (hi >> 5)] & (1u << (hi & 31))) arc_keep[doff[u] + t] = 1;
     }
   }
 }
