@@ -969,8 +969,11 @@ void certify(cds_ctx *c, cudaStream_t s, const CoreOut &co, uint32_t k, const st
     const Comp &h = hc[i];
     const Level &l = hl[i];
     CertAnswer &o = out[i];
-    o.num = l.size ? (int64_t)l.psi : 0;
-    o.den = l.size;
+    if (l.size) {  // (a subset that the component cannot have: as if none had been found)
+      if (!l.psi || l.psi > co.comp_cbeg[i + 1] - co.comp_cbeg[i] || l.size > h.n) continue;
+      o.num = (int64_t)l.psi;
+      o.den = l.size;
+    }
     if (hstate[i] != REACHED) continue;
     const __int128 psi = (__int128)(co.comp_cbeg[i + 1] - co.comp_cbeg[i]);
     const __int128 cap = (__int128)k * l.p * one;  // times q, as all below

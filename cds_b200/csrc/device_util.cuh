@@ -280,9 +280,10 @@ constexpr int SCAN_THREADS = 512;
 constexpr int SCAN_ITEMS = 8;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 
+// (blocks of up to 1,024 threads: 32 warps' prefixes, and the total in a word of its own)
 template <class T>
 __device__ __forceinline__ T block_exclusive_scan(T v, T *total) {
-  __shared__ T s_warp[32];
+  __shared__ T s_warp[33];
   T inc = warp_inclusive_scan(v);
   const int w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
   if (lane_id() == 31) s_warp[w] = inc;
@@ -291,11 +292,11 @@ __device__ __forceinline__ T block_exclusive_scan(T v, T *total) {
     T x = (int)lane_id() < nw ? s_warp[lane_id()] : T(0);
     T xi = warp_inclusive_scan(x);
     if ((int)lane_id() < nw) s_warp[lane_id()] = xi - x;
-    if (lane_id() == 31) s_warp[31] = xi;  // nw <= 31 for blockDim <= 992
+    if (lane_id() == 31) s_warp[32] = xi;
   }
   __syncthreads();
   T r = s_warp[w] + inc - v;
-  if (total) *total = s_warp[31];
+  if (total) *total = s_warp[32];
   __syncthreads();
   return r;
 }

@@ -145,3 +145,39 @@ def test_cores_of_a_batch_side_by_side(both, k):
             b.num, b.den, b.vertices.tolist(), b.pruned_edges, b.n_components, b.core_size)
         g.free()
     assert k == 4 or sum(b.core_size for b in got) > 4096
+
+
+def two_rings(n, near, nearer, seed):
+    """Two rings of n / 2 vertices on mixed ids, one whose vertices are adjacent up to
+    distance `near`, one up to `nearer` < `near` - 1; ten vertices of the second are
+    joined to two neighbours of the first.  The first is the only densest set."""
+    size, rng = n // 2, np.random.default_rng(seed)
+    u, v = [], []
+    for first, m, reach in ((0, size, near), (size, n - size, nearer)):
+        for d in range(1, reach + 1):
+            u.append(first + np.arange(m))
+            v.append(first + (np.arange(m) + d) % m)
+    spread = np.arange(10) * (size // 10)
+    u += [spread, spread + 1]
+    v += [size + spread, size + spread]
+    ids = rng.permutation(n)
+    off, adj = cds.csr_from_edges(n, ids[np.concatenate(u)], ids[np.concatenate(v)])
+    return off, adj, np.sort(ids[:size])
+
+
+# components of a whole block of 1,024 threads, and some of whose last warp is partly or
+# wholly idle: the scan over the order's ranks spans up to 32 warps
+@pytest.mark.parametrize("k", [2, 3])
+@pytest.mark.parametrize("n", [700, 992, 993, 1000, 1023, 1024])
+def test_a_denser_subset_of_a_large_component(both, n, k):
+    off, adj, ring = two_rings(n, 12, 9, n + k)
+    proof = both[0]
+    proof.profile(True)
+    proof.profile_read()
+    a = answer(proof, off, adj, k)
+    launches = proof.profile_read()
+    proof.profile(False)
+    assert a == answer(both[1], off, adj, k)
+    assert a[0] == len(ring) * {2: 12, 3: 66}[k] and a[2] == ring.tolist()
+    assert a[4] == 1  # in one component with the other ring, and no flow was needed
+    assert "certify" in launches and "push_relabel" not in launches
