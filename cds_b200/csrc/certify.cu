@@ -969,6 +969,7 @@ void certify(cds_ctx *c, cudaStream_t s, const CoreOut &co, uint32_t k, const st
     const Comp &h = hc[i];
     const Level &l = hl[i];
     CertAnswer &o = out[i];
+    o.tried = true;
     if (l.size) {  // (a subset that the component cannot have: as if none had been found)
       if (!l.psi || l.psi > co.comp_cbeg[i + 1] - co.comp_cbeg[i] || l.size > h.n) continue;
       o.num = (int64_t)l.psi;

@@ -837,6 +837,7 @@ void exact_search(cds_ctx *c, cudaStream_t s, const CoreOut &co, const Instances
 
   const int G = c->sm_count * 4;
   DBuf<double> known;  // weights of components the proof gave up
+  bool all_known = true;  // of every component that is left to the flows
   DBuf<uint8_t> mark(c, s, nv + 1), fin(c, s, nnet);
   mark.zero();
   // Most components are their own densest set: where that can be proved without a
@@ -860,7 +861,10 @@ void exact_search(cds_ctx *c, cudaStream_t s, const CoreOut &co, const Instances
         cs.lb_d = found[i].den;
         cs.improved = true;
       }
-      if (!found[i].proven) continue;
+      if (!found[i].proven) {
+        if (cs.candidate) all_known = all_known && found[i].tried;
+        continue;
+      }
       cs.done = cs.certify = true;
       ncand--;
       ans.flows = 1;  // an assignment that saturates the network, as one max-flow finds
@@ -897,9 +901,10 @@ void exact_search(cds_ctx *c, cudaStream_t s, const CoreOut &co, const Instances
     DBuf<unsigned long long> cut(c, s, 2 * (size_t)nnet);
     DBuf<unsigned long long> bfsw(c, s, 4);
     // warm start: T - 1 weight updates, then the split (t.flow_warm; < 0: the split
-    // alone from weights that are known, else by size, three for networks of a
-    // million cliques or more; 0: none)
-    const uint32_t T = (uint32_t)std::min(255, t.flow_warm >= 0 ? t.flow_warm : known.p ? 1 : nc >= (1ull << 20) ? 3 : 0);
+    // alone where every network's weights are known, else by size, three for networks
+    // of a million cliques or more; 0: none)
+    const uint32_t T = (uint32_t)std::min(
+        255, t.flow_warm >= 0 ? t.flow_warm : known.p && all_known ? 1 : nc >= (1ull << 20) ? 3 : 0);
     DBuf<float> wgt(c, s, T ? nv + 1 : 0), wl(c, s, T ? nv + 1 : 0);
     DBuf<unsigned long long> wload(c, s, T ? nv + 1 : 0);
     bool wgt_init = false;

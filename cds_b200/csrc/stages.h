@@ -151,6 +151,7 @@ struct CertAsk {
   int64_t p = 0, q = 0;
 };
 struct CertAnswer {
+  bool tried = false;  // the balancing ran for it (weights are known)
   bool proven = false;
   int64_t num = 0, den = 0;
 };

@@ -181,3 +181,22 @@ def test_a_denser_subset_of_a_large_component(both, n, k):
     assert a[0] == len(ring) * {2: 12, 3: 66}[k] and a[2] == ring.tolist()
     assert a[4] == 1  # in one component with the other ring, and no flow was needed
     assert "certify" in launches and "push_relabel" not in launches
+
+
+def test_warm_start_by_the_networks_left(ctx):
+    # a network that the proof never saw (more than 1,024 vertices, few cliques) starts
+    # without a split, whatever else of its batch was proved
+    large = cds.gen_er(3000, 60.0 / 2999, 12)
+    small = cds.gen_plant(*cds.gen_er(2000, 0.004, 0), 40, 0.6, 0)[:2]
+    launches = []
+    for graphs in ((large,), (large, small)):
+        gs = [ctx.graph(off, adj) for off, adj in graphs]
+        ctx.profile(True)
+        ctx.profile_read()
+        ctx.solve_batch([(g, cds.make_params(3)) for g in gs])
+        launches.append(ctx.profile_read())
+        ctx.profile(False)
+        for g in gs:
+            g.free()
+    assert all("push_relabel" in x and "flow_warm" not in x for x in launches)
+    assert "certify" in launches[1] and "certify" not in launches[0]
