@@ -97,6 +97,7 @@ namespace cds {
 // Stream-ordered device allocation against the context budget.
 void *dalloc_bytes(cds_ctx *c, size_t bytes, cudaStream_t s);
 void dfree(cds_ctx *c, void *p, cudaStream_t s);
+void spare_release(cds_ctx *c);  // kept blocks back to the driver (under c->mu)
 
 template <class T>
 struct DBuf {
