@@ -107,3 +107,29 @@ def test_levels_of_long_histograms(ctx, k):
             want = oracle.peel(off, adj, k)["core"]
         assert s.max_core == int(want.max())
         assert s.peel_levels == len(np.unique(want))
+
+
+@pytest.mark.parametrize("gap", [0, 31, 20_000_000])
+def test_long_runs_of_isolated_vertices(ctx, gap):
+    # two triangles, two edges and a fan, whose arcs lie on both sides of the runs
+    first = np.array([0, 0, 1, 3]), np.array([1, 2, 2, 4])
+    fan = np.arange(40)
+    u, v = [first[0], first[0] + 5 + gap], [first[1], first[1] + 5 + gap]
+    base = 10 + 2 * gap
+    u += [np.full(40, base), base + 1 + fan[:-1]]
+    v += [base + 1 + fan, base + 2 + fan[:-1]]
+    n = base + 41
+    off, adj = cds.csr_from_edges(n, np.concatenate(u), np.concatenate(v))
+    g = ctx.graph(off, adj)
+    ctx.profile(True)
+    ctx.profile_read()
+    core, largest, total = ctx.clique_core(g, 3)
+    arcs_ms = ctx.profile_read()["peel_arcs"][1]
+    ctx.profile(False)
+    g.free()
+    want = np.zeros(n, np.int64)
+    want[[0, 1, 2]] = want[np.array([0, 1, 2]) + 5 + gap] = 1
+    want[base:] = 1  # a fan: every core holds a vertex of one triangle
+    assert total == 2 + 39 and largest == 1
+    assert np.array_equal(core.astype(np.int64), want)
+    assert arcs_ms < 100  # (the runs walked one vertex after another: 3,554 ms)
