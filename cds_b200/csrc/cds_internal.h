@@ -66,8 +66,12 @@ struct cds_ctx {
   uint64_t budget = 0;
   std::atomic<uint64_t> in_use{0};
   std::atomic<uint64_t> peak{0};
-  std::mutex mu;  // guards sizes, spare and err
-  std::unordered_map<void *, size_t> sizes;
+  std::mutex mu;  // guards sizes, held, spare and err
+  struct Block {
+    size_t bytes = 0, held = 0;  // asked for; asked of the driver
+  };
+  std::unordered_map<void *, Block> sizes;
+  uint64_t held = 0;  // of all blocks, spare ones too
   std::unordered_map<cudaStream_t, cds::SpareBlocks> spare;
   std::string err;
   cds::Tuning tune[CDS_MAX_K + 1];

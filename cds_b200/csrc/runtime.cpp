@@ -21,9 +21,10 @@ void cuda_check(cudaError_t e, const char *what) {
 // them were a tenth of the smallest solve's time (2,000 vertices: 0.91 -> 0.83 ms).
 // Blocks of up to MAX_BLOCK bytes are therefore kept, by stream and rounded size, when
 // they are freed: what a stream freed, its later work may use in the same order the
-// driver would keep.  At most MAX_BYTES a stream; all of it goes back to the driver
-// when an allocation fails and when the context ends.  The budget counts what is in
-// use, as requested.
+// driver would keep.  At most MAX_BYTES a stream, and no more than the budget leaves
+// beside what is in use; all of it goes back to the driver when it is in the way of an
+// allocation and when the context ends.  The budget is checked against what is in use,
+// as requested (the rounding adds at most a quarter of the small blocks to that).
 namespace {
 
 // index and bytes of the rounded size (at most a quarter more than asked)
@@ -42,91 +43,114 @@ int spare_size(size_t bytes, size_t *rounded) {
   *rounded = (q << e) * 256;
   return 3 + 4 * e + (int)(q - 4);
 }
+size_t class_bytes(int size) {
+  return size < 3 ? 256 * ((size_t)size + 1) : (size_t)(4 + (size - 3) % 4) << ((size - 3) / 4 + 8);
+}
 
 }  // namespace
 
 void spare_release(cds_ctx *c) {
-  for (auto &st : c->spare) {
-    for (auto &v : st.second.blocks) {
+  for (auto &st : c->spare)
+    for (int size = 0; size < SpareBlocks::SIZES; size++) {
+      auto &v = st.second.blocks[size];
       for (void *p : v) cudaFreeAsync(p, st.first);
+      c->held -= v.size() * class_bytes(size);
+      st.second.bytes -= v.size() * class_bytes(size);
       v.clear();
     }
-    st.second.bytes = 0;
-  }
 }
 
 void *dalloc_bytes(cds_ctx *c, size_t bytes, cudaStream_t s) {
   if (bytes == 0) return nullptr;
   bytes = (bytes + 255) & ~size_t(255);
   const uint64_t now = c->in_use.fetch_add(bytes) + bytes;
-  if (now > c->budget) {
-    c->in_use.fetch_sub(bytes);
-    fail(CDS_ERR_OOM, "device memory budget exceeded (" + std::to_string(now) + " > " +
-                          std::to_string(c->budget) + " bytes)");
-  }
-  const auto note_peak = [&] {
-    uint64_t pk = c->peak.load();
-    while (now > pk && !c->peak.compare_exchange_weak(pk, now)) {
-    }
-  };
-  size_t rounded = bytes;
   void *p = nullptr;
-  if (bytes <= SpareBlocks::MAX_BLOCK) {
-    const int size = spare_size(bytes, &rounded);
-    std::lock_guard<std::mutex> g(c->mu);
-    SpareBlocks &sp = c->spare[s];
-    if (!sp.blocks[size].empty()) {
-      p = sp.blocks[size].back();
-      sp.blocks[size].pop_back();
-      sp.bytes -= rounded;
-      c->sizes[p] = bytes;
-      note_peak();
-      return p;
-    }
-  }
-  cudaError_t e = cudaMallocFromPoolAsync(&p, rounded, c->pool, s);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
+  size_t held = 0;  // what the driver was asked for
+  try {
+    if (now > c->budget)
+      fail(CDS_ERR_OOM, "device memory budget exceeded (" + std::to_string(now) + " > " +
+                            std::to_string(c->budget) + " bytes)");
     {
       std::lock_guard<std::mutex> g(c->mu);
-      spare_release(c);
+      size_t want = bytes;
+      if (bytes <= SpareBlocks::MAX_BLOCK) {
+        const int size = spare_size(bytes, &want);
+        SpareBlocks &sp = c->spare[s];
+        auto &v = sp.blocks[size];
+        if (!v.empty()) {
+          c->sizes[v.back()] = {bytes, want};
+          p = v.back();
+          v.pop_back();
+          sp.bytes -= want;
+        }
+      }
+      if (!p) {
+        if (c->held + want > c->budget) spare_release(c);
+        if (c->held + want > c->budget) want = bytes;
+        c->held += held = want;
+      }
     }
-    e = cudaMallocFromPoolAsync(&p, rounded, c->pool, s);
-  }
-  if (e != cudaSuccess) {
+    if (!p) {
+      cudaError_t e = cudaMallocFromPoolAsync(&p, held, c->pool, s);
+      if (e != cudaSuccess) {
+        cudaGetLastError();
+        {
+          std::lock_guard<std::mutex> g(c->mu);
+          spare_release(c);
+        }
+        p = nullptr;
+        e = cudaMallocFromPoolAsync(&p, held, c->pool, s);
+      }
+      if (e != cudaSuccess) {
+        cudaGetLastError();
+        p = nullptr;
+        fail(CDS_ERR_OOM, std::string("device allocation failed: ") + cudaGetErrorString(e));
+      }
+      std::lock_guard<std::mutex> g(c->mu);
+      c->sizes[p] = {bytes, held};
+    }
+  } catch (...) {
+    if (held) {
+      if (p) cudaFreeAsync(p, s);
+      std::lock_guard<std::mutex> g(c->mu);
+      c->held -= held;
+    }
     c->in_use.fetch_sub(bytes);
-    cudaGetLastError();
-    fail(CDS_ERR_OOM, std::string("device allocation failed: ") + cudaGetErrorString(e));
+    throw;
   }
-  note_peak();
-  std::lock_guard<std::mutex> g(c->mu);
-  c->sizes[p] = bytes;
+  uint64_t pk = c->peak.load();
+  while (now > pk && !c->peak.compare_exchange_weak(pk, now)) {
+  }
   return p;
 }
 
+// Called by destructors: where keeping the block takes host memory that is not
+// there, it goes back to the driver.
 void dfree(cds_ctx *c, void *p, cudaStream_t s) {
-  size_t bytes = 0;
+  cds_ctx::Block b;
   bool kept = false;
   {
     std::lock_guard<std::mutex> g(c->mu);
     auto it = c->sizes.find(p);
     if (it != c->sizes.end()) {
-      bytes = it->second;
+      b = it->second;
       c->sizes.erase(it);
     }
-    if (bytes && bytes <= SpareBlocks::MAX_BLOCK) {
-      size_t rounded;
-      const int size = spare_size(bytes, &rounded);
-      SpareBlocks &sp = c->spare[s];
-      if (sp.bytes + rounded <= SpareBlocks::MAX_BYTES) {
-        sp.blocks[size].push_back(p);
-        sp.bytes += rounded;
-        kept = true;
+    size_t rounded = 0;
+    const int size = b.bytes && b.bytes <= SpareBlocks::MAX_BLOCK ? spare_size(b.bytes, &rounded) : -1;
+    if (size >= 0 && b.held == rounded) try {
+        SpareBlocks &sp = c->spare[s];
+        if (sp.bytes + rounded <= SpareBlocks::MAX_BYTES) {
+          sp.blocks[size].push_back(p);
+          sp.bytes += rounded;
+          kept = true;
+        }
+      } catch (const std::bad_alloc &) {
       }
-    }
+    if (!kept) c->held -= b.held;
   }
   if (!kept) cudaFreeAsync(p, s);
-  c->in_use.fetch_sub(bytes);
+  c->in_use.fetch_sub(b.bytes);
 }
 
 namespace {

@@ -42,7 +42,10 @@ const char *cudaGetErrorString(cudaError_t) { return "error"; }
 cudaError_t cudaMallocFromPoolAsync(void **p, size_t n, cudaMemPool_t, cudaStream_t) {
   if (live_bytes + n > driver_limit) return cudaErrorMemoryAllocation;
   *p = std::malloc(1);
+  const long left = news_left;  // (the test's own notes always fit)
+  news_left = -1;
   live[*p] = n;
+  news_left = left;
   live_bytes += n;
   if (live_bytes > live_peak) live_peak = live_bytes;
   driver_calls++;
@@ -116,4 +119,88 @@ def test_nested_reads(tmp_path):
       }
       outer.wait();
       assert(x == 1);
+    """)
+
+
+def test_kept_blocks_stay_within_the_budget(tmp_path):
+    # sizes that are no other's class: what was kept for one does not serve the next
+    run(tmp_path, """
+      cds_ctx c;
+      c.budget = 1 << 20;
+      for (size_t n : {300u << 10, 200u << 10, 150u << 10, 700u << 10, 90u << 10, 1024u << 10}) {
+        std::vector<void *> p;
+        for (size_t i = 0; i < (1u << 20) / n; i++) p.push_back(dalloc_bytes(&c, n, stream(1 + i % 3)));
+        for (size_t i = 0; i < p.size(); i++) dfree(&c, p[i], stream(1 + i % 3));
+        assert(c.in_use.load() == 0);
+      }
+      assert(live_peak <= c.budget + c.budget / 4);  // (rounding, of blocks in use)
+      assert(c.held == live_bytes);
+    """)
+
+
+def test_kept_blocks_serve_their_stream_and_are_bounded(tmp_path):
+    run(tmp_path, """
+      cds_ctx c;
+      c.budget = 1ull << 40;
+      void *a = dalloc_bytes(&c, 1000, stream(1));
+      dfree(&c, a, stream(1));
+      void *b = dalloc_bytes(&c, 1000, stream(2));
+      assert(b != a && driver_calls == 2);
+      assert(dalloc_bytes(&c, 900, stream(1)) == a && driver_calls == 2);
+      dfree(&c, a, stream(1));
+      dfree(&c, b, stream(2));
+      std::vector<void *> p;
+      for (int i = 0; i < 100; i++) p.push_back(dalloc_bytes(&c, 3u << 20, stream(1)));
+      p.push_back(dalloc_bytes(&c, 64u << 20, stream(1)));
+      for (void *q : p) dfree(&c, q, stream(1));
+      assert(live_bytes <= SpareBlocks::MAX_BYTES + 1024);
+      // an allocation that the driver refuses gets everything back first
+      driver_limit = live_bytes + (1u << 20);
+      void *d = dalloc_bytes(&c, 32u << 20, stream(2));
+      assert(live_bytes == 32u << 20);
+      dfree(&c, d, stream(2));
+      bool refused = false;
+      try {
+        dalloc_bytes(&c, 1ull << 30, stream(2));
+      } catch (const Error &e) {
+        refused = e.status == CDS_ERR_OOM;
+      }
+      assert(refused && c.in_use.load() == 0 && live_bytes == 0);
+    """)
+
+
+def test_no_host_memory(tmp_path):
+    # buffers are freed by destructors: a failure to keep a block must not leave them
+    run(tmp_path, """
+      for (long left = 0; left < 4; left++) {
+        cds_ctx c;
+        c.budget = 1ull << 40;
+        std::vector<void *> p;
+        for (int i = 0; i < 40; i++) p.push_back(dalloc_bytes(&c, 4096 << (i % 9), stream(1 + i % 2)));
+        for (int i = 0; i < 40; i++) {
+          news_left = left;
+          dfree(&c, p[i], stream(3 + i % 5));
+          news_left = -1;
+        }
+        assert(c.in_use.load() == 0);
+        size_t before = live_bytes;
+        int refused = 0;
+        for (int i = 0; i < 8; i++) {
+          news_left = i % 2 ? left : 0;
+          try {
+            void *q = dalloc_bytes(&c, 777777 + 4096 * i, stream(9));
+            news_left = -1;
+            dfree(&c, q, stream(9));
+          } catch (...) {
+            news_left = -1;
+            refused++;
+            assert(live_bytes == before);
+          }
+          before = live_bytes;
+          assert(c.in_use.load() == 0);
+        }
+        assert(refused);
+        spare_release(&c);
+        assert(live_bytes == 0);
+      }
     """)
