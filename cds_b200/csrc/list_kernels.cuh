@@ -249,6 +249,25 @@ __device__ void dfs_common(const uint32_t *rows, uint32_t rs, uint32_t W, const 
   }
 }
 
+// Cliques of `size` (2 or more) vertices of mask M, over symmetric rows of one word.
+__device__ __forceinline__ unsigned long long cliques_in_word(const uint32_t *rows, uint32_t M, int size) {
+  uint32_t left[CDS_MAX_K];  // by members chosen: who may be the next
+  unsigned long long total = 0;
+  int l = 0;
+  left[0] = M;
+  for (;;) {
+    const uint32_t m = left[l];
+    if ((int)__popc(m) < size - l) {
+      if (l-- == 0) return total;
+      continue;
+    }
+    left[l] = m & (m - 1);
+    const uint32_t next = left[l] & rows[__ffs(m) - 1];
+    if (l + 2 == size) total += __popc(next);
+    else left[++l] = next;
+  }
+}
+
 // Words from one symmetric row to the next: a row of more than one word is
 // padded with zeros to whole 16-byte pieces, an odd number of them apart, so that
 // eight lanes reading a piece each of different rows meet different banks.
@@ -364,14 +383,16 @@ __device__ void local_count(const uint32_t *A, const uint32_t *hid, uint32_t d, 
     T::sync();
   }
   if (K == 3) return;
-  if (!TB && (K == 4 || K == 5) && W == 1) {
+  if (!TB && W == 1) {
     const uint32_t row = lane < d ? rows[lane * rs] : 0u;
-    uint32_t s = 0;
+    C s = 0;
     if (K == 4) {
       for (uint32_t j = 0; j < d; j++) {
         const uint32_t rj = __shfl_sync(CDS_FULL, row, j);
         if ((row >> j) & 1u) s += __popc(row & rj);
       }
+    } else if (K == 0) {  // each lane the cliques among its own neighbours, no step shared and none atomic
+      s = cliques_in_word(rows, row, kk - 2) * (uint32_t)(kk - 2);
     } else {
       for (uint32_t m = row; m; m &= m - 1) {
         const uint32_t j = __ffs(m) - 1;

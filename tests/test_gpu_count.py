@@ -108,3 +108,19 @@ def test_complete_graphs_past_the_proof(ctx, s):
     g.free()
     assert (sol.total_cliques, sol.num, sol.den) == (comb(s, 3), comb(s, 3), s)
     assert sol.vertices.tolist() == list(range(s))
+
+
+@pytest.mark.parametrize("k", [6, 7, 8, 12, 16])
+def test_one_word_neighbourhoods_of_large_cliques(ctx, k):
+    sizes = (k - 1, k, k + 1, 20) + ((32, 33) if k < 12 else (24,))
+    off, adj = complete(sizes)
+    g = ctx.graph(off, adj)
+    got, deg = ctx.list_cliques(g, k)
+    core, _, _ = ctx.clique_core(g, k)
+    g.free()
+    assert got == sum(comb(s, k) for s in sizes)
+    assert deg.tolist() == [comb(s - 1, k - 1) for s in sizes for _ in range(s)] == core.tolist()
+    off, adj = cds.gen_er(300, 0.0, 1)
+    for i in range(3):
+        off, adj, _ = cds.gen_plant(off, adj, 30, 0.8 if k < 12 else 0.95, 10 * k + i)
+    check(ctx, off, adj, k)
