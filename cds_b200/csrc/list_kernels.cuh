@@ -211,6 +211,7 @@ __device__ __forceinline__ bool heavy_words(const HeavyBits &hb, const uint32_t 
 // Depth-first enumeration of the `depth`-cliques {l1 < l2 < ...} inside mask M
 // from position `first` on, over symmetric rows; leaf(path, s) for each, with
 // s = the vertices adjacent to all of the path inside M.  Only for k >= 6.
+// A path goes on only where the vertices left can complete it and leave one more.
 template <class Leaf>
 __device__ void dfs_common(const uint32_t *rows, uint32_t rs, uint32_t W, const uint32_t *M, uint32_t first,
                            int depth, Leaf leaf) {
@@ -240,16 +241,103 @@ __device__ void dfs_common(const uint32_t *rows, uint32_t rs, uint32_t W, const 
     }
     for (uint32_t w = 0; w < W; w++) {
       stack[lvl + 1][w] = stack[lvl][w] & row[w];
-      c |= stack[lvl + 1][w];
+      c += __popc(stack[lvl + 1][w]);
     }
-    if (c) {
+    if ((int)c >= depth - lvl) {
       lvl++;
       pos[lvl] = found + 1;
     }
   }
 }
 
-// Cliques of `size` (2 or more) vertices of mask M, over symmetric rows of one word.
+// The same in registers, for a path of D vertices over rows of two to four words (the
+// second pair of words zero where there are two; later: the bits of M a path may take
+// next).  Adds what it finds to the path's counts; returns the sum of s.
+struct Bits128 {
+  unsigned long long lo, hi;
+  __device__ __forceinline__ uint32_t size() const { return __popcll(lo) + __popcll(hi); }
+  __device__ __forceinline__ Bits128 operator&(const Bits128 &o) const { return {lo & o.lo, hi & o.hi}; }
+};
+__device__ __forceinline__ Bits128 row_bits(const uint32_t *row) {  // (16-byte rows, padded with zeros)
+  const uint4 x = *reinterpret_cast<const uint4 *>(row);
+  return {(unsigned long long)x.y << 32 | x.x, (unsigned long long)x.w << 32 | x.z};
+}
+template <int D, class C>
+__device__ __forceinline__ uint32_t paths_common(const uint32_t *rows, uint32_t rs, Bits128 M, Bits128 later, C *cnt) {
+  uint32_t sum = 0;
+  while (later.lo | later.hi) {
+    uint32_t l;
+    if (later.lo) {
+      l = __ffsll((long long)later.lo) - 1;
+      later.lo &= later.lo - 1;
+    } else {
+      l = 64 + __ffsll((long long)later.hi) - 1;
+      later.hi &= later.hi - 1;
+    }
+    const Bits128 row = row_bits(rows + l * rs), N = M & row;
+    uint32_t s = N.size();
+    if constexpr (D > 1) s = s >= D ? paths_common<D - 1>(rows, rs, N, later & row, cnt) : 0u;
+    if (s) {
+      atomicAdd(&cnt[l], C(s));
+      sum += s;
+    }
+  }
+  return sum;
+}
+
+// The same for wider rows: the words of the P rows of the pair and the path so far are
+// read again at each step (a stack of masks would be in local memory).
+template <int P, int D, class C>
+__device__ __forceinline__ uint32_t paths_wide(const uint32_t *rows, uint32_t rs, uint32_t W, const uint32_t *(&r)[P],
+                                               uint32_t from, C *cnt) {
+  uint32_t sum = 0;
+  for (uint32_t w = from >> 5; w < W; w++) {
+    uint32_t m = w == (from >> 5) ? 0xFFFFFFFFu << (from & 31) : 0xFFFFFFFFu;
+#pragma unroll
+    for (int x = 0; x < P; x++) m &= r[x][w];
+    for (; m; m &= m - 1) {
+      const uint32_t l = w * 32 + __ffs(m) - 1;
+      const uint32_t *q[P + 1];
+#pragma unroll
+      for (int x = 0; x < P; x++) q[x] = r[x];
+      q[P] = rows + l * rs;
+      uint32_t s = 0;
+      for (uint32_t y = 0; y < W; y += 4) {
+        uint4 a = *reinterpret_cast<const uint4 *>(q[0] + y);
+#pragma unroll
+        for (int x = 1; x <= P; x++) {
+          const uint4 b = *reinterpret_cast<const uint4 *>(q[x] + y);
+          a.x &= b.x;
+          a.y &= b.y;
+          a.z &= b.z;
+          a.w &= b.w;
+        }
+        s += __popc(a.x) + __popc(a.y) + __popc(a.z) + __popc(a.w);
+      }
+      if constexpr (D > 1) s = s >= D ? paths_wide<P + 1, D - 1>(rows, rs, W, q, l + 1, cnt) : 0u;
+      if (s) {
+        atomicAdd(&cnt[l], C(s));
+        sum += s;
+      }
+    }
+  }
+  return sum;
+}
+
+// Cliques of S vertices of mask M, over symmetric rows of one word.
+template <int S>
+__device__ __forceinline__ uint32_t word_cliques(const uint32_t *rows, uint32_t M) {
+  uint32_t total = 0;
+  while (__popc(M) >= S) {
+    const uint32_t l = __ffs(M) - 1;
+    M &= M - 1;
+    const uint32_t N = M & rows[l];
+    if constexpr (S == 2) total += __popc(N);
+    else total += word_cliques<S - 1>(rows, N);
+  }
+  return total;
+}
+// The same for a size (2 or more) that is not known when compiling.
 __device__ __forceinline__ unsigned long long cliques_in_word(const uint32_t *rows, uint32_t M, int size) {
   uint32_t left[CDS_MAX_K];  // by members chosen: who may be the next
   unsigned long long total = 0;
@@ -348,8 +436,10 @@ static_assert(slabs_hold_their_rows(), "rows in global memory leave their block'
 // searched rows), so the step that counts is the row building: by binary
 // search of every out-list 5.9 ms for the 2.29 G 4-cliques of that graph, by
 // bitmap words and ballots 2.2 ms.
-template <int K, bool TB, class C>
-__device__ void local_count(const uint32_t *A, const uint32_t *hid, uint32_t d, const HeavyBits &hb,
+// ONE: d is at most 32 (what the callers of one word never reach is then not compiled
+// into them: with it, the clique-core numbers of R-MAT 8,192 at k = 6 took 10.9 ms, ORDER8K without).
+template <int K, bool TB, class C, bool ONE = false>
+__device__ void local_count(const uint32_t *A, uint32_t *hid, uint32_t d, const HeavyBits &hb,
                             const uint64_t *doff, const uint32_t *dadj, const uint32_t *outdeg, uint32_t *rows,
                             C *cnt, int kk) {
   using T = Team<TB>;
@@ -383,7 +473,8 @@ __device__ void local_count(const uint32_t *A, const uint32_t *hid, uint32_t d, 
     T::sync();
   }
   if (K == 3) return;
-  if (!TB && W == 1) {
+  static_assert(!ONE || !TB, "a warp's");
+  if (!TB && (ONE || W == 1)) {
     const uint32_t row = lane < d ? rows[lane * rs] : 0u;
     C s = 0;
     if (K == 4) {
@@ -392,7 +483,11 @@ __device__ void local_count(const uint32_t *A, const uint32_t *hid, uint32_t d, 
         if ((row >> j) & 1u) s += __popc(row & rj);
       }
     } else if (K == 0) {  // each lane the cliques among its own neighbours, no step shared and none atomic
-      s = cliques_in_word(rows, row, kk - 2) * (uint32_t)(kk - 2);
+      if (kk == 6) s = word_cliques<4>(rows, row);
+      else if (kk == 7) s = word_cliques<5>(rows, row);
+      else if (kk == 8) s = word_cliques<6>(rows, row);
+      else s = cliques_in_word(rows, row, kk - 2);
+      s *= (uint32_t)(kk - 2);
     } else {
       for (uint32_t m = row; m; m &= m - 1) {
         const uint32_t j = __ffs(m) - 1;
@@ -405,7 +500,64 @@ __device__ void local_count(const uint32_t *A, const uint32_t *hid, uint32_t d, 
     T::sync();
     return;
   }
-  for (uint32_t i = T::warp(); i < d; i += T::warps()) {
+  if constexpr (ONE) return;
+  if constexpr (K == 0) {
+    // the pairs i < j, a thread each, by their number in a prefix over the rows: a
+    // pair's search takes from nothing to many steps, and most of a word's lanes would
+    // wait for the longest (the prefix lies where the heavy ids were)
+    uint32_t carry = 0;
+    for (uint32_t i0 = 0; i0 < d; i0 += ts) {
+      const uint32_t i = i0 + tr;
+      uint32_t n = 0, tot;
+      if (i < d)
+        for (uint32_t w = i >> 5; w < W; w++)
+          n += __popc(rows[i * rs + w] & (w == (i >> 5) ? ~((2u << (i & 31)) - 1u) : 0xFFFFFFFFu));
+      const uint32_t ex = T::template scan<uint32_t>(n, &tot);
+      if (i < d) hid[i] = carry + ex;
+      carry += tot;
+    }
+    T::sync();
+    for (uint32_t q = tr; q < carry; q += ts) {
+      const uint32_t i = find_row(hid, d, q);
+      const uint32_t *ri = rows + i * rs;
+      uint32_t r = q - hid[i], w0 = i >> 5, m = ri[w0] & ~((2u << (i & 31)) - 1u);
+      for (; r >= (uint32_t)__popc(m); m = ri[++w0]) r -= __popc(m);
+      const uint32_t j = w0 * 32 + (uint32_t)select_bit(m, (int)r);
+      const uint32_t *rj = rows + j * rs;
+      C sum = 0;
+      if (W == 1 || kk > 7) {
+        uint32_t M[DFS_WMAX];
+        int both = 0;
+        for (uint32_t w = 0; w < W; w++) {
+          M[w] = ri[w] & rj[w];
+          both += __popc(M[w]);
+        }
+        if (both < kk - 3) continue;
+        dfs_common(rows, rs, W, M, j + 1, kk - 4, [&](const uint32_t *path, uint32_t s) {
+          for (int t = 0; t < kk - 4; t++) atomicAdd(&cnt[path[t]], C(s));
+          sum += s;
+        });
+      } else if (W <= 4) {
+        const Bits128 M = row_bits(ri) & row_bits(rj);
+        if ((int)M.size() < kk - 3) continue;
+        const Bits128 later = M & Bits128{j < 63 ? ~0ull << (j + 1) : 0ull,
+                                          j < 63 ? ~0ull : j < 127 ? ~0ull << (j - 63) : 0ull};
+        if (kk == 5) sum = paths_common<1>(rows, rs, M, later, cnt);
+        else if (kk == 6) sum = paths_common<2>(rows, rs, M, later, cnt);
+        else sum = paths_common<3>(rows, rs, M, later, cnt);
+      } else {
+        if ((int)common(ri, rj, W) < kk - 3) continue;
+        const uint32_t *pair[2] = {ri, rj};
+        if (kk == 5) sum = paths_wide<2, 1>(rows, rs, W, pair, j + 1, cnt);
+        else if (kk == 6) sum = paths_wide<2, 2>(rows, rs, W, pair, j + 1, cnt);
+        else sum = paths_wide<2, 3>(rows, rs, W, pair, j + 1, cnt);
+      }
+      if (sum) {
+        atomicAdd(&cnt[i], sum);
+        atomicAdd(&cnt[j], sum);
+      }
+    }
+  } else for (uint32_t i = T::warp(); i < d; i += T::warps()) {
     const uint32_t *ri = rows + i * rs;
     C mine = 0;
     for (uint32_t w0 = i >> 5; w0 < W; w0++) {
@@ -417,7 +569,7 @@ __device__ void local_count(const uint32_t *A, const uint32_t *hid, uint32_t d, 
       C sum = 0;
       if (K == 4) {
         sum = common(ri, rj, W);
-      } else if (K == 5) {
+      } else {  // 5
         uint32_t all = 0;
         for (uint32_t w = w0; w < W; w++) {
           uint32_t m2 = ri[w] & rj[w];
@@ -430,17 +582,6 @@ __device__ void local_count(const uint32_t *A, const uint32_t *hid, uint32_t d, 
           }
         }
         sum = all;
-      } else {
-        uint32_t M[DFS_WMAX], any = 0;
-        for (uint32_t w = 0; w < W; w++) {
-          M[w] = ri[w] & rj[w];
-          any |= M[w];
-        }
-        if (any)
-          dfs_common(rows, rs, W, M, j + 1, kk - 4, [&](const uint32_t *path, uint32_t s) {
-            for (int t = 0; t < kk - 4; t++) atomicAdd(&cnt[path[t]], C(s));
-            sum += s;
-          });
       }
       if (sum) atomicAdd(&cnt[j], sum);
       mine += sum;

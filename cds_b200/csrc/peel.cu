@@ -556,8 +556,8 @@ __global__ void __launch_bounds__(THREADS, 2) k_core(CoreParams p) {
                   hid[lane] = p.dag.heavy.id(a);
                 }
                 __syncwarp();
-                local_count<K, false, C>(A, hid, d, p.dag.heavy, p.dag.doff, p.dag.dadj, p.dag.outdeg,
-                                         rows, cnt, (int)kmin + 1);
+                local_count<K, false, C, true>(A, hid, d, p.dag.heavy, p.dag.doff, p.dag.dadj, p.dag.outdeg,
+                                               rows, cnt, (int)kmin + 1);
                 const unsigned long long total =
                     warp_sum(store_weights<K>(p, b, d, lane, 32, [&](uint32_t) { return pos; }, A, cnt)) / kmin;
                 if (lane == 0) p.R[u] = (uint32_t)total;
