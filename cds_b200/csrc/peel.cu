@@ -313,7 +313,7 @@ __device__ void count_pairs(const CoreParams &p, uint2 item, uint32_t sweep, uin
 template <int K, class Use>
 __device__ __forceinline__ uint32_t row_sum(const CoreParams &p, uint64_t b, uint32_t len, uint32_t t, uint32_t tr,
                                             uint32_t ts, Use use) {
-  constexpr int U = 4;
+  constexpr int U = K == 2 ? 8 : 4;  // (k = 2 has no weights to keep: 8 entries, the star 8.5 -> 7.6 ms)
   uint32_t ge = 0;
   for (uint32_t i0 = tr; i0 < len; i0 += ts * U) {
     uint32_t w[U], c[U], x[U];
@@ -348,8 +348,10 @@ struct BinSearch {
     s = 0;
     while (((hi - lo - 1) >> s) >= BINS) s++;
   }
+  __device__ __forceinline__ bool holds(uint32_t x) const { return x >= lo && x < hi; }
+  __device__ __forceinline__ uint32_t bin_of(uint32_t x) const { return (hi - 1 - x) >> s; }
   __device__ __forceinline__ void add(uint32_t *bin, uint32_t x, uint32_t c) const {
-    if (x >= lo && x < hi && c) atomicAdd(&bin[(hi - 1 - x) >> s], c);
+    if (holds(x) && c) atomicAdd(&bin[bin_of(x)], c);
   }
   // weight Sb at or above bin b's lowest value is enough (or that is below lo)
   __device__ __forceinline__ bool found(uint32_t b, uint32_t Sb) const {
@@ -412,7 +414,19 @@ __device__ __forceinline__ uint32_t lower_block(const CoreParams &p, uint32_t v,
     for (uint32_t i = threadIdx.x; i < BINS_BLOCK; i += blockDim.x) bin[i] = 0;
     if (threadIdx.x == 0) s_first = 0xFFFFFFFFu;
     __syncthreads();
-    row_sum<K>(p, b, len, 0xFFFFFFFFu, threadIdx.x, blockDim.x, [&](uint32_t x, uint32_t c) { bs.add(bin, x, c); });
+    // (a hub's neighbours are mostly of a few small values, so a thread adds up a bin's
+    // weights while they come: a star of 4 M vertices, k = 2, 12.1 -> 8.5 ms)
+    uint32_t at = 0, sum = 0;
+    row_sum<K>(p, b, len, 0xFFFFFFFFu, threadIdx.x, blockDim.x, [&](uint32_t x, uint32_t c) {
+      if (!bs.holds(x) || !c) return;
+      if (bs.bin_of(x) != at) {
+        if (sum) atomicAdd(&bin[at], sum);
+        at = bs.bin_of(x);
+        sum = 0;
+      }
+      sum += c;
+    });
+    if (sum) atomicAdd(&bin[at], sum);
     __syncthreads();
     static_assert(BINS_BLOCK == 2 * THREADS, "two bins a thread");
     const uint32_t b0 = 2 * threadIdx.x, x0 = bin[b0], x1 = bin[b0 + 1];
