@@ -852,7 +852,13 @@ void exact_search(cds_ctx *c, cudaStream_t s, const CoreOut &co, const Instances
     }
     std::vector<CertAnswer> found;
     std::vector<uint8_t> in_set;
-    certify(c, s, co, k, ask, found, in_set, known);
+    try {
+      certify(c, s, co, k, ask, found, in_set, known);
+    } catch (const Error &e) {  // (sparse components' flows take less memory)
+      if (e.status != CDS_ERR_OOM) throw;
+      found.assign(nnet, CertAnswer{});
+      known.release();
+    }
     bool marked = false;
     for (uint32_t i = 0; i < nnet; i++) {
       CompState &cs = st[i];
