@@ -24,13 +24,18 @@ namespace {
 // The heavy vertices and their empty bitmap.  16,384 of them: 32 MB, which stays
 // in L2 beside the lists; on R-MAT scale 18, edge factor 16, 99 % of the out-list
 // entries a listing would search belong to them (8,192: 94 %; 32,768: 99.9 %).
-// A context short of memory takes fewer, or none (every list is then searched).
-constexpr uint32_t HEAVY_MAX = 16384;
+// The bitmap takes at most an eighth of what the budget has left, as the stages to come
+// need memory too (a small graph's needed 32 of 35 MB, and a budget of 34 refused what
+// 2 MB hold): a context short of memory takes fewer, or none (every list is then
+// searched).
+constexpr uint32_t HEAVY_MAX = 16384, HEAVY_SHARE = 8;
 void heavy_vertices(cds_ctx *c, cudaStream_t s, uint32_t n, Dag &dag) {
   dag.hid.c = dag.hbits.c = c;
   dag.hid.s = dag.hbits.s = s;
+  const uint64_t used = c->in_use.load(), share = (c->budget > used ? c->budget - used : 0) / HEAVY_SHARE;
   for (uint32_t cap = std::min(n, HEAVY_MAX); cap >= 256 || cap == n; cap /= 2) {
     const uint32_t words = (cap + 31) / 32;
+    if (4 * (uint64_t)cap * words > share) continue;
     try {
       dag.hbits.alloc((size_t)cap * words);
       if (cap < n) dag.hid.alloc(n);

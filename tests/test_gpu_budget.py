@@ -26,3 +26,20 @@ def test_flows_where_the_proof_does_not_fit():
             g.free()
         assert (got.num, got.den) == (n, n)
         assert np.array_equal(got.vertices, want.vertices)
+
+
+@pytest.mark.parametrize("mb", [4, 6, 33, 34, 36])
+def test_bitmap_leaves_memory_to_the_stages(mb):
+    # all 16,384 vertices could be heavy: a bitmap of 32 MB beside 4 MB of everything else
+    off, adj = cds.gen_er(16384, 4 / 16384, 1)
+    with cds.Context(0) as c:
+        g = c.graph(off, adj)
+        want, (wcore, *wrest) = c.solve(g, 3), c.clique_core(g, 3)
+        g.free()
+    with cds.Context(0, mem_budget=mb << 20) as c:
+        g = c.graph(off, adj)
+        got, (core, *rest) = c.solve(g, 3), c.clique_core(g, 3)
+        g.free()
+    assert (got.num, got.den, got.total_cliques) == (want.num, want.den, want.total_cliques)
+    assert np.array_equal(got.vertices, want.vertices)
+    assert np.array_equal(core, wcore) and rest == wrest
