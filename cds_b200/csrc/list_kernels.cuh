@@ -5,6 +5,8 @@
 #include "dag_kernels.cuh"
 #include "cds.h"
 
+#include <type_traits>
+
 namespace {
 
 constexpr int WARP_DMAX = 128;    // out-degree limit of a warp team
@@ -286,11 +288,15 @@ __device__ __forceinline__ uint32_t paths_common(const uint32_t *rows, uint32_t 
 }
 
 // The same for wider rows: the words of the P rows of the pair and the path so far are
-// read again at each step (a stack of masks would be in local memory).
+// read again at each step (a stack of masks would be in local memory).  Of 1,024 vertices
+// paths of two sum up to 5.3e8, longer ones pass 32 bits.
+template <int D>
+using PathSum = std::conditional_t<(D > 2), unsigned long long, uint32_t>;
 template <int P, int D, class C>
-__device__ __forceinline__ uint32_t paths_wide(const uint32_t *rows, uint32_t rs, uint32_t W, const uint32_t *(&r)[P],
-                                               uint32_t from, C *cnt) {
-  uint32_t sum = 0;
+__device__ __forceinline__ PathSum<D> paths_wide(const uint32_t *rows, uint32_t rs, uint32_t W,
+                                                 const uint32_t *(&r)[P], uint32_t from, C *cnt) {
+  PathSum<D> sum = 0;
+  static_assert(D <= 3, "a step's own sum is held in 32 bits");
   for (uint32_t w = from >> 5; w < W; w++) {
     uint32_t m = w == (from >> 5) ? 0xFFFFFFFFu << (from & 31) : 0xFFFFFFFFu;
 #pragma unroll
