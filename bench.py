@@ -51,12 +51,6 @@ WORKLOAD = {"workload": "rmat18-ef16-plant300-k4-seed4",
             "l2": "L2 flushed (256 MiB write) between steps"}
 SOLVE_ARGS = dict(p_size=8000, cp_size=16000, gl_buffer_size=0, partition_size=30000, early_stop=-1)
 RMAT14_KS = (2, 3, 4)
-# DRAM bytes (read + write) per launch of a kernel on a workload, from one ncu
-# capture each (profiles/ holds the summaries and the commands that made them)
-TRAFFIC = {("rmat18", "push_relabel", 4): 511000000000,  # 509.5 GB read + 1.49 GB written
-           ("rmat14", "push_relabel", 4): 59505920}
-TRAFFIC_SOURCE = {("rmat18", "push_relabel", 4): "profiles/k_flow_rmat18_k4.md",
-                  ("rmat14", "push_relabel", 4): "profiles/k_flow_rmat14_k4.md"}
 # Reciprocals a second of one B200: 16 a clock on each of 148 SMs at 1,965 MHz
 RECIPROCALS = 148 * 16 * 1.965e9
 REASONS = {  # nvidia-smi clocks_event_reasons bits
@@ -203,7 +197,7 @@ def e2e_solves(torch, ctx, off, adj, k, steps, warmup, args=SOLVE_ARGS):
     return (time.perf_counter() - t0) * 1e3, h2d, d2h // max(1, steps)
 
 
-def dominant_roofline(prof, off, adj, k, sol, peaks, traffic_key):
+def dominant_roofline(prof, off, adj, k, sol, peaks):
     """Roofline of the kernel with the largest share of a solve's kernel
     time: its algorithmic bytes per launch over its average launch time."""
     kern = {name: v for name, v in prof.items() if not name.startswith(PSEUDO)}
@@ -239,12 +233,11 @@ def dominant_roofline(prof, off, adj, k, sol, peaks, traffic_key):
                 "peak_source": "16 a clock and SM, 148 SMs, 1,965 MHz (nominal)", "passes": passes,
                 "traffic": None, "traffic_source": "profiles/k_certify_rmat18_k3.md", **split}
     achieved = alg / (avg_ms / 1e3) / 1e9 if avg_ms > 0 else 0.0
-    key = (traffic_key, name, k)
     return {"bound": "hbm", "kernel": f"{name} (k={k})", "launches": nl, "avg_launch_ms": round(avg_ms, 4),
             "algorithmic_bytes": alg, "achieved": round(achieved, 2), "peak": peak, "unit": "GB/s",
             "frac": round(achieved / peak, 5),
             "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)" if peaks else "fallback 6.65 TB/s",
-            "traffic": TRAFFIC.get(key), "traffic_source": TRAFFIC_SOURCE.get(key), **split}
+            "traffic": None, "traffic_source": None, **split}
 
 
 def load_peaks():
@@ -284,7 +277,7 @@ def run_rmat14(torch, ctx, steps, flush, peaks):
     (name, kd), _ = max(((key, v) for key, v in merged.items() if not key[0].startswith(PSEUDO)),
                         key=lambda kv: kv[1][1])
     roof = dominant_roofline({nm: v for (nm, kk), v in merged.items() if kk == kd}, off, adj, kd, last[kd],
-                             peaks, "rmat14")
+                             peaks)
     g.free()
     return {"config": "R-MAT scale 14 (16,384 vertices), edge factor 8, a=0.57 b=c=0.19, seed 1; one step = k=2,3,4",
             "solves_per_s": round(3 * steps / (total / 1e3), 2), "per_k": per_k, "roofline": roof}
@@ -321,11 +314,13 @@ def run_batched(ctx, count=256, seed=2):
     gen_s = time.perf_counter() - t0
     gs = [ctx.graph(o, a) for o, a, _ in inst]
     jobs = [(g, cds.make_params(k)) for g, (_, _, k) in zip(gs, inst)]
-    # warm-up: both paths once, so the device memory pool has grown to the
-    # union's size and neither timed run pays first-touch allocation
-    ctx.solve_batch(jobs)
-    for g, (_, _, k) in zip(gs, inst):
-        ctx.solve(g, k)
+    # warm-up: both paths four times in turn, so that the device memory pool holds what
+    # either needs beside what the other left (after one round the next batched passes took
+    # 0.48, 0.24 and 0.15 s)
+    for _ in range(4):
+        ctx.solve_batch(jobs)
+        for g, (_, _, k) in zip(gs, inst):
+            ctx.solve(g, k)
     # three timed passes of each path, median kept (single runs of the
     # batched union varied by up to 1.7x between passes)
     t_plain_runs, t_batch_runs = [], []
@@ -506,7 +501,7 @@ def run_cds(args):
     psol = ctx.solve(g, k, **SOLVE_ARGS)
     prof = ctx.profile_read()
     ctx.profile(False)
-    roofline = dominant_roofline(prof, off, adj, k, psol, peaks, "rmat18")
+    roofline = dominant_roofline(prof, off, adj, k, psol, peaks)
 
     # end to end through the C ABI from pinned host buffers
     g.free()

@@ -17,7 +17,8 @@
 // approach that like 1/t), accelerated by Anderson's method over the last HIST
 // differences (D. G. Anderson, "Iterative procedures for nonlinear integral
 // equations", J. ACM 12, 1965).  5 to 16 passes over the cliques reach the bound on
-// the R-MAT and planted graphs tried (7 to 36 without the derivative).
+// most R-MAT and planted graphs tried, 20 to 40 where levels split late (7 to 36
+// and more without the derivative).
 //
 // A component that some subset S of it is denser than does not balance, and shows it
 // by the eighth pass.  Its vertices by falling weight are then an order to take them
@@ -48,7 +49,8 @@
 // Measured against network build, warm split and push-relabel: 40 vertices and 1,499
 // triangles 0.39 -> 0.14 ms, 470 vertices and 25,761 edges 0.69 -> 0.25, 112 and
 // 1.18 M 4-cliques 1.5 -> 0.38, 746 and 9.3 M triangles 4.4 -> 1.3, 988 and 1.14 G
-// 4-cliques 295 -> 31 (and 62 GB of records and lists that are not built).
+// 4-cliques 295 -> 31 with nine passes and the integer one (another seed's 1.15 G 36 to
+// 37 with ten), and 62 GB of records and lists that are not built.
 #include "core_rows.cuh"
 #include "device_util.cuh"
 #include "stages.h"
@@ -117,7 +119,11 @@ struct CertParams {
   unsigned long long *phase_ns;  // [3] block 0's time in passes, updates, the integer pass (profiling; null: off)
 };
 enum : uint32_t { BALANCE = 0, REACHED = 1, GIVEN_UP = 2, COUNT = 3, NOT_ASKED = 4 };
-constexpr double LEVEL_GAP = 28.0;  // log of the weights' ratio between the levels, at least
+// Log of the weights' ratio between the levels, at least: a clique that crosses gives the
+// members of S at most e^-28 = 7e-13 of its units a member of the rest, so that 10^9 such
+// cliques stay below a thousandth of one clique, and weights down to the floor
+// of e^-60 keep their shares.
+constexpr double LEVEL_GAP = 28.0;
 constexpr int UNIT_BITS = 46;  // a clique has k 2^46 units
 
 // Shared memory of a block: the component it works on.
@@ -588,7 +594,8 @@ __device__ __noinline__ void update(const CertParams &p, uint32_t ci, uint32_t t
   const uint32_t cur = t % (HIST + 1), age = t - lv.since;
   // differences to combine: none once what does not balance has given no order, as the
   // combined steps scatter its weights (463 vertices, all but two of them S: proven in 16
-  // of 16 runs, in 5 of 12 with the differences kept)
+  // of 16 runs, in 5 of 12 with the differences kept; 124 other R-MAT, planted and random
+  // graphs at k = 2, 3, 4 take the same time and leave the same four to the flows either way)
   const uint32_t m = age > 18 && !lv.split ? 0 : min(age, (uint32_t)HIST);
   const double total = lv.target[0] * c.n;  // (about the units in all, for relative sizes)
   // (read before block_sum's barriers: thread 0 sets it below, and all threads have to
@@ -619,6 +626,9 @@ __device__ __noinline__ void update(const CertParams &p, uint32_t ci, uint32_t t
     if (threadIdx.x == 0) p.state[ci] = GIVEN_UP;
     return;
   }
+  // (124 solves of R-MAT, planted and random graphs at k = 2, 3, 4: 4 go on to the flows;
+  // with orders at ages 5, 9, 13, 17 and 21 9 do, and 24 planted ones take 33.6 ms instead of
+  // 30.2; with ages from 12 to 36 4 do and the same take 35.0)
   const bool slow = (age == 8 && rel > 1e-3) || (age == 13 && rel > 1e-4) || (age == 18 && rel > 1e-5) ||
                     age == 23 || age >= 28;
   if (slow && !(lv.split && age == 8)) {

@@ -844,9 +844,8 @@ void densest_core_and_components(cds_ctx *c, cudaStream_t s, const Dag &gdag, co
   }
 }
 
-void build_networks(cds_ctx *c, cudaStream_t s, const Dag &gdag, const Instances &inst, uint32_t k,
-                    const Tuning &t, CoreOut &out, const std::vector<uint8_t> &open, const CountHook *on_count) {
-  (void)inst;
+void build_networks(cds_ctx *c, cudaStream_t s, const Dag &gdag, uint32_t k, const Tuning &t, CoreOut &out,
+                    const std::vector<uint8_t> &open, const CountHook *on_count) {
   const uint32_t ncomp = out.ncomp, nv = out.comp_vbeg[ncomp];
   const int G = c->sm_count * 8;
   if (!out.listed) {

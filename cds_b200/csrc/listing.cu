@@ -5,22 +5,22 @@
 // writeFinalCliques (cudaCode/src/helpers.cu:175-574, 1098-1137), and the
 // k = 2 path writeEdgeCliques (helpers.cu:576-609).
 //
-// Every vertex u with out-degree d >= k-1 is a root.  A team (one warp for
-// d <= 128, one block above that) stages N+(u) = A[0..d) in shared memory
-// with 128-bit loads and builds the local adjacency bitmap: bit j of row i
-// is set when A[j] is an out-neighbour of A[i] (each lane binary-searches one
-// element of N+(A[i]) in A).  The k-cliques rooted at u are then
-// u, A[i], A[j] plus a (k-3)-clique inside row_i & row_j, found with AND and
-// popcount on the bitmaps.  The (i, j) pairs (the set bits of all rows) are
-// numbered 0..P-1 through a prefix over row popcounts, and the team's threads
-// take consecutive pair numbers, so work is balanced inside a root whatever
-// the row lengths.
+// Every vertex u with out-degree d >= k-1 is a root.  A team (one warp for d up to
+// list_warp_dmax, 32 by default for k >= 3, one block above that) takes N+(u) =
+// A[0..d) and builds the adjacency of G[A] as bitmap rows: pairs of heavy vertices
+// are bits of the graph's bitmap, made into row words by ballots, and the arcs of light
+// vertices come from their short out-lists, each entry searched in A.
 //
-// Pass 1 (count) sums the cliques of each root and accumulates each vertex's
-// clique degree in shared memory before one atomic per vertex and root.
-// Pass 2 (write) re-enumerates and stores clique records (k ids) at the
-// root's offset from the prefix of pass-1 counts, so the record order is the
-// root order: deterministic, independent of scheduling.
+// Pass 1 (k_count) has symmetric rows.  For k = 4, 5 a pair of adjacent vertices
+// adds the bits its rows (and a third's) have in common to its ends, so each clique
+// is met once per edge with no step of its own; k = 3 needs degrees alone; k >= 6 searches
+// from the numbered pairs of a neighbourhood, a thread each.  Every vertex's sum is one
+// atomic to its clique degree per root.
+// Pass 2 (k_list_write) has rows oriented as the DAG.  Its (i, j) pairs (the set bits
+// of all rows) are numbered 0..P-1 through a prefix over row popcounts and taken by
+// consecutive threads; clique records (k ids) go to the root's offset from the prefix of
+// pass-1 counts, so the record order is the root order: deterministic, independent
+// of scheduling.
 #include "device_util.cuh"
 #include "stages.h"
 

@@ -37,7 +37,7 @@
 //           before and after; where its later set changed, small sets are
 //           counted at once by the warp, larger ones queued
 //   count   blocks take the queued roots
-//   lower   (twice) weighted h-index of every vertex a change can have reached
+//   lower   (LOWER times) weighted h-index of every vertex a change can have reached
 // Ties keep the order they had: a vertex that arrives at a value goes behind those
 // that were there (its key's low half holds the sweep it arrived in and how far
 // it fell).  With ids to break ties a plateau of equal values turns around as it
@@ -67,7 +67,6 @@
 #include "list_kernels.cuh"
 
 #include <algorithm>
-#include <cstdio>
 
 namespace {
 

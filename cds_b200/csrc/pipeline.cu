@@ -195,7 +195,7 @@ void run_problem(cds_ctx *c, cudaStream_t s, UnionGraph &u, const cds_params &pr
   if (core_only) core_answer(s, pe, u, fa);
   else
     exact_search(c, s, co, u.inst, k, prm, t,
-                 [&](const std::vector<uint8_t> &open) { build_networks(c, s, dag, u.inst, k, t, co, open, on_count); }, fa);
+                 [&](const std::vector<uint8_t> &open) { build_networks(c, s, dag, k, t, co, open, on_count); }, fa);
   totals.wait();
   const int m5 = clk.mark();
   clk.wait();

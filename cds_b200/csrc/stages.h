@@ -109,8 +109,8 @@ struct CoreOut {
   DBuf<uint32_t> comp;      // [n] smallest vertex of each core vertex's component
   DBuf<uint64_t> cidx;      // [n+1] component index of a smallest vertex
   DBuf<uint32_t> local;     // [n] local vertex of each component vertex
-  // small cores (k <= 5): the pairs that core cliques cover, over core-local ids
-  // (row a, column b > a)
+  // small cores: the pairs that core cliques cover, over core-local ids (row a, column
+  // b > a); `small`: k <= 5 too, and no clique has been listed
   bool small = false;
   uint32_t ncore = 0;
   CoreRows rows;
@@ -137,7 +137,7 @@ void densest_core_and_components(cds_ctx *c, cudaStream_t s, const Dag &dag, con
                                  const Instances &inst, uint32_t k, const Tuning &t, CoreOut &out,
                                  StageClock *clk = nullptr, const CountHook *on_count = nullptr);
 // The flow networks of the components with open[i] != 0: records, incidence lists.
-void build_networks(cds_ctx *c, cudaStream_t s, const Dag &dag, const Instances &inst, uint32_t k,
+void build_networks(cds_ctx *c, cudaStream_t s, const Dag &dag, uint32_t k,
                     const Tuning &t, CoreOut &out, const std::vector<uint8_t> &open,
                     const CountHook *on_count = nullptr);
 
