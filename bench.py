@@ -314,17 +314,17 @@ def run_batched(ctx, count=256, seed=2):
     gen_s = time.perf_counter() - t0
     gs = [ctx.graph(o, a) for o, a, _ in inst]
     jobs = [(g, cds.make_params(k)) for g, (_, _, k) in zip(gs, inst)]
-    # warm-up: both paths four times in turn, so that the device memory pool holds what
-    # either needs beside what the other left (after one round the next batched passes took
-    # 0.48, 0.24 and 0.15 s)
-    for _ in range(4):
-        ctx.solve_batch(jobs)
-        for g, (_, _, k) in zip(gs, inst):
-            ctx.solve(g, k)
-    # three timed passes of each path, median kept (single runs of the
-    # batched union varied by up to 1.7x between passes)
+    # warm-up: both paths once, so the device memory pool has grown to the
+    # union's size and neither timed run pays first-touch allocation
+    ctx.solve_batch(jobs)
+    for g, (_, _, k) in zip(gs, inst):
+        ctx.solve(g, k)
+    # nine timed passes of each path, median kept: a batched pass has the same kernel
+    # time every time, but about one in six takes 0.05 to 1.1 s more on the host (with three
+    # passes the median was now 0.15 and now 0.24 s)
+    passes = 9
     t_plain_runs, t_batch_runs = [], []
-    for _ in range(3):
+    for _ in range(passes):
         t0 = time.perf_counter()
         plain, wall = [], []
         for g, (_, _, k) in zip(gs, inst):
@@ -358,7 +358,7 @@ def run_batched(ctx, count=256, seed=2):
     return {"config": f"{count} instances, n log-uniform [500, 50000], half ER / half R-MAT, "
                       "planted 20-200 @0.5, k in {2,3,4}, seed 2",
             "plain_solves_per_s": round(count / t_plain, 2), "batched_solves_per_s": round(count / t_batch, 2),
-            "speedup": round(t_plain / t_batch, 2), "timed_passes": 3,
+            "speedup": round(t_plain / t_batch, 2), "timed_passes": passes,
             "batched_pass_s": [round(t, 3) for t in t_batch_runs], "identical_answers": same,
             "kcliques": int(sum(s.total_cliques for s in batch)), "generation_s": round(gen_s, 1),
             "plain_breakdown": {
