@@ -575,9 +575,12 @@ __global__ void __launch_bounds__(THREADS, 2) k_core(CoreParams p) {
                     warp_sum(store_weights<K>(p, b, d, lane, 32, [&](uint32_t) { return pos; }, A, cnt)) / kmin;
                 if (lane == 0) p.R[u] = (uint32_t)total;
                 __syncwarp();
-              } else if (lane == 0) {
-                p.dplus[u] = d;
-                queue_root(p, sctl, u, d);
+              } else {
+                if (d > p.dmax) clear_weights(p, u, b, d, lane, 32);  // (its items add to them)
+                if (lane == 0) {
+                  p.dplus[u] = d;
+                  queue_root(p, sctl, u, d);
+                }
               }
             });
       }

@@ -49,3 +49,43 @@ def test_levels_by_deletion(scale, factor, plant, k):
             assert np.array_equal(left_by_deletion(ctx, off, adj, degree, k, level), want)
         # (no core above the largest)
         assert not len(left_by_deletion(ctx, off, adj, degree, k, int(values[-1]) + 1))
+
+
+def hubs_over_blocks(blocks, seed):
+    """Random blocks of 24 vertices, denser and sparser ones; hubs joined to a few vertices
+    of each block, whose values lie among the blocks'; beside them 620 vertices of degree
+    about 590, so many rows of over 512 entries that warps order rows of up to 2,048."""
+    rng = np.random.default_rng(seed)
+    u, v = [], []
+    x, y = np.triu_indices(24, 1)
+    for b in range(blocks):
+        on = rng.random(len(x)) < rng.uniform(0.8, 1.0)
+        u.append(x[on] + 24 * b)
+        v.append(y[on] + 24 * b)
+    n = 24 * blocks
+    for _ in range(6):
+        near = np.concatenate([24 * b + rng.choice(24, rng.integers(3, 5), replace=False) for b in range(blocks)])
+        u.append(np.full(len(near), n))
+        v.append(near)
+        n += 1
+    x, y = np.triu_indices(620, 1)
+    on = rng.random(len(x)) < 0.95
+    u.append(x[on] + n)
+    v.append(y[on] + n)
+    return cds.csr_from_edges(n + 620, np.concatenate(u), np.concatenate(v))
+
+
+@pytest.mark.parametrize("blocks,k", [(260, 4), (300, 4), (380, 4), (300, 3)])
+def test_many_wide_rows_with_later_sets_past_one_team(blocks, k):
+    # hubs' later sets past the 768 vertices that one block counts, recounted as the
+    # blocks' values fall below the hubs'
+    off, adj = hubs_over_blocks(blocks, blocks)
+    with cds.Context(0) as ctx:
+        g = ctx.graph(off, adj)
+        core = ctx.clique_core(g, k)[0].astype(np.int64)
+        degree = ctx.list_cliques(g, k)[1]
+        g.free()
+        values = np.unique(np.r_[core[24 * blocks:24 * blocks + 6], np.unique(core)[[1, -1]]])
+        for level in np.unique(np.r_[values, values + 1]):
+            want = np.flatnonzero(core >= level)
+            assert np.array_equal(left_by_deletion(ctx, off, adj, degree, k, level), want)
