@@ -320,7 +320,7 @@ def run_batched(ctx, count=256, seed=2):
     for g, (_, _, k) in zip(gs, inst):
         ctx.solve(g, k)
     # nine timed passes of each path, median kept: a batched pass has the same kernel
-    # time every time, but about one in six takes 0.05 to 1.1 s more on the host (with three
+    # time every time, but about one in four takes 0.05 to 1.1 s more on the host (with three
     # passes the median was now 0.15 and now 0.24 s)
     passes = 9
     t_plain_runs, t_batch_runs = [], []
